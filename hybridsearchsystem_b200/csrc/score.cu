@@ -15,24 +15,141 @@ namespace hss {
 namespace {
 
 // ---------------------------------------------------------------------------------------------
-// Exact materialised scorer. One thread per doc; the CTA holds kExactQ query rows in shared memory.
+// Exact materialised scorer. Every output is one sequential chain of dim separate multiplies and adds,
+// so the kernel is bound by FP32 issue: 2 m n dim lane operations at 128 per clock per SM (29 us for
+// 32 x 131,072 x 128 at 1965 MHz), with the doc rows' 67 MB behind that (10 us). A thread keeps TQ x TD
+// chains in registers, so a query value from shared memory serves TD docs and a doc value TQ queries:
+// at 8 x 4, 12 16-byte shared loads feed 256 operations (one thread per doc, which re-read its row from
+// L1 for every query and had one chain in flight, took 535 us there; this takes 45 us). Stages of 16
+// dims, or one stage of 32, let 7 CTAs share an SM instead of 5 but took 51 and 53 us (more barriers;
+// spills at 72 registers). Doc rows are copied as they lie (cp.async, two stages of 32 dims) with a
+// row pitch of 36 floats, which keeps the 16-byte reads of 8 neighbouring rows on distinct banks.
+// Packed f32x2 multiplies and adds are not used: they came out contracted into a fused multiply-add,
+// which rounds once where the ground truth rounds twice.
 // ---------------------------------------------------------------------------------------------
-constexpr int kExactDocs = 128;
-constexpr int kExactQ = 8;
+constexpr int kExactT = 128;        // threads: 4 warps, WQ of them side by side over the queries
+constexpr int kExactK = 32;         // dims per stage
+constexpr int kExactPitch = kExactK + 4;
 
-__global__ void __launch_bounds__(kExactDocs) exact_score_kernel(const float* __restrict__ qry,
-                                                                 const float* __restrict__ docs,
-                                                                 float* __restrict__ out, uint32_t m, uint32_t n,
-                                                                 uint32_t dim, uint64_t ldc) {
-    extern __shared__ float sq[];  // [kExactQ][dim]
-    const uint32_t q0 = blockIdx.y * kExactQ;
-    const uint32_t nq = min(static_cast<uint32_t>(kExactQ), m - q0);
-    for (uint32_t i = threadIdx.x; i < nq * dim; i += blockDim.x) sq[i] = qry[static_cast<uint64_t>(q0) * dim + i];
-    __syncthreads();
-    const uint64_t doc = static_cast<uint64_t>(blockIdx.x) * kExactDocs + threadIdx.x;
-    if (doc >= n) return;
-    const float* v = docs + doc * dim;
-    for (uint32_t j = 0; j < nq; ++j) out[(q0 + j) * ldc + doc] = exact_dot(sq + j * dim, v, dim);
+// 16 bytes, or four 4-byte copies where a matrix is only 4-byte aligned (VEC false).
+template <bool VEC>
+__device__ __forceinline__ void copy4_async(float* smem, const float* gmem) {
+    const uint32_t s = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
+    if (VEC) {
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(s), "l"(gmem) : "memory");
+    } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(s + 4u * i), "l"(gmem + i) : "memory");
+    }
+}
+
+template <int TQ, int TD, int WQ>
+struct ExactTile {
+    static constexpr int QT = TQ * WQ;             // queries per CTA
+    static constexpr int DT = 32 * TD * (4 / WQ);  // docs per CTA
+    static constexpr int stage_floats = DT * kExactPitch + QT * kExactK;
+    static constexpr size_t smem = 2 * static_cast<size_t>(stage_floats) * sizeof(float);
+};
+
+template <int TQ, int TD, int WQ, bool VEC>
+__global__ void __launch_bounds__(kExactT) exact_score_kernel(const float* __restrict__ qry,
+                                                              const float* __restrict__ docs, float* __restrict__ out,
+                                                              uint32_t m, uint32_t n, uint32_t dim, uint64_t ldc) {
+    using T = ExactTile<TQ, TD, WQ>;
+    extern __shared__ __align__(16) float exact_smem[];
+    const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const uint32_t wq = warp % WQ, wd = warp / WQ;
+    const uint64_t doc0 = static_cast<uint64_t>(blockIdx.x) * T::DT;
+    const uint32_t q0 = blockIdx.y * T::QT;
+    const uint32_t chunks = (dim + kExactK - 1) / kExactK;
+
+    // rows past the matrices copy the last row instead (in bounds; their outputs are not stored)
+    auto stage = [&](uint32_t c) {
+        float* sd = exact_smem + (c & 1u) * T::stage_floats;
+        float* sq = sd + T::DT * kExactPitch;
+        const uint32_t k0 = c * kExactK, k4 = min(static_cast<uint32_t>(kExactK), dim - k0) / 4;
+        for (uint32_t f = t; f < T::DT * (kExactK / 4); f += kExactT) {
+            const uint32_t r = f / (kExactK / 4), part = f % (kExactK / 4);
+            if (part < k4) {
+                const uint64_t doc = min(doc0 + r, static_cast<uint64_t>(n) - 1);
+                copy4_async<VEC>(sd + r * kExactPitch + part * 4, docs + doc * dim + k0 + part * 4);
+            }
+        }
+        for (uint32_t f = t; f < T::QT * (kExactK / 4); f += kExactT) {
+            const uint32_t r = f / (kExactK / 4), part = f % (kExactK / 4);
+            if (part < k4)
+                copy4_async<VEC>(sq + r * kExactK + part * 4,
+                                 qry + static_cast<uint64_t>(min(q0 + r, m - 1)) * dim + k0 + part * 4);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+
+    float acc[TQ][TD];
+#pragma unroll
+    for (int i = 0; i < TQ; ++i)
+#pragma unroll
+        for (int j = 0; j < TD; ++j) acc[i][j] = 0.0f;
+
+    stage(0);
+    for (uint32_t c = 0; c < chunks; ++c) {
+        if (c + 1 < chunks) {
+            stage(c + 1);
+            asm volatile("cp.async.wait_group 1;" ::: "memory");
+        } else {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+        }
+        __syncthreads();
+        const float* sd = exact_smem + (c & 1u) * T::stage_floats + (wd * 32u * TD + lane) * kExactPitch;
+        const float* sq = exact_smem + (c & 1u) * T::stage_floats + T::DT * kExactPitch + wq * TQ * kExactK;
+        const uint32_t kc = min(static_cast<uint32_t>(kExactK), dim - c * kExactK);
+#pragma unroll 4
+        for (uint32_t k = 0; k < kc; k += 4) {
+            float4 d[TD];
+#pragma unroll
+            for (int j = 0; j < TD; ++j) d[j] = *reinterpret_cast<const float4*>(sd + j * 32 * kExactPitch + k);
+#pragma unroll
+            for (int i = 0; i < TQ; ++i) {
+                const float4 q = *reinterpret_cast<const float4*>(sq + i * kExactK + k);
+#pragma unroll
+                for (int j = 0; j < TD; ++j) {
+                    float s = acc[i][j];
+                    s = __fadd_rn(s, __fmul_rn(q.x, d[j].x));
+                    s = __fadd_rn(s, __fmul_rn(q.y, d[j].y));
+                    s = __fadd_rn(s, __fmul_rn(q.z, d[j].z));
+                    s = __fadd_rn(s, __fmul_rn(q.w, d[j].w));
+                    acc[i][j] = s;
+                }
+            }
+        }
+        __syncthreads();  // the stage is read before the next-but-one chunk is copied into it
+    }
+#pragma unroll
+    for (int i = 0; i < TQ; ++i) {
+        const uint32_t q = q0 + wq * TQ + i;
+        if (q >= m) break;
+#pragma unroll
+        for (int j = 0; j < TD; ++j) {
+            const uint64_t doc = doc0 + wd * 32u * TD + lane + 32u * j;
+            if (doc < n) out[q * ldc + doc] = acc[i][j];
+        }
+    }
+}
+
+template <int TQ, int TD, int WQ>
+cudaError_t launch_exact_tile(const float* qry, const float* docs, float* out, uint32_t m, uint32_t n, uint32_t dim,
+                              uint64_t ldc, cudaStream_t stream) {
+    using T = ExactTile<TQ, TD, WQ>;
+    const bool vec = ((reinterpret_cast<uintptr_t>(qry) | reinterpret_cast<uintptr_t>(docs)) & 15u) == 0;
+    auto kernel = vec ? exact_score_kernel<TQ, TD, WQ, true> : exact_score_kernel<TQ, TD, WQ, false>;
+    if (T::smem > 48 * 1024) {
+        cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             static_cast<int>(T::smem));
+        if (e != cudaSuccess) return e;
+    }
+    const dim3 grid(static_cast<uint32_t>((static_cast<uint64_t>(n) + T::DT - 1) / T::DT), (m + T::QT - 1) / T::QT);
+    kernel<<<grid, kExactT, T::smem, stream>>>(qry, docs, out, m, n, dim, ldc);
+    return cudaGetLastError();
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -177,22 +294,23 @@ __global__ void __launch_bounds__(kCT) cand_simt_kernel(CandLaunch L) {
 
 }  // namespace
 
+// The tile: few queries take narrow ones (the pass is then bound by the doc rows, so no thread should
+// carry chains of absent queries); from 5 queries on, 32 x 128 where that pads the batch to at most a
+// tenth more queries than 16 x 64 does and still gives every SM a CTA, else 16 x 64.
 cudaError_t launch_exact_score(const float* qry, const float* docs, float* out, uint32_t m, uint32_t n, uint32_t dim,
                                uint64_t ldc, cudaStream_t stream) {
     if (m == 0 || n == 0) return cudaSuccess;
-    const size_t smem = static_cast<size_t>(kExactQ) * dim * sizeof(float);
-    if (smem > 48 * 1024) {
-        // one ceiling for every caller (concurrent callers with other dimensions launch it too)
-        constexpr size_t kCeiling = 200 * 1024;
-        if (smem > kCeiling) return cudaErrorInvalidValue;
-        cudaError_t e = cudaFuncSetAttribute(exact_score_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             static_cast<int>(kCeiling));
-        if (e != cudaSuccess) return e;
-    }
-    dim3 grid((n + kExactDocs - 1) / kExactDocs, (m + kExactQ - 1) / kExactQ);
-    if (grid.y > 65535u) return cudaErrorInvalidValue;
-    exact_score_kernel<<<grid, kExactDocs, smem, stream>>>(qry, docs, out, m, n, dim, ldc);
-    return cudaGetLastError();
+    if ((static_cast<uint64_t>(m) + 7) / 8 > 65535u) return cudaErrorInvalidValue;
+    constexpr uint64_t kSms = 148;
+    if (m <= 2) return launch_exact_tile<2, 1, 1>(qry, docs, out, m, n, dim, ldc, stream);
+    if (m <= 4)
+        return n >= kSms * 256 ? launch_exact_tile<4, 2, 1>(qry, docs, out, m, n, dim, ldc, stream)
+                               : launch_exact_tile<4, 1, 1>(qry, docs, out, m, n, dim, ldc, stream);
+    const uint32_t pad32 = (m + 31) / 32 * 32, pad16 = (m + 15) / 16 * 16;
+    const uint64_t ctas = static_cast<uint64_t>(pad32 / 32) * ((static_cast<uint64_t>(n) + 127) / 128);
+    if (10ull * pad32 <= 11ull * pad16 && ctas >= kSms)
+        return launch_exact_tile<8, 4, 4>(qry, docs, out, m, n, dim, ldc, stream);
+    return launch_exact_tile<4, 2, 4>(qry, docs, out, m, n, dim, ldc, stream);
 }
 
 uint32_t cand_simt_segments(uint64_t tile_count, int num_sms, uint32_t cap) {
