@@ -9,8 +9,14 @@
 //    reference's Aggregator operator (kernel_aggregator.h:18-206) without the host count round trip.
 //  * topk_op_kernel: exact top K of a compacted (score, location) list -- the reference's TOPK
 //    operator (kernel_topk.h:27-419), which there is only a pivot pre-select followed by a host sort.
+#include <cooperative_groups.h>
+
+#include <atomic>
+
 #include "hss_device.cuh"
 #include "hss_kernels.h"
+
+namespace cg = cooperative_groups;
 
 namespace hss {
 namespace {
@@ -118,8 +124,10 @@ __device__ uint32_t kth_largest_u32_visit(Visit visit, uint32_t k, SelectSmem& S
 }
 
 // Picks, from the top of a 4096-bin histogram, the bin holding the k-th largest key (blockDim.x ==
-// kST: thread t owns bins 4095 - 4t .. 4092 - 4t). Returns the bin; *krem becomes the rank inside it.
-__device__ inline uint32_t pick_digit4096(const uint32_t* hist, uint32_t* krem, SelectSmem& S) {
+// kST: thread t owns bins 4095 - 4t .. 4092 - 4t). Returns the bin; *krem becomes the rank inside it and
+// *in_bin (if given) the keys it holds.
+__device__ inline uint32_t pick_digit4096(const uint32_t* hist, uint32_t* krem, SelectSmem& S,
+                                          uint32_t* in_bin = nullptr) {
     const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const uint32_t kr = *krem;
     uint32_t h[4], local = 0;
@@ -155,6 +163,7 @@ __device__ inline uint32_t pick_digit4096(const uint32_t* hist, uint32_t* krem, 
             if (cum + h[j] >= kr) {
                 S.bcast[0] = 4095 - 4 * t - j;
                 S.bcast[1] = kr - cum;
+                S.bcast[2] = h[j];
                 break;
             }
             cum += h[j];
@@ -163,6 +172,7 @@ __device__ inline uint32_t pick_digit4096(const uint32_t* hist, uint32_t* krem, 
     __syncthreads();
     const uint32_t d = S.bcast[0];
     *krem = S.bcast[1];
+    if (in_bin) *in_bin = S.bcast[2];
     __syncthreads();
     return d;
 }
@@ -346,81 +356,127 @@ __device__ uint64_t kth_largest_u64(KeyFn key, uint32_t n, uint32_t k, SelectSme
     return prefix;
 }
 
-// Sorts S.sortbuf[0..m) descending; m is a power of two <= kMaxTopK.
-__device__ void bitonic_desc(SelectSmem& S, uint32_t m) {
+// Sorts E keys per thread (key of index t + 1024 e in v[e]) of the first m / E threads descending:
+// a bitonic network whose exchanges over a distance below 32 are shuffles and whose exchanges over 1024
+// and more stay inside a thread, so only distances 32..512 go through shared memory and a barrier of
+// the m / E threads (for 512 keys 10 of the 45 steps).
+template <int E>
+__device__ __forceinline__ void bitonic_regs(unsigned long long* buf, uint32_t m) {
+    const uint32_t t = threadIdx.x, threads = E == 1 ? m : static_cast<uint32_t>(kST);
+    auto bar = [&] { asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory"); };
+    unsigned long long v[E];
+#pragma unroll
+    for (int e = 0; e < E; ++e) v[e] = buf[t + static_cast<uint32_t>(kST) * e];
     for (uint32_t k = 2; k <= m; k <<= 1) {
         for (uint32_t j = k >> 1; j > 0; j >>= 1) {
-            for (uint32_t i = threadIdx.x; i < m; i += blockDim.x) {
-                const uint32_t ixj = i ^ j;
-                if (ixj > i) {
-                    const unsigned long long a = S.sortbuf[i], b = S.sortbuf[ixj];
-                    const bool desc = (i & k) == 0;
-                    if (desc ? (a < b) : (a > b)) {
-                        S.sortbuf[i] = b;
-                        S.sortbuf[ixj] = a;
+            if (E > 1 && j >= static_cast<uint32_t>(kST)) {
+                const uint32_t de = j / static_cast<uint32_t>(kST);
+#pragma unroll
+                for (int e = 0; e < E; ++e) {
+                    const int o = e ^ static_cast<int>(de);
+                    if (o < e || o >= E) continue;
+                    const bool desc = ((t + static_cast<uint32_t>(kST) * e) & k) == 0;
+#pragma unroll
+                    for (int f = 0; f < E; ++f) {  // f == o: a compile-time register index
+                        if (f != o) continue;
+                        const unsigned long long a = v[e], b = v[f];
+                        if (desc ? (a < b) : (a > b)) {
+                            v[e] = b;
+                            v[f] = a;
+                        }
                     }
                 }
+                continue;
             }
-            __syncthreads();
+            unsigned long long o[E];
+            if (j >= 32) {
+                bar();  // the previous step's reads are done
+#pragma unroll
+                for (int e = 0; e < E; ++e) buf[t + static_cast<uint32_t>(kST) * e] = v[e];
+                bar();
+#pragma unroll
+                for (int e = 0; e < E; ++e) o[e] = buf[(t ^ j) + static_cast<uint32_t>(kST) * e];
+            } else {
+#pragma unroll
+                for (int e = 0; e < E; ++e) o[e] = __shfl_xor_sync(0xffffffffu, v[e], j);
+            }
+#pragma unroll
+            for (int e = 0; e < E; ++e) {
+                // the lower index of a descending pair keeps the larger key
+                const uint32_t i = t + static_cast<uint32_t>(kST) * e;
+                const bool larger = ((i & k) == 0) == ((i & j) == 0);
+                if (larger ? (o[e] > v[e]) : (o[e] < v[e])) v[e] = o[e];
+            }
         }
     }
+    bar();
+#pragma unroll
+    for (int e = 0; e < E; ++e) buf[t + static_cast<uint32_t>(kST) * e] = v[e];
 }
 
-__device__ inline uint32_t pow2_at_least(uint32_t x) {
-    uint32_t m = 1;
-    while (m < x) m <<= 1;
+// Sorts S.sortbuf[0..m) descending; m is a power of two, 32 <= m <= kMaxTopK (sort_size).
+__device__ __forceinline__ void bitonic_desc(SelectSmem& S, uint32_t m) {
+    if (m <= static_cast<uint32_t>(kST)) {
+        if (threadIdx.x < m) bitonic_regs<1>(S.sortbuf, m);
+    } else if (m == 2u * kST) {
+        bitonic_regs<2>(S.sortbuf, m);
+    } else {
+        bitonic_regs<4>(S.sortbuf, m);
+    }
+    __syncthreads();
+}
+
+// Keys a sort of n takes: the power of two at least n, at least a warp's 32.
+__device__ inline uint32_t sort_size(uint32_t n) {
+    uint32_t m = 32;
+    while (m < n) m <<= 1;
+    return m;
+}
+
+// Brings the top `kq` (<= kMaxTopK) of n distinct u64 keys key(i) (and possibly more) into S.sortbuf,
+// unsorted, filled up with zeros to sort_size() entries, which it returns.
+template <class KeyFn>
+__device__ __forceinline__ uint32_t gather_top_keys(KeyFn key, uint32_t n, uint32_t kq, SelectSmem& S) {
+    uint32_t got;
+    if (n <= static_cast<uint32_t>(kMaxTopK) && n <= 2 * kq) {
+        for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) S.sortbuf[i] = key(i);
+        got = n;
+    } else {
+        // n <= kMaxTopK: keep only keys whose score half is at least a lower bound of the kq-th best
+        // score (it keeps the top kq and at most the few keys sharing the kq-th's 24-bit prefix beyond
+        // them), then sort those: a bitonic sort over about kq keys instead of n. Longer lists: the
+        // exact kq-th key.
+        const uint64_t lb =
+            n <= static_cast<uint32_t>(kMaxTopK)
+                ? static_cast<uint64_t>(kth_lower_bound_u32_visit(
+                      [&](auto fn) {
+                          for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) fn(static_cast<uint32_t>(key(i) >> 32));
+                      },
+                      kq, S))
+                      << 32
+                : kth_largest_u64(key, n, kq, S);
+        if (threadIdx.x == 0) S.counter = 0;
+        __syncthreads();
+        for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
+            const uint64_t v = key(i);
+            if (v >= lb) {
+                const uint32_t pos = atomicAdd(&S.counter, 1u);
+                if (pos < static_cast<uint32_t>(kMaxTopK)) S.sortbuf[pos] = v;
+            }
+        }
+        __syncthreads();
+        got = min(S.counter, static_cast<uint32_t>(kMaxTopK));
+    }
+    const uint32_t m = sort_size(got);
+    for (uint32_t i = got + threadIdx.x; i < m; i += blockDim.x) S.sortbuf[i] = 0ull;
+    __syncthreads();
     return m;
 }
 
 // Top `kq` (<= kMaxTopK) of n distinct u64 keys key(i), sorted descending into S.sortbuf[0..kq).
 template <class KeyFn>
-__device__ void top_keys(KeyFn key, uint32_t n, uint32_t kq, SelectSmem& S) {
-    if (n <= static_cast<uint32_t>(kMaxTopK) && n > 2 * kq) {
-        // keep only keys whose score half is at least a lower bound of the kq-th best score (it keeps
-        // the top kq and at most the few keys sharing the kq-th's 24-bit prefix beyond them), then
-        // sort those: a bitonic sort over about kq keys instead of n
-        const uint32_t lb = kth_lower_bound_u32_visit(
-            [&](auto fn) {
-                for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) fn(static_cast<uint32_t>(key(i) >> 32));
-            },
-            kq, S);
-        if (threadIdx.x == 0) S.counter = 0;
-        __syncthreads();
-        for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
-            const uint64_t v = key(i);
-            if (static_cast<uint32_t>(v >> 32) >= lb) S.sortbuf[atomicAdd(&S.counter, 1u)] = v;
-        }
-        __syncthreads();
-        const uint32_t got = S.counter;  // >= kq, <= n
-        const uint32_t m = pow2_at_least(got);
-        for (uint32_t i = got + threadIdx.x; i < m; i += blockDim.x) S.sortbuf[i] = 0ull;
-        __syncthreads();
-        bitonic_desc(S, m);
-        return;
-    }
-    if (n <= static_cast<uint32_t>(kMaxTopK)) {
-        const uint32_t m = pow2_at_least(n);
-        for (uint32_t i = threadIdx.x; i < m; i += blockDim.x) S.sortbuf[i] = i < n ? key(i) : 0ull;
-        __syncthreads();
-        bitonic_desc(S, m);
-        return;
-    }
-    const uint64_t kth = kth_largest_u64(key, n, kq, S);
-    if (threadIdx.x == 0) S.counter = 0;
-    __syncthreads();
-    for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
-        const uint64_t v = key(i);
-        if (v >= kth) {
-            const uint32_t pos = atomicAdd(&S.counter, 1u);
-            if (pos < static_cast<uint32_t>(kMaxTopK)) S.sortbuf[pos] = v;
-        }
-    }
-    __syncthreads();
-    const uint32_t got = min(S.counter, static_cast<uint32_t>(kMaxTopK));
-    const uint32_t m = pow2_at_least(got);
-    for (uint32_t i = got + threadIdx.x; i < m; i += blockDim.x) S.sortbuf[i] = 0ull;
-    __syncthreads();
-    bitonic_desc(S, m);
+__device__ __forceinline__ void top_keys(KeyFn key, uint32_t n, uint32_t kq, SelectSmem& S) {
+    bitonic_desc(S, gather_top_keys(key, n, kq, S));
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -659,27 +715,44 @@ __global__ void __launch_bounds__(kST) select_topk_kernel(SelectLaunch L) {
 }
 
 // ---------------------------------------------------------------------------------------------
-// Aggregator: stable compaction in three launches (count per block, scan, scatter).
-constexpr int kAggT = 1024;  // docs per aggregation block (one per thread)
+// Aggregator: stable compaction. A CTA scatters 4,096 docs (64 bitmap words); where they go needs the
+// kept docs before them, which it finds by
+//   own     counting the bitmap's earlier words itself (one launch),
+//   sums    adding up the earlier blocks' counts, which aggregate_count_kernel left (two launches), or
+//   scanned reading its offset after aggregate_scan_kernel (three launches, very long lists).
+// All three are bound by launches and one dependent chain of loads, not by bandwidth, at the sizes of a
+// query's docs: 1.3M docs, a tenth kept, 15 us in three launches with 1,024 docs a CTA, now 8 us; 10M
+// docs 24 us. (8,192 docs a CTA of 1,024 threads: one CTA per SM at 56 registers, 28 us at 10M; held to
+// 32 registers it spills, 27 us.) The rule is at launch_aggregate.
+constexpr int kAggT = 512;                  // threads of a scatter CTA
+constexpr uint32_t kAggWords = 64;          // bitmap words a scatter CTA covers
+constexpr uint32_t kAggDocs = kAggWords * 64;
+enum AggPrefix : int { kAggOwn = 0, kAggSums = 1, kAggScanned = 2 };
 
-__global__ void __launch_bounds__(kAggT) aggregate_count_kernel(const uint64_t* __restrict__ bits, uint32_t n,
-                                                                 uint32_t* __restrict__ block_count) {
-    __shared__ uint32_t part[kAggT / 32];
-    const uint32_t doc = blockIdx.x * kAggT + threadIdx.x;
-    const bool hit = doc < n && ((bits[doc >> 6] >> (doc & 63)) & 1ull);
-    const uint32_t c = __popc(__ballot_sync(0xffffffffu, hit));
-    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = c;
-    __syncthreads();
-    if (threadIdx.x < 32) {
-        uint32_t v = part[threadIdx.x];
-        v = warp_sum(v);
-        if (threadIdx.x == 0) block_count[blockIdx.x] = v;
-    }
+// Bitmap word w of n docs, docs past n cleared.
+__device__ __forceinline__ uint64_t agg_word(const uint64_t* bits, uint64_t w, uint32_t n) {
+    const uint64_t d0 = w * 64;
+    if (d0 >= n) return 0;
+    const uint64_t left = n - d0;
+    const uint64_t v = bits[w];
+    return left >= 64 ? v : v & ((1ull << left) - 1);
 }
 
-// Exclusive scan of nb block counts in place (one CTA); writes the total to *total.
-__global__ void __launch_bounds__(1024) aggregate_scan_kernel(uint32_t* __restrict__ block_count, uint32_t nb,
-                                                              uint32_t* __restrict__ total) {
+// Kept docs of each block of kAggDocs docs, one warp per block.
+__global__ void __launch_bounds__(256) aggregate_count_kernel(const uint64_t* __restrict__ bits, uint32_t n,
+                                                              uint32_t nb, uint32_t* __restrict__ block_count) {
+    const uint32_t b = blockIdx.x * 8u + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+    if (b >= nb) return;
+    uint32_t c = 0;
+#pragma unroll
+    for (uint32_t i = 0; i < kAggWords / 32; ++i)
+        c += __popcll(agg_word(bits, static_cast<uint64_t>(b) * kAggWords + lane + 32u * i, n));
+    c = warp_sum(c);
+    if (lane == 0) block_count[b] = c;
+}
+
+// Exclusive scan of nb block counts in place (one CTA).
+__global__ void __launch_bounds__(1024) aggregate_scan_kernel(uint32_t* __restrict__ block_count, uint32_t nb) {
     __shared__ uint32_t warp_tot[32];
     __shared__ uint32_t carry;
     if (threadIdx.x == 0) carry = 0;
@@ -713,41 +786,102 @@ __global__ void __launch_bounds__(1024) aggregate_scan_kernel(uint32_t* __restri
         if (threadIdx.x == blockDim.x - 1) carry = excl + v;
         __syncthreads();
     }
-    if (threadIdx.x == 0) *total = carry;
 }
 
+template <int MODE>
 __global__ void __launch_bounds__(kAggT) aggregate_scatter_kernel(const uint64_t* __restrict__ bits,
                                                                   const float* __restrict__ scores,
                                                                   const uint32_t* __restrict__ loc_in, uint32_t n,
-                                                                  const uint32_t* __restrict__ block_off,
+                                                                  const uint32_t* __restrict__ blocks,
                                                                   float* __restrict__ out_scores,
-                                                                  uint32_t* __restrict__ out_loc) {
-    __shared__ uint32_t woff[kAggT / 32];
-    const uint32_t doc = blockIdx.x * kAggT + threadIdx.x;
-    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const bool hit = doc < n && ((bits[doc >> 6] >> (doc & 63)) & 1ull);
-    const uint32_t m = __ballot_sync(0xffffffffu, hit);
-    if (lane == 0) woff[warp] = __popc(m);
-    __syncthreads();
-    if (warp == 0) {
-        uint32_t v = woff[lane], x = v;
+                                                                  uint32_t* __restrict__ out_loc,
+                                                                  uint32_t* __restrict__ total) {
+    __shared__ uint32_t wsum[kAggT / 32];
+    __shared__ uint32_t woff[kAggWords];
+    __shared__ uint64_t wbits[kAggWords];
+    const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5, b = blockIdx.x;
+    // kept docs before this block: this thread's share of them
+    uint32_t before = 0;
+    if (MODE == kAggOwn) {
+        // whole words below the block; the bitmap is only 8-byte aligned
+        const uint32_t words = b * kAggWords;
+#pragma unroll 8
+        for (uint32_t w = t; w < words; w += kAggT) before += __popcll(__ldg(bits + w));
+    } else if (MODE == kAggSums) {
+        for (uint32_t i = t; i < b; i += kAggT) before += blocks[i];
+    } else if (t == 0) {
+        before = blocks[b];
+    }
+    uint32_t c = 0;
+    if (t < kAggWords) {
+        const uint64_t v = agg_word(bits, static_cast<uint64_t>(b) * kAggWords + t, n);
+        wbits[t] = v;
+        c = static_cast<uint32_t>(__popcll(v));
+    }
+    // exclusive offsets of the block's words (the first four warps), and the sum of every thread's share
+    uint32_t x = c;
+    if (t < kAggWords) {
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
             if (lane >= static_cast<uint32_t>(o)) x += y;
         }
-        woff[lane] = x - v;
+        woff[t] = x - c;
     }
+    before = warp_sum(before);
+    __shared__ uint32_t qsum[kAggWords / 32];
+    if (lane == 31 && warp < kAggWords / 32) qsum[warp] = x;
+    if (lane == 0) wsum[warp] = before;
     __syncthreads();
-    if (hit) {
-        const uint32_t pos = block_off[blockIdx.x] + woff[warp] + __popc(m & ((1u << lane) - 1u));
-        out_scores[pos] = scores[doc];
-        out_loc[pos] = loc_in ? loc_in[doc] : doc;
+    const uint32_t base = warp_sum(lane < kAggT / 32 ? wsum[lane] : 0u);
+    // a warp takes four words (256 docs): 8 coalesced loads per thread in flight, only for kept docs
+    const uint32_t w0 = warp * 4u;
+    uint32_t off = base;
+#pragma unroll
+    for (uint32_t i = 0; i < kAggWords / 32; ++i)
+        if (i < w0 / 32u) off += qsum[i];
+    float s[8];
+    uint32_t l[8], at[8];
+    uint32_t hits = 0;
+#pragma unroll
+    for (uint32_t j = 0; j < 8; ++j) {
+        const uint64_t wv = wbits[w0 + j / 2];
+        const uint32_t low = static_cast<uint32_t>(wv);
+        const uint32_t half = j & 1u ? static_cast<uint32_t>(wv >> 32) : low;
+        const uint64_t doc = static_cast<uint64_t>(b) * kAggDocs + (w0 + j / 2) * 64u + (j & 1u) * 32u + lane;
+        at[j] = off + woff[w0 + j / 2] + (j & 1u ? __popc(low) : 0) + __popc(half & ((1u << lane) - 1u));
+        if ((half >> lane) & 1u) {
+            hits |= 1u << j;
+            s[j] = scores[doc];
+            l[j] = loc_in ? loc_in[doc] : static_cast<uint32_t>(doc);
+        }
+    }
+#pragma unroll
+    for (uint32_t j = 0; j < 8; ++j)
+        if ((hits >> j) & 1u) {
+            out_scores[at[j]] = s[j];
+            out_loc[at[j]] = l[j];
+        }
+    if (b == gridDim.x - 1 && t == 0) {
+        uint32_t sum = base;
+#pragma unroll
+        for (uint32_t i = 0; i < kAggWords / 32; ++i) sum += qsum[i];
+        *total = sum;
     }
 }
 
 // ---------------------------------------------------------------------------------------------
-// TOPK operator: exact top K of one compacted list, one CTA.
+// TOPK operator: exact top K of one compacted list, one thread-block cluster. The list's length is only
+// known on the device and the caller gives no scratch, so the CTAs of one cluster work together through
+// distributed shared memory: a 12-bit digit histogram of the keys per CTA, summed over the cluster,
+// picks the digit of the K-th key; as soon as the keys at or above its bucket fit the sort buffer they
+// go to the first CTA, which sorts them. For real scores that is one digit: the scores are read twice.
+// A list longer than kTopkSample is first bounded from below by an evenly spaced sample, so that the
+// histogram only counts keys that can still be among the top K (shared-memory atomics on a few crowded
+// bins would bound the pass otherwise). One CTA over eight digits took 357 us for the top 100 of
+// 131,072 scores; 16 CTAs take 11 us.
+constexpr uint32_t kTopkSample = 65536;
+
 __global__ void __launch_bounds__(kST) topk_op_kernel(const float* __restrict__ scores,
                                                       const uint32_t* __restrict__ locs,
                                                       const uint32_t* __restrict__ count, uint32_t k,
@@ -755,19 +889,125 @@ __global__ void __launch_bounds__(kST) topk_op_kernel(const float* __restrict__ 
                                                       uint32_t* __restrict__ out_count) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     SelectSmem& S = *reinterpret_cast<SelectSmem*>(smem_raw);
+    cg::cluster_group cluster = cg::this_cluster();
+    const uint32_t C = cluster.num_blocks(), rank = cluster.block_rank(), t = threadIdx.x;
     const uint32_t n = *count;
     const uint32_t kq = min(k, n);
-    if (kq == 0) {
-        if (threadIdx.x == 0) *out_count = 0;
-        return;
+    uint32_t m;  // keys to sort
+    if (kq == 0 || n <= static_cast<uint32_t>(kMaxTopK)) {  // uniform over the cluster: no remote access follows
+        if (rank != 0) return;
+        if (kq == 0) {
+            if (t == 0) *out_count = 0;
+            return;
+        }
+        m = gather_top_keys([&](uint32_t i) { return result_key(scores[i], locs[i]); }, n, kq, S);
+    } else {
+        uint32_t* hist = &S.hist[0][0];
+        const uint32_t gt = rank * kST + t, gthreads = C * kST;
+        // fn(index, score) for the entries mul * i, i < cnt, 4 loads in flight
+        auto visit = [&](uint32_t cnt, uint32_t mul, auto fn) {
+            for (uint64_t i = gt; i < cnt; i += 4ull * gthreads) {
+                float v[4];
+#pragma unroll
+                for (uint32_t u = 0; u < 4; ++u) {
+                    const uint64_t at = i + static_cast<uint64_t>(u) * gthreads;
+                    v[u] = at < cnt ? scores[at * mul] : 0.0f;
+                }
+#pragma unroll
+                for (uint32_t u = 0; u < 4; ++u) {
+                    const uint64_t at = i + static_cast<uint64_t>(u) * gthreads;
+                    if (at < cnt) fn(static_cast<uint32_t>(at * mul), v[u]);
+                }
+            }
+        };
+        // the histograms of all CTAs summed into every CTA's own: each sums a slice of the bins, then
+        // gathers the others' slices (a CTA's histogram and slice are not written again before every
+        // CTA has read them: the next pass writes its histogram after the second barrier, its slice
+        // after the next pass's first)
+        auto sum_cluster = [&] {
+            cluster.sync();
+            const uint32_t slice = 4096u / C;
+            if (t < slice) {
+                uint32_t s = 0;
+                for (uint32_t r = 0; r < C; ++r) s += cluster.map_shared_rank(hist, r)[rank * slice + t];
+                S.segn[t] = s;
+            }
+            cluster.sync();
+            for (uint32_t i = t; i < 4096u; i += kST) hist[i] = cluster.map_shared_rank(S.segn, i / slice)[i % slice];
+            __syncthreads();
+        };
+        auto clear = [&] {
+            for (uint32_t i = t; i < 4096u; i += kST) hist[i] = 0;
+            __syncthreads();
+        };
+        uint32_t floor_key = 0;  // keys below it are not among the top K
+        if (n > 2u * kTopkSample) {
+            clear();
+            visit(kTopkSample, n / kTopkSample, [&](uint32_t, float v) { atomicAdd(&hist[float_key(v) >> 20], 1u); });
+            sum_cluster();
+            uint32_t kr = kq;  // kq <= kMaxTopK < kTopkSample
+            floor_key = pick_digit4096(hist, &kr, S) << 20;
+        }
+        uint64_t prefix = 0, mask = 0;
+        uint32_t krem = kq, in_bin = 0;
+        const int shifts[6] = {52, 40, 32, 20, 8, 0};
+        bool fits = false;
+        for (int p = 0; p < 6 && !fits; ++p) {
+            const int shift = shifts[p];
+            const uint64_t digit = p == 2 || p == 5 ? 255ull : 4095ull;
+            clear();
+            visit(n, 1u, [&](uint32_t i, float v) {
+                const uint32_t hi = float_key(v);
+                if (hi < floor_key || ((static_cast<uint64_t>(hi) << 32) & mask) >> 32 != prefix >> 32) return;
+                uint64_t key = static_cast<uint64_t>(hi) << 32;
+                if (p >= 3) {
+                    key = result_key(v, locs[i]);
+                    if ((key & mask) != prefix) return;
+                }
+                atomicAdd(&hist[(key >> shift) & digit], 1u);
+            });
+            sum_cluster();
+            const uint64_t d = pick_digit4096(hist, &krem, S, &in_bin);
+            prefix |= d << shift;
+            mask |= digit << shift;
+            fits = (kq - krem) + in_bin <= static_cast<uint32_t>(kMaxTopK);
+        }
+        // the keys above the bucket (kq - krem of them), then the bucket's own, into the first CTA's
+        // buffer: all of them when they fit; otherwise every bit is fixed, the bucket holds copies of
+        // one key (an entry listed more than once) and the first krem of them are as good as any
+        if (t == 0) {
+            S.counter = 0;
+            S.total = 0;
+        }
+        cluster.sync();
+        SelectSmem* S0 = cluster.map_shared_rank(&S, 0);
+        const uint32_t above = kq - krem;
+        visit(n, 1u, [&](uint32_t i, float v) {
+            const uint32_t hi = float_key(v);
+            if (hi < static_cast<uint32_t>(prefix >> 32)) return;
+            const uint64_t key = result_key(v, locs[i]);
+            if ((key & mask) < prefix) return;
+            if ((key & mask) > prefix) {
+                S0->sortbuf[atomicAdd(&S0->counter, 1u)] = key;
+            } else {
+                const uint32_t at = above + atomicAdd(&S0->total, 1u);
+                if (at < static_cast<uint32_t>(kMaxTopK)) S0->sortbuf[at] = key;
+            }
+        });
+        cluster.sync();
+        if (rank != 0) return;
+        const uint32_t got = min(above + S.total, static_cast<uint32_t>(kMaxTopK));
+        m = sort_size(got);
+        for (uint32_t i = got + t; i < m; i += kST) S.sortbuf[i] = 0ull;
+        __syncthreads();
     }
-    top_keys([&](uint32_t i) { return result_key(scores[i], locs[i]); }, n, kq, S);
-    for (uint32_t i = threadIdx.x; i < kq; i += blockDim.x) {
+    bitonic_desc(S, m);
+    for (uint32_t i = t; i < kq; i += kST) {
         const uint64_t key = S.sortbuf[i];
         out_scores[i] = result_key_score(key);
         out_locs[i] = result_key_loc(key);
     }
-    if (threadIdx.x == 0) *out_count = kq;
+    if (t == 0) *out_count = kq;
 }
 
 // Per-query error bounds: eps = c * ||q||_2 * max_doc ||v||_2 (Cauchy-Schwarz on sum |q_i v_i|),
@@ -842,31 +1082,69 @@ cudaError_t launch_query_eps(const float* qry, const uint32_t* qlist, uint32_t n
 }
 
 size_t aggregate_workspace_bytes(uint32_t n) {
-    const size_t nb = (static_cast<size_t>(n) + kAggT - 1) / kAggT;
+    const size_t nb = (static_cast<size_t>(n) + 1023) / 1024;
     return (nb > 0 ? nb : 1) * sizeof(uint32_t);
 }
 
+// One launch while a CTA counts the bitmap below it about as fast as a second launch starts (the last
+// CTA's chain is the longest, 4 KB of words a step, 128 KB at 2^20 docs: 8.0 us there against 9.3 us for
+// two launches at 1.5M, 6.7 us below 500,000); block counts added up by every CTA while they are few; a
+// scan of them beyond.
 cudaError_t launch_aggregate(const uint64_t* bits, const float* scores, const uint32_t* loc_in, uint32_t n,
                              float* out_scores, uint32_t* out_loc, uint32_t* total, uint32_t* workspace,
                              cudaStream_t stream) {
-    const uint32_t nb = (n + kAggT - 1) / kAggT;
+    constexpr uint32_t kOwnDocs = 1u << 20;
+    constexpr uint32_t kSumBlocks = 16384;
+    const uint32_t nb = static_cast<uint32_t>((static_cast<uint64_t>(n) + kAggDocs - 1) / kAggDocs);
     if (nb == 0) return cudaMemsetAsync(total, 0, sizeof(uint32_t), stream);
-    aggregate_count_kernel<<<nb, kAggT, 0, stream>>>(bits, n, workspace);
-    aggregate_scan_kernel<<<1, 1024, 0, stream>>>(workspace, nb, total);
-    aggregate_scatter_kernel<<<nb, kAggT, 0, stream>>>(bits, scores, loc_in, n, workspace, out_scores, out_loc);
+    if (n <= kOwnDocs) {
+        aggregate_scatter_kernel<kAggOwn>
+            <<<nb, kAggT, 0, stream>>>(bits, scores, loc_in, n, workspace, out_scores, out_loc, total);
+        return cudaGetLastError();
+    }
+    aggregate_count_kernel<<<(nb + 7) / 8, 256, 0, stream>>>(bits, n, nb, workspace);
+    if (nb <= kSumBlocks) {
+        aggregate_scatter_kernel<kAggSums>
+            <<<nb, kAggT, 0, stream>>>(bits, scores, loc_in, n, workspace, out_scores, out_loc, total);
+        return cudaGetLastError();
+    }
+    aggregate_scan_kernel<<<1, 1024, 0, stream>>>(workspace, nb);
+    aggregate_scatter_kernel<kAggScanned>
+        <<<nb, kAggT, 0, stream>>>(bits, scores, loc_in, n, workspace, out_scores, out_loc, total);
     return cudaGetLastError();
 }
 
-// Scratch of the allocation-free aggregator: one block count per kAggT docs, kAggStaticBlocks of
-// them (64 KB, docNumber <= 16,777,216). Module-scope, so it exists once per device for the life of
+// Scratch of the allocation-free aggregator: one word per 1,024 docs, kAggStaticBlocks of them (64 KB,
+// docNumber <= 16,777,216; the count kernel writes one per kAggDocs docs). Module-scope, so it exists once per device for the life of
 // the process and every call on that device shares it. The count kernel writes every entry a call
 // reads before the scan reads it, so a call never sees an earlier call's contents and nothing has to
 // be cleared; two calls that overlap on the GPU (different streams, no ordering) do race on it.
 static __device__ __align__(256) uint32_t g_aggregate_scratch[kAggStaticBlocks];
-static_assert(kAggStaticMaxDocs == kAggStaticBlocks * static_cast<uint32_t>(kAggT), "one block count per kAggT docs");
+static_assert(kAggStaticMaxDocs == kAggStaticBlocks * 1024u && kAggDocs >= 1024u, "a block count per 1,024 docs at most");
 
 cudaError_t aggregate_static_scratch(uint32_t** scratch) {
     return cudaGetSymbolAddress(reinterpret_cast<void**>(scratch), g_aggregate_scratch);
+}
+
+// CTAs of the TOPK operator's cluster on the current device: 16 where a GPC holds them, else the portable
+// 8. A property of the device, asked once (the query costs more host time than the launch).
+static unsigned topk_cluster(cudaLaunchConfig_t& cfg, cudaLaunchAttribute& attr) {
+    constexpr int kDevices = 64;
+    static std::atomic<unsigned> known[kDevices];
+    int dev = 0;
+    const bool keep = cudaGetDevice(&dev) == cudaSuccess && dev >= 0 && dev < kDevices;
+    unsigned size = keep ? known[dev].load(std::memory_order_relaxed) : 0u;
+    if (size) return size;
+    size = 16;
+    attr.val.clusterDim.x = size;
+    cfg.gridDim = dim3(size, 1, 1);
+    int clusters = 0;
+    if (cudaOccupancyMaxActiveClusters(&clusters, topk_op_kernel, &cfg) != cudaSuccess || clusters < 1) {
+        cudaGetLastError();
+        size = 8;
+    }
+    if (keep) known[dev].store(size, std::memory_order_relaxed);
+    return size;
 }
 
 cudaError_t launch_topk_op(const float* scores, const uint32_t* locs, const uint32_t* count, uint32_t k,
@@ -874,9 +1152,23 @@ cudaError_t launch_topk_op(const float* scores, const uint32_t* locs, const uint
     if (k > static_cast<uint32_t>(kMaxTopK)) return cudaErrorInvalidValue;
     const size_t smem = sizeof(SelectSmem);
     cudaError_t e = set_smem(topk_op_kernel, smem);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(topk_op_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e != cudaSuccess) return e;
-    topk_op_kernel<<<1, kST, smem, stream>>>(scores, locs, count, k, out_scores, out_locs, out_count);
-    return cudaGetLastError();
+    cudaLaunchConfig_t cfg{};
+    cfg.blockDim = dim3(kST, 1, 1);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    const unsigned size = topk_cluster(cfg, attr[0]);
+    attr[0].val.clusterDim.x = size;
+    cfg.gridDim = dim3(size, 1, 1);
+    return cudaLaunchKernelEx(&cfg, topk_op_kernel, scores, locs, count, k, out_scores, out_locs, out_count);
 }
 
 
