@@ -1178,6 +1178,12 @@ cudaError_t launch_topk_op(const float* scores, const uint32_t* locs, const uint
 // shard first (within a shard, list order). Every entry finds its output position directly: its
 // index in its own list plus, for every other shard, how many of that shard's entries precede it
 // (a binary search on the score), so one thread places one entry and no thread waits on another.
+// Only entries that can be among the top K take part: where m shards hold at least j = ceil(K / m)
+// entries, K entries score at least tau, the least of those shards' j-th scores, and a list's entries
+// from tau up are a prefix of it. The prefixes (a little over K entries in all when the shards are
+// alike) are ranked in shared memory, where the searches' instructions bound the kernel: eight lists of
+// 1,000 for 256 queries took 98 us when every entry searched every list in global memory, 29 us with the
+// prefixes in shared memory and general binary searches, and take 17 us with padded lists of keys.
 namespace {
 // Entries of a list sorted by score descending that come before score x: those with score > x, or
 // with score >= x when `ties_first` (a lower shard).
@@ -1194,38 +1200,123 @@ __device__ inline uint32_t preceding(const float* sc, uint32_t n, float x, bool 
     return lo;
 }
 
-__global__ void __launch_bounds__(256) merge_shards_kernel(const __grid_constant__ ShardMergeLaunch L) {
-    const uint32_t q = blockIdx.x;
-    __shared__ uint32_t s_n[kMaxShards], s_off[kMaxShards + 1];
-    if (threadIdx.x == 0) {
-        uint32_t total = 0;
-        for (uint32_t s = 0; s < L.shards; ++s) {
-            uint32_t c = L.counts[s][q];
-            c = min(c, min(L.in_stride, L.topk));
-            s_n[s] = c;
-            s_off[s] = total;
-            total += c;
+constexpr int kMergeT = 1024;
+constexpr uint32_t kMergeCap = 12000;  // keys held in shared memory (with the rest within 48 KB)
+
+__global__ void __launch_bounds__(kMergeT) merge_shards_kernel(const __grid_constant__ ShardMergeLaunch L) {
+    extern __shared__ __align__(16) uint32_t merge_key[];  // [shards][P]
+    __shared__ uint32_t s_n[kMaxShards];
+    __shared__ float s_tau;
+    __shared__ int s_all;
+    const uint32_t q = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint64_t row = static_cast<uint64_t>(q) * L.in_stride;
+    if (warp == 0) {
+        // lane l holds the counts of shards l and l + 32
+        const uint32_t most = min(L.in_stride, L.topk);
+        const uint32_t c0 = lane < L.shards ? min(L.counts[lane][q], most) : 0u;
+        const uint32_t c1 = lane + 32 < L.shards ? min(L.counts[lane + 32][q], most) : 0u;
+        const uint32_t total = warp_sum(c0 + c1);
+        // the most shards m that hold ceil(topk / m) entries each
+        uint32_t j = 0;
+        if (total > L.topk)
+            for (uint32_t m = L.shards; m > 0 && j == 0; --m) {
+                const uint32_t want = (L.topk + m - 1) / m;
+                const uint32_t have = __popc(__ballot_sync(0xffffffffu, c0 >= want)) +
+                                      __popc(__ballot_sync(0xffffffffu, c1 >= want));
+                if (want > 0 && have >= m) j = want;
+            }
+        float tau = INFINITY;
+        if (j > 0) {
+            const float a = c0 >= j ? L.scores[lane][row + j - 1] : INFINITY;
+            const float b = c1 >= j ? L.scores[lane + 32][row + j - 1] : INFINITY;
+            tau = fminf(a, b);
         }
-        s_off[L.shards] = total;
-        L.out_count[q] = min(total, L.topk);
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) tau = fminf(tau, __shfl_xor_sync(0xffffffffu, tau, o));
+        s_n[lane] = c0;
+        s_n[lane + 32] = c1;
+        if (lane == 0) {
+            s_tau = tau;
+            s_all = j == 0;
+            L.out_count[q] = min(total, L.topk);
+        }
     }
     __syncthreads();
-    const uint32_t total = s_off[L.shards];
-    for (uint32_t e = threadIdx.x; e < total; e += blockDim.x) {
-        uint32_t s = 0;
-        while (e >= s_off[s + 1]) ++s;
-        const uint32_t i = e - s_off[s];
-        const uint64_t row = static_cast<uint64_t>(q) * L.in_stride;
-        const float x = L.scores[s][row + i];
-        uint32_t pos = i;
-        for (uint32_t t = 0; t < L.shards && pos < L.topk; ++t)
-            if (t != s) pos += preceding(L.scores[t] + row, s_n[t], x, t < s);
-        if (pos < L.topk) {
-            const uint64_t o = static_cast<uint64_t>(q) * L.out_stride + pos;
-            L.out_score[o] = x;
-            L.out_id[o] = L.ids[s][row + i];
+    if (!s_all) {
+        // each list's entries that are not below tau: a 32-way search per warp (a NaN is not below it)
+        const float tau = s_tau;
+        for (uint32_t s = warp; s < L.shards; s += kMergeT / 32) {
+            const float* sc = L.scores[s] + row;
+            uint32_t lo = 0, hi = s_n[s];  // entries before lo are in, those from hi on are out
+            while (lo < hi) {
+                const uint32_t step = (hi - lo + 31) / 32;
+                const uint32_t at = lo + lane * step;
+                const bool in = at < hi && !(sc[at] < tau);
+                const uint32_t ins = __popc(__ballot_sync(0xffffffffu, in));  // a prefix of the lanes
+                if (ins == 0) {
+                    hi = lo;
+                } else {
+                    hi = min(hi, lo + ins * step);
+                    lo = lo + (ins - 1) * step + 1;
+                }
+            }
+            __syncwarp();
+            if (lane == 0) s_n[s] = lo;
         }
+        __syncthreads();
     }
+    // The prefixes' scores as order-preserving keys, each list padded with zeros to the same power of two:
+    // a search for how many keys of list t exceed a key is then log2(P) identical steps. An equal key of a
+    // lower shard precedes: it exceeds the key minus one.
+    uint32_t longest = max(s_n[lane], s_n[lane + 32]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) longest = max(longest, __shfl_xor_sync(0xffffffffu, longest, o));
+    if (longest == 0) return;
+    const uint32_t log_p = 32u - __clz(longest), P = 1u << log_p;  // P > longest: the search can pass every entry
+    if (L.shards * static_cast<uint64_t>(P) <= kMergeCap) {
+        for (uint32_t e = threadIdx.x; e < L.shards * P; e += kMergeT) {
+            const uint32_t s = e >> log_p, i = e & (P - 1u);
+            merge_key[e] = i < s_n[s] ? float_key(L.scores[s][row + i]) : 0u;
+        }
+        __syncthreads();
+        for (uint32_t e = threadIdx.x; e < L.shards * P; e += kMergeT) {
+            const uint32_t s = e >> log_p, i = e & (P - 1u);
+            if (i >= s_n[s]) continue;
+            const uint32_t key = merge_key[e];
+            const int64_t id = L.ids[s][row + i];
+            uint32_t pos = i;
+            for (uint32_t t = 0; t < L.shards; t += 2) {  // two searches at a time
+                const bool b = t + 1 < L.shards;
+                const uint32_t ka = key - (t < s ? 1u : 0u), kb = key - (t + 1 < s ? 1u : 0u);
+                const uint32_t *pa = merge_key + t * P - 1, *pb = b ? pa + P : pa;
+                uint32_t na = 0, nb = 0;
+                for (uint32_t step = P >> 1; step > 0; step >>= 1) {
+                    na += pa[na + step] > ka ? step : 0u;
+                    nb += pb[nb + step] > kb ? step : 0u;
+                }
+                pos += (t != s ? na : 0u) + (b && t + 1 != s ? nb : 0u);
+            }
+            if (pos < L.topk) {
+                const uint64_t o = static_cast<uint64_t>(q) * L.out_stride + pos;
+                L.out_score[o] = L.scores[s][row + i];
+                L.out_id[o] = id;
+            }
+        }
+        return;
+    }
+    // prefixes past the buffer: searched in global memory
+    for (uint32_t s = 0; s < L.shards; ++s)
+        for (uint32_t i = threadIdx.x; i < s_n[s]; i += kMergeT) {
+            const float x = L.scores[s][row + i];
+            uint32_t pos = i;
+            for (uint32_t t = 0; t < L.shards && pos < L.topk; ++t)
+                if (t != s) pos += preceding(L.scores[t] + row, s_n[t], x, t < s);
+            if (pos < L.topk) {
+                const uint64_t o = static_cast<uint64_t>(q) * L.out_stride + pos;
+                L.out_score[o] = x;
+                L.out_id[o] = L.ids[s][row + i];
+            }
+        }
 }
 }  // namespace
 
@@ -1236,7 +1327,7 @@ cudaError_t launch_merge_shards(const ShardMergeLaunch& L, cudaStream_t stream) 
         return cudaErrorInvalidValue;
     for (uint32_t s = 0; s < L.shards; ++s)
         if (!L.scores[s] || !L.ids[s] || !L.counts[s]) return cudaErrorInvalidValue;
-    merge_shards_kernel<<<L.nq, 256, 0, stream>>>(L);
+    merge_shards_kernel<<<L.nq, kMergeT, kMergeCap * sizeof(uint32_t), stream>>>(L);
     return cudaGetLastError();
 }
 
