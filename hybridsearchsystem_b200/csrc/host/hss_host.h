@@ -398,8 +398,7 @@ class ThresholdModel {
     size_t OffW3() const { return OffB2() + m_h; }
     size_t OffB3() const { return OffW3() + m_h; }
     bool Reserve(uint32_t batch);
-    cudaError_t ForwardInto(const float* dX, uint32_t B, cudaStream_t s);
-    cudaError_t Backward(const float* dX, const float* dT, uint32_t B, cudaStream_t s);
+    cudaError_t TrainPass(const float* dX, const float* dT, uint32_t B, cudaStream_t s);
     int Finish(cudaError_t e, float* hLoss, uint32_t B, cudaStream_t s);
 
     int32_t m_deviceId;
@@ -412,7 +411,7 @@ class ThresholdModel {
     uint32_t m_cap = 0;
     float *m_dP = nullptr, *m_dG = nullptr, *m_dM = nullptr, *m_dV = nullptr;
     float *m_dZ1 = nullptr, *m_dA1 = nullptr, *m_dZ2 = nullptr, *m_dA2 = nullptr;
-    float *m_dY = nullptr, *m_dDy = nullptr, *m_dD1 = nullptr, *m_dD2 = nullptr, *m_dSq = nullptr;
+    float *m_dDy = nullptr, *m_dD1 = nullptr, *m_dD2 = nullptr, *m_dSq = nullptr;
 };
 
 class FullRecallSearcher {

@@ -55,7 +55,7 @@ ThresholdModel::ThresholdModel(int32_t deviceId, uint32_t din, uint32_t hidden, 
 
 ThresholdModel::~ThresholdModel() {
     cudaSetDevice(m_deviceId);
-    float* bufs[] = {m_dP, m_dG, m_dM, m_dV, m_dZ1, m_dA1, m_dZ2, m_dA2, m_dY, m_dDy, m_dD1, m_dD2, m_dSq};
+    float* bufs[] = {m_dP, m_dG, m_dM, m_dV, m_dZ1, m_dA1, m_dZ2, m_dA2, m_dDy, m_dD1, m_dD2, m_dSq};
     for (float* b : bufs)
         if (b) cudaFree(b);
 }
@@ -63,7 +63,7 @@ ThresholdModel::~ThresholdModel() {
 bool ThresholdModel::Reserve(uint32_t batch) {
     if (batch <= m_cap) return true;
     float** acts[] = {&m_dZ1, &m_dA1, &m_dZ2, &m_dA2, &m_dD1, &m_dD2};
-    float** vecs[] = {&m_dY, &m_dDy, &m_dSq};
+    float** vecs[] = {&m_dDy, &m_dSq};
     for (float** a : acts) {
         if (*a) cudaFree(*a);
         *a = nullptr;
@@ -87,43 +87,27 @@ bool ThresholdModel::Reserve(uint32_t batch) {
     return true;
 }
 
-cudaError_t ThresholdModel::ForwardInto(const float* dX, uint32_t B, cudaStream_t s) {
-    const int H = static_cast<int>(m_h), D = static_cast<int>(m_din), n = static_cast<int>(B);
-    cudaError_t e =
-        launch_gemm(false, false, dX, m_dP + OffW1(), m_dA1, n, H, D, D, H, H, m_dP + OffB1(), 1, m_dZ1, false, s);
-    if (e == cudaSuccess)
-        e = launch_gemm(false, false, m_dA1, m_dP + OffW2(), m_dA2, n, H, H, H, H, H, m_dP + OffB2(), 1, m_dZ2, false,
-                        s);
-    if (e == cudaSuccess)
-        e = launch_gemm(false, false, m_dA2, m_dP + OffW3(), m_dY, n, 1, H, H, 1, 1, m_dP + OffB3(), 0, nullptr, false,
-                        s);
-    return e;
-}
-
-// Gradients of the loss (mean squared error, or the pinball loss of the tau-quantile) after
-// ForwardInto, into m_dG (same layout as the parameters).
-cudaError_t ThresholdModel::Backward(const float* dX, const float* dT, uint32_t B, cudaStream_t s) {
-    const int H = static_cast<int>(m_h), D = static_cast<int>(m_din), n = static_cast<int>(B);
-    cudaError_t e = launch_loss_grad(m_dY, dT, n, m_tau, m_dDy, m_dSq, s);
-    // output layer: dw3 = A2^T dy, db3 = sum dy, dA2 = dy w3^T
-    if (e == cudaSuccess)
-        e = launch_gemm(true, false, m_dA2, m_dDy, m_dG + OffW3(), H, 1, n, H, 1, 1, nullptr, 0, nullptr, false, s);
-    if (e == cudaSuccess) e = launch_colsum(m_dDy, n, 1, 1, m_dG + OffB3(), s);
-    if (e == cudaSuccess)
-        e = launch_gemm(false, true, m_dDy, m_dP + OffW3(), m_dD2, n, H, 1, 1, 1, H, nullptr, 0, nullptr, false, s);
-    // hidden 2: dZ2 = dA2 * gelu'(Z2); dW2 = A1^T dZ2; db2 = colsum; dA1 = dZ2 W2^T
-    if (e == cudaSuccess) e = launch_gelu_backward(m_dD2, m_dZ2, static_cast<int64_t>(n) * H, s);
-    if (e == cudaSuccess)
-        e = launch_gemm(true, false, m_dA1, m_dD2, m_dG + OffW2(), H, H, n, H, H, H, nullptr, 0, nullptr, false, s);
-    if (e == cudaSuccess) e = launch_colsum(m_dD2, n, H, H, m_dG + OffB2(), s);
-    if (e == cudaSuccess)
-        e = launch_gemm(false, true, m_dD2, m_dP + OffW2(), m_dD1, n, H, H, H, H, H, nullptr, 0, nullptr, false, s);
-    // hidden 1: dZ1 = dA1 * gelu'(Z1); dW1 = X^T dZ1; db1 = colsum
-    if (e == cudaSuccess) e = launch_gelu_backward(m_dD1, m_dZ1, static_cast<int64_t>(n) * H, s);
-    if (e == cudaSuccess)
-        e = launch_gemm(true, false, dX, m_dD1, m_dG + OffW1(), D, H, n, D, H, H, nullptr, 0, nullptr, false, s);
-    if (e == cudaSuccess) e = launch_colsum(m_dD1, n, H, H, m_dG + OffB1(), s);
-    return e;
+// Forward pass, loss terms (into m_dSq) and gradients of the loss (mean squared error, or the pinball
+// loss of the tau-quantile) into m_dG (same layout as the parameters).
+cudaError_t ThresholdModel::TrainPass(const float* dX, const float* dT, uint32_t B, cudaStream_t s) {
+    TrainLaunch L{};
+    L.X = dX;
+    L.T = dT;
+    L.B = static_cast<int>(B);
+    L.D = static_cast<int>(m_din);
+    L.H = static_cast<int>(m_h);
+    L.tau = m_tau;
+    L.P = m_dP;
+    L.G = m_dG;
+    L.Z1 = m_dZ1;
+    L.A1 = m_dA1;
+    L.Z2 = m_dZ2;
+    L.A2 = m_dA2;
+    L.dZ1 = m_dD1;
+    L.dZ2 = m_dD2;
+    L.dy = m_dDy;
+    L.term = m_dSq;
+    return launch_train_gradients(L, s);
 }
 
 int ThresholdModel::Finish(cudaError_t e, float* hLoss, uint32_t B, cudaStream_t s) {
@@ -162,8 +146,7 @@ int ThresholdModel::Gradients(const float* dX, const float* dT, uint32_t B, floa
                               cudaStream_t s) {
     if (!m_ok || B == 0) return -1;
     if (cudaSetDevice(m_deviceId) != cudaSuccess || !Reserve(B)) return -1;
-    cudaError_t e = ForwardInto(dX, B, s);
-    if (e == cudaSuccess) e = Backward(dX, dT, B, s);
+    cudaError_t e = TrainPass(dX, dT, B, s);
     if (e == cudaSuccess && hGrad) e = cudaMemcpyAsync(hGrad, m_dG, m_np * sizeof(float), cudaMemcpyDeviceToHost, s);
     return Finish(e, hLoss, B, s);
 }
@@ -171,8 +154,7 @@ int ThresholdModel::Gradients(const float* dX, const float* dT, uint32_t B, floa
 int ThresholdModel::TrainStep(const float* dX, const float* dT, uint32_t B, float lr, float* hLoss, cudaStream_t s) {
     if (!m_ok || B == 0) return -1;
     if (cudaSetDevice(m_deviceId) != cudaSuccess || !Reserve(B)) return -1;
-    cudaError_t e = ForwardInto(dX, B, s);
-    if (e == cudaSuccess) e = Backward(dX, dT, B, s);
+    cudaError_t e = TrainPass(dX, dT, B, s);
     if (e == cudaSuccess)
         e = launch_adam(m_dP, m_dG, m_dM, m_dV, static_cast<int64_t>(m_np), lr, 0.9f, 0.999f, 1e-8f, ++m_step, s);
     return Finish(e, hLoss, B, s);

@@ -257,17 +257,21 @@ cudaError_t launch_aggregate(const uint64_t* bits, const float* scores, const ui
                              float* out_scores, uint32_t* out_loc, uint32_t* total, uint32_t* workspace,
                              cudaStream_t stream);
 // Learned threshold predictor (mlp.cu).
-// C = op(A) op(B) (+ C) (+ bias), then act (0 identity, 1 GELU); pre receives the value before act.
-cudaError_t launch_gemm(bool ta, bool tb, const float* A, const float* B, float* C, int M, int N, int K, int lda,
-                        int ldb, int ldc, const float* bias, int act, float* pre, bool accumulate,
-                        cudaStream_t stream);
-cudaError_t launch_gelu_backward(float* dA, const float* Z, int64_t n, cudaStream_t stream);
-cudaError_t launch_colsum(const float* G, int M, int N, int ld, float* out, cudaStream_t stream);
-// dL/dy and the per-row loss terms: squared error (tau = 0) or the pinball loss of the tau-quantile.
-cudaError_t launch_loss_grad(const float* y, const float* t, int B, float tau, float* dy, float* term,
-                             cudaStream_t stream);
+// One training pass over a batch: forward, loss terms and the gradient of every parameter, P and G in
+// ThresholdModel's layout. The loss: squared error (tau = 0) or the pinball loss of the tau-quantile.
+struct TrainLaunch {
+    const float *X, *T;            // [B][D] features, [B] targets
+    int B, D, H;
+    float tau;
+    const float* P;
+    float* G;
+    float *Z1, *A1, *Z2, *A2;      // [B][H] pre-activations and activations
+    float *dZ1, *dZ2;              // [B][H]
+    float *dy, *term;              // [B] the loss's gradient and each row's loss term
+};
+cudaError_t launch_train_gradients(const TrainLaunch& L, cudaStream_t stream);
 // The whole inference forward pass of the MLP (parameters P in ThresholdModel's layout) in one launch;
-// bit-identical to the three-GEMM pass. H <= 1024, 4 (D + 2H) floats of shared memory <= 48 KB.
+// bit-identical to the training pass's outputs. H <= 1024, 4 (D + 2H) floats of shared memory <= 48 KB.
 cudaError_t launch_mlp_forward(const float* X, int B, int D, int H, const float* P, float* y, cudaStream_t stream);
 cudaError_t launch_adam(float* p, const float* g, float* m, float* v, int64_t n, float lr, float b1, float b2,
                         float eps, int step, cudaStream_t stream);

@@ -5,8 +5,14 @@
 //   backward  from dL/dy: the gradients of every parameter (GEMMs with transposed operands, GELU'
 //             from the stored pre-activations, bias gradients as column sums)
 //   adam      one Adam step over the flat parameter vector
-// FP32 throughout. The GEMMs are small (batch x ~400 x 256): a shared-memory tiled SIMT GEMM with a
-// fused bias + activation epilogue is enough; they are nowhere near the search's critical path.
+// FP32 throughout. The products of a training step are small (512 x 397 x 256 at most at its usual batch,
+// 0.4 GFLOP in all, 6 us at the FP32 rate), so the step is bound by latency: few CTAs, dependent launches
+// and the load latency of each k step. Hence five launches instead of fourteen (each pass's elementwise
+// work in its epilogue, independent products side by side in one grid, bias gradients from the tiles that
+// a product already stages), 32 x 32 output tiles (at least 100 CTAs) and operands copied by cp.async
+// three k steps ahead; the gradients' products, whose sums may take any order, split k four ways inside a
+// CTA. The forward pass keeps one sum per output over k ascending. At a batch of 512, 397 features and
+// 256 hidden units the kernels took 432 us (64 x 64 tiles on 4 to 32 CTAs) and take 45 us.
 #include <algorithm>
 
 #include "hss_device.cuh"
@@ -14,9 +20,6 @@
 
 namespace hss {
 namespace {
-
-constexpr int kTM = 64, kTN = 64, kTK = 16;  // block tile
-constexpr int kGT = 256;                     // threads: 16 x 16, 4 x 4 outputs each
 
 __device__ inline float gelu(float z) { return 0.5f * z * (1.0f + erff(z * 0.70710678118654752f)); }
 __device__ inline float gelu_grad(float z) {
@@ -26,107 +29,341 @@ __device__ inline float gelu_grad(float z) {
     return cdf + z * pdf;
 }
 
-// C = op(A) op(B) (+ C when accumulate) (+ bias[n]), then the activation; pre (if given) receives the
-// value before the activation. op(A)(m, k) = TA ? A[k * lda + m] : A[m * lda + k], likewise B with
-// (k, n). act: 0 identity, 1 GELU.
-template <bool TA, bool TB>
-__global__ void __launch_bounds__(kGT) gemm_kernel(const float* __restrict__ A, const float* __restrict__ B,
-                                                  float* __restrict__ C, int M, int N, int K, int lda, int ldb,
-                                                  int ldc, const float* __restrict__ bias, int act,
-                                                  float* __restrict__ pre, int accumulate) {
-    __shared__ float sA[kTK][kTM + 4];
-    __shared__ float sB[kTK][kTN + 4];
-    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-    const int m0 = blockIdx.y * kTM, n0 = blockIdx.x * kTN;
-    float acc[4][4] = {};
-    for (int k0 = 0; k0 < K; k0 += kTK) {
-        for (int i = threadIdx.x; i < kTK * kTM; i += kGT) {
-            const int kk = TA ? i / kTM : i % kTK;
-            const int mm = TA ? i % kTM : i / kTK;
-            const int m = m0 + mm, k = k0 + kk;
-            sA[kk][mm] = (m < M && k < K) ? (TA ? A[static_cast<int64_t>(k) * lda + m]
-                                                 : A[static_cast<int64_t>(m) * lda + k])
-                                           : 0.0f;
-        }
-        for (int i = threadIdx.x; i < kTK * kTN; i += kGT) {
-            const int kk = TB ? i % kTK : i / kTN;
-            const int nn = TB ? i / kTK : i % kTN;
-            const int n = n0 + nn, k = k0 + kk;
-            sB[kk][nn] = (n < N && k < K) ? (TB ? B[static_cast<int64_t>(n) * ldb + k]
-                                                 : B[static_cast<int64_t>(k) * ldb + n])
-                                           : 0.0f;
-        }
-        __syncthreads();
+constexpr int kTile = 32;          // output tile: 32 x 32, 2 x 4 outputs per thread of a group
+constexpr int kTileK = 32;         // k per stage
+constexpr int kGroup = 128;        // threads that share one k range
+constexpr int kPitch = kTile + 4;  // staged rows of 36 floats: 16-byte reads
+constexpr int kStageFloats = 2 * kTile * kPitch;
+constexpr int kGradSplit = 4;      // k split of the gradients' products
+constexpr int kGradThreads = kGroup * kGradSplit;
+constexpr int kFwdStages = 4, kGradStages = 3;
+constexpr size_t kFwdSmem = static_cast<size_t>(kFwdStages) * kStageFloats * sizeof(float);
+constexpr size_t kGradSmem = static_cast<size_t>(kGradSplit) * kGradStages * kStageFloats * sizeof(float);
+
+// One product's operands: C[M][N] = op(A) op(B) over K.
+struct Product {
+    const float *A, *B;
+    int M, N, K, lda, ldb;
+};
+
+// min(words, `width`) floats (width 4: 16-byte aligned addresses; 1: any), zeros in the rest of width.
+template <int width>
+__device__ __forceinline__ void copy_async(float* smem, const float* gmem, int words) {
+    const uint32_t dst = static_cast<uint32_t>(__cvta_generic_to_shared(smem));
+    const int bytes = 4 * max(0, min(words, width));
+    if (width == 4)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(gmem), "r"(bytes) : "memory");
+    else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(gmem), "r"(bytes) : "memory");
+}
+
+// A 32 x 32 block of a row-major matrix [rows][cols] (pitch ld) from (r0, c0), to smem rows of kPitch;
+// zeros outside the matrix. 16-byte copies where the matrix allows them.
+__device__ __forceinline__ void copy_block(float* smem, const float* M, int rows, int cols, int ld, int r0, int c0,
+                                           int t, bool vec) {
+    if (vec) {
 #pragma unroll
-        for (int kk = 0; kk < kTK; ++kk) {
-            float a[4], b[4];
+        for (int i = 0; i < kTile * kTileK / 4 / kGroup; ++i) {
+            const int f = t + kGroup * i, r = f / 8, c = f % 8 * 4;
+            const bool in = r0 + r < rows && c0 + c < cols;
+            copy_async<4>(smem + r * kPitch + c, in ? M + static_cast<int64_t>(r0 + r) * ld + c0 + c : M,
+                          in ? cols - c0 - c : 0);
+        }
+    } else {
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                a[i] = sA[kk][ty * 4 + i];
-                b[i] = sB[kk][tx * 4 + i];
+        for (int i = 0; i < kTile * kTileK / kGroup; ++i) {
+            const int f = t + kGroup * i, r = f / 32, c = f % 32;
+            const bool in = r0 + r < rows && c0 + c < cols;
+            copy_async<1>(smem + r * kPitch + c, in ? M + static_cast<int64_t>(r0 + r) * ld + c0 + c : M, in ? 1 : 0);
+        }
+    }
+}
+
+__device__ __forceinline__ bool rows_of_16_bytes(const float* M, int ld) {
+    return (reinterpret_cast<uintptr_t>(M) & 15u) == 0 && (ld & 3) == 0;
+}
+
+// The tile at (m0, n0) of one product, into acc of group 0's threads: thread t has rows
+// 2 (t / 8) + {0, 1} and columns tile_col(t % 8, {0..3}). KS groups of 128 threads take every KS-th stage
+// of k and are summed in group order. op(A)(m, k) = TA ? A[k * lda + m] : A[m * lda + k], likewise
+// op(B)(k, n) = TB ? B[n * ldb + k] : B[k * ldb + n]; both are staged as they lie, and four k at a time
+// are read from an operand whose rows run along k. With colsum (TB false), thread t < 32 of group 0 also
+// gets the sum over k of op(B)'s column n0 + t in *colsum.
+template <bool TB>
+__device__ __forceinline__ int tile_col(int tx, int j) {
+    return TB ? tx + 8 * j : 4 * tx + j;  // TB: the 8 rows a read takes are neighbours (distinct banks)
+}
+
+template <bool TA, bool TB, int KS, int ST>
+__device__ __forceinline__ void product_tile(const Product& P, int m0, int n0, float* smem, float (&acc)[2][4],
+                                             float* colsum) {
+    const int g = threadIdx.x / kGroup, t = threadIdx.x % kGroup;
+    const int tx = t % 8, ty = t / 8;
+    float* ring = smem + g * ST * kStageFloats;
+    const int chunks = (P.K + kTileK - 1) / kTileK;
+    const int steps = (chunks + KS - 1) / KS;
+    const bool vecA = rows_of_16_bytes(P.A, P.lda), vecB = rows_of_16_bytes(P.B, P.ldb);
+    auto load = [&](int step) {
+        float* sA = ring + (step % ST) * kStageFloats;
+        float* sB = sA + kTile * kPitch;
+        const int k0 = (step * KS + g) * kTileK;
+        copy_block(sA, P.A, TA ? P.K : P.M, TA ? P.M : P.K, P.lda, TA ? k0 : m0, TA ? m0 : k0, t, vecA);
+        copy_block(sB, P.B, TB ? P.N : P.K, TB ? P.K : P.N, P.ldb, TB ? n0 : k0, TB ? k0 : n0, t, vecB);
+    };
+    auto commit = [] { asm volatile("cp.async.commit_group;" ::: "memory"); };
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f;
+    float cs = 0.0f;
+    for (int s = 0; s < ST - 1; ++s) {
+        if (s < steps) load(s);
+        commit();
+    }
+    for (int step = 0; step < steps; ++step) {
+        asm volatile("cp.async.wait_group %0;" ::"n"(ST - 2) : "memory");
+        __syncthreads();  // the stage has landed, and the one loaded next has been read by every thread
+        if (step + ST - 1 < steps) load(step + ST - 1);
+        commit();
+        const float* sA = ring + (step % ST) * kStageFloats;
+        const float* sB = sA + kTile * kPitch;
+#pragma unroll 4
+        for (int k = 0; k < kTileK; k += 4) {
+            float a[2][4], b[4][4];  // [row][k], [k][column]
+            if (TA) {
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const float2 x = *reinterpret_cast<const float2*>(sA + (k + u) * kPitch + 2 * ty);
+                    a[0][u] = x.x;
+                    a[1][u] = x.y;
+                }
+            } else {
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {
+                    const float4 x = *reinterpret_cast<const float4*>(sA + (2 * ty + i) * kPitch + k);
+                    a[i][0] = x.x;
+                    a[i][1] = x.y;
+                    a[i][2] = x.z;
+                    a[i][3] = x.w;
+                }
             }
 #pragma unroll
-            for (int i = 0; i < 4; ++i)
+            for (int u = 0; u < 4; ++u) {
+                const float4 x = *reinterpret_cast<const float4*>(TB ? sB + tile_col<TB>(tx, u) * kPitch + k
+                                                                     : sB + (k + u) * kPitch + 4 * tx);
+                if (TB) {
+                    b[0][u] = x.x;
+                    b[1][u] = x.y;
+                    b[2][u] = x.z;
+                    b[3][u] = x.w;
+                } else {
+                    b[u][0] = x.x;
+                    b[u][1] = x.y;
+                    b[u][2] = x.z;
+                    b[u][3] = x.w;
+                }
+            }
 #pragma unroll
-                for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+            for (int u = 0; u < 4; ++u)
+#pragma unroll
+                for (int i = 0; i < 2; ++i)
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(a[i][u], b[u][j], acc[i][j]);
+        }
+        if (colsum && t < kTile) {
+#pragma unroll 8
+            for (int kk = 0; kk < kTileK; ++kk) cs += sB[kk * kPitch + t];
+        }
+    }
+    if (KS > 1) {
+        asm volatile("cp.async.wait_all;" ::: "memory");
+        __syncthreads();
+        float* part = smem;  // [KS - 1][9][kGroup]
+        if (g > 0) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) part[((g - 1) * 9 + j) * kGroup + t] = acc[j / 4][j % 4];
+            part[((g - 1) * 9 + 8) * kGroup + t] = cs;
+        }
+        __syncthreads();
+        if (g == 0) {
+#pragma unroll
+            for (int s = 0; s < KS - 1; ++s) {
+#pragma unroll
+                for (int j = 0; j < 8; ++j) acc[j / 4][j % 4] += part[(s * 9 + j) * kGroup + t];
+                cs += part[(s * 9 + 8) * kGroup + t];
+            }
+        }
+    }
+    if (colsum) *colsum = cs;
+}
+
+// fn(index into C, row, column, value) for the outputs of a tile that lie inside [M][N] (group 0 only).
+template <bool TB, class Fn>
+__device__ __forceinline__ void store_tile(const Product& P, int m0, int n0, const float (&acc)[2][4], Fn fn) {
+    if (threadIdx.x >= kGroup) return;
+    const int tx = threadIdx.x % 8, ty = threadIdx.x / 8;
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const int m = m0 + 2 * ty + i;
+        if (m >= P.M) continue;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int n = n0 + tile_col<TB>(tx, j);
+            if (n < P.N) fn(static_cast<int64_t>(m) * P.N + n, n, acc[i][j]);
+        }
+    }
+}
+
+__device__ __forceinline__ void tile_of(int64_t tile, int N, int* m0, int* n0) {
+    const int across = (N + kTile - 1) / kTile;
+    *m0 = static_cast<int>(tile / across) * kTile;
+    *n0 = static_cast<int>(tile % across) * kTile;
+}
+
+// A hidden layer of the training pass: Z = A W + b, act = gelu(Z).
+__global__ void __launch_bounds__(kGroup) layer_forward_kernel(Product P, const float* __restrict__ bias,
+                                                               float* __restrict__ Z, float* __restrict__ act) {
+    extern __shared__ __align__(16) float gsm[];
+    int m0, n0;
+    tile_of(blockIdx.x, P.N, &m0, &n0);
+    float acc[2][4];
+    product_tile<false, false, 1, kFwdStages>(P, m0, n0, gsm, acc, nullptr);
+    store_tile<false>(P, m0, n0, acc, [&](int64_t at, int n, float v) {
+        const float z = v + bias[n];
+        Z[at] = z;
+        act[at] = gelu(z);
+    });
+}
+
+// The output layer, the loss and the way back to the second hidden layer, for kHeadRows rows:
+// y = A2 w3 + b3 (each row's sum over k ascending), the loss's gradient dy and term, and
+// dZ2 = (dy w3^T) * gelu'(Z2). tau = 0: mean squared error, dy = 2 (y - t) / B, term (y - t)^2. tau in
+// (0, 1): the pinball loss of the tau-quantile, term tau (t - y) when t >= y and (1 - tau) (y - t)
+// otherwise, dy = (y > t ? 1 - tau : -tau) / B (the network then predicts a conditional tau-quantile of
+// the target).
+constexpr int kHeadRows = 8;
+constexpr int kHeadT = 256;
+constexpr int kHeadK = 256;
+
+__global__ void __launch_bounds__(kHeadT) head_kernel(const float* __restrict__ A2, const float* __restrict__ Z2,
+                                                      const float* __restrict__ w3, const float* __restrict__ b3,
+                                                      const float* __restrict__ target, int B, int H, float tau,
+                                                      float* __restrict__ dy, float* __restrict__ term,
+                                                      float* __restrict__ dZ2) {
+    __shared__ float sa[kHeadRows][kHeadK + 1];
+    __shared__ float sw[kHeadK];
+    __shared__ float sdy[kHeadRows];
+    const int r0 = blockIdx.x * kHeadRows, t = threadIdx.x;
+    const int rows = min(kHeadRows, B - r0);
+    float acc = 0.0f;
+    for (int k0 = 0; k0 < H; k0 += kHeadK) {
+        const int kc = min(kHeadK, H - k0);
+        if (t < kc) sw[t] = w3[k0 + t];
+#pragma unroll
+        for (int r = 0; r < kHeadRows; ++r)
+            if (t < kc && r < rows) sa[r][t] = A2[static_cast<int64_t>(r0 + r) * H + k0 + t];
+        __syncthreads();
+        if (t < rows) {
+#pragma unroll 16
+            for (int k = 0; k < kc; ++k) acc = fmaf(sa[t][k], sw[k], acc);
         }
         __syncthreads();
     }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int m = m0 + ty * 4 + i;
-        if (m >= M) continue;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-            const int n = n0 + tx * 4 + j;
-            if (n >= N) continue;
-            const int64_t at = static_cast<int64_t>(m) * ldc + n;
-            float v = acc[i][j];
-            if (accumulate) v += C[at];
-            if (bias) v += bias[n];
-            if (pre) pre[at] = v;
-            C[at] = act == 1 ? gelu(v) : v;
+    if (t < rows) {
+        const float d = acc + b3[0] - target[r0 + t];
+        float g, l;
+        if (tau <= 0.0f) {
+            g = 2.0f * d / static_cast<float>(B);
+            l = d * d;
+        } else {
+            g = (d > 0.0f ? 1.0f - tau : -tau) / static_cast<float>(B);
+            l = d > 0.0f ? (1.0f - tau) * d : -tau * d;
         }
+        sdy[t] = g;
+        dy[r0 + t] = g;
+        term[r0 + t] = l;
+    }
+    __syncthreads();
+    for (int j = t; j < H; j += kHeadT) {
+        const float w = w3[j];
+#pragma unroll
+        for (int r = 0; r < kHeadRows; ++r)
+            if (r < rows) {
+                const int64_t at = static_cast<int64_t>(r0 + r) * H + j;
+                dZ2[at] = sdy[r] * w * gelu_grad(Z2[at]);
+            }
     }
 }
 
-// dZ = dA * gelu'(Z), in place on dA.
-__global__ void gelu_backward_kernel(float* __restrict__ dA, const float* __restrict__ Z, int64_t n) {
-    const int64_t i = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-    if (i < n) dA[i] *= gelu_grad(Z[i]);
-}
-
-// out[n] = sum_m G[m * ld + n] (bias gradients), one thread per column.
-__global__ void colsum_kernel(const float* __restrict__ G, int M, int N, int ld, float* __restrict__ out) {
-    const int n = blockIdx.x * blockDim.x + threadIdx.x;
-    if (n >= N) return;
-    float s = 0.0f;
-    for (int m = 0; m < M; ++m) s += G[static_cast<int64_t>(m) * ld + n];
-    out[n] = s;
-}
-
-// The loss's gradient dL/dy and each row's loss term. tau = 0: mean squared error, dy = 2 (y - t) / B,
-// term (y - t)^2. tau in (0, 1): the pinball loss of the tau-quantile, term tau (t - y) when t >= y and
-// (1 - tau) (y - t) otherwise, dy = (y > t ? 1 - tau : -tau) / B (the network then predicts a
-// conditional tau-quantile of the target).
-__global__ void loss_grad_kernel(const float* __restrict__ y, const float* __restrict__ t, int B, float tau,
-                                 float* __restrict__ dy, float* __restrict__ term) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= B) return;
-    const float d = y[i] - t[i];
-    if (tau <= 0.0f) {
-        dy[i] = 2.0f * d / static_cast<float>(B);
-        if (term) term[i] = d * d;
-    } else {
-        dy[i] = (d > 0.0f ? 1.0f - tau : -tau) / static_cast<float>(B);
-        if (term) term[i] = d > 0.0f ? (1.0f - tau) * d : -tau * d;
+// Gradients of the output and second hidden layer, one grid: tiles [0, tilesA) dZ1 = (dZ2 W2^T) *
+// gelu'(Z1), then tilesW of dW2 = A1^T dZ2 (those of the first 32 rows also db2, the columns' sums of
+// dZ2), then blocks of 32 outputs of dw3 = A2^T dy (the first also db3 = sum dy).
+__global__ void __launch_bounds__(kGradThreads) grad_hidden_kernel(Product dA, const float* __restrict__ Z1,
+                                                                   float* __restrict__ dZ1, int64_t tilesA, Product dW,
+                                                                   float* __restrict__ gW2, float* __restrict__ gb2,
+                                                                   int64_t tilesW, const float* __restrict__ A2,
+                                                                   const float* __restrict__ dy, int B, int H,
+                                                                   float* __restrict__ gw3, float* __restrict__ gb3) {
+    extern __shared__ __align__(16) float gsm[];
+    int64_t tile = blockIdx.x;
+    int m0, n0;
+    float acc[2][4];
+    if (tile < tilesA) {
+        tile_of(tile, dA.N, &m0, &n0);
+        product_tile<false, true, kGradSplit, kGradStages>(dA, m0, n0, gsm, acc, nullptr);
+        store_tile<true>(dA, m0, n0, acc, [&](int64_t at, int, float v) { dZ1[at] = v * gelu_grad(Z1[at]); });
+        return;
     }
+    tile -= tilesA;
+    if (tile < tilesW) {
+        tile_of(tile, dW.N, &m0, &n0);
+        float cs = 0.0f;
+        product_tile<true, false, kGradSplit, kGradStages>(dW, m0, n0, gsm, acc, m0 == 0 ? &cs : nullptr);
+        store_tile<false>(dW, m0, n0, acc, [&](int64_t at, int, float v) { gW2[at] = v; });
+        if (m0 == 0 && threadIdx.x < kTile && n0 + static_cast<int>(threadIdx.x) < dW.N) gb2[n0 + threadIdx.x] = cs;
+        return;
+    }
+    tile -= tilesW;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, j = static_cast<int>(tile) * 32 + lane;
+    constexpr int kWarps = kGradThreads / 32;
+    float s = 0.0f, sd = 0.0f;
+#pragma unroll 4
+    for (int m = warp; m < B; m += kWarps) {
+        const float g = dy[m];
+        if (j < H) s = fmaf(A2[static_cast<int64_t>(m) * H + j], g, s);
+        sd += g;
+    }
+    gsm[warp * 32 + lane] = s;
+    if (lane == 0) gsm[kWarps * 32 + warp] = sd;
+    __syncthreads();
+    if (warp == 0) {
+        float v = 0.0f, d = 0.0f;
+        for (int w = 0; w < kWarps; ++w) {
+            v += gsm[w * 32 + lane];
+            d += gsm[kWarps * 32 + w];
+        }
+        if (j < H) gw3[j] = v;
+        if (tile == 0 && lane == 0) gb3[0] = d;
+    }
+}
+
+// dW1 = X^T dZ1, db1 = the columns' sums of dZ1.
+__global__ void __launch_bounds__(kGradThreads) grad_input_kernel(Product dW, float* __restrict__ gW1,
+                                                                  float* __restrict__ gb1) {
+    extern __shared__ __align__(16) float gsm[];
+    int m0, n0;
+    tile_of(blockIdx.x, dW.N, &m0, &n0);
+    float acc[2][4];
+    float cs = 0.0f;
+    product_tile<true, false, kGradSplit, kGradStages>(dW, m0, n0, gsm, acc, m0 == 0 ? &cs : nullptr);
+    store_tile<false>(dW, m0, n0, acc, [&](int64_t at, int, float v) { gW1[at] = v; });
+    if (m0 == 0 && threadIdx.x < kTile && n0 + static_cast<int>(threadIdx.x) < dW.N) gb1[n0 + threadIdx.x] = cs;
 }
 
 // Inference forward pass fused into one launch: a CTA takes kFwdRows feature rows, thread j computes
 // hidden unit j of both layers for all of them, and thread r < kFwdRows the output of row r. Every sum
-// runs over k in ascending order with fmaf, the bias added after, as gemm_kernel does: the outputs equal
-// the three-GEMM forward pass (ForwardInto) bit for bit.
+// runs over k in ascending order with fmaf, the bias added after, as layer_forward_kernel and head_kernel
+// do: the outputs equal the training pass's (launch_train_gradients) bit for bit.
 constexpr int kFwdRows = 4;
 constexpr int kFwdUnroll = 64;  // weight loads in flight per thread
 
@@ -258,41 +495,44 @@ __global__ void predict_theta_kernel(const float* y, const float* __restrict__ e
 
 }  // namespace
 
-cudaError_t launch_gemm(bool ta, bool tb, const float* A, const float* B, float* C, int M, int N, int K, int lda,
-                        int ldb, int ldc, const float* bias, int act, float* pre, bool accumulate,
-                        cudaStream_t stream) {
-    if (M <= 0 || N <= 0 || K <= 0) return cudaSuccess;
-    const dim3 grid((N + kTN - 1) / kTN, (M + kTM - 1) / kTM);
-    if (grid.y > 65535u) return cudaErrorInvalidValue;
-    const int acc = accumulate ? 1 : 0;
-    if (!ta && !tb)
-        gemm_kernel<false, false><<<grid, kGT, 0, stream>>>(A, B, C, M, N, K, lda, ldb, ldc, bias, act, pre, acc);
-    else if (ta && !tb)
-        gemm_kernel<true, false><<<grid, kGT, 0, stream>>>(A, B, C, M, N, K, lda, ldb, ldc, bias, act, pre, acc);
-    else if (!ta && tb)
-        gemm_kernel<false, true><<<grid, kGT, 0, stream>>>(A, B, C, M, N, K, lda, ldb, ldc, bias, act, pre, acc);
-    else
-        gemm_kernel<true, true><<<grid, kGT, 0, stream>>>(A, B, C, M, N, K, lda, ldb, ldc, bias, act, pre, acc);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_gelu_backward(float* dA, const float* Z, int64_t n, cudaStream_t stream) {
-    if (n <= 0) return cudaSuccess;
-    gelu_backward_kernel<<<static_cast<unsigned>((n + 255) / 256), 256, 0, stream>>>(dA, Z, n);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_colsum(const float* G, int M, int N, int ld, float* out, cudaStream_t stream) {
-    if (N <= 0) return cudaSuccess;
-    colsum_kernel<<<(N + 127) / 128, 128, 0, stream>>>(G, M, N, ld, out);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_loss_grad(const float* y, const float* t, int B, float tau, float* dy, float* term,
-                             cudaStream_t stream) {
-    if (B <= 0) return cudaSuccess;
-    if (!(tau >= 0.0f && tau < 1.0f)) return cudaErrorInvalidValue;
-    loss_grad_kernel<<<(B + 255) / 256, 256, 0, stream>>>(y, t, B, tau, dy, term);
+cudaError_t launch_train_gradients(const TrainLaunch& L, cudaStream_t stream) {
+    if (L.B <= 0) return cudaSuccess;
+    if (!(L.tau >= 0.0f && L.tau < 1.0f)) return cudaErrorInvalidValue;
+    const int B = L.B, D = L.D, H = L.H;
+    auto tiles = [](int m, int n) {
+        return static_cast<int64_t>((m + kTile - 1) / kTile) * ((n + kTile - 1) / kTile);
+    };
+    const float* W1 = L.P;
+    const float* b1 = W1 + static_cast<int64_t>(D) * H;
+    const float* W2 = b1 + H;
+    const float* b2 = W2 + static_cast<int64_t>(H) * H;
+    const float* w3 = b2 + H;
+    const float* b3 = w3 + H;
+    float* gW1 = L.G;
+    float* gb1 = gW1 + static_cast<int64_t>(D) * H;
+    float* gW2 = gb1 + H;
+    float* gb2 = gW2 + static_cast<int64_t>(H) * H;
+    float* gw3 = gb2 + H;
+    float* gb3 = gw3 + H;
+    const int64_t tF = tiles(B, H), tW2 = tiles(H, H), tW1 = tiles(D, H), tw3 = (H + 31) / 32;
+    if (tF + tW2 + tw3 > 0x7fffffff || tW1 > 0x7fffffff) return cudaErrorInvalidValue;
+    for (const void* k : {reinterpret_cast<const void*>(grad_hidden_kernel),
+                          reinterpret_cast<const void*>(grad_input_kernel)}) {
+        cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             static_cast<int>(kGradSmem));
+        if (e != cudaSuccess) return e;
+    }
+    layer_forward_kernel<<<static_cast<unsigned>(tF), kGroup, kFwdSmem, stream>>>(Product{L.X, W1, B, H, D, D, H}, b1,
+                                                                                 L.Z1, L.A1);
+    layer_forward_kernel<<<static_cast<unsigned>(tF), kGroup, kFwdSmem, stream>>>(Product{L.A1, W2, B, H, H, H, H}, b2,
+                                                                                 L.Z2, L.A2);
+    head_kernel<<<(B + kHeadRows - 1) / kHeadRows, kHeadT, 0, stream>>>(L.A2, L.Z2, w3, b3, L.T, B, H, L.tau, L.dy,
+                                                                        L.term, L.dZ2);
+    grad_hidden_kernel<<<static_cast<unsigned>(tF + tW2 + tw3), kGradThreads, kGradSmem, stream>>>(
+        Product{L.dZ2, W2, B, H, H, H, H}, L.Z1, L.dZ1, tF, Product{L.A1, L.dZ2, H, H, B, H, H}, gW2, gb2, tW2, L.A2,
+        L.dy, B, H, gw3, gb3);
+    grad_input_kernel<<<static_cast<unsigned>(tW1), kGradThreads, kGradSmem, stream>>>(
+        Product{L.X, L.dZ1, D, H, B, D, H}, gW1, gb1);
     return cudaGetLastError();
 }
 
