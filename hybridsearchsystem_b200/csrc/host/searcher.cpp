@@ -117,8 +117,9 @@ SearcherConfig Normalised(SearcherConfig c) {
 uint32_t SampleCap(const DataTable& T, const SearcherConfig& c) {
     const uint64_t forK = (4ull * 1024 * T.GetDocNum() + c.candidateCap - 1) / c.candidateCap;
     return static_cast<uint32_t>(
-        std::min<uint64_t>(std::max<uint64_t>({forK, c.sampleDocs, static_cast<uint64_t>(kMaxTopK)}), 1u << 19) +
-        128ull * kMaxCandSegs);
+        AlignUp(std::min<uint64_t>(std::max<uint64_t>({forK, c.sampleDocs, static_cast<uint64_t>(kMaxTopK)}), 1u << 19) +
+                    128ull * kMaxCandSegs,
+                4));  // a row of group maxima starts on 16 bytes
 }
 }  // namespace
 
@@ -564,7 +565,7 @@ void FullRecallSearcher::Stage(const uint32_t* dList, uint32_t rows) {
 // SIMT pass and the single-SM tensor-core pass, 256 for the SM-pair pass.
 void FullRecallSearcher::Cand(const float* theta, float* score, uint32_t* loc, uint32_t* count, uint32_t cap,
                               uint32_t segBase, uint32_t segCap, uint64_t begin, uint64_t step, uint32_t skip,
-                              uint64_t countTiles, const uint32_t* dList, uint32_t rows, bool simt) {
+                              uint64_t countTiles, const uint32_t* dList, uint32_t rows, bool simt, float* best) {
     const DataTable& T = *m_table;
     const uint32_t g = CtasOf(rows, countTiles, cap, simt);
     if (UseSimt(simt)) {
@@ -583,6 +584,7 @@ void FullRecallSearcher::Cand(const float* theta, float* score, uint32_t* loc, u
         C.segs = g;
         C.seg_cap = segCap;
         C.seg_base = segBase;
+        C.best = best;
         C.dim = T.GetDimension();
         C.tile_begin = begin;
         C.tile_step = step;
@@ -609,6 +611,7 @@ void FullRecallSearcher::Cand(const float* theta, float* score, uint32_t* loc, u
     C.ctas = g;
     C.seg_cap = segCap;
     C.seg_base = segBase;
+    C.best = best;
     C.tile_begin = begin;
     C.tile_step = step;
     C.tile_count = countTiles;
@@ -635,6 +638,14 @@ void FullRecallSearcher::SampleTiles(uint64_t want, uint32_t rows, bool simt, ui
     *count = std::min<uint64_t>(sampTiles, (tilesU + *step - 1) / *step);
 }
 
+// Groups of a sample of `count` tiles that is kept as group maxima, 0 where it is kept as lists of docs: a
+// K past half the groups would find its threshold far below the docs' K-th best (at K = groups it is
+// the least maximum).
+uint32_t FullRecallSearcher::MaximaGroups(uint32_t rows, uint64_t count, bool simt) const {
+    const uint64_t groups = count * (UnitOf(rows, simt) / (UseSimt(simt) ? kSimtGroup : kTcGroup));
+    return groups >= 2ull * m_b.maxK && groups <= m_sampCap ? static_cast<uint32_t>(groups) : 0u;
+}
+
 uint64_t FullRecallSearcher::Sample(const uint32_t* dList, uint32_t rows, bool simt, bool raiseOnly, float* stats,
                                     float* thetaCopy, const float* emitTheta) {
     const StageLayout SL = MakeLayout(m_cfg.maxBatch);
@@ -644,6 +655,23 @@ uint64_t FullRecallSearcher::Sample(const uint32_t* dList, uint32_t rows, bool s
     const uint32_t segs = SegsOf(rows, count, m_sampCap, simt);
     const uint32_t segCap = SegCapOf(rows, count, m_sampCap, segs, simt);
     auto* dSampCount = reinterpret_cast<uint32_t*>(D + SL.sampCount);
+    if (const uint32_t groups = MaximaGroups(rows, count, simt); groups && !stats && !raiseOnly) {
+        Cand(reinterpret_cast<const float*>(D + SL.negInf), m_dSampScore, m_dSampLoc, dSampCount, m_sampCap, 0, segCap, 0,
+             step, 0, count, dList, rows, simt, m_dSampScore);
+        MaximaThresholdLaunch MT{};
+        MT.best = m_dSampScore;
+        MT.cap = m_sampCap;
+        MT.groups = groups;
+        MT.topk = reinterpret_cast<const uint32_t*>(D + SL.topk);
+        MT.eps_sample = reinterpret_cast<const float*>(D + SL.epsSamp);
+        MT.eps_main = reinterpret_cast<const float*>(D + SL.epsMain);
+        MT.theta = reinterpret_cast<float*>(D + SL.theta);
+        MT.theta_also = thetaCopy;
+        MT.qlist = dList;
+        MT.nq_list = rows;
+        Ck(launch_maxima_threshold(MT, m_b.stream));
+        return count;
+    }
     Cand(emitTheta ? emitTheta : reinterpret_cast<const float*>(D + SL.negInf), m_dSampScore, m_dSampLoc, dSampCount,
          m_sampCap, 0, segCap, 0, step, 0, count, dList, rows, simt);
     SampleThresholdLaunch ST{};
@@ -888,7 +916,7 @@ int FullRecallSearcher::EnqueueAttempt(uint32_t nq, const BatchInputs& in, float
     const DataTable& T = *m_table;
     const uint64_t words = T.GetBitmapWords();
     if (m_timing) Ck(cudaEventRecord(m_ev[0], stream));
-    const uint32_t maxK = in.maxK;
+    const uint32_t maxK = m_b.maxK = in.maxK;
     if (EnqueueFilter(nq, in, m_dBits, words, stream) != 0) Ck(cudaErrorUnknown);
     ++m_b.launches;
     Stage(nullptr, nq);
@@ -907,9 +935,10 @@ int FullRecallSearcher::EnqueueAttempt(uint32_t nq, const BatchInputs& in, float
     // the sample's proven thresholds (theta_1) are also kept in theta1, copied to the host with the
     // statuses (a copy here would stall the stream between the sample and the passes)
     auto* dTheta1 = reinterpret_cast<float*>(D + SL.theta1);
-    uint64_t sampCount;
-    if (m_b.want > m_cfg.sampleDocs) {
-        // A sample grown with K in two steps: the sample_docs sample's proven threshold first, then the
+    uint64_t sampCount = 0, grownStep = 1;
+    SampleTiles(m_b.want, nq, false, &sampCount, &grownStep);
+    if (m_b.want > m_cfg.sampleDocs && !MaximaGroups(nq, sampCount, false)) {
+        // A sample grown with K, kept as lists, in two steps: the sample_docs sample's proven threshold first, then the
         // grown sample keeps only the docs above it. Its K-th best is the same whenever it has K docs
         // above that threshold (and raises theta_1 then); otherwise theta_1 stays. Every doc of the
         // grown sample is otherwise stored and walked (K = 1000 at 10M: about 76k per query).

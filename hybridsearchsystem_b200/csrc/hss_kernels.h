@@ -89,10 +89,14 @@ struct CandLaunch {
     uint32_t cap;
     uint32_t segs, seg_cap;    // CTAs of the launch (cand_simt_segments) and entries per segment
     uint32_t seg_base;         // first segment this pass writes
+    // [nq][cap] or null: instead of candidates the pass writes, for the it-th tile it visits, the best
+    // score of each kSimtGroup docs whose filter bit is set (-inf: none) at it * (128 / kSimtGroup) + group
+    float* best;
     uint32_t dim;              // multiple of 4
     uint64_t tile_begin, tile_step, tile_count;
     uint32_t tile_skip;
 };
+constexpr uint32_t kSimtGroup = 4, kTcGroup = 8;  // docs per group maximum
 // Largest query count of one SIMT candidate pass (its per-query counts live in shared memory).
 constexpr uint32_t kMaxSimtBatch = 4096;
 // CTAs of a SIMT candidate pass over tile_count tiles into lists of `cap` entries (one list segment
@@ -130,6 +134,21 @@ struct SampleThresholdLaunch {
     float* stats;              // [nq][kSampleStats] or null (layout at kSampleStats)
 };
 
+// Threshold from a doc sample's group maxima (a candidate pass with `best` set): theta = (a lower bound of
+// the K-th best maximum) - eps_sample - eps_main, -inf where fewer than K groups hold a filtered doc.
+struct MaximaThresholdLaunch {
+    const float* best;         // [nq][cap], `groups` of each row in use; 16-byte aligned
+    uint32_t cap, groups;      // multiples of 4
+    const uint32_t* topk;      // [nq]
+    const float* eps_sample;
+    const float* eps_main;
+    float* theta;              // [nq] out
+    float* theta_also;         // [nq] or null: a copy of theta
+    const uint32_t* qlist;
+    uint32_t nq_list;
+};
+cudaError_t launch_maxima_threshold(const MaximaThresholdLaunch& L, cudaStream_t stream);
+
 struct SelectLaunch {
     const float* vec;
     const float* qry;
@@ -155,7 +174,7 @@ struct SelectLaunch {
     int32_t* status;
     const uint32_t* qlist;
     uint32_t nq_list;
-    int fast_large;            // hold up to 32,768 candidate scores in shared memory (else 12,288)
+    int fast_large;            // hold up to 32,768 candidate scores in shared memory (else 8,192)
 };
 
 // Tensor-core candidate pass (score_tc.cu).
@@ -182,6 +201,7 @@ struct TcCandLaunch {
     uint32_t cap;
     uint32_t ctas, seg_cap;    // CTAs of the launch (tc_cand_ctas); entries per list segment
     uint32_t seg_base;         // first segment this pass writes (it writes 2 per CTA)
+    float* best;               // or null: group maxima instead of candidates, as in CandLaunch (kTcGroup docs)
     uint64_t tile_begin, tile_step, tile_count;  // tiles of tc_tile_docs(nq_rows, kblocks) docs
     uint32_t tile_skip;
     uint64_t tiles128;         // 128-doc tiles of the corpus (rows of the tensor map / 128)

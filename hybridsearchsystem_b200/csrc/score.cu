@@ -160,9 +160,12 @@ cudaError_t launch_exact_tile(const float* qry, const float* docs, float* out, u
 constexpr int kCT = 256;
 constexpr int kCQ = 64;   // queries per chunk
 constexpr int kCK = 32;   // dims per smem stage
+static_assert(kSimtGroup == 4, "a thread's docs of a tile are one group");
 constexpr int kDPad = kDocTile + 4;
 constexpr int kQPad = kCQ + 4;
 
+// MAXIMA: the pass writes group maxima (CandLaunch::best) instead of candidates.
+template <bool MAXIMA>
 __global__ void __launch_bounds__(kCT) cand_simt_kernel(CandLaunch L) {
     extern __shared__ uint32_t sCount[];  // [nq_list] candidates this CTA found per query
     __shared__ __align__(16) float sD[kCK][kDPad];
@@ -261,6 +264,16 @@ __global__ void __launch_bounds__(kCT) cand_simt_kernel(CandLaunch L) {
                 if (qi == 0xffffffffu) continue;  // warp-uniform
                 const float th = sTheta[qq];
                 const uint64_t w0 = sBits[qq][0], w1 = sBits[qq][1];
+                if constexpr (MAXIMA) {
+                    float b = -INFINITY;
+#pragma unroll
+                    for (int r = 0; r < 4; ++r) {
+                        const uint32_t dl = dg * 4 + r;
+                        if (((dl < 64 ? w0 : w1) >> (dl & 63)) & 1ull) b = fmaxf(b, acc[r][j]);
+                    }
+                    L.best[static_cast<uint64_t>(qi) * L.cap + it * (kDocTile / kSimtGroup) + dg] = b;
+                    continue;
+                }
                 const uint64_t seg =
                     static_cast<uint64_t>(qi) * L.cap + static_cast<uint64_t>(L.seg_base + blockIdx.x) * L.seg_cap;
 #pragma unroll
@@ -285,6 +298,7 @@ __global__ void __launch_bounds__(kCT) cand_simt_kernel(CandLaunch L) {
             }
         }
     }
+    if (MAXIMA) return;
     __syncthreads();
     for (uint32_t i = tid; i < L.nq_list; i += kCT) {
         const uint32_t qi = L.qlist ? L.qlist[i] : i;
@@ -329,7 +343,8 @@ cudaError_t launch_cand_simt(const CandLaunch& L, int num_sms, cudaStream_t stre
         !tile_walk_fits(L.tile_begin, L.tile_step, L.tile_skip, L.tile_count, L.segs))
         return cudaErrorInvalidValue;
     const size_t smem = static_cast<size_t>(L.nq_list) * sizeof(uint32_t);
-    cand_simt_kernel<<<L.segs, kCT, smem, stream>>>(L);
+    if (L.best && L.tile_count * (kDocTile / kSimtGroup) > L.cap) return cudaErrorInvalidValue;
+    (L.best ? cand_simt_kernel<true> : cand_simt_kernel<false>)<<<L.segs, kCT, smem, stream>>>(L);
     return cudaGetLastError();
 }
 

@@ -388,7 +388,31 @@ __device__ __forceinline__ void emit_chunk(bool live, uint32_t m, const uint32_t
     }
 }
 
-template <int F, int H>
+// One 32-doc chunk's group maxima (the doc sample): the best score of each kTcGroup docs whose filter bit is
+// set, -inf where none is, as one 16-byte store. live: the chunk was read (some lane has a bit).
+template <int F>
+__device__ __forceinline__ void store_maxima(bool live, uint32_t m, const uint32_t (&v)[32], float qs,
+                                             const float* doc_scale, uint64_t doc0, float* out) {
+    float g[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+    if (live) {
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+            float x[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+                float s = __uint_as_float(v[8 * k + j]);
+                if (F == kTcE4M3) s = s * qs * __ldg(doc_scale + doc0 + 8 * k + j);
+                x[j] = (m >> (8 * k + j)) & 1u ? s : -INFINITY;
+            }
+            g[k] = max3(max3(x[0], x[1], x[2]), max3(x[3], x[4], x[5]), fmaxf(x[6], x[7]));
+        }
+    }
+    *reinterpret_cast<float4*>(out) = make_float4(g[0], g[1], g[2], g[3]);
+}
+static_assert(kTcGroup == 8, "a chunk of 32 docs holds 4 groups");
+
+// MAXIMA: the pass writes group maxima (TcCandLaunch::best) instead of candidates.
+template <int F, int H, bool MAXIMA>
 __global__ void __launch_bounds__(64 + 256 * H, 1) tc_cand_kernel(const __grid_constant__ CUtensorMap doc_map,
                                                                   const __grid_constant__ CUtensorMap qry_map,
                                                                   TcCandLaunch L) {
@@ -563,7 +587,11 @@ __global__ void __launch_bounds__(64 + 256 * H, 1) tc_cand_kernel(const __grid_c
 #pragma unroll
             for (int c = 0; c < 2; ++c) {
                 const uint64_t doc0 = tile * kRows + colh * 64u + c * 32u;
-                if constexpr (F == kTcE4M3) {
+                if constexpr (MAXIMA) {
+                    if (valid)
+                        store_maxima<F>(live[c], m[c], v[c], qs, L.doc_scale, doc0,
+                                        L.best + static_cast<uint64_t>(qi) * L.cap + it * 16u + colh * 8u + c * 4u);
+                } else if constexpr (F == kTcE4M3) {
                     emit_chunk<F>(live[c], m[c], v[c], t, theta, qs, L.doc_scale, doc0, out_score, out_loc, seg_cap,
                                   ncand);
                 } else if (live[c]) {
@@ -571,7 +599,7 @@ __global__ void __launch_bounds__(64 + 256 * H, 1) tc_cand_kernel(const __grid_c
                 }
             }
         }
-        if (valid) L.cand_count[static_cast<uint64_t>(qi) * kMaxCandSegs + segment] = ncand;
+        if (valid && !MAXIMA) L.cand_count[static_cast<uint64_t>(qi) * kMaxCandSegs + segment] = ncand;
     }
     __syncthreads();
     if (threadIdx.x == 0 && S.n_consumed < S.n_issued) {
@@ -640,7 +668,11 @@ __device__ inline bool pair_wait(unsigned long long* bar, uint32_t parity, PairS
 
 // SQ (streamed queries, long vectors): no resident query tile; each stage holds the query k-block
 // (16 KB, from the L2-resident staged queries) followed by the doc k-block, loaded together.
-template <int F, bool SQ, bool WIDE>
+// EMIT: kEmitHot for a pass that keeps few docs, kEmitMost for the doc sample's lists (most docs kept),
+// kEmitMaxima for its group maxima (TcCandLaunch::best).
+enum PairEmit : int { kEmitHot = 0, kEmitMost = 1, kEmitMaxima = 2 };
+
+template <int F, bool SQ, int EMIT>
 __global__ void __launch_bounds__(kPairThreads, 1) tc2_cand_kernel(const __grid_constant__ CUtensorMap doc_map,
                                                                   const __grid_constant__ CUtensorMap qry_map,
                                                                   TcCandLaunch L) {
@@ -830,7 +862,7 @@ __global__ void __launch_bounds__(kPairThreads, 1) tc2_cand_kernel(const __grid_
             if (!__all_sync(0xffffffffu, ready)) break;
             fence_after();
             const uint32_t tbase = tmem + ((sub * 32u) << 16) + buf * 256u + g * 64u;
-            if constexpr (WIDE) {
+            if constexpr (EMIT == kEmitMost) {
                 // a pass that keeps most docs (the doc sample): both chunks in registers, the buffer
                 // back to the issuer before the long emission (spills a little at 96 registers)
                 uint32_t v[2][32];
@@ -869,7 +901,12 @@ __global__ void __launch_bounds__(kPairThreads, 1) tc2_cand_kernel(const __grid_
                         if (lane == 0) mbar_arrive_cluster(buf ? acc_empty_addr1 : acc_empty_addr0);
                     }
                     const uint64_t doc0 = tile * 256u + g * 64u + c * 32u;
-                    if constexpr (F == kTcE4M3) {
+                    if constexpr (EMIT == kEmitMaxima) {
+                        // (E4M3: no scales past the corpus rows, whose bits are clear)
+                        if (valid)
+                            store_maxima<F>(live[c] && doc0 < L.tiles128 * 128u, m[c], v, qs, L.doc_scale, doc0,
+                                            L.best + static_cast<uint64_t>(qi) * L.cap + it * 32u + g * 8u + c * 4u);
+                    } else if constexpr (F == kTcE4M3) {
                         emit_chunk<F>(live[c], m[c], v, t, theta, qs, L.doc_scale, doc0, out_score, out_loc, seg_cap,
                                       ncand);
                     } else if (live[c]) {
@@ -878,7 +915,7 @@ __global__ void __launch_bounds__(kPairThreads, 1) tc2_cand_kernel(const __grid_
                 }
             }
         }
-        if (valid) L.cand_count[static_cast<uint64_t>(qi) * kMaxCandSegs + segment] = ncand;
+        if (valid && EMIT != kEmitMaxima) L.cand_count[static_cast<uint64_t>(qi) * kMaxCandSegs + segment] = ncand;
     }
     __syncthreads();
     if (threadIdx.x == 0 && S.n_consumed < S.n_issued) {
@@ -903,7 +940,8 @@ template <int F, bool SQ>
 cudaError_t launch_tc2_typed(const TcCandLaunch& L, const CUtensorMap& dmap, const CUtensorMap& qmap,
                              cudaStream_t stream) {
     const size_t smem = tc_pair_smem_bytes(L.kblocks, L.stages, L.group);
-    auto kernel = L.emit_all ? tc2_cand_kernel<F, SQ, true> : tc2_cand_kernel<F, SQ, false>;
+    auto kernel = L.best ? tc2_cand_kernel<F, SQ, kEmitMaxima>
+                         : L.emit_all ? tc2_cand_kernel<F, SQ, kEmitMost> : tc2_cand_kernel<F, SQ, kEmitHot>;
     // the ceiling, not this launch's size: searchers of other tables launch it concurrently
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          static_cast<int>(kTcSmemCeiling));
@@ -927,10 +965,11 @@ template <int F>
 cudaError_t launch_tc1_typed(const TcCandLaunch& L, const CUtensorMap& dmap, const CUtensorMap& qmap,
                              cudaStream_t stream) {
     const size_t smem = tc_smem_bytes(1, L.kblocks, L.stages, L.group);
-    cudaError_t e = cudaFuncSetAttribute(tc_cand_kernel<F, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    auto kernel = L.best ? tc_cand_kernel<F, 1, true> : tc_cand_kernel<F, 1, false>;
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          static_cast<int>(kTcSmemCeiling));
     if (e != cudaSuccess) return e;
-    tc_cand_kernel<F, 1><<<L.ctas, 64 + 256, smem, stream>>>(dmap, qmap, L);
+    kernel<<<L.ctas, 64 + 256, smem, stream>>>(dmap, qmap, L);
     return cudaGetLastError();
 }
 
@@ -999,6 +1038,10 @@ cudaError_t launch_tc_cand(const TcCandLaunch& Lin, const CUtensorMap& doc_map, 
     const uint64_t seg_end = static_cast<uint64_t>(L.seg_base) + 2ull * L.ctas;
     if (L.ctas != tc_cand_ctas(L.nq_rows, L.kblocks, L.tile_count, sms, L.cap) || L.seg_cap == 0 || seg_end > kMaxCandSegs ||
         seg_end * L.seg_cap > L.cap)
+        return cudaErrorInvalidValue;
+    // a tile's group maxima stay inside a query's row, in 16-byte stores
+    if (L.best && (L.tile_count * (tc_tile_docs(L.nq_rows, L.kblocks) / kTcGroup) > L.cap || L.cap % 4 ||
+                   (reinterpret_cast<uintptr_t>(L.best) & 15u)))
         return cudaErrorInvalidValue;
     switch (L.format) {
         case kTcTF32: return sq ? launch_tc2_typed<kTcTF32, true>(L, doc_map, qry_map, stream)

@@ -21,120 +21,55 @@ namespace cg = cooperative_groups;
 namespace hss {
 namespace {
 
-constexpr int kST = 1024;             // threads of the selection CTAs
-constexpr int kHist = 16;             // radix histograms per CTA (warp w adds to hist[w % kHist])
-// candidate scores a select CTA holds in shared memory: kSelFast, or kSelFastLarge for batches whose
-// lists run long (large K). The larger buffer leaves less of the SM's memory to L1, which costs the
-// short lists' select step (K = 100: 0.098 -> 0.112 ms at 10M), so it is taken only where asked.
-constexpr uint32_t kSelFast = 12288;
-constexpr uint32_t kSelFastLarge = 32768;
+constexpr int kST = 1024;             // threads of the TOPK operator's CTAs and of the large select form
+constexpr int kSelT = 512;            // threads of the threshold kernel and of the usual select form
+constexpr int kBins = 4096;           // histogram bins: 12-bit digits
+// candidate scores a CTA holds in shared memory: the usual select form (two CTAs of 512 threads per SM),
+// the form for batches whose lists run long (large K; one CTA of 1,024), the threshold kernel (two CTAs)
+constexpr uint32_t kFast = 8192;
+constexpr uint32_t kFastLarge = 32768;
+constexpr uint32_t kFastSample = 20480;
 
-struct SelectSmem {
-    uint32_t hist[kHist][256];                  // radix histograms
-    unsigned long long sortbuf[kMaxTopK];       // bitonic sort buffer
-    uint32_t segn[kMaxCandSegs];                // stored entries of each candidate segment
-    uint32_t segoff[kMaxCandSegs];              // their exclusive prefix sum (scan_segments)
+struct HistSmem {
+    __align__(16) uint32_t hist[kBins];
+    uint32_t wsum[32], wmax[32];
     uint32_t bcast[4];
-    uint32_t counter;
-    uint32_t total;                             // stored entries (load_segments)
-    uint32_t wsum[kST / 32];
+    uint32_t counter, total, lost;
 };
 
-// Merges the histograms into hist[0] and picks, from the top, the digit holding the k-th
-// largest key. Returns the digit and updates *krem to the rank inside that digit.
-__device__ inline uint32_t pick_digit(SelectSmem& S, uint32_t* krem) {
-    const uint32_t tid = threadIdx.x;
-    if (tid < 256) {
-        uint32_t s = 0;
-        for (int w = 0; w < kHist; ++w) s += S.hist[w][tid];
-        S.hist[0][tid] = s;
-    }
-    __syncthreads();
-    if (tid < 32) {
-        // warp 0 scans the 256 digits from the top: lane l owns digits 255 - 8l .. 248 - 8l
-        const uint32_t lane = tid;
-        const uint32_t kr = *krem;
-        uint32_t h[8], local = 0;
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-            h[i] = S.hist[0][255 - 8 * lane - i];
-            local += h[i];
-        }
-        uint32_t incl = local;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= static_cast<uint32_t>(o)) incl += y;
-        }
-        const uint32_t excl = incl - local;
-        // the first lane whose digits bring the running count to kr holds the k-th largest key
-        const uint32_t hit = __ballot_sync(0xffffffffu, excl < kr && incl >= kr);
-        if (hit && lane == static_cast<uint32_t>(__ffs(hit) - 1)) {
-            uint32_t cum = excl;
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-                if (cum + h[i] >= kr) {
-                    S.bcast[0] = 255 - 8 * lane - i;
-                    S.bcast[1] = kr - cum;
-                    break;
-                }
-                cum += h[i];
-            }
-        }
-    }
-    __syncthreads();
-    const uint32_t chosen = S.bcast[0];
-    *krem = S.bcast[1];
-    __syncthreads();
-    return chosen;
+struct SelectSmem : HistSmem {
+    __align__(16) unsigned long long sortbuf[kMaxTopK];  // keys to sort
+    uint32_t locs[kMaxTopK];  // select: locations of the first list entries; TOPK: a slice of the bins
+};
+
+// The next place of a list counted in shared memory, one addition per warp for its active lanes.
+__device__ __forceinline__ uint32_t next_place(uint32_t* counter) {
+    const uint32_t active = __activemask(), lane = threadIdx.x & 31;
+    const uint32_t leader = __ffs(active) - 1;
+    uint32_t base = 0;
+    if (lane == leader) base = atomicAdd(counter, static_cast<uint32_t>(__popc(active)));
+    return __shfl_sync(active, base, leader) + __popc(active & ((1u << lane) - 1u));
 }
 
-// Counts digit d (< 256; 256 = nothing) of each calling lane into hist_row. Lanes holding the same
-// digit add once, together: candidate scores cluster (a query's nearest cluster scores within a few
-// hundredths), so most of a warp's keys share their leading digits and 32 increments of one
-// shared-memory word would serialise.
-__device__ __forceinline__ void hist_add(uint32_t* hist_row, uint32_t d) {
-    const uint32_t active = __activemask();
-    const uint32_t grp = __match_any_sync(active, d);
-    if (d < 256u && (threadIdx.x & 31u) == static_cast<uint32_t>(__ffs(grp) - 1))
-        atomicAdd(&hist_row[d], static_cast<uint32_t>(__popc(grp)));
-}
-
-__device__ inline void clear_hist(SelectSmem& S) {
-    for (uint32_t i = threadIdx.x; i < kHist * 256; i += blockDim.x) (&S.hist[0][0])[i] = 0;
-    __syncthreads();
-}
-
-// k-th largest (1-based, k <= the number of keys) of the u32 keys that visit(fn) hands to fn.
-template <class Visit>
-__device__ uint32_t kth_largest_u32_visit(Visit visit, uint32_t k, SelectSmem& S) {
-    uint32_t prefix = 0, mask = 0, krem = k;
-    const uint32_t warp = threadIdx.x >> 5;
-    for (int shift = 24; shift >= 0; shift -= 8) {
-        clear_hist(S);
-        visit([&](uint32_t v) {
-            hist_add(S.hist[warp % kHist], (v & mask) == prefix ? ((v >> shift) & 255u) : 256u);
-        });
-        __syncthreads();
-        const uint32_t d = pick_digit(S, &krem);
-        prefix |= d << shift;
-        mask |= 255u << shift;
-    }
-    return prefix;
-}
-
-// Picks, from the top of a 4096-bin histogram, the bin holding the k-th largest key (blockDim.x ==
-// kST: thread t owns bins 4095 - 4t .. 4092 - 4t). Returns the bin; *krem becomes the rank inside it and
-// *in_bin (if given) the keys it holds.
-__device__ inline uint32_t pick_digit4096(const uint32_t* hist, uint32_t* krem, SelectSmem& S,
+// Picks, from the top of a 4096-bin histogram, the bin holding the k-th largest key (blockDim.x == NT:
+// thread t owns the 4096 / NT bins below 4096 (NT - t) / NT). Returns the bin; *krem becomes the rank
+// inside it and *in_bin (if given) the keys it holds. The caller has synchronised after the last
+// addition; a synchronisation lies between this and the next use of S.wsum and S.bcast.
+template <int NT>
+__device__ inline uint32_t pick_digit4096(const uint32_t* hist, uint32_t* krem, HistSmem& S,
                                           uint32_t* in_bin = nullptr) {
+    constexpr int B = kBins / NT;
     const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
     const uint32_t kr = *krem;
-    uint32_t h[4], local = 0;
+    uint32_t h[B], local = 0;  // h[j]: bin kBins - 1 - B t - j
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-        h[j] = hist[4095 - 4 * t - j];
-        local += h[j];
+    for (int j = 0; j < B; j += 4) {
+        const uint4 x = *reinterpret_cast<const uint4*>(hist + kBins - B * t - j - 4);
+        h[j] = x.w;
+        h[j + 1] = x.z;
+        h[j + 2] = x.y;
+        h[j + 3] = x.x;
+        local += x.x + x.y + x.z + x.w;
     }
     uint32_t x = local;
 #pragma unroll
@@ -144,24 +79,15 @@ __device__ inline uint32_t pick_digit4096(const uint32_t* hist, uint32_t* krem, 
     }
     if (lane == 31) S.wsum[warp] = x;
     __syncthreads();
-    if (warp == 0) {
-        const uint32_t w = S.wsum[lane];
-        uint32_t z = w;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, z, o);
-            if (lane >= static_cast<uint32_t>(o)) z += y;
-        }
-        S.wsum[lane] = z - w;  // exclusive over warps
-    }
-    __syncthreads();
-    const uint32_t incl = S.wsum[warp] + x, excl = incl - local;
+    // every warp adds up the warps before it
+    const uint32_t before = warp_sum(lane < warp ? S.wsum[lane] : 0u);
+    const uint32_t incl = before + x, excl = incl - local;
     if (excl < kr && incl >= kr) {  // exactly one thread
         uint32_t cum = excl;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
+        for (int j = 0; j < B; ++j) {
             if (cum + h[j] >= kr) {
-                S.bcast[0] = 4095 - 4 * t - j;
+                S.bcast[0] = kBins - 1 - B * t - j;
                 S.bcast[1] = kr - cum;
                 S.bcast[2] = h[j];
                 break;
@@ -170,258 +96,299 @@ __device__ inline uint32_t pick_digit4096(const uint32_t* hist, uint32_t* krem, 
         }
     }
     __syncthreads();
-    const uint32_t d = S.bcast[0];
     *krem = S.bcast[1];
     if (in_bin) *in_bin = S.bcast[2];
+    return S.bcast[0];
+}
+
+template <int NT>
+__device__ __forceinline__ void clear_hist(HistSmem& S) {
+    for (uint32_t i = threadIdx.x; i < kBins / 4; i += NT) reinterpret_cast<uint4*>(S.hist)[i] = make_uint4(0, 0, 0, 0);
+}
+
+// Adds digits to a histogram, each thread merging its runs of equal digits before it does (keys of one
+// query cluster, so consecutive keys mostly share a digit). flush() before the histogram is read.
+struct RunAdder {
+    uint32_t* hist;
+    uint32_t cur = 0, cnt = 0;
+    __device__ __forceinline__ explicit RunAdder(uint32_t* h) : hist(h) {}
+    __device__ __forceinline__ void add(uint32_t d) {
+        if (d != cur) {
+            if (cnt) atomicAdd(&hist[cur], cnt);
+            cur = d;
+            cnt = 0;
+        }
+        ++cnt;
+    }
+    __device__ __forceinline__ void flush() {
+        if (cnt) atomicAdd(&hist[cur], cnt);
+        cnt = 0;
+    }
+};
+
+// Smallest and largest of the block's u32 keys (each thread's in lo, hi; none: lo > hi), in every
+// thread afterwards. S.wsum and S.wmax are used, once between two synchronisations.
+template <int NT>
+__device__ __forceinline__ void block_minmax(uint32_t& lo, uint32_t& hi, HistSmem& S) {
+    lo = __reduce_min_sync(0xffffffffu, lo);
+    hi = __reduce_max_sync(0xffffffffu, hi);
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (lane == 0) {
+        S.wsum[warp] = lo;
+        S.wmax[warp] = hi;
+    }
     __syncthreads();
-    return d;
+    lo = __reduce_min_sync(0xffffffffu, lane < NT / 32 ? S.wsum[lane] : 0xffffffffu);
+    hi = __reduce_max_sync(0xffffffffu, lane < NT / 32 ? S.wmax[lane] : 0u);
 }
 
 // A lower bound of the k-th largest (1-based, k <= the number of keys) of the u32 keys that visit(fn)
-// hands to fn: the k-th largest key's top 24 bits with the low 8 bits cleared. Every key sharing that
-// prefix is >= the result, so at least k keys are >= it -- all a proven threshold or a rescoring cut
-// needs -- and as an order-preserving float key it is at most 2^-15 (relative) below the k-th
-// largest. Two passes of 12-bit digits over one 4096-bin histogram; each thread merges runs of equal
-// digits before adding them (keys of one query cluster, so consecutive keys mostly share a digit).
-template <class Visit>
-__device__ uint32_t kth_lower_bound_u32_visit(Visit visit, uint32_t k, SelectSmem& S) {
-    uint32_t* hist = &S.hist[0][0];
-    static_assert(sizeof(S.hist) / sizeof(uint32_t) >= 4096, "4096-bin histogram");
-    uint32_t prefix = 0, mask = 0, krem = k;
+// hands to fn, all of them in [lo, hi]: at least k keys are >= it -- all a proven threshold or a
+// rescoring cut needs -- and it shares the k-th key's top 24 bits at least (as an order-preserving float
+// key it is at most 2^-15, relatively, below). Two passes over a 4096-bin histogram: the bins of the first
+// divide [lo, hi], those of the second the k-th key's bin. Digits of the keys themselves would crowd a few
+// bins, whose shared-memory additions serialise: a query's scores share their exponents.
+template <int NT, class Visit>
+__device__ __forceinline__ uint32_t kth_lower_bound(Visit visit, uint32_t k, uint32_t lo, uint32_t hi, HistSmem& S) {
+    uint32_t krem = k;
+#pragma unroll 1
     for (int pass = 0; pass < 2; ++pass) {
-        const int shift = pass == 0 ? 20 : 8;
-        for (uint32_t i = threadIdx.x; i < 4096; i += blockDim.x) hist[i] = 0;
+        const int bits = 32 - __clz(hi - lo);
+        const int shift = bits > 12 ? bits - 12 : 0;
         __syncthreads();
-        uint32_t cur = 0, cnt = 0;
+        clear_hist<NT>(S);
+        __syncthreads();
+        RunAdder add(S.hist);
         visit([&](uint32_t v) {
-            if ((v & mask) != prefix) return;
-            const uint32_t d = (v >> shift) & 4095u;
-            if (d != cur) {
-                if (cnt) atomicAdd(&hist[cur], cnt);
-                cur = d;
-                cnt = 0;
-            }
-            ++cnt;
+            if (v - lo <= hi - lo) add.add((v - lo) >> shift);
         });
-        if (cnt) atomicAdd(&hist[cur], cnt);
+        add.flush();
         __syncthreads();
-        const uint32_t d = pick_digit4096(hist, &krem, S);
+        lo += pick_digit4096<NT>(S.hist, &krem, S) << shift;
+        hi = lo + ((1u << shift) - 1u);
+        if (shift == 0) break;
+    }
+    return lo;
+}
+
+// A lower bound of the k-th largest (1-based) of the finite scores that visit(fn) hands to fn, all of them
+// in [lo, hi], k <= their number: at least k of them are >= it. The 4096 bins divide [lo, hi] evenly (a
+// monotone map, so a score in a higher bin is a higher score): scores of both signs, whose keys would
+// crowd the bins of a few exponents, spread over them. The bound is the least score of the k-th's bin;
+// where that bin is crowded (an outlier stretches the range, or many equal scores) it is refined by keys.
+template <int NT, class Visit>
+__device__ __forceinline__ float kth_score_bound(Visit visit, uint32_t k, float lo, float hi, HistSmem& S) {
+    const float scale = 4096.0f / (hi - lo);
+    uint32_t krem = k, in_bin = 0;
+    uint32_t key_lo = float_key(lo), key_hi = float_key(hi);
+    if (scale > 0.0f && scale < 1e30f) {  // else: equal scores, or a range past the floats
+        auto bin = [&](float v) { return min(static_cast<uint32_t>((v - lo) * scale), 4095u); };
+        __syncthreads();
+        clear_hist<NT>(S);
+        __syncthreads();
+        visit([&](float v) { atomicAdd(&S.hist[bin(v)], 1u); });
+        __syncthreads();
+        const uint32_t d = pick_digit4096<NT>(S.hist, &krem, S, &in_bin);
+        uint32_t a = 0xffffffffu, b = 0;
+        visit([&](float v) {
+            if (bin(v) == d) {
+                a = min(a, float_key(v));
+                b = max(b, float_key(v));
+            }
+        });
+        block_minmax<NT>(a, b, S);
+        if (in_bin <= 64u) return key_float(a);
+        key_lo = a;
+        key_hi = b;
+    }
+    return key_float(kth_lower_bound<NT>([&](auto fn) { visit([&](float v) { fn(float_key(v)); }); }, krem, key_lo,
+                                         key_hi, S));
+}
+
+// A lower bound of the k-th largest of n u64 keys key(i) that at most kMaxTopK keys reach, where there is
+// one (else the k-th largest itself).
+template <int NT, class KeyFn>
+__device__ __forceinline__ uint64_t kth_bound_u64(KeyFn key, uint32_t n, uint32_t k, HistSmem& S) {
+    uint64_t prefix = 0, mask = 0;
+    uint32_t krem = k, in_bin = 0;
+    const int shifts[6] = {52, 40, 32, 20, 8, 0};
+#pragma unroll 1
+    for (int p = 0; p < 6; ++p) {
+        const int shift = shifts[p];
+        const uint64_t digit = p == 2 || p == 5 ? 255ull : 4095ull;
+        __syncthreads();
+        clear_hist<NT>(S);
+        __syncthreads();
+        RunAdder add(S.hist);
+        for (uint32_t i = threadIdx.x; i < n; i += NT) {
+            const uint64_t v = key(i);
+            if ((v & mask) == prefix) add.add(static_cast<uint32_t>((v >> shift) & digit));
+        }
+        add.flush();
+        __syncthreads();
+        const uint64_t d = pick_digit4096<NT>(S.hist, &krem, S, &in_bin);
         prefix |= d << shift;
-        mask |= 4095u << shift;
+        mask |= digit << shift;
+        if ((k - krem) + in_bin <= static_cast<uint32_t>(kMaxTopK)) break;
     }
     return prefix;
 }
 
-// k-th largest (1-based, k <= n) of n u32 keys produced by key(i).
-template <class KeyFn>
-__device__ uint32_t kth_largest_u32(KeyFn key, uint32_t n, uint32_t k, SelectSmem& S) {
-    return kth_largest_u32_visit(
-        [&](auto fn) {
-            for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) fn(key(i));
-        },
-        k, S);
-}
-
-// S.segoff[g] = entries stored in segments before g (exclusive prefix sum of S.segn[0..segs)).
-// segs <= kMaxCandSegs = blockDim.x.
-__device__ inline void scan_segments(SelectSmem& S, uint32_t segs) {
-    const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5;
-    const uint32_t v = t < segs ? S.segn[t] : 0u;
-    uint32_t x = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-        if (lane >= static_cast<uint32_t>(o)) x += y;
-    }
-    if (lane == 31) S.wsum[warp] = x;
-    __syncthreads();
-    if (warp == 0) {
-        const uint32_t w = lane < (blockDim.x >> 5) ? S.wsum[lane] : 0u;
-        uint32_t z = w;
+// Calls fn(index, valid, score) for every stored entry of a query's segmented list of scores src (counts:
+// per-segment counts, seg_cap the most a segment stores), in no particular order. A warp takes up to 32
+// segments at a time, a lane each, and walks their entries flattened: lane l's entry belongs to the last
+// segment that starts at or before it, found by five shuffles, so the loads are coalesced within a
+// segment, independent and eight per thread in flight, and no block-wide scan or barrier is needed. Every
+// call is made by a full warp (valid = false past the end), so fn may use warp collectives; begin(m) is
+// called by the full warp before a group's m entries. Returns whether a segment of this lane lost entries.
+template <int NT, class Begin, class Fn>
+__device__ __forceinline__ bool walk_segments(const uint32_t* counts, uint32_t segs, uint32_t seg_cap, const float* src,
+                                              Begin begin, Fn fn) {
+    constexpr uint32_t U = 8, kWarps = NT / 32;
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // segments per warp and round: as even a share as 32 lanes allow
+    const uint32_t rounds = (segs + 32 * kWarps - 1) / (32 * kWarps);
+    const uint32_t per = (segs + kWarps * rounds - 1) / (kWarps * rounds);
+    bool lost = false;
+    for (uint32_t g0 = warp * per; g0 < segs; g0 += kWarps * per) {
+        uint32_t c = lane < per && g0 + lane < segs ? counts[g0 + lane] : 0u;
+        lost |= c > seg_cap;
+        c = min(c, seg_cap);
+        uint32_t x = c;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(0xffffffffu, z, o);
-            if (lane >= static_cast<uint32_t>(o)) z += y;
+            const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= static_cast<uint32_t>(o)) x += y;
         }
-        S.wsum[lane] = z - w;  // exclusive over warps
-    }
-    __syncthreads();
-    if (t < segs) S.segoff[t] = S.wsum[warp] + x - v;
-    __syncthreads();
-}
-
-// Loads the per-segment counts of one query's segmented candidate list (kMaxCandSegs layout) into
-// S.segn (clamped to seg_cap) and their prefix sums into S.segoff. Returns the stored total (also in
-// S.total); *overflow = some segment lost entries. segs <= blockDim.x.
-__device__ uint32_t load_segments(SelectSmem& S, const uint32_t* counts, uint32_t segs, uint32_t seg_cap,
-                                  bool* overflow) {
-    if (threadIdx.x == 0) {
-        S.bcast[2] = 0;
-        S.bcast[3] = 0;
-    }
-    __syncthreads();
-    for (uint32_t g = threadIdx.x; g < segs; g += blockDim.x) {
-        const uint32_t c = counts[g];
-        const uint32_t st = min(c, seg_cap);
-        S.segn[g] = st;
-        if (st) atomicAdd(&S.bcast[2], st);
-        if (c > seg_cap) atomicOr(&S.bcast[3], 1u);
-    }
-    __syncthreads();
-    const uint32_t n = S.bcast[2];
-    *overflow = S.bcast[3] != 0;
-    if (threadIdx.x == 0) S.total = n;
-    scan_segments(S, segs);  // synchronises
-    return n;
-}
-
-// Storage index of the idx-th stored entry (idx < S.total) of a segmented list: the last segment
-// starting at or before idx, by binary search over S.segoff (empty segments share their successor's
-// start, so the last such segment is the non-empty one holding idx).
-__device__ __forceinline__ uint64_t segment_entry(const SelectSmem& S, uint32_t segs, uint32_t seg_cap, uint32_t idx) {
-    uint32_t lo = 0, hi = segs;
-    while (hi - lo > 1) {
-        const uint32_t mid = (lo + hi) >> 1;
-        if (S.segoff[mid] <= idx) lo = mid;
-        else hi = mid;
-    }
-    return static_cast<uint64_t>(lo) * seg_cap + (idx - S.segoff[lo]);
-}
-
-// Calls fn(index, valid, score) for every stored entry of a segmented list of scores src (after
-// load_segments). Short segments (a candidate list's: a few entries each): a warp takes 4 x 32
-// consecutive entries of the flattened list per round: lanes read consecutive entries (coalesced
-// within a segment), and each lane's 4 segment lookups and loads are independent, so a thread keeps 4
-// loads in flight instead of one dependent chain per entry. Long segments: walked segment by segment.
-// Every call is made by a full warp (valid = false past the end), so fn may use warp collectives.
-template <class Fn>
-__device__ inline void for_each_segment_entry(const SelectSmem& S, uint32_t segs, uint32_t seg_cap,
-                                              const float* src, Fn fn) {
-    constexpr uint32_t U = 4;
-    const uint32_t n = S.total, lane = threadIdx.x & 31;
-    if (n >= 32u * segs) {
-        // long segments (a doc sample's lists): warp w walks segments w, w + 32, ..., 4 x 32 entries
-        // a round, with no per-entry segment lookup
-        for (uint32_t g = threadIdx.x >> 5; g < segs; g += blockDim.x >> 5) {
-            const uint32_t cnt = S.segn[g];
-            const uint64_t base = static_cast<uint64_t>(g) * seg_cap;
-            for (uint32_t o = 0; o < cnt; o += 32u * U) {
-                bool ok[U];
-                float v[U];
+        const uint32_t off = x - c, total = __shfl_sync(0xffffffffu, x, 31);
+        if (total == 0) continue;
+        begin(total);
+        for (uint32_t b = 0; b < total; b += 32 * U) {
+            uint32_t at[U];
+            float v[U];
 #pragma unroll
-                for (uint32_t u = 0; u < U; ++u) {
-                    const uint32_t e = o + 32u * u + lane;
-                    ok[u] = e < cnt;
-                    v[u] = ok[u] ? src[base + e] : 0.0f;
+            for (uint32_t u = 0; u < U; ++u) {
+                const uint32_t idx = b + 32 * u + lane;
+                uint32_t lo = 0;
+#pragma unroll
+                for (uint32_t step = 16; step > 0; step >>= 1) {
+                    const uint32_t o = __shfl_sync(0xffffffffu, off, lo + step);
+                    if (o <= idx) lo += step;
                 }
+                at[u] = (g0 + lo) * seg_cap + idx - __shfl_sync(0xffffffffu, off, lo);
+                v[u] = idx < total ? src[at[u]] : 0.0f;
+            }
 #pragma unroll
-                for (uint32_t u = 0; u < U; ++u) fn(static_cast<uint32_t>(base + o + 32u * u + lane), ok[u], v[u]);
+            for (uint32_t u = 0; u < U; ++u) {
+                if (b + 32 * u >= total) break;  // warp-uniform
+                fn(at[u], b + 32 * u + lane < total, v[u]);
             }
         }
-        return;
     }
-    for (uint32_t b = (threadIdx.x >> 5) * 32u * U; b < n; b += blockDim.x * U) {
-        uint64_t i[U];
-        bool ok[U];
-        float v[U];
-#pragma unroll
-        for (uint32_t u = 0; u < U; ++u) {
-            const uint32_t idx = b + 32u * u + lane;
-            ok[u] = idx < n;
-            i[u] = ok[u] ? segment_entry(S, segs, seg_cap, idx) : 0ull;
-        }
-#pragma unroll
-        for (uint32_t u = 0; u < U; ++u) v[u] = ok[u] ? src[i[u]] : 0.0f;
-#pragma unroll
-        for (uint32_t u = 0; u < U; ++u) fn(static_cast<uint32_t>(i[u]), ok[u], v[u]);
-    }
+    return lost;
 }
 
-template <class KeyFn>
-__device__ uint64_t kth_largest_u64(KeyFn key, uint32_t n, uint32_t k, SelectSmem& S) {
-    uint64_t prefix = 0, mask = 0;
-    uint32_t krem = k;
-    const uint32_t warp = threadIdx.x >> 5;
-    for (int shift = 56; shift >= 0; shift -= 8) {
-        clear_hist(S);
-        for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
-            const uint64_t v = key(i);
-            hist_add(S.hist[warp % kHist], (v & mask) == prefix ? static_cast<uint32_t>((v >> shift) & 255u) : 256u);
-        }
-        __syncthreads();
-        const uint64_t d = pick_digit(S, &krem);
-        prefix |= d << shift;
-        mask |= 255ull << shift;
+// The first walk of a list: scores into `cache` (as many as fit), where locs is given the locations of the
+// first kMaxTopK too, and the smallest and largest key. Returns the number of entries; *overflow = some
+// segment lost entries. Synchronised at its end.
+template <int NT>
+__device__ __forceinline__ uint32_t load_list(HistSmem& S, const uint32_t* counts, uint32_t segs, uint32_t seg_cap,
+                                              const float* src, const uint32_t* loc_src, float* cache, uint32_t cap,
+                                              uint32_t* locs, bool* overflow, uint32_t* key_lo, uint32_t* key_hi) {
+    if (threadIdx.x == 0) {
+        S.counter = 0;
+        S.lost = 0;
     }
-    return prefix;
+    __syncthreads();
+    uint32_t pos = 0, lo = 0xffffffffu, hi = 0;
+    const uint32_t lane = threadIdx.x & 31;
+    const bool lost = walk_segments<NT>(
+        counts, segs, seg_cap, src,
+        [&](uint32_t m) {
+            if (lane == 0) pos = atomicAdd(&S.counter, m);
+            pos = __shfl_sync(0xffffffffu, pos, 0) + lane;
+        },
+        [&](uint32_t at, bool ok, float v) {
+            if (ok) {
+                if (locs && pos < static_cast<uint32_t>(kMaxTopK)) locs[pos] = loc_src[at];
+                if (pos < cap) cache[pos] = v;
+                const uint32_t key = float_key(v);
+                lo = min(lo, key);
+                hi = max(hi, key);
+            }
+            pos += 32;
+        });
+    if (lost) S.lost = 1;
+    block_minmax<NT>(lo, hi, S);
+    *key_lo = lo;
+    *key_hi = hi;
+    *overflow = S.lost != 0;
+    return S.counter;
 }
 
-// Sorts E keys per thread (key of index t + 1024 e in v[e]) of the first m / E threads descending:
-// a bitonic network whose exchanges over a distance below 32 are shuffles and whose exchanges over 1024
-// and more stay inside a thread, so only distances 32..512 go through shared memory and a barrier of
+// Sorts E keys per thread (key of index t + NT e in v[e]) of the first m / E threads descending:
+// a bitonic network whose exchanges over a distance below 32 are shuffles and whose exchanges over NT
+// and more stay inside a thread, so only the distances between go through shared memory and a barrier of
 // the m / E threads (for 512 keys 10 of the 45 steps).
-template <int E>
+template <int NT, int E>
 __device__ __forceinline__ void bitonic_regs(unsigned long long* buf, uint32_t m) {
-    const uint32_t t = threadIdx.x, threads = E == 1 ? m : static_cast<uint32_t>(kST);
+    const uint32_t t = threadIdx.x, threads = E == 1 ? m : static_cast<uint32_t>(NT);
     auto bar = [&] { asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory"); };
     unsigned long long v[E];
 #pragma unroll
-    for (int e = 0; e < E; ++e) v[e] = buf[t + static_cast<uint32_t>(kST) * e];
+    for (int e = 0; e < E; ++e) v[e] = buf[t + static_cast<uint32_t>(NT) * e];
     for (uint32_t k = 2; k <= m; k <<= 1) {
         for (uint32_t j = k >> 1; j > 0; j >>= 1) {
-            if (E > 1 && j >= static_cast<uint32_t>(kST)) {
-                const uint32_t de = j / static_cast<uint32_t>(kST);
+            if (E > 1 && j >= static_cast<uint32_t>(NT)) {
 #pragma unroll
-                for (int e = 0; e < E; ++e) {
-                    const int o = e ^ static_cast<int>(de);
-                    if (o < e || o >= E) continue;
-                    const bool desc = ((t + static_cast<uint32_t>(kST) * e) & k) == 0;
+                for (int de = E / 2; de > 0; de >>= 1) {  // compile-time register indices
+                    if (j != static_cast<uint32_t>(NT) * de) continue;
 #pragma unroll
-                    for (int f = 0; f < E; ++f) {  // f == o: a compile-time register index
-                        if (f != o) continue;
-                        const unsigned long long a = v[e], b = v[f];
+                    for (int e = 0; e < E; ++e) {
+                        if (e & de) continue;
+                        const bool desc = ((t + static_cast<uint32_t>(NT) * e) & k) == 0;
+                        const unsigned long long a = v[e], b = v[e + de];
                         if (desc ? (a < b) : (a > b)) {
                             v[e] = b;
-                            v[f] = a;
+                            v[e + de] = a;
                         }
                     }
                 }
                 continue;
             }
-            unsigned long long o[E];
             if (j >= 32) {
                 bar();  // the previous step's reads are done
 #pragma unroll
-                for (int e = 0; e < E; ++e) buf[t + static_cast<uint32_t>(kST) * e] = v[e];
+                for (int e = 0; e < E; ++e) buf[t + static_cast<uint32_t>(NT) * e] = v[e];
                 bar();
-#pragma unroll
-                for (int e = 0; e < E; ++e) o[e] = buf[(t ^ j) + static_cast<uint32_t>(kST) * e];
-            } else {
-#pragma unroll
-                for (int e = 0; e < E; ++e) o[e] = __shfl_xor_sync(0xffffffffu, v[e], j);
             }
 #pragma unroll
             for (int e = 0; e < E; ++e) {
+                const unsigned long long o = j >= 32 ? buf[(t ^ j) + static_cast<uint32_t>(NT) * e]
+                                                     : __shfl_xor_sync(0xffffffffu, v[e], j);
                 // the lower index of a descending pair keeps the larger key
-                const uint32_t i = t + static_cast<uint32_t>(kST) * e;
+                const uint32_t i = t + static_cast<uint32_t>(NT) * e;
                 const bool larger = ((i & k) == 0) == ((i & j) == 0);
-                if (larger ? (o[e] > v[e]) : (o[e] < v[e])) v[e] = o[e];
+                if (larger ? (o > v[e]) : (o < v[e])) v[e] = o;
             }
         }
     }
     bar();
 #pragma unroll
-    for (int e = 0; e < E; ++e) buf[t + static_cast<uint32_t>(kST) * e] = v[e];
+    for (int e = 0; e < E; ++e) buf[t + static_cast<uint32_t>(NT) * e] = v[e];
 }
 
 // Sorts S.sortbuf[0..m) descending; m is a power of two, 32 <= m <= kMaxTopK (sort_size).
+template <int NT>
 __device__ __forceinline__ void bitonic_desc(SelectSmem& S, uint32_t m) {
-    if (m <= static_cast<uint32_t>(kST)) {
-        if (threadIdx.x < m) bitonic_regs<1>(S.sortbuf, m);
-    } else if (m == 2u * kST) {
-        bitonic_regs<2>(S.sortbuf, m);
-    } else {
-        bitonic_regs<4>(S.sortbuf, m);
+    if (m <= static_cast<uint32_t>(NT)) {
+        if (threadIdx.x < m) bitonic_regs<NT, 1>(S.sortbuf, m);
+    } else if (m == 2u * NT) {
+        bitonic_regs<NT, 2>(S.sortbuf, m);
+    } else if (m == 4u * NT) {
+        bitonic_regs<NT, 4>(S.sortbuf, m);
+    } else if constexpr (kMaxTopK > 4 * NT) {
+        bitonic_regs<NT, 8>(S.sortbuf, m);
     }
     __syncthreads();
 }
@@ -433,148 +400,285 @@ __device__ inline uint32_t sort_size(uint32_t n) {
     return m;
 }
 
-// Brings the top `kq` (<= kMaxTopK) of n distinct u64 keys key(i) (and possibly more) into S.sortbuf,
-// unsorted, filled up with zeros to sort_size() entries, which it returns.
-template <class KeyFn>
+// Sorts n (<= kRankSort) distinct keys of S.sortbuf into `out` by counting, for each, the keys that precede
+// it, NT / 256 threads to a key: no barrier between steps (256 keys: 1 us against 2 us by the network).
+constexpr uint32_t kRankSort = 256;
+template <int NT>
+__device__ __forceinline__ void rank_sort(const SelectSmem& S, uint32_t n, unsigned long long* out) {
+    constexpr uint32_t W = NT / kRankSort;  // 2 or 4 neighbouring lanes
+    const uint32_t i = threadIdx.x / W, w = threadIdx.x % W;
+    const unsigned long long key = i < n ? S.sortbuf[i] : 0ull;
+    uint32_t before = 0;
+    if (i < n) {
+#pragma unroll 4
+        for (uint32_t j = w; j < n; j += W) {
+            const unsigned long long o = S.sortbuf[j];
+            before += o > key || (o == key && j < i) ? 1u : 0u;
+        }
+    }
+#pragma unroll
+    for (uint32_t o = 1; o < W; o <<= 1) before += __shfl_xor_sync(0xffffffffu, before, o);
+    if (i < n && w == 0) out[before] = key;
+    __syncthreads();
+}
+
+// Zeros after the first `got` (<= kMaxTopK) keys of S.sortbuf up to the sort's size, which it returns.
+template <int NT>
+__device__ __forceinline__ uint32_t pad_sort(SelectSmem& S, uint32_t got) {
+    const uint32_t m = sort_size(got);
+    for (uint32_t i = got + threadIdx.x; i < m; i += NT) S.sortbuf[i] = 0ull;
+    __syncthreads();
+    return m;
+}
+
+// Brings the top `kq` (<= kMaxTopK) of n u64 keys key(i) (and possibly more) into S.sortbuf, unsorted,
+// filled up with zeros to sort_size() entries, which it returns. Long lists are cut at a lower bound of
+// the kq-th key first, so that the sort takes about kq keys.
+template <int NT, class KeyFn>
 __device__ __forceinline__ uint32_t gather_top_keys(KeyFn key, uint32_t n, uint32_t kq, SelectSmem& S) {
     uint32_t got;
-    if (n <= static_cast<uint32_t>(kMaxTopK) && n <= 2 * kq) {
-        for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) S.sortbuf[i] = key(i);
+    if (n <= static_cast<uint32_t>(NT) || (n <= static_cast<uint32_t>(kMaxTopK) && n <= 2 * kq)) {
+        for (uint32_t i = threadIdx.x; i < n; i += NT) S.sortbuf[i] = key(i);
         got = n;
     } else {
-        // n <= kMaxTopK: keep only keys whose score half is at least a lower bound of the kq-th best
-        // score (it keeps the top kq and at most the few keys sharing the kq-th's 24-bit prefix beyond
-        // them), then sort those: a bitonic sort over about kq keys instead of n. Longer lists: the
-        // exact kq-th key.
         const uint64_t lb =
             n <= static_cast<uint32_t>(kMaxTopK)
-                ? static_cast<uint64_t>(kth_lower_bound_u32_visit(
+                ? static_cast<uint64_t>(kth_lower_bound<NT>(
                       [&](auto fn) {
-                          for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) fn(static_cast<uint32_t>(key(i) >> 32));
+                          for (uint32_t i = threadIdx.x; i < n; i += NT) fn(static_cast<uint32_t>(key(i) >> 32));
                       },
-                      kq, S))
+                      kq, 0u, 0xffffffffu, S))
                       << 32
-                : kth_largest_u64(key, n, kq, S);
+                : kth_bound_u64<NT>(key, n, kq, S);
         if (threadIdx.x == 0) S.counter = 0;
         __syncthreads();
-        for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) {
+        for (uint32_t i = threadIdx.x; i < n; i += NT) {
             const uint64_t v = key(i);
             if (v >= lb) {
-                const uint32_t pos = atomicAdd(&S.counter, 1u);
+                const uint32_t pos = next_place(&S.counter);
                 if (pos < static_cast<uint32_t>(kMaxTopK)) S.sortbuf[pos] = v;
             }
         }
         __syncthreads();
         got = min(S.counter, static_cast<uint32_t>(kMaxTopK));
     }
-    const uint32_t m = sort_size(got);
-    for (uint32_t i = got + threadIdx.x; i < m; i += blockDim.x) S.sortbuf[i] = 0ull;
-    __syncthreads();
-    return m;
-}
-
-// Top `kq` (<= kMaxTopK) of n distinct u64 keys key(i), sorted descending into S.sortbuf[0..kq).
-template <class KeyFn>
-__device__ __forceinline__ void top_keys(KeyFn key, uint32_t n, uint32_t kq, SelectSmem& S) {
-    bitonic_desc(S, gather_top_keys(key, n, kq, S));
+    return pad_sort<NT>(S, got);
 }
 
 // ---------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(kST) sample_threshold_kernel(SampleThresholdLaunch L) {
+// The threshold of a sample or of a first candidate pass. One CTA per query; bound by a chain of
+// dependent steps (counts, entries, two digits), so the list is read once, into shared memory where it
+// fits (kFastSample entries), with the first digit counted on the way.
+template <int NT>
+__global__ void __launch_bounds__(NT, 1024 / NT) sample_threshold_kernel(SampleThresholdLaunch L) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    SelectSmem& S = *reinterpret_cast<SelectSmem*>(smem_raw);
+    HistSmem& S = *reinterpret_cast<HistSmem*>(smem_raw);
+    float* cs = reinterpret_cast<float*>(smem_raw + sizeof(HistSmem));
     const uint32_t qi = L.qlist ? L.qlist[blockIdx.x] : blockIdx.x;
     const uint32_t k = L.topk[qi];
+    const uint32_t* counts = L.count + static_cast<uint64_t>(qi) * kMaxCandSegs;
+    const float* sc = L.score + static_cast<uint64_t>(qi) * L.cap;
     bool lost = false;  // a sample segment that overflowed only lowers the sample's K-th best
-    const uint32_t n = load_segments(S, L.count + static_cast<uint64_t>(qi) * kMaxCandSegs, L.segs, L.seg_cap, &lost);
-    float theta = L.raise_only ? L.theta[qi] : -INFINITY;
-    if (L.stats) {
-        // the sample's best scores at ranks 1, 2, 4, ..., 64: a lower bound of the key at rank
-        // r = min(64, n) (its 24-bit prefix, two walks of the list), then the (fewer than r) keys above
-        // that prefix's bucket, each placed by counting the keys that precede it; a rank inside the
-        // bucket gets the bound (at most 2^-15 relative below the score)
-        float* st = L.stats + static_cast<uint64_t>(qi) * kSampleStats;
-        const float* sc = L.score + static_cast<uint64_t>(qi) * L.cap;
-        const uint32_t r = min(n, 64u);
-        uint32_t key_r = 0;
-        if (r > 0)
-            key_r = kth_lower_bound_u32_visit(
-                [&](auto fn) {
-                    for_each_segment_entry(S, L.segs, L.seg_cap, sc, [&](uint32_t, bool ok, float v) {
-                        if (ok) fn(float_key(v));
-                    });
-                },
-                r, S);
-        const uint32_t bucket_top = key_r | 0xFFu;
-        if (threadIdx.x == 0) S.counter = 0;
-        __syncthreads();
-        if (r > 0)
-            for_each_segment_entry(S, L.segs, L.seg_cap, sc, [&](uint32_t, bool ok, float v) {
-                const uint32_t key = ok ? float_key(v) : 0u;
-                if (ok && key > bucket_top) {
-                    const uint32_t slot = atomicAdd(&S.counter, 1u);
-                    if (slot < 64u) S.sortbuf[slot] = key;
-                }
+    uint32_t key_lo, key_hi;
+    const uint32_t n = load_list<NT>(S, counts, L.segs, L.seg_cap, sc, nullptr, cs, kFastSample, nullptr, &lost, &key_lo,
+                                     &key_hi);
+    auto visit = [&](auto fn) {
+        if (n <= kFastSample) {
+            for (uint32_t i = threadIdx.x; i < n; i += NT) fn(float_key(cs[i]));
+        } else {
+            walk_segments<NT>(counts, L.segs, L.seg_cap, sc, [](uint32_t) {}, [&](uint32_t, bool ok, float v) {
+                if (ok) fn(float_key(v));
             });
-        __syncthreads();
-        const uint32_t c = min(S.counter, 64u);  // < r unless keys were lost
-        if (threadIdx.x < c) {
-            const unsigned long long key = S.sortbuf[threadIdx.x];
-            uint32_t rank = 0;
-            for (uint32_t j = 0; j < c; ++j) {
-                const unsigned long long o = S.sortbuf[j];
-                rank += (o > key || (o == key && j < threadIdx.x)) ? 1u : 0u;
-            }
-            S.sortbuf[64 + rank] = key;
         }
-        __syncthreads();
-        if (threadIdx.x < kSampleRanks) {
-            const uint32_t rho = 1u << threadIdx.x;
-            float v = -2.0f;
-            if (rho <= r) v = key_float(rho <= c ? static_cast<uint32_t>(S.sortbuf[64 + rho - 1]) : key_r);
-            st[threadIdx.x] = v;
-        } else if (threadIdx.x == kSampleRanks) {
-            st[kSampleRanks] = -2.0f;  // the K-th best, set below when the sample holds K docs
-            st[kSampleRanks + 1] = static_cast<float>(n);
-            for (uint32_t j = kSampleRanks + 2; j < kSampleStats; ++j) st[j] = 0.0f;
-        }
-        __syncthreads();
+    };
+    // with statistics, absolute digits: the features keep the 24-bit prefixes of the keys they stand for
+    if (L.stats) {
+        key_lo = 0;
+        key_hi = 0xffffffffu;
     }
+    float theta = L.raise_only ? L.theta[qi] : -INFINITY;
     if (k > 0 && n >= k) {
-        const float* sc = L.score + static_cast<uint64_t>(qi) * L.cap;
         // a lower bound of the K-th best serves the proof below as well as the K-th best itself
-        const uint32_t kk = kth_lower_bound_u32_visit(
-            [&](auto fn) {
-                for_each_segment_entry(S, L.segs, L.seg_cap, sc, [&](uint32_t, bool ok, float v) {
-                    if (ok) fn(float_key(v));
-                });
-            },
-            k, S);
+        const uint32_t kk = kth_lower_bound<NT>(visit, k, key_lo, key_hi, S);
         // k sample docs score >= t approximately, so the true K-th best exact score is >= t - eps_s;
         // a true top-K doc therefore scores >= t - eps_s - eps_m under the main pass's arithmetic.
         const float t = __fsub_rd(__fsub_rd(key_float(kk), L.eps_sample[qi]), L.eps_main[qi]);
         theta = L.raise_only ? fmaxf(theta, t) : t;
         if (L.stats && threadIdx.x == 0) L.stats[static_cast<uint64_t>(qi) * kSampleStats + kSampleRanks] = key_float(kk);
         if (L.theta_also && L.raise_only && threadIdx.x == 0) L.theta_also[qi] = fmaxf(L.theta_also[qi], t);
+    } else if (L.stats && threadIdx.x == 0) {
+        L.stats[static_cast<uint64_t>(qi) * kSampleStats + kSampleRanks] = -2.0f;  // no K-th best
     }
     __syncthreads();  // every thread has read the old theta
     if (threadIdx.x == 0) {
         L.theta[qi] = theta;
         if (L.theta_also && !L.raise_only) L.theta_also[qi] = theta;
     }
+    if (L.stats) {
+        // the sample's best scores at ranks 1, 2, 4, ..., 64: a lower bound of the key at rank
+        // r = min(64, n) (its 24-bit prefix), then the (fewer than r) keys above that prefix's bucket,
+        // each placed by counting the keys that precede it; a rank inside the bucket gets the bound (at
+        // most 2^-15 relative below the score)
+        float* st = L.stats + static_cast<uint64_t>(qi) * kSampleStats;
+        const uint32_t r = min(n, 64u);
+        uint32_t key_r = 0;
+        if (r > 0) key_r = kth_lower_bound<NT>(visit, r, key_lo, key_hi, S);
+        const uint32_t bucket_top = key_r | 0xFFu;
+        __shared__ uint32_t above[64], ranked[64];
+        if (threadIdx.x == 0) S.counter = 0;
+        __syncthreads();
+        if (r > 0)
+            visit([&](uint32_t key) {
+                if (key > bucket_top) {
+                    const uint32_t slot = atomicAdd(&S.counter, 1u);
+                    if (slot < 64u) above[slot] = key;
+                }
+            });
+        __syncthreads();
+        const uint32_t c = min(S.counter, 64u);  // < r unless keys were lost
+        if (threadIdx.x < c) {
+            const uint32_t key = above[threadIdx.x];
+            uint32_t rank = 0;
+            for (uint32_t j = 0; j < c; ++j) {
+                const uint32_t o = above[j];
+                rank += (o > key || (o == key && j < threadIdx.x)) ? 1u : 0u;
+            }
+            ranked[rank] = key;
+        }
+        __syncthreads();
+        if (threadIdx.x < kSampleRanks) {
+            const uint32_t rho = 1u << threadIdx.x;
+            float v = -2.0f;
+            if (rho <= r) v = key_float(rho <= c ? ranked[rho - 1] : key_r);
+            st[threadIdx.x] = v;
+        } else if (threadIdx.x == kSampleRanks) {
+            st[kSampleRanks + 1] = static_cast<float>(n);
+            for (uint32_t j = kSampleRanks + 2; j < kSampleStats; ++j) st[j] = 0.0f;
+        }
+    }
 }
 
-// Byte offset of the shared-memory candidate arrays of select_topk_kernel: after SelectSmem and the
-// query (dim floats), 16-byte aligned.
+// The threshold of a doc sample whose pass wrote, for every query, the best score of each small group of
+// sample docs (-inf for a group without a filtered doc). The group maxima are scores of distinct docs, so
+// their K-th best bounds the docs' K-th best from below as a sample's K-th best does; where K is at most
+// half the groups it lies at a rank not far past K (K = 100 of 4,096 groups: about 101). A dense array of
+// an eighth of the docs replaces lists of all filtered docs with their counts and locations.
+template <int NT>
+__global__ void __launch_bounds__(NT, 1024 / NT) maxima_threshold_kernel(MaximaThresholdLaunch L) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    HistSmem& S = *reinterpret_cast<HistSmem*>(smem_raw);
+    float4* cs = reinterpret_cast<float4*>(smem_raw + sizeof(HistSmem));
+    const uint32_t qi = L.qlist ? L.qlist[blockIdx.x] : blockIdx.x;
+    const uint32_t k = L.topk[qi];
+    const float eps_s = L.eps_sample[qi], eps_m = L.eps_main[qi];
+    const float4* src = reinterpret_cast<const float4*>(L.best + static_cast<uint64_t>(qi) * L.cap);
+    const uint32_t quads = L.groups / 4, cached = min(quads, kFastSample / 4);
+    float lo = INFINITY, hi = -INFINITY;
+    uint32_t n = 0;
+    auto each = [](const float4& v, auto fn) {
+        if (v.x > -INFINITY) fn(v.x);
+        if (v.y > -INFINITY) fn(v.y);
+        if (v.z > -INFINITY) fn(v.z);
+        if (v.w > -INFINITY) fn(v.w);
+    };
+#pragma unroll 4
+    for (uint32_t i = threadIdx.x; i < quads; i += NT) {
+        const float4 v = src[i];
+        if (i < cached) cs[i] = v;
+        each(v, [&](float x) {
+            lo = fminf(lo, x);
+            hi = fmaxf(hi, x);
+            ++n;
+        });
+    }
+    if (threadIdx.x == 0) S.counter = 0;
+    __syncthreads();
+    n = warp_sum(n);
+    if ((threadIdx.x & 31) == 0 && n) atomicAdd(&S.counter, n);
+    uint32_t a = float_key(lo), b = float_key(hi);  // no score: +inf, -inf
+    block_minmax<NT>(a, b, S);
+    float theta = -INFINITY;
+    if (k > 0 && S.counter >= k) {
+        const float t = kth_score_bound<NT>(
+            [&](auto fn) {
+                for (uint32_t i = threadIdx.x; i < cached; i += NT) each(cs[i], fn);
+                for (uint32_t i = cached + threadIdx.x; i < quads; i += NT) each(src[i], fn);
+            },
+            k, key_float(a), key_float(b), S);
+        theta = __fsub_rd(__fsub_rd(t, eps_s), eps_m);  // as in sample_threshold_kernel
+    }
+    if (threadIdx.x == 0) {
+        L.theta[qi] = theta;
+        if (L.theta_also) L.theta_also[qi] = theta;
+    }
+}
+
+// Byte offsets of the query and of the cached scores in select_topk_kernel's shared memory.
 __host__ __device__ inline size_t select_cand_offset(uint32_t dim) {
     return (sizeof(SelectSmem) + static_cast<size_t>(dim) * sizeof(float) + 15) & ~static_cast<size_t>(15);
 }
 
+// Exact scores of list(i), i < m, by groups of four lanes: lane j of a group holds floats 4 j .. 4 j + 3 of
+// every 16 of its row (eight 16-byte loads in flight, 128 dims of the row), and the running sum goes
+// round the four lanes, so that it still adds the products one by one in ascending order, as the ground
+// truth does. put(i, location, score) is called by one lane per row.
+template <int NT, class List, class Put>
+__device__ __forceinline__ void rescore_rows(const float* sq, const float* vec, uint32_t dim, uint32_t m, List list,
+                                             Put put) {
+    const uint32_t lane = threadIdx.x & 31, j = lane & 3;
+    const uint32_t quads = dim / 4;
+    for (uint32_t r0 = (threadIdx.x >> 5) * 8; r0 < m; r0 += NT / 4) {
+        const uint32_t r = r0 + (lane >> 2);
+        const bool ok = r < m;
+        const uint32_t loc = list(ok ? r : r0);
+        const float4* row = reinterpret_cast<const float4*>(vec + static_cast<uint64_t>(loc) * dim);
+        float s = 0.0f;
+        for (uint32_t f0 = 0; f0 < quads; f0 += 32) {
+            float4 v[8];
+#pragma unroll
+            for (uint32_t i = 0; i < 8; ++i) {
+                const uint32_t f = f0 + 4 * i + j;
+                v[i] = f < quads ? __ldg(row + f) : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+#pragma unroll
+            for (uint32_t i = 0; i < 8; ++i) {
+                if (f0 + 4 * i >= quads) break;  // uniform
+                const uint32_t f = f0 + 4 * i + j;
+                float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (f < quads) q = *reinterpret_cast<const float4*>(sq + 4 * f);
+                const float a = __fmul_rn(q.x, v[i].x), b = __fmul_rn(q.y, v[i].y);
+                const float c = __fmul_rn(q.z, v[i].z), d = __fmul_rn(q.w, v[i].w);
+#pragma unroll
+                for (uint32_t turn = 0; turn < 4; ++turn) {
+                    // in turn u lane u of the group holds the sum so far and adds its four products
+                    float n = __fadd_rn(s, a);
+                    n = __fadd_rn(n, b);
+                    n = __fadd_rn(n, c);
+                    n = __fadd_rn(n, d);
+                    if (f0 + 4 * i + turn < quads) s = __shfl_sync(0xffffffffu, n, turn, 4);
+                }
+            }
+        }
+        if (ok && j == 0) put(r, loc, s);
+    }
+}
+
 // ---------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(kST) select_topk_kernel(SelectLaunch L) {
+// The select step, one CTA per query: a chain of dependent steps and the rescoring's row reads bound it.
+//   * The list's scores are read once into shared memory (`fast` entries), the first locations with them.
+//   * A list of at most kSelT entries is rescored whole; a longer one is cut: t~ bounds the K-th
+//     best approximate score from below, so only entries of at least t~ - 2 eps can be in the top K. Where
+//     those are more than kSelT, the entries of at least t~ (K of them at least) are rescored
+//     first: the least of their exact scores, s, bounds the K-th exact score, and the rest needs only
+//     s - eps, about half the band.
+//   * Survivors are packed before they are rescored, so that every lane group has a row.
+template <int NT, uint32_t FAST>
+__global__ void __launch_bounds__(NT, NT == kSelT ? 2 : 1) select_topk_kernel(SelectLaunch L) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     SelectSmem& S = *reinterpret_cast<SelectSmem*>(smem_raw);
     float* sq = reinterpret_cast<float*>(smem_raw + sizeof(SelectSmem));
+    float* cs = reinterpret_cast<float*>(smem_raw + select_cand_offset(L.dim));
+    uint32_t* surv = S.hist;  // survivors' locations: after the last digit
     const uint32_t qi = L.qlist ? L.qlist[blockIdx.x] : blockIdx.x;
     const uint32_t tid = threadIdx.x;
     const uint32_t k = L.topk[qi];
@@ -586,23 +690,29 @@ __global__ void __launch_bounds__(kST) select_topk_kernel(SelectLaunch L) {
         }
         return;
     }
-    bool overflow = false;
-    const uint32_t n =
-        load_segments(S, L.cand_count + static_cast<uint64_t>(qi) * kMaxCandSegs, L.segs, L.seg_cap, &overflow);
+    const uint32_t* counts = L.cand_count + static_cast<uint64_t>(qi) * kMaxCandSegs;
     const float* sc = L.cand_score + row;
     const uint32_t* lc = L.cand_loc + row;
     const float eps = L.eps_main[qi];
-    auto visit_scores = [&](auto fn) {
-        for_each_segment_entry(S, L.segs, L.seg_cap, sc, [&](uint32_t, bool ok, float v) {
-            if (ok) fn(float_key(v));
-        });
+    const float theta_q = L.theta[qi];
+    for (uint32_t i = tid; i < L.dim; i += NT) sq[i] = L.qry[static_cast<uint64_t>(qi) * L.dim + i];
+    bool overflow = false;
+    uint32_t key_lo, key_hi;
+    const uint32_t n = load_list<NT>(S, counts, L.segs, L.seg_cap, sc, lc, cs, FAST, S.locs, &overflow, &key_lo, &key_hi);
+    auto visit_keys = [&](auto fn) {
+        if (n <= FAST) {
+            for (uint32_t i = tid; i < n; i += NT) fn(float_key(cs[i]));
+        } else {
+            walk_segments<NT>(counts, L.segs, L.seg_cap, sc, [](uint32_t) {}, [&](uint32_t, bool ok, float v) {
+                if (ok) fn(float_key(v));
+            });
+        }
     };
     // A threshold above the proven one (a prediction) has to be checked: the list holds every doc
     // with s~ >= theta, so a doc left out scores s < theta + eps, and the K best candidates are the
     // K best docs when their K-th exact score s_K >= theta + eps. A query that fails goes back to a
     // proven threshold: the larger of its proven one and s_K - eps (every true top-K doc scores at
     // least s_K, the candidates' K-th best, hence s~ >= s_K - eps).
-    const float theta_q = L.theta[qi];
     const bool unproven = L.theta_proven != nullptr && theta_q > L.theta_proven[qi];
     auto threshold_miss = [&](float raised) {
         if (tid == 0) {
@@ -618,9 +728,10 @@ __global__ void __launch_bounds__(kST) select_topk_kernel(SelectLaunch L) {
         // the true K-th best from below: raise the threshold and let the host re-run this query.
         float theta = unproven ? L.theta_proven[qi] : theta_q;
         if (n >= k && k > 0) {
-            const uint32_t kk = kth_lower_bound_u32_visit(visit_scores, k, S);
+            const uint32_t kk = kth_lower_bound<NT>(visit_keys, k, key_lo, key_hi, S);
             theta = fmaxf(theta, __fsub_rd(key_float(kk), 2.0f * eps));
         }
+        __syncthreads();  // every thread has read the old thresholds
         if (tid == 0) {
             L.theta[qi] = theta;
             if (L.theta_proven) L.theta_proven[qi] = theta;
@@ -638,80 +749,137 @@ __global__ void __launch_bounds__(kST) select_topk_kernel(SelectLaunch L) {
         return;
     }
     const uint32_t kq = min(k, n);
-    for (uint32_t i = tid; i < L.dim; i += blockDim.x) sq[i] = L.qry[static_cast<uint64_t>(qi) * L.dim + i];
-    // A list that fits is gathered into shared memory once (scores only: the few rescored entries
-    // look their location up again); the selection and rescoring passes then read shared memory
-    // instead of walking the segments again.
-    const bool fast = n <= (L.fast_large ? kSelFastLarge : kSelFast);
-    float* cs = reinterpret_cast<float*>(smem_raw + select_cand_offset(L.dim));
-    if (fast) {
-        for (uint32_t idx = tid; idx < n; idx += blockDim.x) cs[idx] = sc[segment_entry(S, L.segs, L.seg_cap, idx)];
-        __syncthreads();
-    }
-    float thr = -INFINITY;
-    if (n > kq) {
-        // a lower bound of the K-th best approximate score only widens the rescoring cut
-        const uint32_t kk = fast ? kth_lower_bound_u32_visit(
-                                       [&](auto fn) {
-                                           for (uint32_t i = threadIdx.x; i < n; i += blockDim.x) fn(float_key(cs[i]));
-                                       },
-                                       kq, S)
-                                 : kth_lower_bound_u32_visit(visit_scores, kq, S);
-        thr = __fsub_rd(key_float(kk), 2.0f * eps);
-    }
-    if (tid == 0) S.counter = 0;
-    __syncthreads();
     unsigned long long* ws = L.work + row;
-    // rescoring of one entry (score s, location loc; warp-collective): kept entries are appended to ws
-    auto rescore = [&](bool ok, float s, uint32_t loc) {
-        bool take = false;
-        unsigned long long key = 0;
-        if (ok && s >= thr) {
-            const float e = exact_dot(sq, L.vec + static_cast<uint64_t>(loc) * L.dim, L.dim);
-            key = result_key(e, loc);
-            take = true;
-        }
-        const uint32_t mask = __ballot_sync(0xffffffffu, take);
-        if (mask) {
-            const uint32_t lane = tid & 31;
-            const uint32_t leader = __ffs(mask) - 1;
-            uint32_t base = 0;
-            if (lane == leader) base = atomicAdd(&S.counter, __popc(mask));
-            base = __shfl_sync(0xffffffffu, base, leader);
-            if (take) ws[base + __popc(mask & ((1u << lane) - 1u))] = key;
-        }
-    };
-    if (fast) {
-        for (uint32_t b = tid & ~31u; b < n; b += blockDim.x) {  // warp-uniform bounds
-            const uint32_t idx = b + (tid & 31);
-            const bool ok = idx < n;
-            const float v = ok ? cs[idx] : 0.0f;
-            rescore(ok, v, ok && v >= thr ? lc[segment_entry(S, L.segs, L.seg_cap, idx)] : 0u);
-        }
+    uint32_t nf;
+    bool in_smem;  // the keys: S.sortbuf or ws
+    if (n <= static_cast<uint32_t>(kSelT)) {
+        rescore_rows<NT>(sq, L.vec, L.dim, n, [&](uint32_t i) { return S.locs[i]; },
+                         [&](uint32_t i, uint32_t loc, float e) { S.sortbuf[i] = result_key(e, loc); });
+        nf = n;
+        in_smem = true;
     } else {
-        for_each_segment_entry(S, L.segs, L.seg_cap, sc, [&](uint32_t i, bool ok, float v) {
-            rescore(ok, v, ok && v >= thr ? lc[i] : 0u);
-        });
+        const float t = n > kq ? key_float(kth_lower_bound<NT>(visit_keys, kq, key_lo, key_hi, S)) : -INFINITY;
+        const float cut2 = __fsub_rd(t, 2.0f * eps);
+        // fn(score, location) of every entry
+        auto visit_entries = [&](auto fn) {
+            if (n <= min(FAST, static_cast<uint32_t>(kMaxTopK))) {
+                for (uint32_t i = tid; i < n; i += NT) fn(cs[i], [&] { return S.locs[i]; });
+            } else {
+                walk_segments<NT>(counts, L.segs, L.seg_cap, sc, [](uint32_t) {}, [&](uint32_t at, bool ok, float v) {
+                    if (ok) fn(v, [&] { return lc[at]; });
+                });
+            }
+        };
+        // how many clear the cut at all
+        if (tid == 0) S.counter = 0;
+        __syncthreads();
+        uint32_t mine = 0;
+        visit_keys([&](uint32_t key) { mine += key_float(key) >= cut2 ? 1u : 0u; });
+        mine = warp_sum(mine);
+        if ((tid & 31) == 0 && mine) atomicAdd(&S.counter, mine);
+        __syncthreads();
+        const uint32_t all = S.counter;
+        const bool two = all > static_cast<uint32_t>(kSelT) && all > kq && t > -INFINITY;
+        float lo = two ? t : cut2, hi = INFINITY, low_exact = INFINITY;
+        nf = 0;
+        in_smem = all <= static_cast<uint32_t>(kMaxTopK);
+        for (int wave = 0; wave < (two ? 2 : 1); ++wave) {
+            __syncthreads();  // the survivors' list is free
+            if (tid == 0) S.total = 0;
+            __syncthreads();
+            const bool last = !two || wave == 1;
+            visit_entries([&](float v, auto loc) {
+                if (v >= lo && (wave == 0 || v < hi)) {
+                    const uint32_t at = next_place(&S.total);
+                    if (in_smem)
+                        surv[at] = loc();
+                    else
+                        ws[nf + at] = loc();
+                }
+            });
+            __syncthreads();
+            const uint32_t m = S.total;
+            float least = INFINITY;
+            rescore_rows<NT>(
+                sq, L.vec, L.dim, m,
+                [&](uint32_t i) { return in_smem ? surv[i] : static_cast<uint32_t>(ws[nf + i]); },
+                [&](uint32_t i, uint32_t loc, float e) {
+                    const unsigned long long key = result_key(e, loc);
+                    if (in_smem)
+                        S.sortbuf[nf + i] = key;
+                    else
+                        ws[nf + i] = key;
+                    least = fminf(least, e);
+                });
+            nf += m;
+            if (last) break;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) least = fminf(least, __shfl_xor_sync(0xffffffffu, least, o));
+            if ((tid & 31) == 0) S.wsum[tid >> 5] = float_bits(least);
+            __syncthreads();
+            for (int w = 0; w < NT / 32; ++w) low_exact = fminf(low_exact, bits_float(S.wsum[w]));
+            hi = t;
+            lo = fmaxf(cut2, __fsub_rd(low_exact, eps));
+        }
     }
     __syncthreads();
-    const uint32_t nf = S.counter;
-    __syncthreads();
-    top_keys([&](uint32_t i) { return static_cast<uint64_t>(ws[i]); }, nf, kq, S);
+    uint32_t m;
+    const unsigned long long* sorted = S.sortbuf;
+    if (in_smem && nf <= kRankSort) {
+        unsigned long long* out = reinterpret_cast<unsigned long long*>(S.hist);  // free: the last list is read
+        rank_sort<NT>(S, nf, out);
+        sorted = out;
+        m = 0;
+    } else if (in_smem && (nf <= static_cast<uint32_t>(kSelT) || nf <= 2 * kq)) {
+        m = pad_sort<NT>(S, nf);
+    } else if (in_smem) {
+        // more keys than a short sort takes: cut in place (each thread's keys go to registers first)
+        constexpr int kOwn = kMaxTopK / NT;
+        unsigned long long own[kOwn];
+#pragma unroll
+        for (int i = 0; i < kOwn; ++i) own[i] = tid + NT * i < nf ? S.sortbuf[tid + NT * i] : 0ull;
+        uint32_t lo = 0xffffffffu, hi = 0;
+#pragma unroll
+        for (int i = 0; i < kOwn; ++i)
+            if (tid + NT * i < nf) {
+                lo = min(lo, static_cast<uint32_t>(own[i] >> 32));
+                hi = max(hi, static_cast<uint32_t>(own[i] >> 32));
+            }
+        block_minmax<NT>(lo, hi, S);
+        const uint32_t lb = kth_lower_bound<NT>(
+            [&](auto fn) {
+#pragma unroll
+                for (int i = 0; i < kOwn; ++i)
+                    if (tid + NT * i < nf) fn(static_cast<uint32_t>(own[i] >> 32));
+            },
+            kq, lo, hi, S);
+        if (tid == 0) S.counter = 0;
+        __syncthreads();
+#pragma unroll
+        for (int i = 0; i < kOwn; ++i)
+            if (tid + NT * i < nf && static_cast<uint32_t>(own[i] >> 32) >= lb) S.sortbuf[next_place(&S.counter)] = own[i];
+        __syncthreads();
+        m = pad_sort<NT>(S, S.counter);
+    } else {
+        m = gather_top_keys<NT>([&](uint32_t i) { return static_cast<uint64_t>(ws[i]); }, nf, kq, S);
+    }
+    if (m) bitonic_desc<NT>(S, m);
     if (unproven) {
-        const float lo = kq == k ? __fsub_rd(result_key_score(S.sortbuf[kq - 1]), eps) : -INFINITY;
+        const float lo = kq == k && nf >= kq ? __fsub_rd(result_key_score(sorted[kq - 1]), eps) : -INFINITY;
         if (!(lo >= theta_q)) {
             threshold_miss(lo);
             return;
         }
     }
+    const uint32_t kout = min(kq, nf);  // kq, unless the bound is not a number
     const uint64_t orow = static_cast<uint64_t>(qi) * L.out_stride;
-    for (uint32_t i = tid; i < kq; i += blockDim.x) {
-        const uint64_t key = S.sortbuf[i];
+    for (uint32_t i = tid; i < kout; i += NT) {
+        const uint64_t key = sorted[i];
         const uint32_t loc = result_key_loc(key);
         L.out_score[orow + i] = result_key_score(key);
         L.out_id[orow + i] = L.gdocid ? L.gdocid[loc] : static_cast<int64_t>(loc);
     }
-    if (tid == 0) L.out_count[qi] = kq;
+    if (tid == 0) L.out_count[qi] = kout;
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -900,9 +1068,9 @@ __global__ void __launch_bounds__(kST) topk_op_kernel(const float* __restrict__ 
             if (t == 0) *out_count = 0;
             return;
         }
-        m = gather_top_keys([&](uint32_t i) { return result_key(scores[i], locs[i]); }, n, kq, S);
+        m = gather_top_keys<kST>([&](uint32_t i) { return result_key(scores[i], locs[i]); }, n, kq, S);
     } else {
-        uint32_t* hist = &S.hist[0][0];
+        uint32_t* hist = S.hist;
         const uint32_t gt = rank * kST + t, gthreads = C * kST;
         // fn(index, score) for the entries mul * i, i < cnt, 4 loads in flight
         auto visit = [&](uint32_t cnt, uint32_t mul, auto fn) {
@@ -930,10 +1098,10 @@ __global__ void __launch_bounds__(kST) topk_op_kernel(const float* __restrict__ 
             if (t < slice) {
                 uint32_t s = 0;
                 for (uint32_t r = 0; r < C; ++r) s += cluster.map_shared_rank(hist, r)[rank * slice + t];
-                S.segn[t] = s;
+                S.locs[t] = s;
             }
             cluster.sync();
-            for (uint32_t i = t; i < 4096u; i += kST) hist[i] = cluster.map_shared_rank(S.segn, i / slice)[i % slice];
+            for (uint32_t i = t; i < 4096u; i += kST) hist[i] = cluster.map_shared_rank(S.locs, i / slice)[i % slice];
             __syncthreads();
         };
         auto clear = [&] {
@@ -946,7 +1114,7 @@ __global__ void __launch_bounds__(kST) topk_op_kernel(const float* __restrict__ 
             visit(kTopkSample, n / kTopkSample, [&](uint32_t, float v) { atomicAdd(&hist[float_key(v) >> 20], 1u); });
             sum_cluster();
             uint32_t kr = kq;  // kq <= kMaxTopK < kTopkSample
-            floor_key = pick_digit4096(hist, &kr, S) << 20;
+            floor_key = pick_digit4096<kST>(hist, &kr, S) << 20;
         }
         uint64_t prefix = 0, mask = 0;
         uint32_t krem = kq, in_bin = 0;
@@ -967,7 +1135,7 @@ __global__ void __launch_bounds__(kST) topk_op_kernel(const float* __restrict__ 
                 atomicAdd(&hist[(key >> shift) & digit], 1u);
             });
             sum_cluster();
-            const uint64_t d = pick_digit4096(hist, &krem, S, &in_bin);
+            const uint64_t d = pick_digit4096<kST>(hist, &krem, S, &in_bin);
             prefix |= d << shift;
             mask |= digit << shift;
             fits = (kq - krem) + in_bin <= static_cast<uint32_t>(kMaxTopK);
@@ -997,11 +1165,9 @@ __global__ void __launch_bounds__(kST) topk_op_kernel(const float* __restrict__ 
         cluster.sync();
         if (rank != 0) return;
         const uint32_t got = min(above + S.total, static_cast<uint32_t>(kMaxTopK));
-        m = sort_size(got);
-        for (uint32_t i = got + t; i < m; i += kST) S.sortbuf[i] = 0ull;
-        __syncthreads();
+        m = pad_sort<kST>(S, got);
     }
-    bitonic_desc(S, m);
+    bitonic_desc<kST>(S, m);
     for (uint32_t i = t; i < kq; i += kST) {
         const uint64_t key = S.sortbuf[i];
         out_scores[i] = result_key_score(key);
@@ -1039,7 +1205,7 @@ __global__ void query_eps_kernel(const float* __restrict__ qry, const uint32_t* 
 // could drop below another caller's launch.
 template <class K>
 cudaError_t set_smem(K kernel, size_t bytes) {
-    constexpr size_t kCeiling = 200 * 1024;
+    constexpr size_t kCeiling = 216 * 1024;
     if (bytes <= 48 * 1024) return cudaSuccess;
     if (bytes > kCeiling) return cudaErrorInvalidValue;
     return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kCeiling));
@@ -1053,23 +1219,44 @@ bool bad_segments(uint32_t segs, uint32_t seg_cap, uint32_t cap) {
 }
 }  // namespace
 
+// Up to this many queries every CTA has an SM to itself: the selection kernels then take 1,024 threads
+// (more, and two CTAs of 512 threads per SM hide each other's steps better).
+constexpr uint32_t kWideQueries = 148;
+
 cudaError_t launch_sample_threshold(const SampleThresholdLaunch& L, cudaStream_t stream) {
     if (L.nq_list == 0) return cudaSuccess;
     if (bad_segments(L.segs, L.seg_cap, L.cap)) return cudaErrorInvalidValue;
-    const size_t smem = sizeof(SelectSmem);
-    cudaError_t e = set_smem(sample_threshold_kernel, smem);
+    const size_t smem = sizeof(HistSmem) + kFastSample * sizeof(float);
+    const bool wide = L.nq_list <= kWideQueries;
+    auto kernel = wide ? sample_threshold_kernel<kST> : sample_threshold_kernel<kSelT>;
+    cudaError_t e = set_smem(kernel, smem);
     if (e != cudaSuccess) return e;
-    sample_threshold_kernel<<<L.nq_list, kST, smem, stream>>>(L);
+    kernel<<<L.nq_list, wide ? kST : kSelT, smem, stream>>>(L);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_maxima_threshold(const MaximaThresholdLaunch& L, cudaStream_t stream) {
+    if (L.nq_list == 0) return cudaSuccess;
+    if (L.groups == 0 || L.groups % 4 || L.cap % 4 || L.groups > L.cap || (reinterpret_cast<uintptr_t>(L.best) & 15u))
+        return cudaErrorInvalidValue;
+    const size_t smem = sizeof(HistSmem) + (L.groups < kFastSample ? L.groups : kFastSample) * sizeof(float);
+    const bool wide = L.nq_list <= kWideQueries;
+    auto kernel = wide ? maxima_threshold_kernel<kST> : maxima_threshold_kernel<kSelT>;
+    cudaError_t e = set_smem(kernel, smem);
+    if (e != cudaSuccess) return e;
+    kernel<<<L.nq_list, wide ? kST : kSelT, smem, stream>>>(L);
     return cudaGetLastError();
 }
 
 cudaError_t launch_select_topk(const SelectLaunch& L, cudaStream_t stream) {
     if (L.nq_list == 0) return cudaSuccess;
     if (bad_segments(L.segs, L.seg_cap, L.cap) || L.segs > static_cast<uint32_t>(kST)) return cudaErrorInvalidValue;
-    const size_t smem = select_cand_offset(L.dim) + (L.fast_large ? kSelFastLarge : kSelFast) * sizeof(float);
-    cudaError_t e = set_smem(select_topk_kernel, smem);
+    const bool wide = L.fast_large || L.nq_list <= kWideQueries;
+    const size_t smem = select_cand_offset(L.dim) + (wide ? kFastLarge : kFast) * sizeof(float);
+    auto kernel = wide ? select_topk_kernel<kST, kFastLarge> : select_topk_kernel<kSelT, kFast>;
+    cudaError_t e = set_smem(kernel, smem);
     if (e != cudaSuccess) return e;
-    select_topk_kernel<<<L.nq_list, kST, smem, stream>>>(L);
+    kernel<<<L.nq_list, wide ? kST : kSelT, smem, stream>>>(L);
     return cudaGetLastError();
 }
 

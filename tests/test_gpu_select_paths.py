@@ -1,0 +1,59 @@
+"""The selection kernels' paths against the oracle, ids and scores bit for bit: K on both sides of half the
+sample's groups (group maxima, lists of docs), lists rescored whole, cut in one wave and in two, cached and
+walked, few and many queries (one CTA per SM or two), dims that are no multiple of 16, filters that leave
+fewer docs than K."""
+import numpy as np
+import pytest
+
+import hybridsearchsystem_b200 as hss
+import oracle
+from hybridsearchsystem_b200 import data
+
+pytestmark = pytest.mark.gpu
+
+_WORLD = {}
+
+
+def _world(n, dim):
+    if (n, dim) not in _WORLD:
+        mix = data.Mixture(dim, 48, (2e-4, 0.6), n_clusters=40, seed=9)
+        vec, bits, _ = mix.corpus(n, seed=10)
+        vec[n // 3] = vec[n // 2] = vec[n - 1]  # equal scores
+        _WORLD[(n, dim)] = (mix, vec, bits, hss.DataTable.build(vec, bits, 48, device=0, doc_num_per_segment=16384))
+    return _WORLD[(n, dim)]
+
+
+def _check(n, dim, method, nq, topks, sample_docs=32768, cap=1 << 18):
+    mix, vec, bits, table = _world(n, dim)
+    q = mix.queries(nq, seed=nq + 11)
+    exprs = data.make_filters(mix, nq, n_tags=(1, 5), seed=nq + 12)
+    exprs[0] = ""
+    exprs[-1] = "NOT 5"
+    topks = np.resize(np.asarray(topks, np.uint32), nq)
+    s = hss.FullRecallSearcher(table, max_batch=nq, method=method, sample_docs=sample_docs, candidate_cap=cap)
+    for a, e, k in zip(q, exprs, topks):
+        s.add_query(e, a, int(k))
+    scores, ids, counts = s.batch_search(out_stride=int(topks.max()))
+    want_s, want_i, want_c = oracle.topk(q, exprs, topks.astype(np.int32), vec, bits, threads=8)
+    for i in range(nq):
+        c = int(want_c[i])
+        assert int(counts[i]) == c, (i, exprs[i])
+        assert (ids[i, :c] == want_i[i, :c]).all(), (i, exprs[i])
+        assert (scores[i, :c].view(np.uint32) == want_s[i, :c].view(np.uint32)).all()
+
+
+@pytest.mark.parametrize("method", [0, 1, 2, 3], ids=["simt", "tf32", "bf16", "e4m3"])
+@pytest.mark.parametrize("nq,k", [(1, 1), (5, 100), (9, 2048), (9, 2049), (150, 513), (3, 4096)])
+def test_select_paths_match_the_oracle(torch_cuda, method, nq, k):
+    _check(60001, 128, method, nq, [k])
+
+
+@pytest.mark.parametrize("method,dim", [(0, 100), (0, 36), (1, 32), (1, 352), (2, 64), (2, 704)])
+def test_select_paths_at_other_dims(torch_cuda, method, dim):
+    _check(20003, dim, method, 40, [1, 10, 300, 1000])
+
+
+@pytest.mark.parametrize("method", [0, 2, 3], ids=["simt", "bf16", "e4m3"])
+@pytest.mark.parametrize("sample_docs,cap", [(512, 1 << 18), (4096, 8192), (60001, 1 << 18)])
+def test_small_samples_and_lists(torch_cuda, method, sample_docs, cap):
+    _check(60001, 128, method, 17, [3, 128, 256, 257, 1024], sample_docs=sample_docs, cap=cap)
