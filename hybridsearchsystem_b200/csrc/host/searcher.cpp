@@ -565,7 +565,7 @@ void FullRecallSearcher::Stage(const uint32_t* dList, uint32_t rows) {
 // SIMT pass and the single-SM tensor-core pass, 256 for the SM-pair pass.
 void FullRecallSearcher::Cand(const float* theta, float* score, uint32_t* loc, uint32_t* count, uint32_t cap,
                               uint32_t segBase, uint32_t segCap, uint64_t begin, uint64_t step, uint32_t skip,
-                              uint64_t countTiles, const uint32_t* dList, uint32_t rows, bool simt, float* best) {
+                              uint64_t countTiles, const uint32_t* dList, uint32_t rows, bool simt, float* best, bool coarse) {
     const DataTable& T = *m_table;
     const uint32_t g = CtasOf(rows, countTiles, cap, simt);
     if (UseSimt(simt)) {
@@ -612,6 +612,7 @@ void FullRecallSearcher::Cand(const float* theta, float* score, uint32_t* loc, u
     C.seg_cap = segCap;
     C.seg_base = segBase;
     C.best = best;
+    C.coarse = coarse ? 1 : 0;
     C.tile_begin = begin;
     C.tile_step = step;
     C.tile_count = countTiles;
@@ -640,9 +641,13 @@ void FullRecallSearcher::SampleTiles(uint64_t want, uint32_t rows, bool simt, ui
 
 // Groups of a sample of `count` tiles that is kept as group maxima, 0 where it is kept as lists of docs: a
 // K past half the groups would find its threshold far below the docs' K-th best (at K = groups it is
-// the least maximum).
-uint32_t FullRecallSearcher::MaximaGroups(uint32_t rows, uint64_t count, bool simt) const {
-    const uint64_t groups = count * (UnitOf(rows, simt) / (UseSimt(simt) ? kSimtGroup : kTcGroup));
+// the least maximum). *docs: docs of a group. Coarse groups, a quarter of the stores and of the
+// threshold's entries, where K is an eighth of them at most (the K-th maximum is then at rank 1.07 K or
+// better among the docs).
+uint32_t FullRecallSearcher::MaximaGroups(uint32_t rows, uint64_t count, bool simt, uint32_t* docs) const {
+    const uint64_t all = count * UnitOf(rows, simt);
+    *docs = UseSimt(simt) ? kSimtGroup : all / kTcCoarseGroup >= 8ull * m_b.maxK ? kTcCoarseGroup : kTcGroup;
+    const uint64_t groups = all / *docs;
     return groups >= 2ull * m_b.maxK && groups <= m_sampCap ? static_cast<uint32_t>(groups) : 0u;
 }
 
@@ -655,9 +660,10 @@ uint64_t FullRecallSearcher::Sample(const uint32_t* dList, uint32_t rows, bool s
     const uint32_t segs = SegsOf(rows, count, m_sampCap, simt);
     const uint32_t segCap = SegCapOf(rows, count, m_sampCap, segs, simt);
     auto* dSampCount = reinterpret_cast<uint32_t*>(D + SL.sampCount);
-    if (const uint32_t groups = MaximaGroups(rows, count, simt); groups && !stats && !raiseOnly) {
+    uint32_t groupDocs = 0;
+    if (const uint32_t groups = MaximaGroups(rows, count, simt, &groupDocs); groups && !stats && !raiseOnly) {
         Cand(reinterpret_cast<const float*>(D + SL.negInf), m_dSampScore, m_dSampLoc, dSampCount, m_sampCap, 0, segCap, 0,
-             step, 0, count, dList, rows, simt, m_dSampScore);
+             step, 0, count, dList, rows, simt, m_dSampScore, groupDocs == kTcCoarseGroup);
         MaximaThresholdLaunch MT{};
         MT.best = m_dSampScore;
         MT.cap = m_sampCap;
@@ -789,6 +795,37 @@ uint64_t FullRecallSearcher::SampleWant(uint32_t maxK) const {
     // the doc sample whose threshold keeps the full pass within the list capacity
     return std::max<uint64_t>(m_cfg.sampleDocs, (4ull * std::max<uint32_t>(maxK, 1u) * m_table->GetDocNum() +
                                                  m_cfg.candidateCap - 1) / m_cfg.candidateCap);
+}
+
+// The doc sample, as group maxima, that balances its own cost against what a tighter threshold saves: with s
+// sample docs the two passes keep about 2 K sqrt(N / s) docs per query, so the best s grows with
+// (queries * K * sqrt(N))^(2/3), less for longer rows. The constant from 10M docs x 128 (BF16, 256
+// queries, K = 100): N / 305 (the 32,768 minimum) 1058 us a batch, N / 128 1038, N / 64 1016, N / 32
+// 1029, N / 16 1076; 2.5M, 64 queries, K = 1000: N / 64 428, N / 32 411, N / 16 402. The 8-bit form's
+// thresholds are its error band below the K-th score, where a rank more or less matters more: N / 16
+// (1M docs, 128 queries, K = 10: 477 us against 510 at the minimum). The FP32 SIMT form's sample
+// costs as much per doc as its passes do: the minimum. So does a configuration below the default minimum,
+// which asks for small samples.
+uint64_t FullRecallSearcher::SampleOptimum(uint32_t nq, uint32_t maxK) const {
+    if (m_tcFormat < 0 || m_cfg.sampleDocs < SearcherConfig{}.sampleDocs) return 0;
+    const double n = static_cast<double>(m_table->GetDocNum());
+    const double rows = std::max(1.0, m_tcKblocks / 2.0);  // row length, in 256-byte units
+    double s = std::pow(0.763 * nq * std::max<uint32_t>(maxK, 1u) * std::sqrt(n) / rows, 2.0 / 3.0);
+    if (m_tcFormat == kTcE4M3) s = std::max(s, n / 16);
+    return static_cast<uint64_t>(std::min(s, n / 8));
+}
+
+// Whether the corpus is passed over once, at the sample's threshold, instead of in two parts with the
+// threshold raised between them. One pass keeps about K N / s docs per query, two 2 K sqrt(N / s); the
+// second launch, the raise and the gap cost about as much as keeping 400,000 more docs (300,000 docs, 256
+// queries, K = 100: 165 -> 146 us; 131,072 docs, 32 queries: 108 -> 92; 1M x 768, 256 queries, 570,000
+// more docs: 551 -> 557). Not where the lists would fill past an eighth, nor for the 8-bit form (1M docs,
+// 128 queries: 512 -> 675 us: its band keeps far more than that estimate).
+bool FullRecallSearcher::OnePass(uint32_t nq, uint32_t maxK, uint64_t sampled) const {
+    if (m_tcFormat == kTcE4M3 || sampled == 0) return false;
+    const double ratio = static_cast<double>(m_table->GetDocNum()) / static_cast<double>(sampled);
+    const double more = static_cast<double>(nq) * maxK * (ratio - 2.0 * std::sqrt(ratio));
+    return more <= 300e3 && 8.0 * maxK * ratio <= m_cfg.candidateCap;
 }
 
 uint32_t FullRecallSearcher::PlanTopK(uint32_t maxK) const {
@@ -935,9 +972,12 @@ int FullRecallSearcher::EnqueueAttempt(uint32_t nq, const BatchInputs& in, float
     // the sample's proven thresholds (theta_1) are also kept in theta1, copied to the host with the
     // statuses (a copy here would stall the stream between the sample and the passes)
     auto* dTheta1 = reinterpret_cast<float*>(D + SL.theta1);
+    if (!wantStats) m_b.want = std::max<uint64_t>(m_b.want, SampleOptimum(nq, maxK));
     uint64_t sampCount = 0, grownStep = 1;
+    uint32_t groupDocs = 0;
     SampleTiles(m_b.want, nq, false, &sampCount, &grownStep);
-    if (m_b.want > m_cfg.sampleDocs && !MaximaGroups(nq, sampCount, false)) {
+    if (m_b.want > m_cfg.sampleDocs && !MaximaGroups(nq, sampCount, false, &groupDocs)) {
+        m_b.want = m_b.wantRerun;
         // A sample grown with K, kept as lists, in two steps: the sample_docs sample's proven threshold first, then the
         // grown sample keeps only the docs above it. Its K-th best is the same whenever it has K docs
         // above that threshold (and raises theta_1 then); otherwise theta_1 stays. Every doc of the
@@ -988,6 +1028,7 @@ int FullRecallSearcher::EnqueueAttempt(uint32_t nq, const BatchInputs& in, float
     }
     uint32_t split = static_cast<uint32_t>(std::sqrt(static_cast<double>(tilesM) / static_cast<double>(splitSample)));
     split = std::min<uint32_t>(split, 64);
+    if (!learned && OnePass(nq, maxK, std::min<uint64_t>(sampCount * UnitOf(nq, false), T.GetDocNum()))) split = 1;
     SelectLaunch& SE = m_b.se;
     SE.vec = T.DeviceVectors();
     SE.qry = dQueries;

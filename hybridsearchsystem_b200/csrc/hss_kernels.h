@@ -96,7 +96,7 @@ struct CandLaunch {
     uint64_t tile_begin, tile_step, tile_count;
     uint32_t tile_skip;
 };
-constexpr uint32_t kSimtGroup = 4, kTcGroup = 8;  // docs per group maximum
+constexpr uint32_t kSimtGroup = 4, kTcGroup = 8, kTcCoarseGroup = 32;  // docs per group maximum
 // Largest query count of one SIMT candidate pass (its per-query counts live in shared memory).
 constexpr uint32_t kMaxSimtBatch = 4096;
 // CTAs of a SIMT candidate pass over tile_count tiles into lists of `cap` entries (one list segment
@@ -201,7 +201,8 @@ struct TcCandLaunch {
     uint32_t cap;
     uint32_t ctas, seg_cap;    // CTAs of the launch (tc_cand_ctas); entries per list segment
     uint32_t seg_base;         // first segment this pass writes (it writes 2 per CTA)
-    float* best;               // or null: group maxima instead of candidates, as in CandLaunch (kTcGroup docs)
+    float* best;               // or null: group maxima instead of candidates, as in CandLaunch
+    int coarse;                // their groups: kTcGroup docs (0) or kTcCoarseGroup (1)
     uint64_t tile_begin, tile_step, tile_count;  // tiles of tc_tile_docs(nq_rows, kblocks) docs
     uint32_t tile_skip;
     uint64_t tiles128;         // 128-doc tiles of the corpus (rows of the tensor map / 128)

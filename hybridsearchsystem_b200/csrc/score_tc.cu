@@ -389,10 +389,12 @@ __device__ __forceinline__ void emit_chunk(bool live, uint32_t m, const uint32_t
 }
 
 // One 32-doc chunk's group maxima (the doc sample): the best score of each kTcGroup docs whose filter bit is
-// set, -inf where none is, as one 16-byte store. live: the chunk was read (some lane has a bit).
+// set, -inf where none is, as one 16-byte store at out[4 * chunk]; coarse: of the whole chunk, at
+// out[chunk]. live: the chunk was read (some lane has a bit).
 template <int F>
 __device__ __forceinline__ void store_maxima(bool live, uint32_t m, const uint32_t (&v)[32], float qs,
-                                             const float* doc_scale, uint64_t doc0, float* out) {
+                                             const float* doc_scale, uint64_t doc0, float* out, uint32_t chunk,
+                                             bool coarse) {
     float g[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
     if (live) {
 #pragma unroll
@@ -407,9 +409,12 @@ __device__ __forceinline__ void store_maxima(bool live, uint32_t m, const uint32
             g[k] = max3(max3(x[0], x[1], x[2]), max3(x[3], x[4], x[5]), fmaxf(x[6], x[7]));
         }
     }
-    *reinterpret_cast<float4*>(out) = make_float4(g[0], g[1], g[2], g[3]);
+    if (coarse)
+        out[chunk] = fmaxf(max3(g[0], g[1], g[2]), g[3]);
+    else
+        *reinterpret_cast<float4*>(out + 4u * chunk) = make_float4(g[0], g[1], g[2], g[3]);
 }
-static_assert(kTcGroup == 8, "a chunk of 32 docs holds 4 groups");
+static_assert(kTcGroup == 8 && kTcCoarseGroup == 32, "a chunk of 32 docs holds 4 groups, or is one");
 
 // MAXIMA: the pass writes group maxima (TcCandLaunch::best) instead of candidates.
 template <int F, int H, bool MAXIMA>
@@ -590,7 +595,8 @@ __global__ void __launch_bounds__(64 + 256 * H, 1) tc_cand_kernel(const __grid_c
                 if constexpr (MAXIMA) {
                     if (valid)
                         store_maxima<F>(live[c], m[c], v[c], qs, L.doc_scale, doc0,
-                                        L.best + static_cast<uint64_t>(qi) * L.cap + it * 16u + colh * 8u + c * 4u);
+                                        L.best + static_cast<uint64_t>(qi) * L.cap,
+                                        static_cast<uint32_t>(it) * 4u + colh * 2u + c, L.coarse != 0);
                 } else if constexpr (F == kTcE4M3) {
                     emit_chunk<F>(live[c], m[c], v[c], t, theta, qs, L.doc_scale, doc0, out_score, out_loc, seg_cap,
                                   ncand);
@@ -905,7 +911,7 @@ __global__ void __launch_bounds__(kPairThreads, 1) tc2_cand_kernel(const __grid_
                         // (E4M3: no scales past the corpus rows, whose bits are clear)
                         if (valid)
                             store_maxima<F>(live[c] && doc0 < L.tiles128 * 128u, m[c], v, qs, L.doc_scale, doc0,
-                                            L.best + static_cast<uint64_t>(qi) * L.cap + it * 32u + g * 8u + c * 4u);
+                                            L.best + static_cast<uint64_t>(qi) * L.cap, it * 8u + g * 2u + c, L.coarse != 0);
                     } else if constexpr (F == kTcE4M3) {
                         emit_chunk<F>(live[c], m[c], v, t, theta, qs, L.doc_scale, doc0, out_score, out_loc, seg_cap,
                                       ncand);
@@ -1040,7 +1046,7 @@ cudaError_t launch_tc_cand(const TcCandLaunch& Lin, const CUtensorMap& doc_map, 
         seg_end * L.seg_cap > L.cap)
         return cudaErrorInvalidValue;
     // a tile's group maxima stay inside a query's row, in 16-byte stores
-    if (L.best && (L.tile_count * (tc_tile_docs(L.nq_rows, L.kblocks) / kTcGroup) > L.cap || L.cap % 4 ||
+    if (L.best && (L.tile_count * (tc_tile_docs(L.nq_rows, L.kblocks) / (L.coarse ? kTcCoarseGroup : kTcGroup)) > L.cap || L.cap % 4 ||
                    (reinterpret_cast<uintptr_t>(L.best) & 15u)))
         return cudaErrorInvalidValue;
     switch (L.format) {
