@@ -235,6 +235,7 @@ __global__ void __launch_bounds__(kTile) filter_batch_kernel(FilterLaunch L) {
     __shared__ uint32_t s_prog[kMaxProgram];
     __shared__ int s_bad;
 
+    launch_dependents();
     const uint32_t q = blockIdx.x;
     const uint32_t t = threadIdx.x;
     const uint32_t seg_words = L.docs_per_seg / 64;
@@ -384,6 +385,7 @@ __global__ void __launch_bounds__(kDenseT) filter_dense_kernel(DenseFilterLaunch
     __shared__ uint32_t s_prog[kMaxProgram];
     __shared__ uint32_t s_row[kMaxOperands];
 
+    launch_dependents();
     const uint32_t q = blockIdx.x;
     const uint32_t t = threadIdx.x;
     const uint32_t seg_words = L.seg_words;
@@ -621,6 +623,7 @@ __global__ void __launch_bounds__(kWideT, kWideCtasPerSm) filter_dense_wide_kern
     __shared__ const uint64_t* s_base[kWideMaxOpnd];
     __shared__ int s_ok;
 
+    launch_dependents();
     const uint32_t q = blockIdx.x;
     const uint32_t t = threadIdx.x;
     const uint32_t seg_words = L.seg_words;

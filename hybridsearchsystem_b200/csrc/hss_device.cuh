@@ -66,6 +66,13 @@ __host__ __device__ inline uint64_t result_key(float s, uint32_t loc) {
 __host__ __device__ inline uint32_t result_key_loc(uint64_t k) { return 0xffffffffu - static_cast<uint32_t>(k); }
 __host__ __device__ inline float result_key_score(uint64_t k) { return key_float(static_cast<uint32_t>(k >> 32)); }
 
+// Programmatic dependent launch: a kernel launched by launch_dependent (hss_kernels.h) may start while the
+// kernel before it on the stream still runs, as soon as each of that kernel's CTAs has called
+// launch_dependents() or returned. Until wait_for_previous() returns, it must not touch global memory
+// that an earlier kernel reads or writes; after it, every earlier kernel has completed.
+__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 __device__ inline uint32_t warp_sum(uint32_t v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);

@@ -7,8 +7,32 @@
 
 #include <cstddef>
 #include <cstdint>
+#include <utility>
 
 namespace hss {
+
+// Launches a kernel that calls wait_for_previous() (hss_device.cuh), so that its launch and its
+// set-up overlap the end of the kernel before it: a batch's chain of short kernels otherwise idles
+// 1 to 3 us between each two. cluster > 1: clusters of that many CTAs along x.
+template <class... Params, class... Args>
+cudaError_t launch_dependent(void (*kernel)(Params...), dim3 grid, unsigned block, size_t smem, cudaStream_t stream,
+                             unsigned cluster, Args&&... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(block, 1, 1);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = cluster;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = cluster > 1 ? 2 : 1;
+    return cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+}
 
 // Batched postfix filter (filter.cu). Operand i of query q at segment s is the posting at device
 // address table[row * row_stride + s * seg_stride], row = opnd_row[opnd_off[q] + i] (or i when

@@ -224,6 +224,8 @@ __device__ __forceinline__ void tile_of(int64_t tile, int N, int* m0, int* n0) {
 __global__ void __launch_bounds__(kGroup) layer_forward_kernel(Product P, const float* __restrict__ bias,
                                                                float* __restrict__ Z, float* __restrict__ act) {
     extern __shared__ __align__(16) float gsm[];
+    launch_dependents();
+    wait_for_previous();
     int m0, n0;
     tile_of(blockIdx.x, P.N, &m0, &n0);
     float acc[2][4];
@@ -253,6 +255,8 @@ __global__ void __launch_bounds__(kHeadT) head_kernel(const float* __restrict__ 
     __shared__ float sa[kHeadRows][kHeadK + 1];
     __shared__ float sw[kHeadK];
     __shared__ float sdy[kHeadRows];
+    launch_dependents();
+    wait_for_previous();
     const int r0 = blockIdx.x * kHeadRows, t = threadIdx.x;
     const int rows = min(kHeadRows, B - r0);
     float acc = 0.0f;
@@ -305,6 +309,8 @@ __global__ void __launch_bounds__(kGradThreads) grad_hidden_kernel(Product dA, c
                                                                    const float* __restrict__ dy, int B, int H,
                                                                    float* __restrict__ gw3, float* __restrict__ gb3) {
     extern __shared__ __align__(16) float gsm[];
+    launch_dependents();
+    wait_for_previous();
     int64_t tile = blockIdx.x;
     int m0, n0;
     float acc[2][4];
@@ -351,6 +357,8 @@ __global__ void __launch_bounds__(kGradThreads) grad_hidden_kernel(Product dA, c
 __global__ void __launch_bounds__(kGradThreads) grad_input_kernel(Product dW, float* __restrict__ gW1,
                                                                   float* __restrict__ gb1) {
     extern __shared__ __align__(16) float gsm[];
+    launch_dependents();
+    wait_for_previous();
     int m0, n0;
     tile_of(blockIdx.x, dW.N, &m0, &n0);
     float acc[2][4];
@@ -522,18 +530,23 @@ cudaError_t launch_train_gradients(const TrainLaunch& L, cudaStream_t stream) {
                                              static_cast<int>(kGradSmem));
         if (e != cudaSuccess) return e;
     }
-    layer_forward_kernel<<<static_cast<unsigned>(tF), kGroup, kFwdSmem, stream>>>(Product{L.X, W1, B, H, D, D, H}, b1,
-                                                                                 L.Z1, L.A1);
-    layer_forward_kernel<<<static_cast<unsigned>(tF), kGroup, kFwdSmem, stream>>>(Product{L.A1, W2, B, H, H, H, H}, b2,
-                                                                                 L.Z2, L.A2);
-    head_kernel<<<(B + kHeadRows - 1) / kHeadRows, kHeadT, 0, stream>>>(L.A2, L.Z2, w3, b3, L.T, B, H, L.tau, L.dy,
-                                                                        L.term, L.dZ2);
-    grad_hidden_kernel<<<static_cast<unsigned>(tF + tW2 + tw3), kGradThreads, kGradSmem, stream>>>(
-        Product{L.dZ2, W2, B, H, H, H, H}, L.Z1, L.dZ1, tF, Product{L.A1, L.dZ2, H, H, B, H, H}, gW2, gb2, tW2, L.A2,
-        L.dy, B, H, gw3, gb3);
-    grad_input_kernel<<<static_cast<unsigned>(tW1), kGradThreads, kGradSmem, stream>>>(
-        Product{L.X, L.dZ1, D, H, B, D, H}, gW1, gb1);
-    return cudaGetLastError();
+    const dim3 gF(static_cast<unsigned>(tF));
+    cudaError_t e = launch_dependent(layer_forward_kernel, gF, kGroup, kFwdSmem, stream, 1, Product{L.X, W1, B, H, D, D, H},
+                                     b1, L.Z1, L.A1);
+    if (e == cudaSuccess)
+        e = launch_dependent(layer_forward_kernel, gF, kGroup, kFwdSmem, stream, 1, Product{L.A1, W2, B, H, H, H, H}, b2,
+                             L.Z2, L.A2);
+    if (e == cudaSuccess)
+        e = launch_dependent(head_kernel, dim3((B + kHeadRows - 1) / kHeadRows), kHeadT, 0, stream, 1, L.A2, L.Z2, w3, b3,
+                             L.T, B, H, L.tau, L.dy, L.term, L.dZ2);
+    if (e == cudaSuccess)
+        e = launch_dependent(grad_hidden_kernel, dim3(static_cast<unsigned>(tF + tW2 + tw3)), kGradThreads, kGradSmem,
+                             stream, 1, Product{L.dZ2, W2, B, H, H, H, H}, L.Z1, L.dZ1, tF,
+                             Product{L.A1, L.dZ2, H, H, B, H, H}, gW2, gb2, tW2, L.A2, L.dy, B, H, gw3, gb3);
+    if (e == cudaSuccess)
+        e = launch_dependent(grad_input_kernel, dim3(static_cast<unsigned>(tW1)), kGradThreads, kGradSmem, stream, 1,
+                             Product{L.X, L.dZ1, D, H, B, D, H}, gW1, gb1);
+    return e;
 }
 
 cudaError_t launch_mlp_forward(const float* X, int B, int D, int H, const float* P, float* y, cudaStream_t stream) {

@@ -116,9 +116,10 @@ __global__ void tile_minmax_kernel(const float* __restrict__ scale, uint64_t til
     if (lane == 0) out[t] = make_float2(lo, hi);
 }
 
-__global__ void stage_queries_kernel(StageQueriesLaunch L) {
-    const uint32_t r = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
-    if (r >= L.rows_alloc) return;
+// Runs beside the batch's filter, the kernel before it: it reads and writes nothing of the filter's (the
+// queries are complete before the filter starts), and waits for it only at its end, so that what is
+// launched after it finds both complete.
+__device__ __forceinline__ void stage_row(const StageQueriesLaunch& L, uint32_t r) {
     const uint32_t elem = L.format == kTcBF16 ? 2u : (L.format == kTcE4M3 ? 1u : 4u);
     uint8_t* row = static_cast<uint8_t*>(L.staged) + static_cast<uint64_t>(r) * L.dim * elem;
     const uint32_t lane = threadIdx.x & 31;
@@ -147,6 +148,13 @@ __global__ void stage_queries_kernel(StageQueriesLaunch L) {
     }
 }
 
+__global__ void stage_queries_kernel(StageQueriesLaunch L) {
+    launch_dependents();
+    const uint32_t r = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
+    if (r < L.rows_alloc) stage_row(L, r);
+    wait_for_previous();
+}
+
 }  // namespace
 
 cudaError_t launch_quantize_docs(const float* vec, uint64_t rows, uint64_t valid_rows, uint32_t dim, int format,
@@ -166,8 +174,7 @@ cudaError_t launch_tile_scale_minmax(const float* scale, uint64_t tiles, float2*
 
 cudaError_t launch_stage_queries(const StageQueriesLaunch& L, cudaStream_t stream) {
     if (L.rows_alloc == 0) return cudaSuccess;
-    stage_queries_kernel<<<(L.rows_alloc + 7) / 8, 256, 0, stream>>>(L);
-    return cudaGetLastError();
+    return launch_dependent(stage_queries_kernel, dim3((L.rows_alloc + 7) / 8), 256, 0, stream, 1, L);
 }
 
 }  // namespace hss

@@ -179,6 +179,8 @@ __global__ void __launch_bounds__(kCT) cand_simt_kernel(CandLaunch L) {
     const uint32_t qg = tid >> 5;  // warp
     const uint32_t nchunks = (L.nq_list + kCQ - 1) / kCQ;
     const uint32_t kchunks = (L.dim + kCK - 1) / kCK;
+    launch_dependents();
+    wait_for_previous();
     for (uint32_t i = tid; i < L.nq_list; i += kCT) sCount[i] = 0;
 
     TileWalk walk(L.tile_begin, L.tile_step, L.tile_skip, blockIdx.x, gridDim.x);
@@ -344,8 +346,8 @@ cudaError_t launch_cand_simt(const CandLaunch& L, int num_sms, cudaStream_t stre
         return cudaErrorInvalidValue;
     const size_t smem = static_cast<size_t>(L.nq_list) * sizeof(uint32_t);
     if (L.best && L.tile_count * (kDocTile / kSimtGroup) > L.cap) return cudaErrorInvalidValue;
-    (L.best ? cand_simt_kernel<true> : cand_simt_kernel<false>)<<<L.segs, kCT, smem, stream>>>(L);
-    return cudaGetLastError();
+    return launch_dependent(L.best ? cand_simt_kernel<true> : cand_simt_kernel<false>, dim3(L.segs), kCT, smem, stream,
+                            1, L);
 }
 
 }  // namespace hss

@@ -458,18 +458,25 @@ __global__ void __launch_bounds__(64 + 256 * H, 1) tc_cand_kernel(const __grid_c
     }
     __syncthreads();
     fence_after();
+    launch_dependents();
     const uint32_t tmem = S.tmem_base;
     const uint64_t ntiles = L.tile_count;
     const long long budget = L.wait_budget > 0 ? L.wait_budget : kWaitBudget;
 
     if (warp == 0) {
         if (lane == 0) {
-            // queries once
-            mbar_expect_tx(&S.qbar, static_cast<uint32_t>(H) * kb_n * kStageBytes);
-            for (int h = 0; h < H; ++h)
-                for (uint32_t kb = 0; kb < kb_n; ++kb)
-                    tma_load_2d(qsm + (static_cast<size_t>(h) * kb_n + kb) * kStageBytes, &qry_map,
-                                static_cast<int>(kb * (128 / Fmt<F>::elem)), h * kRows, &S.qbar);
+            // queries once, when the kernel that staged them has completed; the ring is filled first (the
+            // corpus is no earlier kernel's output)
+            bool queries = false;
+            auto load_queries = [&] {
+                queries = true;
+                wait_for_previous();
+                mbar_expect_tx(&S.qbar, static_cast<uint32_t>(H) * kb_n * kStageBytes);
+                for (int h = 0; h < H; ++h)
+                    for (uint32_t kb = 0; kb < kb_n; ++kb)
+                        tma_load_2d(qsm + (static_cast<size_t>(h) * kb_n + kb) * kStageBytes, &qry_map,
+                                    static_cast<int>(kb * (128 / Fmt<F>::elem)), h * kRows, &S.qbar);
+            };
             uint32_t n = 0;
             bool held = false;
             TileWalk walk(L.tile_begin, L.tile_step, L.tile_skip, blockIdx.x, gridDim.x);
@@ -481,6 +488,7 @@ __global__ void __launch_bounds__(64 + 256 * H, 1) tc_cand_kernel(const __grid_c
                         held = true;
                         break;
                     }
+                    if (n == stages) load_queries();
                     if (!mbar_wait(&S.empty[s], ph ^ 1u, S, L.error, 1, budget)) break;
                     mbar_expect_tx(&S.full[s], static_cast<uint32_t>(stage_bytes));
                     for (uint32_t j = 0; j < G; ++j)
@@ -488,6 +496,7 @@ __global__ void __launch_bounds__(64 + 256 * H, 1) tc_cand_kernel(const __grid_c
                                     static_cast<int>((g * G + j) * (128 / Fmt<F>::elem)), y, &S.full[s]);
                 }
             }
+            if (!queries) load_queries();
             S.n_issued = n;
         }
     } else if (warp == 1) {
@@ -535,6 +544,7 @@ __global__ void __launch_bounds__(64 + 256 * H, 1) tc_cand_kernel(const __grid_c
         // the two groups of a half split its 128 doc columns (64 each). A thread owns one staged query
         // row and one column half for the whole launch: its candidate count lives in a register and
         // its candidates go to its own segment (2 per CTA) of the query's list, no atomics.
+        wait_for_previous();
         const uint32_t g = (warp - 2) / 4;
         const uint32_t half = g / 2;
         const uint32_t colh = g % 2;
@@ -724,22 +734,30 @@ __global__ void __launch_bounds__(kPairThreads, 1) tc2_cand_kernel(const __grid_
     __syncthreads();
     cluster_sync();  // both CTAs' barriers are initialised before any remote arrive
     fence_after();
+    launch_dependents();
     const uint32_t tmem = S.tmem_base;
     const uint64_t ntiles = L.tile_count;
 
     if (warp == 0) {
         if (lane == 0) {
-            if (!SQ) {
+            // as in tc_cand_kernel: the ring first, then (resident) queries; streamed ones come with the docs
+            bool queries = false;
+            auto load_queries = [&] {
+                queries = true;
+                wait_for_previous();
+                if (SQ) return;
                 mbar_expect_tx(&S.qbar, kb_n * kStageBytes);
                 for (uint32_t kb = 0; kb < kb_n; ++kb)
                     tma_load_2d(qsm + static_cast<size_t>(kb) * kStageBytes, &qry_map,
                                 static_cast<int>(kb * (128 / Fmt<F>::elem)), static_cast<int>(rank * kRows), &S.qbar);
-            }
+            };
+            if (SQ) load_queries();
             uint32_t n = 0, s = 0, ph = 0;  // stages issued; ring slot and phase of the next
             TileWalk walk(L.tile_begin, L.tile_step, L.tile_skip, pair, npairs);
             for (uint64_t it = pair; it < ntiles && !S.abort; it += npairs, walk.advance()) {
                 const int y = static_cast<int>(walk.tile() * 2 * kRows + rank * kRows);
                 for (uint32_t g = 0; g < sg_n; ++g, ++n, s = s + 1 == stages ? 0 : s + 1, ph ^= s == 0 ? 1u : 0u) {
+                    if (!SQ && n == stages) load_queries();
                     if (!pair_wait<F>(&S.empty[s], ph ^ 1u, S, L.error, 1, false)) break;
                     unsigned char* st = ring + static_cast<size_t>(s) * kStage;
                     mbar_expect_tx(&S.full[s], static_cast<uint32_t>(kStage));
@@ -755,6 +773,7 @@ __global__ void __launch_bounds__(kPairThreads, 1) tc2_cand_kernel(const __grid_
                     }
                 }
             }
+            if (!queries) load_queries();
             S.n_issued = n;
         }
     } else if (warp == 1) {
@@ -820,6 +839,7 @@ __global__ void __launch_bounds__(kPairThreads, 1) tc2_cand_kernel(const __grid_
         // Epilogue: warp w reads TMEM lanes 32 (w % 4) .. +31 (query rows) and doc columns
         // [64 g, 64 g + 64) of the 256, g = (w - 2) / 4. A thread owns one query row and one 64-doc
         // column group for the whole launch: candidates go to its own list segment, no atomics.
+        wait_for_previous();
         const uint32_t g = (warp - 2) / 4;
         const uint32_t sub = warp & 3u;
         const uint32_t row = rank * 128u + sub * 32u + lane;
@@ -952,19 +972,7 @@ cudaError_t launch_tc2_typed(const TcCandLaunch& L, const CUtensorMap& dmap, con
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          static_cast<int>(kTcSmemCeiling));
     if (e != cudaSuccess) return e;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(L.ctas, 1, 1);
-    cfg.blockDim = dim3(kPairThreads, 1, 1);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, kernel, dmap, qmap, L);
+    return launch_dependent(kernel, dim3(L.ctas), kPairThreads, smem, stream, 2, dmap, qmap, L);
 }
 
 template <int F>
@@ -975,8 +983,7 @@ cudaError_t launch_tc1_typed(const TcCandLaunch& L, const CUtensorMap& dmap, con
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          static_cast<int>(kTcSmemCeiling));
     if (e != cudaSuccess) return e;
-    kernel<<<L.ctas, 64 + 256, smem, stream>>>(dmap, qmap, L);
-    return cudaGetLastError();
+    return launch_dependent(kernel, dim3(L.ctas), 64 + 256, smem, stream, 1, dmap, qmap, L);
 }
 
 constexpr size_t kSmemBudget = 232448;  // dynamic shared memory of one CTA

@@ -474,6 +474,8 @@ __global__ void __launch_bounds__(NT, 1024 / NT) sample_threshold_kernel(SampleT
     extern __shared__ __align__(16) unsigned char smem_raw[];
     HistSmem& S = *reinterpret_cast<HistSmem*>(smem_raw);
     float* cs = reinterpret_cast<float*>(smem_raw + sizeof(HistSmem));
+    launch_dependents();
+    wait_for_previous();
     const uint32_t qi = L.qlist ? L.qlist[blockIdx.x] : blockIdx.x;
     const uint32_t k = L.topk[qi];
     const uint32_t* counts = L.count + static_cast<uint64_t>(qi) * kMaxCandSegs;
@@ -568,6 +570,8 @@ __global__ void __launch_bounds__(NT, 1024 / NT) maxima_threshold_kernel(MaximaT
     extern __shared__ __align__(16) unsigned char smem_raw[];
     HistSmem& S = *reinterpret_cast<HistSmem*>(smem_raw);
     float4* cs = reinterpret_cast<float4*>(smem_raw + sizeof(HistSmem));
+    launch_dependents();
+    wait_for_previous();
     const uint32_t qi = L.qlist ? L.qlist[blockIdx.x] : blockIdx.x;
     const uint32_t k = L.topk[qi];
     const float eps_s = L.eps_sample[qi], eps_m = L.eps_main[qi];
@@ -679,6 +683,8 @@ __global__ void __launch_bounds__(NT, NT == kSelT ? 2 : 1) select_topk_kernel(Se
     float* sq = reinterpret_cast<float*>(smem_raw + sizeof(SelectSmem));
     float* cs = reinterpret_cast<float*>(smem_raw + select_cand_offset(L.dim));
     uint32_t* surv = S.hist;  // survivors' locations: after the last digit
+    launch_dependents();
+    wait_for_previous();
     const uint32_t qi = L.qlist ? L.qlist[blockIdx.x] : blockIdx.x;
     const uint32_t tid = threadIdx.x;
     const uint32_t k = L.topk[qi];
@@ -909,6 +915,7 @@ __device__ __forceinline__ uint64_t agg_word(const uint64_t* bits, uint64_t w, u
 // Kept docs of each block of kAggDocs docs, one warp per block.
 __global__ void __launch_bounds__(256) aggregate_count_kernel(const uint64_t* __restrict__ bits, uint32_t n,
                                                               uint32_t nb, uint32_t* __restrict__ block_count) {
+    launch_dependents();
     const uint32_t b = blockIdx.x * 8u + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (b >= nb) return;
     uint32_t c = 0;
@@ -923,6 +930,8 @@ __global__ void __launch_bounds__(256) aggregate_count_kernel(const uint64_t* __
 __global__ void __launch_bounds__(1024) aggregate_scan_kernel(uint32_t* __restrict__ block_count, uint32_t nb) {
     __shared__ uint32_t warp_tot[32];
     __shared__ uint32_t carry;
+    launch_dependents();
+    wait_for_previous();
     if (threadIdx.x == 0) carry = 0;
     __syncthreads();
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -967,6 +976,8 @@ __global__ void __launch_bounds__(kAggT) aggregate_scatter_kernel(const uint64_t
     __shared__ uint32_t wsum[kAggT / 32];
     __shared__ uint32_t woff[kAggWords];
     __shared__ uint64_t wbits[kAggWords];
+    launch_dependents();
+    wait_for_previous();
     const uint32_t t = threadIdx.x, lane = t & 31, warp = t >> 5, b = blockIdx.x;
     // kept docs before this block: this thread's share of them
     uint32_t before = 0;
@@ -1059,6 +1070,7 @@ __global__ void __launch_bounds__(kST) topk_op_kernel(const float* __restrict__ 
     SelectSmem& S = *reinterpret_cast<SelectSmem*>(smem_raw);
     cg::cluster_group cluster = cg::this_cluster();
     const uint32_t C = cluster.num_blocks(), rank = cluster.block_rank(), t = threadIdx.x;
+    wait_for_previous();
     const uint32_t n = *count;
     const uint32_t kq = min(k, n);
     uint32_t m;  // keys to sort
@@ -1182,9 +1194,14 @@ __global__ void __launch_bounds__(kST) topk_op_kernel(const float* __restrict__ 
 __global__ void query_eps_kernel(const float* __restrict__ qry, const uint32_t* __restrict__ qlist, uint32_t nq,
                                  uint32_t dim, float max_norm, double c_main, double c_sample,
                                  float* __restrict__ eps_main, float* __restrict__ eps_sample) {
+    // beside the batch's filter, as stage_queries_kernel
+    launch_dependents();
     const uint32_t r = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
     const uint32_t lane = threadIdx.x & 31;
-    if (r >= nq) return;
+    if (r >= nq) {
+        wait_for_previous();
+        return;
+    }
     const uint32_t q = qlist ? qlist[r] : r;
     double s = 0.0;
     for (uint32_t d = lane; d < dim; d += 32) {
@@ -1198,6 +1215,7 @@ __global__ void query_eps_kernel(const float* __restrict__ qry, const uint32_t* 
         eps_main[q] = __double2float_ru(c_main * base + 1e-30);
         eps_sample[q] = __double2float_ru(c_sample * base + 1e-30);
     }
+    wait_for_previous();
 }
 
 // Opts a kernel into more than 48 KB of dynamic shared memory, always to the same ceiling: searchers
@@ -1231,8 +1249,7 @@ cudaError_t launch_sample_threshold(const SampleThresholdLaunch& L, cudaStream_t
     auto kernel = wide ? sample_threshold_kernel<kST> : sample_threshold_kernel<kSelT>;
     cudaError_t e = set_smem(kernel, smem);
     if (e != cudaSuccess) return e;
-    kernel<<<L.nq_list, wide ? kST : kSelT, smem, stream>>>(L);
-    return cudaGetLastError();
+    return launch_dependent(kernel, dim3(L.nq_list), wide ? kST : kSelT, smem, stream, 1, L);
 }
 
 cudaError_t launch_maxima_threshold(const MaximaThresholdLaunch& L, cudaStream_t stream) {
@@ -1244,8 +1261,7 @@ cudaError_t launch_maxima_threshold(const MaximaThresholdLaunch& L, cudaStream_t
     auto kernel = wide ? maxima_threshold_kernel<kST> : maxima_threshold_kernel<kSelT>;
     cudaError_t e = set_smem(kernel, smem);
     if (e != cudaSuccess) return e;
-    kernel<<<L.nq_list, wide ? kST : kSelT, smem, stream>>>(L);
-    return cudaGetLastError();
+    return launch_dependent(kernel, dim3(L.nq_list), wide ? kST : kSelT, smem, stream, 1, L);
 }
 
 cudaError_t launch_select_topk(const SelectLaunch& L, cudaStream_t stream) {
@@ -1256,16 +1272,14 @@ cudaError_t launch_select_topk(const SelectLaunch& L, cudaStream_t stream) {
     auto kernel = wide ? select_topk_kernel<kST, kFastLarge> : select_topk_kernel<kSelT, kFast>;
     cudaError_t e = set_smem(kernel, smem);
     if (e != cudaSuccess) return e;
-    kernel<<<L.nq_list, wide ? kST : kSelT, smem, stream>>>(L);
-    return cudaGetLastError();
+    return launch_dependent(kernel, dim3(L.nq_list), wide ? kST : kSelT, smem, stream, 1, L);
 }
 
 cudaError_t launch_query_eps(const float* qry, const uint32_t* qlist, uint32_t nq, uint32_t dim, float max_norm,
                              double c_main, double c_sample, float* eps_main, float* eps_sample, cudaStream_t stream) {
     if (nq == 0) return cudaSuccess;
-    query_eps_kernel<<<(nq + 7) / 8, 256, 0, stream>>>(qry, qlist, nq, dim, max_norm, c_main, c_sample, eps_main,
-                                                       eps_sample);
-    return cudaGetLastError();
+    return launch_dependent(query_eps_kernel, dim3((nq + 7) / 8), 256, 0, stream, 1, qry, qlist, nq, dim, max_norm,
+                            c_main, c_sample, eps_main, eps_sample);
 }
 
 size_t aggregate_workspace_bytes(uint32_t n) {
@@ -1285,20 +1299,18 @@ cudaError_t launch_aggregate(const uint64_t* bits, const float* scores, const ui
     const uint32_t nb = static_cast<uint32_t>((static_cast<uint64_t>(n) + kAggDocs - 1) / kAggDocs);
     if (nb == 0) return cudaMemsetAsync(total, 0, sizeof(uint32_t), stream);
     if (n <= kOwnDocs) {
-        aggregate_scatter_kernel<kAggOwn>
-            <<<nb, kAggT, 0, stream>>>(bits, scores, loc_in, n, workspace, out_scores, out_loc, total);
-        return cudaGetLastError();
+        return launch_dependent(aggregate_scatter_kernel<kAggOwn>, dim3(nb), kAggT, 0, stream, 1, bits, scores, loc_in, n,
+                                workspace, out_scores, out_loc, total);
     }
     aggregate_count_kernel<<<(nb + 7) / 8, 256, 0, stream>>>(bits, n, nb, workspace);
     if (nb <= kSumBlocks) {
-        aggregate_scatter_kernel<kAggSums>
-            <<<nb, kAggT, 0, stream>>>(bits, scores, loc_in, n, workspace, out_scores, out_loc, total);
-        return cudaGetLastError();
+        return launch_dependent(aggregate_scatter_kernel<kAggSums>, dim3(nb), kAggT, 0, stream, 1, bits, scores, loc_in,
+                                n, workspace, out_scores, out_loc, total);
     }
-    aggregate_scan_kernel<<<1, 1024, 0, stream>>>(workspace, nb);
-    aggregate_scatter_kernel<kAggScanned>
-        <<<nb, kAggT, 0, stream>>>(bits, scores, loc_in, n, workspace, out_scores, out_loc, total);
-    return cudaGetLastError();
+    cudaError_t e = launch_dependent(aggregate_scan_kernel, dim3(1), 1024, 0, stream, 1, workspace, nb);
+    if (e != cudaSuccess) return e;
+    return launch_dependent(aggregate_scatter_kernel<kAggScanned>, dim3(nb), kAggT, 0, stream, 1, bits, scores, loc_in, n,
+                            workspace, out_scores, out_loc, total);
 }
 
 // Scratch of the allocation-free aggregator: one word per 1,024 docs, kAggStaticBlocks of them (64 KB,
@@ -1353,9 +1365,8 @@ cudaError_t launch_topk_op(const float* scores, const uint32_t* locs, const uint
     cfg.attrs = attr;
     cfg.numAttrs = 1;
     const unsigned size = topk_cluster(cfg, attr[0]);
-    attr[0].val.clusterDim.x = size;
-    cfg.gridDim = dim3(size, 1, 1);
-    return cudaLaunchKernelEx(&cfg, topk_op_kernel, scores, locs, count, k, out_scores, out_locs, out_count);
+    return launch_dependent(topk_op_kernel, dim3(size), kST, smem, stream, size, scores, locs, count, k, out_scores,
+                            out_locs, out_count);
 }
 
 
