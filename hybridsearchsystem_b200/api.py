@@ -455,7 +455,7 @@ class ThresholdModel:
         return loss.value
 
     def gradients(self, d_x, d_t, batch, stream=0):
-        g = np.zeros(self.param_count, np.float32)
+        g = np.empty(self.param_count, np.float32)  # written whole
         loss = ctypes.c_float()
         check(_lib.load().hss_model_gradients(self._h, d_x, d_t, batch, _np_ptr(g), ctypes.byref(loss), stream))
         return g, loss.value

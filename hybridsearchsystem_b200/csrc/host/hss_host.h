@@ -399,7 +399,7 @@ class ThresholdModel {
     size_t OffB3() const { return OffW3() + m_h; }
     bool Reserve(uint32_t batch);
     cudaError_t TrainPass(const float* dX, const float* dT, uint32_t B, cudaStream_t s);
-    int Finish(cudaError_t e, float* hLoss, uint32_t B, cudaStream_t s);
+    int Finish(cudaError_t e, float* hGrad, float* hLoss, uint32_t B, cudaStream_t s);
 
     int32_t m_deviceId;
     uint32_t m_din, m_h;
@@ -411,6 +411,8 @@ class ThresholdModel {
     uint32_t m_cap = 0;
     float *m_dP = nullptr, *m_dG = nullptr, *m_dM = nullptr, *m_dV = nullptr;
     float *m_dZ1 = nullptr, *m_dA1 = nullptr, *m_dZ2 = nullptr, *m_dA2 = nullptr;
+    float* m_hPin = nullptr;  // pinned: gradient and loss terms on their way out
+    size_t m_pinFloats = 0;
     float *m_dDy = nullptr, *m_dD1 = nullptr, *m_dD2 = nullptr, *m_dSq = nullptr;
 };
 
@@ -534,8 +536,8 @@ class FullRecallSearcher {
 
    private:
     struct ArenaLayout {
-        size_t bits, candScore, candLoc, work, sampScore, sampLoc, stage, queries, outScore, outId, outCount, stats,
-            features, predictions, staged, qScale, error, total;
+        size_t bits, candScore, candLoc, work, sampScore, sampLoc, stage, queries, out, stats, features, predictions,
+            staged, qScale, total;
         size_t stageBytes;
         uint32_t sampCap;
     };
@@ -646,12 +648,9 @@ class FullRecallSearcher {
     size_t m_stageBytes = 0;
     uint8_t* m_hStage = nullptr;  // pinned host copy
     float* m_dQueries = nullptr;  // for BatchSearch
-    float* m_dOutScore = nullptr;
-    int64_t* m_dOutId = nullptr;
-    uint32_t* m_dOutCount = nullptr;
-    float* m_hOutScore = nullptr;
-    int64_t* m_hOutId = nullptr;
-    uint32_t* m_hOutCount = nullptr;
+    uint8_t* m_dOut = nullptr;  // BatchSearch's packed results
+    uint8_t* m_hOut = nullptr;  // their pinned host copy
+    float* m_hQueries = nullptr;  // pinned: BatchSearch's query vectors
     // tensor-core pass
     int m_tcFormat = -1;  // TcFormat, or -1 for the SIMT pass
     uint32_t m_tcKblocks = 0;

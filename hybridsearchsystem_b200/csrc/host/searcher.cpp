@@ -84,11 +84,11 @@ StageLayout MakeLayout(uint32_t B) {
     L.theta = take(B * 4ull);
     L.thetaPr = take(B * 4ull);  // proven thresholds beside predicted ones (learned threshold)
     L.qlist = take(B * 4ull);
-    L.errWord = take(4);  // host copy of the tensor-core pass's error bits
-    L.counters = at;  // zeroed per batch: passCount, status and theta1
+    L.counters = at;  // zeroed per batch: passCount, status, theta1 and errWord
     L.passCount = take(B * 4ull);
     L.status = take(B * 4ull);
     L.theta1 = take(B * 4ull);  // the doc sample's proven thresholds, copied out with the statuses
+    L.errWord = take(4);  // the tensor-core pass's error bits, likewise
     // the programs, then their operand rows (one host-to-device copy of [0, prog + words))
     L.prog = take(static_cast<size_t>(B) * (kMaxProgram + kMaxOperands) * 4ull);
     L.opnd = take(static_cast<size_t>(B) * kMaxOperands * 4ull);  // host only: operands while programs are laid out
@@ -121,6 +121,8 @@ uint32_t SampleCap(const DataTable& T, const SearcherConfig& c) {
                     128ull * kMaxCandSegs,
                 4));  // a row of group maxima starts on 16 bytes
 }
+// BatchSearch's packed results at most: scores, ids (on 8 bytes) and counts of a full batch.
+size_t OutBytes(uint32_t B) { return static_cast<size_t>(B) * (kMaxTopK * 12ull + 4) + 8; }
 }  // namespace
 
 // Byte offsets of every device buffer of a searcher inside its arena (256-byte aligned).
@@ -144,16 +146,13 @@ FullRecallSearcher::ArenaLayout FullRecallSearcher::Layout(const DataTable& T, c
     A.stageBytes = MakeLayout(c.maxBatch).total;
     A.stage = take(A.stageBytes);
     A.queries = take(B * dim * 4);
-    A.outScore = take(B * kMaxTopK * 4ull);
-    A.outId = take(B * kMaxTopK * 8ull);
-    A.outCount = take(B * 4);
+    A.out = take(OutBytes(c.maxBatch));
     A.stats = take(B * static_cast<uint64_t>(kSampleStats) * sizeof(float));
     A.features = take(B * (dim + T.PostingRows() + kFeatureTail) * sizeof(float));
     A.predictions = take(B * sizeof(float));
     if (c.method != ScoreMethod::SIMT_FP32) {
         A.staged = take(256ull * dim * 4);
         A.qScale = take(256 * sizeof(float));
-        A.error = take(sizeof(int32_t));
     }
     A.total = at;
     return A;
@@ -176,7 +175,7 @@ FullRecallSearcher::FullRecallSearcher(int32_t deviceId, std::shared_ptr<DataTab
 FullRecallSearcher::~FullRecallSearcher() {
     cudaSetDevice(m_deviceId);
     if (m_arenaOwned && m_dArena) cudaFree(m_dArena);
-    void* hptrs[] = {m_hStage, m_hOutScore, m_hOutId, m_hOutCount, m_hThetaA};
+    void* hptrs[] = {m_hStage, m_hOut, m_hQueries, m_hThetaA};
     for (void* p : hptrs)
         if (p) cudaFreeHost(p);
     for (auto& e : m_ev)
@@ -242,9 +241,7 @@ bool FullRecallSearcher::Allocate(void* dArena, size_t arenaBytes) {
     m_dSampLoc = reinterpret_cast<uint32_t*>(W + A.sampLoc);
     m_dStage = W + A.stage;
     m_dQueries = reinterpret_cast<float*>(W + A.queries);
-    m_dOutScore = reinterpret_cast<float*>(W + A.outScore);
-    m_dOutId = reinterpret_cast<int64_t*>(W + A.outId);
-    m_dOutCount = reinterpret_cast<uint32_t*>(W + A.outCount);
+    m_dOut = W + A.out;
     m_dStats = reinterpret_cast<float*>(W + A.stats);
     m_dX = reinterpret_cast<float*>(W + A.features);
     m_dYp = reinterpret_cast<float*>(W + A.predictions);
@@ -255,9 +252,8 @@ bool FullRecallSearcher::Allocate(void* dArena, size_t arenaBytes) {
     const StageLayout L = MakeLayout(static_cast<uint32_t>(B));
     float* negInf = reinterpret_cast<float*>(m_hStage + L.negInf);
     for (uint64_t i = 0; i < B; ++i) negInf[i] = -INFINITY;
-    if (!ck(cudaMallocHost(&m_hOutScore, B * kMaxTopK * 4ull), "cudaMallocHost results")) return false;
-    if (!ck(cudaMallocHost(&m_hOutId, B * kMaxTopK * 8ull), "cudaMallocHost results")) return false;
-    if (!ck(cudaMallocHost(&m_hOutCount, B * 4ull), "cudaMallocHost results")) return false;
+    if (!ck(cudaMallocHost(&m_hOut, OutBytes(m_cfg.maxBatch)), "cudaMallocHost results")) return false;
+    if (!ck(cudaMallocHost(&m_hQueries, B * m_table->GetDimension() * 4ull), "cudaMallocHost queries")) return false;
     if (!ck(cudaMallocHost(&m_hThetaA, B * sizeof(float)), "cudaMallocHost thresholds")) return false;
     for (auto& e : m_ev)
         if (!ck(cudaEventCreate(&e), "cudaEventCreate")) return false;
@@ -265,8 +261,7 @@ bool FullRecallSearcher::Allocate(void* dArena, size_t arenaBytes) {
         const uint32_t dim = m_table->GetDimension();
         m_dStaged = W + A.staged;
         m_dQScale = reinterpret_cast<float*>(W + A.qScale);
-        m_dError = reinterpret_cast<int32_t*>(W + A.error);
-        if (!ck(cudaMemset(m_dError, 0, sizeof(int32_t)), "cudaMemset error word")) return false;
+        m_dError = reinterpret_cast<int32_t*>(m_dStage + L.errWord);
         if (!make_tc_map(&m_docMap, m_tcFormat, m_table->DeviceRows(m_tcFormat), m_table->GetTileNum() * 128, dim) ||
             !make_tc_map(&m_qryMap, m_tcFormat, m_dStaged, 256, dim)) {
             m_err = "cuTensorMapEncodeTiled failed";
@@ -1096,9 +1091,8 @@ int FullRecallSearcher::EnqueueAttempt(uint32_t nq, const BatchInputs& in, float
     if (m_timing) Ck(cudaEventRecord(m_ev[4], stream));
     // the statuses that decide re-runs (and the tensor-core pass's error bits), on the host when
     // m_evStatus (recorded by the caller) completes
-    // one copy for the statuses and theta_1 (theta1 follows status in the staging layout)
-    Ck(cudaMemcpyAsync(H + SL.status, dStatus, (SL.theta1 - SL.status) + nq * 4ull, cudaMemcpyDeviceToHost, stream));
-    if (m_tcFormat >= 0) Ck(cudaMemcpyAsync(H + SL.errWord, m_dError, 4, cudaMemcpyDeviceToHost, stream));
+    // one copy for the statuses, theta_1 and the error bits (one after the other in the staging layout)
+    Ck(cudaMemcpyAsync(H + SL.status, dStatus, SL.errWord - SL.status + 4, cudaMemcpyDeviceToHost, stream));
     // the model's thresholds (m_dYp is not written after the prediction)
     if (learned) Ck(cudaMemcpyAsync(m_hThetaA, m_dYp, nq * 4ull, cudaMemcpyDeviceToHost, stream));
     return 0;
@@ -1313,22 +1307,35 @@ bool FullRecallSearcher::BatchSearch(std::vector<std::shared_ptr<FullRecallResul
         }
         cudaStream_t stream = nullptr;
         if (cudaSetDevice(m_deviceId) != cudaSuccess) return finish(false);
-        if (cudaMemcpyAsync(m_dQueries, m_queryVectors.data() + static_cast<size_t>(b0) * dim, nb * dim * 4ull,
-                            cudaMemcpyHostToDevice, stream) != cudaSuccess)
+        // the batch's results lie packed in the arena's result block (scores, ids, counts; rows of the
+        // largest K), so that one copy, queued behind the batch, brings them
+        uint32_t stride = 1;
+        for (uint32_t i = 0; i < nb; ++i)
+            stride = std::max(stride, std::min(m_topKs[b0 + i], static_cast<uint32_t>(kMaxTopK)));
+        const size_t idOff = AlignUp(static_cast<size_t>(nb) * stride * 4, 8);
+        const size_t countOff = idOff + static_cast<size_t>(nb) * stride * 8, bytes = countOff + nb * 4ull;
+        std::memcpy(m_hQueries, m_queryVectors.data() + static_cast<size_t>(b0) * dim, nb * dim * 4ull);
+        if (cudaMemcpyAsync(m_dQueries, m_hQueries, nb * dim * 4ull, cudaMemcpyHostToDevice, stream) != cudaSuccess)
             return finish(false);
-        const int rc = SearchDevice(m_dQueries, nb, ptrs.data(), m_topKs.data() + b0, m_dOutScore, m_dOutId,
-                                    m_dOutCount, kMaxTopK, stream);
-        if (rc < 0) return finish(false);
-        cudaMemcpyAsync(m_hOutCount, m_dOutCount, nb * 4ull, cudaMemcpyDeviceToHost, stream);
-        cudaMemcpyAsync(m_hOutScore, m_dOutScore, nb * kMaxTopK * 4ull, cudaMemcpyDeviceToHost, stream);
-        cudaMemcpyAsync(m_hOutId, m_dOutId, nb * kMaxTopK * 8ull, cudaMemcpyDeviceToHost, stream);
-        if (cudaStreamSynchronize(stream) != cudaSuccess) return finish(false);
+        int rc = SearchEnqueue(m_dQueries, nb, ptrs.data(), m_topKs.data() + b0, reinterpret_cast<float*>(m_dOut),
+                               reinterpret_cast<int64_t*>(m_dOut + idOff), reinterpret_cast<uint32_t*>(m_dOut + countOff),
+                               stride, stream);
+        if (rc == 0 && m_b.pending) {
+            cudaMemcpyAsync(m_hOut, m_dOut, bytes, cudaMemcpyDeviceToHost, stream);
+            rc = SearchFinish();
+            // queries that were re-run have changed since
+            if (rc >= 0 && m_times.retries > 0) cudaMemcpyAsync(m_hOut, m_dOut, bytes, cudaMemcpyDeviceToHost, stream);
+        }
+        if (cudaStreamSynchronize(stream) != cudaSuccess || rc < 0) return finish(false);
+        const float* outScore = reinterpret_cast<const float*>(m_hOut);
+        const int64_t* outId = reinterpret_cast<const int64_t*>(m_hOut + idOff);
+        const uint32_t* outCount = reinterpret_cast<const uint32_t*>(m_hOut + countOff);
         for (uint32_t i = 0; i < nb; ++i) {
             auto r = std::make_shared<FullRecallResult>();
             r->isMultiShard = isMultiShard;
-            const uint32_t c = m_lastStatus[i] ? 0u : m_hOutCount[i];
-            const float* sc = m_hOutScore + static_cast<size_t>(i) * kMaxTopK;
-            const int64_t* id = m_hOutId + static_cast<size_t>(i) * kMaxTopK;
+            const uint32_t c = m_lastStatus[i] ? 0u : outCount[i];
+            const float* sc = outScore + static_cast<size_t>(i) * stride;
+            const int64_t* id = outId + static_cast<size_t>(i) * stride;
             for (uint32_t j = 0; j < c; ++j) {
                 if (isMultiShard) {
                     ScoreWithIndex s(sc[j], static_cast<uint32_t>(id[j] - static_cast<int64_t>(m_table->GetConfig().docOffset)));

@@ -58,6 +58,7 @@ ThresholdModel::~ThresholdModel() {
     float* bufs[] = {m_dP, m_dG, m_dM, m_dV, m_dZ1, m_dA1, m_dZ2, m_dA2, m_dDy, m_dD1, m_dD2, m_dSq};
     for (float* b : bufs)
         if (b) cudaFree(b);
+    if (m_hPin) cudaFreeHost(m_hPin);
 }
 
 bool ThresholdModel::Reserve(uint32_t batch) {
@@ -110,20 +111,29 @@ cudaError_t ThresholdModel::TrainPass(const float* dX, const float* dT, uint32_t
     return launch_train_gradients(L, s);
 }
 
-int ThresholdModel::Finish(cudaError_t e, float* hLoss, uint32_t B, cudaStream_t s) {
-    std::vector<float> sq;
-    if (e == cudaSuccess && hLoss) {
-        sq.resize(B);
-        e = cudaMemcpyAsync(sq.data(), m_dSq, B * sizeof(float), cudaMemcpyDeviceToHost, s);
+// The host copies of a training pass (the gradient where asked for, the loss terms), through one pinned
+// buffer: a copy into the caller's pageable memory waits for the pass and is staged by the driver.
+int ThresholdModel::Finish(cudaError_t e, float* hGrad, float* hLoss, uint32_t B, cudaStream_t s) {
+    const size_t grads = hGrad ? m_np : 0, terms = hLoss ? B : 0;
+    if (e == cudaSuccess && grads + terms > m_pinFloats) {
+        if (m_hPin) cudaFreeHost(m_hPin);
+        m_hPin = nullptr;
+        m_pinFloats = 0;
+        e = cudaMallocHost(&m_hPin, (grads + terms) * sizeof(float));
+        if (e == cudaSuccess) m_pinFloats = grads + terms;
     }
+    if (e == cudaSuccess && terms)
+        e = cudaMemcpyAsync(m_hPin + grads, m_dSq, terms * sizeof(float), cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess && grads) e = cudaMemcpyAsync(m_hPin, m_dG, grads * sizeof(float), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     if (e != cudaSuccess) {
         m_err = cudaGetErrorString(e);
         return -2;
     }
+    if (hGrad) std::memcpy(hGrad, m_hPin, grads * sizeof(float));
     if (hLoss) {
         double l = 0;
-        for (float v : sq) l += v;
+        for (size_t i = 0; i < terms; ++i) l += m_hPin[grads + i];
         *hLoss = static_cast<float>(l / B);
     }
     return 0;
@@ -147,8 +157,7 @@ int ThresholdModel::Gradients(const float* dX, const float* dT, uint32_t B, floa
     if (!m_ok || B == 0) return -1;
     if (cudaSetDevice(m_deviceId) != cudaSuccess || !Reserve(B)) return -1;
     cudaError_t e = TrainPass(dX, dT, B, s);
-    if (e == cudaSuccess && hGrad) e = cudaMemcpyAsync(hGrad, m_dG, m_np * sizeof(float), cudaMemcpyDeviceToHost, s);
-    return Finish(e, hLoss, B, s);
+    return Finish(e, hGrad, hLoss, B, s);
 }
 
 int ThresholdModel::TrainStep(const float* dX, const float* dT, uint32_t B, float lr, float* hLoss, cudaStream_t s) {
@@ -157,7 +166,7 @@ int ThresholdModel::TrainStep(const float* dX, const float* dT, uint32_t B, floa
     cudaError_t e = TrainPass(dX, dT, B, s);
     if (e == cudaSuccess)
         e = launch_adam(m_dP, m_dG, m_dM, m_dV, static_cast<int64_t>(m_np), lr, 0.9f, 0.999f, 1e-8f, ++m_step, s);
-    return Finish(e, hLoss, B, s);
+    return Finish(e, nullptr, hLoss, B, s);
 }
 
 int ThresholdModel::SetQuantile(float tau) {
