@@ -153,159 +153,213 @@ cudaError_t launch_exact_tile(const float* qry, const float* docs, float* out, u
 }
 
 // ---------------------------------------------------------------------------------------------
-// SIMT candidate pass.
-// 256 threads = 32 doc groups (4 docs each) x 8 query groups (8 queries each); a warp is one query
-// group, so the epilogue's per-query ballots are warp-uniform.
+// SIMT candidate pass, bound by the FP32 pipe: 2 nq n dim flop at 74 TFLOP/s (64 queries x 1M docs x 128:
+// 220 us). A CTA of 8 warps scores 128 docs for 8 TQ queries at a time: a warp is one group of TQ queries
+// (so the epilogue's per-query ballots are warp-uniform), a lane has docs lane + 32 r, r < 4. Rows are
+// staged as they lie (cp.async, three stages of 32 dims, a pitch of 36 floats: the 16-byte reads of 8
+// neighbouring rows fall on distinct banks) and products are taken two dims at a time by packed
+// multiply-adds: an accumulator holds the even and the odd dims' sums, added at the end (the pass's error
+// bound holds for any order of summation). A packed instruction takes the pipe as long as two plain ones
+// but one issue slot (in registers alone 4 x 8 outputs run at 63 TFLOP/s this way, 44 with plain
+// multiply-adds). 64 queries x 1M docs x 128: 670 us with 4-byte transposed stores, one stage and plain
+// multiply-adds, 455 us now (two stages with two barriers each: 468; 16 queries a thread in CTAs of 4 warps:
+// 485, too few warps to hide the reads).
 // ---------------------------------------------------------------------------------------------
-constexpr int kCT = 256;
-constexpr int kCQ = 64;   // queries per chunk
-constexpr int kCK = 32;   // dims per smem stage
+constexpr int kCT = 256;           // threads: 8 warps
+constexpr uint32_t kCWarps = kCT / 32;
+constexpr int kCK = 32;            // dims per stage
+constexpr int kCPitch = kCK + 4;
 static_assert(kSimtGroup == 4, "a thread's docs of a tile are one group");
-constexpr int kDPad = kDocTile + 4;
-constexpr int kQPad = kCQ + 4;
+
+__device__ __forceinline__ void fma2(unsigned long long& acc, unsigned long long a, unsigned long long b) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
+}
+
+template <int TQ>
+struct SimtTile {
+    static constexpr uint32_t QT = kCWarps * TQ;  // queries per chunk
+    static constexpr uint32_t stage_floats = (kDocTile + QT) * kCPitch;
+    // three stages, four chunks' filter words; then the queries' counts and thresholds
+    static constexpr size_t fixed = 3 * stage_floats * sizeof(float) + 4 * QT * 16;
+};
 
 // MAXIMA: the pass writes group maxima (CandLaunch::best) instead of candidates.
-template <bool MAXIMA>
-__global__ void __launch_bounds__(kCT) cand_simt_kernel(CandLaunch L) {
-    extern __shared__ uint32_t sCount[];  // [nq_list] candidates this CTA found per query
-    __shared__ __align__(16) float sD[kCK][kDPad];
-    __shared__ __align__(16) float sQ[kCK][kQPad];
-    __shared__ uint64_t sBits[kCQ][2];
-    __shared__ float sTheta[kCQ];
-    __shared__ uint32_t sQi[kCQ];
+template <int TQ, bool MAXIMA>
+__global__ void __launch_bounds__(kCT, 2) cand_simt_kernel(CandLaunch L) {
+    using T = SimtTile<TQ>;
+    extern __shared__ __align__(16) unsigned char simt_smem[];
+    float* ring = reinterpret_cast<float*>(simt_smem);
+    uint4* sBits = reinterpret_cast<uint4*>(ring + 3 * T::stage_floats);  // [4][QT]: 128 docs' filter bits
+    uint32_t* sCount = reinterpret_cast<uint32_t*>(sBits + 4 * T::QT);  // [nq_list] candidates found per query
+    float* sTheta = reinterpret_cast<float*>(sCount + L.nq_list);
 
-    const uint32_t tid = threadIdx.x;
-    const uint32_t dg = tid & 31;  // lane
-    const uint32_t qg = tid >> 5;  // warp
-    const uint32_t nchunks = (L.nq_list + kCQ - 1) / kCQ;
+    const uint32_t tid = threadIdx.x, lane = tid & 31, qg = tid >> 5;
+    const uint32_t nchunks = (L.nq_list + T::QT - 1) / T::QT;
     const uint32_t kchunks = (L.dim + kCK - 1) / kCK;
     launch_dependents();
     wait_for_previous();
-    for (uint32_t i = tid; i < L.nq_list; i += kCT) sCount[i] = 0;
+    for (uint32_t i = tid; i < L.nq_list; i += kCT) {
+        sCount[i] = 0;
+        sTheta[i] = L.theta[L.qlist ? L.qlist[i] : i];
+    }
 
-    TileWalk walk(L.tile_begin, L.tile_step, L.tile_skip, blockIdx.x, gridDim.x);
-    for (uint64_t it = blockIdx.x; it < L.tile_count; it += gridDim.x, walk.advance()) {
-        const uint64_t tile = walk.tile();
-        const uint64_t doc0 = tile * kDocTile;
-        for (uint32_t chunk = 0; chunk < nchunks; ++chunk) {
-            float acc[4][8];
+    auto copy16 = [](void* smem, const void* gmem) {
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                         static_cast<uint32_t>(__cvta_generic_to_shared(smem))),
+                     "l"(gmem)
+                     : "memory");
+    };
+    // dims [32 kc, +32) of a tile's docs and a chunk's queries; with kc = 0 the chunk's filter words too
+    auto copy_stage = [&](uint32_t tile, uint32_t chunk, uint32_t kc, uint32_t stage, uint32_t bits) {
+        const uint32_t k0 = kc * kCK, part = tid & 7;
+        float* sd = ring + stage * T::stage_floats + (tid >> 3) * kCPitch + part * 4;
+        if (part * 4 < L.dim - k0) {
+            const float* v = L.vec + (static_cast<uint64_t>(tile) * kDocTile + (tid >> 3)) * L.dim + k0 + part * 4;
+#pragma unroll
+            for (uint32_t i = 0; i < kDocTile * 8 / kCT; ++i)
+                copy16(sd + i * (kCT / 8) * kCPitch, v + static_cast<uint64_t>(i * (kCT / 8)) * L.dim);
+#pragma unroll
+            for (uint32_t i = 0; i < (T::QT * 8 + kCT - 1) / kCT; ++i) {
+                const uint32_t r = (tid >> 3) + i * (kCT / 8);
+                const uint32_t li = min(chunk * T::QT + r, L.nq_list - 1);  // past the list: not emitted
+                const uint32_t qi = L.qlist ? L.qlist[li] : li;
+                if (r < T::QT)
+                    copy16(sd + (kDocTile + i * (kCT / 8)) * kCPitch,
+                           L.qry + static_cast<uint64_t>(qi) * L.dim + k0 + part * 4);
+            }
+        }
+        if (kc == 0 && tid < T::QT) {
+            const uint32_t li = min(chunk * T::QT + tid, L.nq_list - 1);
+            const uint32_t qi = L.qlist ? L.qlist[li] : li;
+            // bitmap rows and tiles are multiples of 16 bytes (segments of 128 docs)
+            copy16(sBits + bits * T::QT + tid, L.bits + static_cast<uint64_t>(qi) * L.bits_stride + tile * 2ull);
+        }
+    };
+    auto commit = [] { asm volatile("cp.async.commit_group;" ::: "memory"); };
+
+    // The it-th tile of the pass (32-bit: the launcher checks tile_walk_fits).
+    auto tile_at = [&](uint32_t it) {
+        return L.tile_skip >= 2 ? it + it / (L.tile_skip - 1) + 1
+                                : static_cast<uint32_t>(L.tile_begin) + it * static_cast<uint32_t>(L.tile_step);
+    };
+    // Stages in order, tile by tile, chunk by chunk, k by k, are copied two ahead into a ring of three. The
+    // next one to copy:
+    const uint32_t count = static_cast<uint32_t>(L.tile_count);
+    uint32_t c_it = blockIdx.x, c_chunk = 0, c_k = 0, c_stage = 0, c_bits = 0;
+    auto copy_next = [&] {
+        if (c_it < count) {
+            copy_stage(tile_at(c_it), c_chunk, c_k, c_stage, c_bits);
+            c_stage = c_stage == 2 ? 0 : c_stage + 1;
+            if (++c_k == kchunks) {
+                c_k = 0;
+                c_bits = (c_bits + 1) & 3;
+                if (++c_chunk == nchunks) {
+                    c_chunk = 0;
+                    c_it += gridDim.x;
+                }
+            }
+        }
+        commit();
+    };
+    copy_next();
+    copy_next();
+    uint32_t stage = 0, bits = 0;
+    for (uint32_t it = blockIdx.x; it < count; it += gridDim.x) {
+        const uint32_t doc0 = tile_at(it) * kDocTile;
+        for (uint32_t chunk = 0; chunk < nchunks; ++chunk, bits = (bits + 1) & 3) {
+            unsigned long long acc[4][TQ];
 #pragma unroll
             for (int r = 0; r < 4; ++r)
 #pragma unroll
-                for (int j = 0; j < 8; ++j) acc[r][j] = 0.0f;
-
-            for (uint32_t kc = 0; kc < kchunks; ++kc) {
-                __syncthreads();
-                const uint32_t k0 = kc * kCK;
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const uint32_t f = tid + kCT * i;
-                    const uint32_t doc = f >> 3, part = f & 7;
-                    const uint32_t k = k0 + part * 4;
-                    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-                    if (k < L.dim) v = *reinterpret_cast<const float4*>(L.vec + (doc0 + doc) * L.dim + k);
-                    sD[part * 4 + 0][doc] = v.x;
-                    sD[part * 4 + 1][doc] = v.y;
-                    sD[part * 4 + 2][doc] = v.z;
-                    sD[part * 4 + 3][doc] = v.w;
-                }
-#pragma unroll
-                for (int i = 0; i < 2; ++i) {
-                    const uint32_t f = tid + kCT * i;
-                    const uint32_t qq = f >> 3, part = f & 7;
-                    const uint32_t k = k0 + part * 4;
-                    const uint32_t li = chunk * kCQ + qq;
-                    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-                    if (li < L.nq_list && k < L.dim) {
-                        const uint32_t qi = L.qlist ? L.qlist[li] : li;
-                        v = *reinterpret_cast<const float4*>(L.qry + static_cast<uint64_t>(qi) * L.dim + k);
-                    }
-                    sQ[part * 4 + 0][qq] = v.x;
-                    sQ[part * 4 + 1][qq] = v.y;
-                    sQ[part * 4 + 2][qq] = v.z;
-                    sQ[part * 4 + 3][qq] = v.w;
-                }
-                if (kc == 0 && tid < kCQ) {
-                    const uint32_t li = chunk * kCQ + tid;
-                    uint64_t b0 = 0, b1 = 0;
-                    float th = INFINITY;
-                    uint32_t qi = 0xffffffffu;
-                    if (li < L.nq_list) {
-                        qi = L.qlist ? L.qlist[li] : li;
-                        const uint64_t* brow = L.bits + static_cast<uint64_t>(qi) * L.bits_stride + tile * 2;
-                        b0 = brow[0];
-                        b1 = brow[1];
-                        th = L.theta[qi];
-                    }
-                    sBits[tid][0] = b0;
-                    sBits[tid][1] = b1;
-                    sTheta[tid] = th;
-                    sQi[tid] = qi;
-                }
-                __syncthreads();
-#pragma unroll 8
-                for (int k = 0; k < kCK; ++k) {
-                    const float4 d4 = *reinterpret_cast<const float4*>(&sD[k][dg * 4]);
-                    const float4 qa = *reinterpret_cast<const float4*>(&sQ[k][qg * 8]);
-                    const float4 qb = *reinterpret_cast<const float4*>(&sQ[k][qg * 8 + 4]);
-                    const float dv[4] = {d4.x, d4.y, d4.z, d4.w};
-                    const float qv[8] = {qa.x, qa.y, qa.z, qa.w, qb.x, qb.y, qb.z, qb.w};
+                for (int j = 0; j < TQ; ++j) acc[r][j] = 0;
+            for (uint32_t kc = 0; kc < kchunks; ++kc, stage = stage == 2 ? 0 : stage + 1) {
+                asm volatile("cp.async.wait_group 1;" ::: "memory");
+                __syncthreads();  // the stage has landed; the one copied into next was read by every warp
+                copy_next();
+                const float* sd = ring + stage * T::stage_floats + lane * kCPitch;
+                const float* sq = ring + stage * T::stage_floats + (kDocTile + qg * TQ) * kCPitch;
+                const uint32_t kn = min(static_cast<uint32_t>(kCK), L.dim - kc * kCK);
+#pragma unroll 2
+                for (uint32_t k = 0; k < kn; k += 4) {
+                    ulonglong2 d[4];
 #pragma unroll
                     for (int r = 0; r < 4; ++r)
+                        d[r] = *reinterpret_cast<const ulonglong2*>(sd + r * 32 * kCPitch + k);
 #pragma unroll
-                        for (int j = 0; j < 8; ++j) acc[r][j] = fmaf(dv[r], qv[j], acc[r][j]);
+                    for (int j = 0; j < TQ; ++j) {
+                        const ulonglong2 q = *reinterpret_cast<const ulonglong2*>(sq + j * kCPitch + k);
+#pragma unroll
+                        for (int r = 0; r < 4; ++r) fma2(acc[r][j], d[r].x, q.x);
+#pragma unroll
+                        for (int r = 0; r < 4; ++r) fma2(acc[r][j], d[r].y, q.y);
+                    }
                 }
             }
 
             // Epilogue: filter bit && score >= theta -> append (score, location) to this CTA's segment
             // of the query's list (a shared-memory count per query; no global atomics).
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                const uint32_t qq = qg * 8 + j;
-                const uint32_t qi = sQi[qq];
-                if (qi == 0xffffffffu) continue;  // warp-uniform
-                const float th = sTheta[qq];
-                const uint64_t w0 = sBits[qq][0], w1 = sBits[qq][1];
-                if constexpr (MAXIMA) {
-                    float b = -INFINITY;
+            for (int j = 0; j < TQ; ++j) {
+                const uint32_t li = chunk * T::QT + qg * TQ + j;
+                if (li >= L.nq_list) break;  // warp-uniform
+                const uint4 w = sBits[bits * T::QT + qg * TQ + j];
+                const uint32_t word[4] = {w.x, w.y, w.z, w.w};
+                float s[4];
 #pragma unroll
-                    for (int r = 0; r < 4; ++r) {
-                        const uint32_t dl = dg * 4 + r;
-                        if (((dl < 64 ? w0 : w1) >> (dl & 63)) & 1ull) b = fmaxf(b, acc[r][j]);
-                    }
-                    L.best[static_cast<uint64_t>(qi) * L.cap + it * (kDocTile / kSimtGroup) + dg] = b;
+                for (int r = 0; r < 4; ++r) {
+                    const float2 x = *reinterpret_cast<const float2*>(&acc[r][j]);
+                    s[r] = (word[r] >> lane) & 1u ? x.x + x.y : -INFINITY;
+                }
+                if constexpr (MAXIMA) {
+                    const uint32_t qi = L.qlist ? L.qlist[li] : li;
+                    L.best[static_cast<uint64_t>(qi) * L.cap + it * (kDocTile / kSimtGroup) + lane] =
+                        fmaxf(fmaxf(s[0], s[1]), fmaxf(s[2], s[3]));
                     continue;
                 }
+                const float th = sTheta[li];
+                if (!__any_sync(0xffffffffu, fmaxf(fmaxf(s[0], s[1]), fmaxf(s[2], s[3])) >= th)) continue;
+                const uint32_t qi = L.qlist ? L.qlist[li] : li;
                 const uint64_t seg =
                     static_cast<uint64_t>(qi) * L.cap + static_cast<uint64_t>(L.seg_base + blockIdx.x) * L.seg_cap;
 #pragma unroll
                 for (int r = 0; r < 4; ++r) {
-                    const uint32_t dl = dg * 4 + r;
-                    const uint64_t w = dl < 64 ? w0 : w1;
-                    const bool pred = ((w >> (dl & 63)) & 1ull) && acc[r][j] >= th;
+                    const bool pred = ((word[r] >> lane) & 1u) && s[r] >= th;
                     const uint32_t mask = __ballot_sync(0xffffffffu, pred);
                     if (mask == 0) continue;
-                    uint32_t base = 0;
-                    const uint32_t leader = __ffs(mask) - 1;
-                    if (dg == leader) base = atomicAdd(&sCount[chunk * kCQ + qq], __popc(mask));
-                    base = __shfl_sync(0xffffffffu, base, leader);
+                    // the query is this warp's alone: no atomic
+                    const uint32_t base = sCount[li];
+                    __syncwarp();
+                    if (lane == 0) sCount[li] = base + __popc(mask);
+                    __syncwarp();
                     if (pred) {
-                        const uint32_t idx = base + __popc(mask & ((1u << dg) - 1u));
+                        const uint32_t idx = base + __popc(mask & ((1u << lane) - 1u));
                         if (idx < L.seg_cap) {
-                            L.cand_score[seg + idx] = acc[r][j];
-                            L.cand_loc[seg + idx] = static_cast<uint32_t>(doc0 + dl);
+                            L.cand_score[seg + idx] = s[r];
+                            L.cand_loc[seg + idx] = doc0 + 32u * r + lane;
                         }
                     }
                 }
             }
         }
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");
     if (MAXIMA) return;
     __syncthreads();
     for (uint32_t i = tid; i < L.nq_list; i += kCT) {
         const uint32_t qi = L.qlist ? L.qlist[i] : i;
         L.cand_count[static_cast<uint64_t>(qi) * kMaxCandSegs + L.seg_base + blockIdx.x] = sCount[i];
     }
+}
+
+template <int TQ>
+cudaError_t launch_cand_simt_tile(const CandLaunch& L, cudaStream_t stream) {
+    const size_t smem = SimtTile<TQ>::fixed + static_cast<size_t>(L.nq_list) * 8;
+    // the most any caller's batch needs: searchers on other threads launch the same kernel
+    constexpr size_t kCeiling = SimtTile<TQ>::fixed + static_cast<size_t>(kMaxSimtBatch) * 8;
+    auto kernel = L.best ? cand_simt_kernel<TQ, true> : cand_simt_kernel<TQ, false>;
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kCeiling));
+    if (e != cudaSuccess) return e;
+    return launch_dependent(kernel, dim3(L.segs), kCT, smem, stream, 1, L);
 }
 
 }  // namespace
@@ -330,7 +384,7 @@ cudaError_t launch_exact_score(const float* qry, const float* docs, float* out, 
 }
 
 uint32_t cand_simt_segments(uint64_t tile_count, int num_sms, uint32_t cap) {
-    uint64_t g = static_cast<uint64_t>(num_sms) * 3;
+    uint64_t g = static_cast<uint64_t>(num_sms) * 2;  // the CTAs resident at a time
     g = tile_count < g ? tile_count : g;
     g = g < kMaxCandSegs / 2 ? g : kMaxCandSegs / 2;  // one segment per CTA, room for two passes
     const uint64_t by_cap = cap / (2 * kMinSegCap) > 0 ? cap / (2 * kMinSegCap) : 1;
@@ -344,10 +398,16 @@ cudaError_t launch_cand_simt(const CandLaunch& L, int num_sms, cudaStream_t stre
         seg_end * L.seg_cap > L.cap || L.nq_list > kMaxSimtBatch ||
         !tile_walk_fits(L.tile_begin, L.tile_step, L.tile_skip, L.tile_count, L.segs))
         return cudaErrorInvalidValue;
-    const size_t smem = static_cast<size_t>(L.nq_list) * sizeof(uint32_t);
     if (L.best && L.tile_count * (kDocTile / kSimtGroup) > L.cap) return cudaErrorInvalidValue;
-    return launch_dependent(L.best ? cand_simt_kernel<true> : cand_simt_kernel<false>, dim3(L.segs), kCT, smem, stream,
-                            1, L);
+    // the filter words and rows are copied 16 bytes at a time
+    if ((L.bits_stride & 1u) || (reinterpret_cast<uintptr_t>(L.bits) & 15u) || (reinterpret_cast<uintptr_t>(L.vec) & 15u) ||
+        (reinterpret_cast<uintptr_t>(L.qry) & 15u))
+        return cudaErrorInvalidValue;
+    // chunks as narrow as the batch: a chunk's pipe time is that of all its queries
+    if (L.nq_list <= 8) return launch_cand_simt_tile<1>(L, stream);
+    if (L.nq_list <= 16) return launch_cand_simt_tile<2>(L, stream);
+    if (L.nq_list <= 32) return launch_cand_simt_tile<4>(L, stream);
+    return launch_cand_simt_tile<8>(L, stream);
 }
 
 }  // namespace hss
