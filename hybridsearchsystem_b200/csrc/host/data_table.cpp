@@ -308,8 +308,6 @@ bool DataTable::EnableFormat(int format, std::string* err) {
     if (ok) ok = CudaOk(cudaMemcpy(hn.data(), norm, rows * 4, cudaMemcpyDeviceToHost), err, "download norms");
     if (ok) ok = CudaOk(cudaMemcpy(he.data(), errn, rows * 4, cudaMemcpyDeviceToHost), err, "download norms");
     if (ok && format == kTcE4M3) {
-        ok = CudaOk(cudaMalloc(&m_dTileScale, GetTileNum() * sizeof(float2)), err, "cudaMalloc tile scales") &&
-             CudaOk(launch_tile_scale_minmax(scale, GetTileNum(), m_dTileScale, nullptr), err, "tile scales");
         m_dDocScale = scale;
         scale = nullptr;
     }
@@ -398,9 +396,7 @@ void DataTable::Release() {
         m_dQuant[f] = nullptr;
     }
     if (m_dDocScale) cudaFree(m_dDocScale);
-    if (m_dTileScale) cudaFree(m_dTileScale);
     m_dDocScale = nullptr;
-    m_dTileScale = nullptr;
     if (m_dVectors) cudaFree(m_dVectors);
     if (m_dArena) cudaFree(m_dArena);
     if (m_dPostingTable) cudaFree(m_dPostingTable);

@@ -256,7 +256,6 @@ class DataTable {
     bool HasFormat(int format) const { return format >= 0 && format < 3 && m_fmtReady[format]; }
     const void* DeviceRows(int format) const { return format == 0 ? static_cast<const void*>(m_dVectors) : m_dQuant[format]; }
     const float* DeviceDocScale() const { return m_dDocScale; }
-    const float2* DeviceTileScale() const { return m_dTileScale; }
     double NormMax(int format) const { return m_fmtNormMax[format]; }
     double ErrMax(int format) const { return m_fmtErrMax[format]; }
 
@@ -311,7 +310,6 @@ class DataTable {
     float* m_dVectors = nullptr;
     void* m_dQuant[3] = {nullptr, nullptr, nullptr};
     float* m_dDocScale = nullptr;
-    float2* m_dTileScale = nullptr;
     bool m_fmtReady[3] = {false, false, false};
     double m_fmtNormMax[3] = {0, 0, 0};
     double m_fmtErrMax[3] = {0, 0, 0};

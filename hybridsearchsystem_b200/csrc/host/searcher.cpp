@@ -592,7 +592,6 @@ void FullRecallSearcher::Cand(const float* theta, float* score, uint32_t* loc, u
     C.format = m_tcFormat;
     C.kblocks = m_tcKblocks;
     C.doc_scale = T.DeviceDocScale();
-    C.tile_scale = T.DeviceTileScale();
     C.q_scale = m_dQScale;
     C.bits = m_dBits;
     C.bits_stride = T.GetBitmapWords();

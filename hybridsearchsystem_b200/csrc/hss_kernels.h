@@ -212,7 +212,6 @@ struct TcCandLaunch {
     uint32_t group;            // corpus k-blocks per ring stage (set by launch_tc_cand; 1 or 2)
     int emit_all;              // every row's threshold is -inf (the doc sample): most docs are kept
     const float* doc_scale;    // E4M3: per-doc dequantisation scale
-    const float2* tile_scale;  // E4M3: per 128-doc tile (min, max) of doc_scale
     const float* q_scale;      // E4M3: per staged query row
     const uint64_t* bits;      // [nq][bits_stride] filter bitmaps
     uint64_t bits_stride;
@@ -263,7 +262,6 @@ bool make_tc_map(CUtensorMap* map, int format, const void* base, uint64_t rows, 
 // per-doc scale (e4m3), per-doc norm and quantisation-error norm (FP64, rounded up to float).
 cudaError_t launch_quantize_docs(const float* vec, uint64_t rows, uint64_t valid_rows, uint32_t dim, int format,
                                  void* out, float* scale, float* norm, float* err_norm, cudaStream_t stream);
-cudaError_t launch_tile_scale_minmax(const float* scale, uint64_t tiles, float2* out, cudaStream_t stream);
 // Stage a batch of queries in a tensor-core format (rows past nq zero) and compute the per-query error
 // bounds of the candidate pass (see score_tc.cu / searcher.cpp).
 struct StageQueriesLaunch {

@@ -98,24 +98,6 @@ __global__ void quantize_docs_kernel(const float* __restrict__ vec, uint64_t row
     }
 }
 
-__global__ void tile_minmax_kernel(const float* __restrict__ scale, uint64_t tiles, float2* __restrict__ out) {
-    const uint64_t t = static_cast<uint64_t>(blockIdx.x) * (blockDim.x / 32) + (threadIdx.x >> 5);
-    if (t >= tiles) return;
-    const uint32_t lane = threadIdx.x & 31;
-    float lo = INFINITY, hi = 0.0f;
-    for (uint32_t i = lane; i < 128; i += 32) {
-        const float s = scale[t * 128 + i];
-        lo = fminf(lo, s);
-        hi = fmaxf(hi, s);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
-        hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
-    }
-    if (lane == 0) out[t] = make_float2(lo, hi);
-}
-
 // Runs beside the batch's filter, the kernel before it: it reads and writes nothing of the filter's (the
 // queries are complete before the filter starts), and waits for it only at its end, so that what is
 // launched after it finds both complete.
@@ -163,12 +145,6 @@ cudaError_t launch_quantize_docs(const float* vec, uint64_t rows, uint64_t valid
     const uint64_t blocks = (rows + 7) / 8;
     quantize_docs_kernel<<<static_cast<unsigned>(blocks), 256, 0, stream>>>(vec, rows, valid_rows, dim, format, out,
                                                                            scale, norm, err_norm);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_tile_scale_minmax(const float* scale, uint64_t tiles, float2* out, cudaStream_t stream) {
-    if (tiles == 0) return cudaSuccess;
-    tile_minmax_kernel<<<static_cast<unsigned>((tiles + 7) / 8), 256, 0, stream>>>(scale, tiles, out);
     return cudaGetLastError();
 }
 

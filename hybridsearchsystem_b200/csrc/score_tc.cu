@@ -276,19 +276,6 @@ __device__ inline float max3(float a, float b, float c) {
     return d;
 }
 
-// Maximum of a lane's 32 scores as a tree of three-input maxima (four dependent steps, not sixteen:
-// the epilogue warps have little else to hide the latency behind).
-__device__ inline float max32(const uint32_t (&r)[32]) {
-    float a[11];
-#pragma unroll
-    for (int i = 0; i < 10; ++i)
-        a[i] = max3(__uint_as_float(r[3 * i]), __uint_as_float(r[3 * i + 1]), __uint_as_float(r[3 * i + 2]));
-    a[10] = fmaxf(__uint_as_float(r[30]), __uint_as_float(r[31]));
-    const float b0 = max3(a[0], a[1], a[2]), b1 = max3(a[3], a[4], a[5]), b2 = max3(a[6], a[7], a[8]);
-    const float b3 = fmaxf(a[9], a[10]);
-    return fmaxf(max3(b0, b1, b2), b3);
-}
-
 // Maximum of the 8 scores v[8k .. 8k + 7] (three steps).
 __device__ __forceinline__ float max8(const uint32_t (&v)[32], int k) {
     const float a = max3(__uint_as_float(v[8 * k]), __uint_as_float(v[8 * k + 1]), __uint_as_float(v[8 * k + 2]));
@@ -306,12 +293,39 @@ __device__ __forceinline__ uint32_t pick8(const uint32_t (&v)[32], int k, uint32
     return (j & 1u) ? b[1] : b[0];
 }
 
-// One 32-doc chunk of a thread's TF32 / BF16 scores (its query): the docs whose filter bit (m) is set
-// and whose approximate score clears the threshold t go to the thread's list segment, in doc order.
+// E4M3: a chunk's raw accumulators times their docs' scales (the lanes share the docs, so the loads are
+// broadcasts), which leaves only the query's own scale, folded into the threshold. With a bound per
+// 128-doc tile instead (the tile's largest scale) a third of the chunks cleared it for nothing and took
+// the emission path: 1M docs, 128 queries, 364 us for the passes against 146 us now.
+__device__ __forceinline__ void scale_chunk(uint32_t (&v)[32], const float* __restrict__ doc_scale, uint64_t doc0) {
+    const float4* s = reinterpret_cast<const float4*>(doc_scale + doc0);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+        const float4 x = __ldg(s + k);
+        v[4 * k + 0] = __float_as_uint(__uint_as_float(v[4 * k + 0]) * x.x);
+        v[4 * k + 1] = __float_as_uint(__uint_as_float(v[4 * k + 1]) * x.y);
+        v[4 * k + 2] = __float_as_uint(__uint_as_float(v[4 * k + 2]) * x.z);
+        v[4 * k + 3] = __float_as_uint(__uint_as_float(v[4 * k + 3]) * x.w);
+    }
+}
+
+// Threshold on scaled accumulators: every x with x * qs >= theta (qs > 0, rounded) has x >= the returned
+// value: the quotient, rounded to nearest, lowered by a relative 2^-20 and a tiny absolute step. NaN (no
+// query) gives -inf.
+__device__ __forceinline__ float e4m3_threshold(float theta, float qs) {
+    const float t = theta / qs;
+    if (!(t == t)) return -INFINITY;
+    return __fsub_rd(t, __fmaf_ru(fabsf(t), 0x1p-20f, 1e-30f));
+}
+
+// One 32-doc chunk of a thread's scores (its query): the docs whose filter bit (m) is set and whose
+// approximate score clears the threshold t go to the thread's list segment, in doc order. E4M3: v are
+// scaled accumulators (scale_chunk), t is on those, and the score is v * qs.
 // The epilogue runs on the ALU pipe (compares, maxima, selects), so the chunk is tested as four 8-doc
 // groups: only a group whose maximum clears t builds a keep mask, and a kept doc is picked from its
 // group's 8 registers. The loop runs once per kept doc (typically zero or one per chunk).
-__device__ __forceinline__ void emit_lane(uint32_t m, const uint32_t (&v)[32], float t, uint64_t doc0,
+template <int F>
+__device__ __forceinline__ void emit_lane(uint32_t m, const uint32_t (&v)[32], float t, float qs, uint64_t doc0,
                                           float* out_score, uint32_t* out_loc, uint32_t seg_cap, uint32_t& ncand) {
     if (m == 0u) return;
     float g[4];
@@ -330,58 +344,9 @@ __device__ __forceinline__ void emit_lane(uint32_t m, const uint32_t (&v)[32], f
             const uint32_t j = static_cast<uint32_t>(__ffs(pass) - 1);
             pass &= pass - 1u;
             if (ncand < seg_cap) {
-                out_score[ncand] = __uint_as_float(pick8(v, k, j));
+                const float s = __uint_as_float(pick8(v, k, j));
+                out_score[ncand] = F == kTcE4M3 ? s * qs : s;
                 out_loc[ncand] = static_cast<uint32_t>(doc0 + 8u * k + j);
-            }
-            ++ncand;
-        }
-    }
-}
-
-// Threshold on a tile's raw E4M3 accumulators: every doc of the tile whose dequantised score
-// acc * qs * ds (ds in [mm.x, mm.y], both positive) reaches theta has acc >= the returned value.
-// The two divisions round to nearest; the result is then lowered by a relative 2^-20 (plus a tiny
-// absolute step) whatever its sign, so it stays below the exact quotient. NaN (no query) gives -inf.
-__device__ __forceinline__ float e4m3_tile_threshold(float theta, float qs, float2 mm) {
-    const float tq = theta / qs;
-    float t = tq > 0.0f ? tq / mm.y : tq / mm.x;
-    if (!(t == t)) return -INFINITY;
-    return __fsub_rd(t, __fmaf_ru(fabsf(t), 0x1p-20f, 1e-30f));
-}
-
-// One 32-doc chunk of a thread's E4M3 scores (its query, raw accumulators v): the docs whose filter
-// bit (m) is set and whose dequantised score clears the threshold go to the thread's list segment.
-// Warp-collective: the warp leaves at once when no lane's chunk clears its tile threshold t, and the
-// emission loop visits only doc positions that some lane keeps (E4M3's wide bound lets many chunks
-// through; for TF32 / BF16 the per-lane form in the kernels measured faster).
-template <int F>
-__device__ __forceinline__ void emit_chunk(bool live, uint32_t m, const uint32_t (&v)[32], float t, float theta,
-                                           float qs, const float* doc_scale, uint64_t doc0, float* out_score,
-                                           uint32_t* out_loc, uint32_t seg_cap, uint32_t& ncand) {
-    const bool hot = live && m != 0u && max32(v) >= t;
-    if (!__any_sync(0xffffffffu, hot)) return;
-    uint32_t pass = 0;
-    if (hot) {
-#pragma unroll
-        for (int j = 0; j < 32; ++j) pass |= (__uint_as_float(v[j]) >= t ? 1u : 0u) << j;
-        pass &= m;
-        if (F == kTcE4M3) {  // the tile threshold is conservative: apply the doc's own scale
-#pragma unroll
-            for (int j = 0; j < 32; ++j)
-                if (((pass >> j) & 1u) && !(__uint_as_float(v[j]) * qs * doc_scale[doc0 + j] >= theta))
-                    pass &= ~(1u << j);
-        }
-    }
-    const uint32_t any = __reduce_or_sync(0xffffffffu, pass);
-#pragma unroll
-    for (int j = 0; j < 32; ++j) {
-        if (!((any >> j) & 1u)) continue;  // warp-uniform
-        if ((pass >> j) & 1u) {
-            float sc = __uint_as_float(v[j]);
-            if (F == kTcE4M3) sc = sc * qs * doc_scale[doc0 + j];
-            if (ncand < seg_cap) {
-                out_score[ncand] = sc;
-                out_loc[ncand] = static_cast<uint32_t>(doc0 + j);
             }
             ++ncand;
         }
@@ -392,9 +357,8 @@ __device__ __forceinline__ void emit_chunk(bool live, uint32_t m, const uint32_t
 // set, -inf where none is, as one 16-byte store at out[4 * chunk]; coarse: of the whole chunk, at
 // out[chunk]. live: the chunk was read (some lane has a bit).
 template <int F>
-__device__ __forceinline__ void store_maxima(bool live, uint32_t m, const uint32_t (&v)[32], float qs,
-                                             const float* doc_scale, uint64_t doc0, float* out, uint32_t chunk,
-                                             bool coarse) {
+__device__ __forceinline__ void store_maxima(bool live, uint32_t m, const uint32_t (&v)[32], float qs, float* out,
+                                             uint32_t chunk, bool coarse) {
     float g[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
     if (live) {
 #pragma unroll
@@ -403,7 +367,7 @@ __device__ __forceinline__ void store_maxima(bool live, uint32_t m, const uint32
 #pragma unroll
             for (int j = 0; j < 8; ++j) {
                 float s = __uint_as_float(v[8 * k + j]);
-                if (F == kTcE4M3) s = s * qs * __ldg(doc_scale + doc0 + 8 * k + j);
+                if (F == kTcE4M3) s *= qs;
                 x[j] = (m >> (8 * k + j)) & 1u ? s : -INFINITY;
             }
             g[k] = max3(max3(x[0], x[1], x[2]), max3(x[3], x[4], x[5]), fmaxf(x[6], x[7]));
@@ -554,6 +518,7 @@ __global__ void __launch_bounds__(64 + 256 * H, 1) tc_cand_kernel(const __grid_c
         const uint32_t qi = valid ? (L.qlist ? L.qlist[row] : row) : 0u;
         const float theta = valid ? L.theta[qi] : INFINITY;
         const float qs = (F == kTcE4M3 && valid) ? L.q_scale[row] : 1.0f;
+        const float t = F == kTcE4M3 ? e4m3_threshold(theta, qs) : theta;
         const uint64_t* brow = L.bits + static_cast<uint64_t>(qi) * L.bits_stride;
         const uint32_t segment = L.seg_base + 2u * blockIdx.x + colh;
         const uint64_t seg = static_cast<uint64_t>(qi) * L.cap + static_cast<uint64_t>(segment) * L.seg_cap;
@@ -575,8 +540,6 @@ __global__ void __launch_bounds__(64 + 256 * H, 1) tc_cand_kernel(const __grid_c
             walk.advance();
             tile_next = walk.tile();
             if (valid && it + gridDim.x < ntiles) fw_next = brow[tile_next * 2 + colh];
-            // threshold on the raw accumulator: acc * qs * ds >= theta
-            const float t = F == kTcE4M3 ? e4m3_tile_threshold(theta, qs, L.tile_scale[tile]) : theta;
             const uint32_t m[2] = {static_cast<uint32_t>(fw), static_cast<uint32_t>(fw >> 32)};
             // 32-doc chunks that no query of the warp lets through are not read from TMEM at all
             bool live[2];
@@ -602,16 +565,13 @@ __global__ void __launch_bounds__(64 + 256 * H, 1) tc_cand_kernel(const __grid_c
 #pragma unroll
             for (int c = 0; c < 2; ++c) {
                 const uint64_t doc0 = tile * kRows + colh * 64u + c * 32u;
+                if (F == kTcE4M3 && live[c]) scale_chunk(v[c], L.doc_scale, doc0);
                 if constexpr (MAXIMA) {
                     if (valid)
-                        store_maxima<F>(live[c], m[c], v[c], qs, L.doc_scale, doc0,
-                                        L.best + static_cast<uint64_t>(qi) * L.cap,
+                        store_maxima<F>(live[c], m[c], v[c], qs, L.best + static_cast<uint64_t>(qi) * L.cap,
                                         static_cast<uint32_t>(it) * 4u + colh * 2u + c, L.coarse != 0);
-                } else if constexpr (F == kTcE4M3) {
-                    emit_chunk<F>(live[c], m[c], v[c], t, theta, qs, L.doc_scale, doc0, out_score, out_loc, seg_cap,
-                                  ncand);
                 } else if (live[c]) {
-                    emit_lane(m[c], v[c], t, doc0, out_score, out_loc, seg_cap, ncand);
+                    emit_lane<F>(m[c], v[c], t, qs, doc0, out_score, out_loc, seg_cap, ncand);
                 }
             }
         }
@@ -847,6 +807,7 @@ __global__ void __launch_bounds__(kPairThreads, 1) tc2_cand_kernel(const __grid_
         const uint32_t qi = valid ? (L.qlist ? L.qlist[row] : row) : 0u;
         const float theta = valid ? L.theta[qi] : INFINITY;
         const float qs = (F == kTcE4M3 && valid) ? L.q_scale[row] : 1.0f;
+        const float t = F == kTcE4M3 ? e4m3_threshold(theta, qs) : theta;
         const uint64_t* brow = L.bits + static_cast<uint64_t>(qi) * L.bits_stride;
         const uint32_t segment = L.seg_base + 4u * pair + g;
         const uint64_t seg = static_cast<uint64_t>(qi) * L.cap + static_cast<uint64_t>(segment) * L.seg_cap;
@@ -874,12 +835,6 @@ __global__ void __launch_bounds__(kPairThreads, 1) tc2_cand_kernel(const __grid_
             walk.advance();
             tile_next = static_cast<uint32_t>(walk.tile());
             if (it + npairs < nt) fw_next = word_of(tile_next);
-            float t = theta;
-            if (F == kTcE4M3) {
-                uint64_t ts = tile * 2 + g / 2;  // 128-doc tile holding this thread's docs
-                ts = ts < L.tiles128 ? ts : L.tiles128 - 1;
-                t = e4m3_tile_threshold(theta, qs, L.tile_scale[ts]);
-            }
             const uint32_t m[2] = {static_cast<uint32_t>(fw), static_cast<uint32_t>(fw >> 32)};
             bool live[2];
 #pragma unroll
@@ -904,11 +859,9 @@ __global__ void __launch_bounds__(kPairThreads, 1) tc2_cand_kernel(const __grid_
 #pragma unroll
                 for (int c = 0; c < 2; ++c) {
                     const uint64_t doc0 = tile * 256u + g * 64u + c * 32u;
-                    if constexpr (F == kTcE4M3) {
-                        emit_chunk<F>(live[c], m[c], v[c], t, theta, qs, L.doc_scale, doc0, out_score, out_loc,
-                                      seg_cap, ncand);
-                    } else if (live[c]) {
-                        emit_lane(m[c], v[c], t, doc0, out_score, out_loc, seg_cap, ncand);
+                    if (live[c]) {
+                        if (F == kTcE4M3) scale_chunk(v[c], L.doc_scale, doc0);
+                        emit_lane<F>(m[c], v[c], t, qs, doc0, out_score, out_loc, seg_cap, ncand);
                     }
                 }
             } else {
@@ -927,16 +880,14 @@ __global__ void __launch_bounds__(kPairThreads, 1) tc2_cand_kernel(const __grid_
                         if (lane == 0) mbar_arrive_cluster(buf ? acc_empty_addr1 : acc_empty_addr0);
                     }
                     const uint64_t doc0 = tile * 256u + g * 64u + c * 32u;
+                    // (a live chunk has a filtered doc, so its docs are rows of the corpus and have scales)
+                    if (F == kTcE4M3 && live[c]) scale_chunk(v, L.doc_scale, doc0);
                     if constexpr (EMIT == kEmitMaxima) {
-                        // (E4M3: no scales past the corpus rows, whose bits are clear)
                         if (valid)
-                            store_maxima<F>(live[c] && doc0 < L.tiles128 * 128u, m[c], v, qs, L.doc_scale, doc0,
-                                            L.best + static_cast<uint64_t>(qi) * L.cap, it * 8u + g * 2u + c, L.coarse != 0);
-                    } else if constexpr (F == kTcE4M3) {
-                        emit_chunk<F>(live[c], m[c], v, t, theta, qs, L.doc_scale, doc0, out_score, out_loc, seg_cap,
-                                      ncand);
+                            store_maxima<F>(live[c], m[c], v, qs, L.best + static_cast<uint64_t>(qi) * L.cap,
+                                            it * 8u + g * 2u + c, L.coarse != 0);
                     } else if (live[c]) {
-                        emit_lane(m[c], v, t, doc0, out_score, out_loc, seg_cap, ncand);
+                        emit_lane<F>(m[c], v, t, qs, doc0, out_score, out_loc, seg_cap, ncand);
                     }
                 }
             }
