@@ -25,7 +25,6 @@ struct OperandInfo {
     uint32_t layout;  // kEmpty for an all-zero or absent posting
     uint32_t plen;    // payload bytes (clamped to what the layout can legally hold)
     uint32_t k;       // sparse entries
-    int32_t lo, hi;   // sparse entries whose unit falls in this tile
 };
 constexpr uint32_t kEmpty = 0xffu;
 
@@ -81,30 +80,14 @@ __device__ inline uint32_t max_payload(uint32_t layout, uint32_t seg_docs) {
     return 0;
 }
 
-// First sparse entry whose unit index is >= u (entries are sorted by unit, posting_serializer.cpp).
-__device__ inline int32_t sparse_lower_bound(const OperandInfo& o, uint32_t u) {
-    int32_t lo = 0, hi = static_cast<int32_t>(o.k);
-    while (lo < hi) {
-        const int32_t mid = (lo + hi) >> 1;
-        const uint32_t unit = o.layout == kSparseBitmap ? ld32(o.addr + 8 + 4u * mid) / 2u
-                                                          : ld32(o.addr + 8 + 4u * mid) >> 16;
-        if (unit < u)
-            lo = mid + 1;
-        else
-            hi = mid;
-    }
-    return lo;
-}
-
-__device__ inline void resolve_operand(OperandInfo& o, const uint8_t* addr, uint32_t seg_docs, uint32_t unit_lo,
-                                       uint32_t unit_hi, int* bad) {
+__device__ inline void resolve_operand(OperandInfo& o, const uint8_t* addr, uint32_t seg_docs, int* bad) {
     o.addr = addr;
     o.layout = kEmpty;
     o.plen = 0;
     o.k = 0;
-    o.lo = o.hi = 0;
     if (addr == nullptr) return;
-    const uint32_t head = ld32(addr);
+    const uint64_t both = ld64(addr);  // [layout:4|hits:28] and the payload's bytes
+    const uint32_t head = static_cast<uint32_t>(both);
     const uint32_t hits = head & 0x0fffffffu;
     const uint32_t layout = head >> 28;
     if (layout > kSparsePacked) {
@@ -113,17 +96,10 @@ __device__ inline void resolve_operand(OperandInfo& o, const uint8_t* addr, uint
     }
     if (hits == 0) return;  // all-zero posting: identity of OR, annihilator of AND
     o.layout = layout;
-    o.plen = min(ld32(addr + 4), max_payload(layout, seg_docs));
+    o.plen = min(static_cast<uint32_t>(both >> 32), max_payload(layout, seg_docs));
     if (layout == kSparseBitmap) o.k = o.plen / 6;
     if (layout == kSparsePacked) o.k = o.plen / 4;
     if (layout == kSparseIdList) o.k = o.plen / 4;
-    if (layout == kSparseBitmap || layout == kSparsePacked) {
-        // a tile spanning the whole segment needs every entry: no search (each step of it is a
-        // dependent global load)
-        const uint32_t units = (seg_docs + 15) / 16;
-        o.lo = unit_lo == 0 ? 0 : sparse_lower_bound(o, unit_lo);
-        o.hi = unit_hi >= units ? static_cast<int32_t>(o.k) : sparse_lower_bound(o, unit_hi);
-    }
 }
 
 __device__ inline uint64_t tail_mask(uint64_t gw, uint64_t doc_num) {
@@ -138,14 +114,16 @@ __device__ inline uint64_t tail_mask(uint64_t gw, uint64_t doc_num) {
 // the next postingNum operands with stackNum popped results, [CONJUNCTION, parts, n_1..n_parts] ANDs
 // the ORs of consecutive operand groups. Every op is decoded and checked once and applied to all W
 // words, so the per-op decode cost is shared. Returns false for a malformed program.
-template <int W>
-__device__ inline bool eval_words(const uint32_t* prog, uint32_t plen, const uint64_t* slots, uint32_t slot_stride,
-                                  uint32_t w0, uint32_t step, uint32_t nop, uint64_t (&result)[W]) {
+//
+// operand(i, v) loads this thread's W words of operand i.
+template <int W, class Operand>
+__device__ __forceinline__ bool eval_words(const uint32_t* prog, uint32_t plen, Operand operand, uint32_t nop,
+                                           uint64_t (&result)[W]) {
     uint64_t st[kMaxStack][W];
     uint32_t sp = 0, next = 0, pc = 0;
     while (pc < plen) {
         const uint32_t op = prog[pc];
-        uint64_t acc[W];
+        uint64_t acc[W], v[W];
         if (op == kOpAnd || op == kOpOr || op == kOpNot) {
             if (pc + 2 >= plen) return false;
             const uint32_t pn = prog[pc + 1], sn = prog[pc + 2];
@@ -154,37 +132,30 @@ __device__ inline bool eval_words(const uint32_t* prog, uint32_t plen, const uin
             // caller's device buffer): next <= nop always holds
             const bool ok = op == kOpNot ? ((pn == 1 && sn == 0) || (pn == 0 && sn == 1)) : (pn != 0 || sn != 0);
             if (!ok || pn > nop - next || sn > sp) return false;
-            const uint64_t* row = slots + static_cast<uint64_t>(next) * slot_stride + w0;
             if (op == kOpNot) {
                 if (pn) {
-#pragma unroll
-                    for (int k = 0; k < W; ++k) acc[k] = ~row[k * step];
+                    operand(next, acc);
                 } else {
                     --sp;
 #pragma unroll
-                    for (int k = 0; k < W; ++k) acc[k] = ~st[sp][k];
+                    for (int k = 0; k < W; ++k) acc[k] = st[sp][k];
                 }
-            } else if (op == kOpAnd) {
 #pragma unroll
-                for (int k = 0; k < W; ++k) acc[k] = ~0ull;
-                for (uint32_t j = 0; j < pn; ++j, row += slot_stride)
-#pragma unroll
-                    for (int k = 0; k < W; ++k) acc[k] &= row[k * step];
-                for (uint32_t j = 0; j < sn; ++j) {
-                    --sp;
-#pragma unroll
-                    for (int k = 0; k < W; ++k) acc[k] &= st[sp][k];
-                }
+                for (int k = 0; k < W; ++k) acc[k] = ~acc[k];
             } else {
+                const bool is_and = op == kOpAnd;
 #pragma unroll
-                for (int k = 0; k < W; ++k) acc[k] = 0ull;
-                for (uint32_t j = 0; j < pn; ++j, row += slot_stride)
+                for (int k = 0; k < W; ++k) acc[k] = is_and ? ~0ull : 0ull;
+#pragma unroll 2  // two operands' loads in flight
+                for (uint32_t j = 0; j < pn; ++j) {
+                    operand(next + j, v);
 #pragma unroll
-                    for (int k = 0; k < W; ++k) acc[k] |= row[k * step];
+                    for (int k = 0; k < W; ++k) acc[k] = is_and ? (acc[k] & v[k]) : (acc[k] | v[k]);
+                }
                 for (uint32_t j = 0; j < sn; ++j) {
                     --sp;
 #pragma unroll
-                    for (int k = 0; k < W; ++k) acc[k] |= st[sp][k];
+                    for (int k = 0; k < W; ++k) acc[k] = is_and ? (acc[k] & st[sp][k]) : (acc[k] | st[sp][k]);
                 }
             }
             next += pn;
@@ -200,10 +171,12 @@ __device__ inline bool eval_words(const uint32_t* prog, uint32_t plen, const uin
                 uint64_t o[W];
 #pragma unroll
                 for (int k = 0; k < W; ++k) o[k] = 0ull;
-                const uint64_t* row = slots + static_cast<uint64_t>(next) * slot_stride + w0;
-                for (uint32_t j = 0; j < pn; ++j, row += slot_stride)
+#pragma unroll 2
+                for (uint32_t j = 0; j < pn; ++j) {
+                    operand(next + j, v);
 #pragma unroll
-                    for (int k = 0; k < W; ++k) o[k] |= row[k * step];
+                    for (int k = 0; k < W; ++k) o[k] |= v[k];
+                }
 #pragma unroll
                 for (int k = 0; k < W; ++k) acc[k] &= o[k];
                 next += pn;
@@ -223,12 +196,17 @@ __device__ inline bool eval_words(const uint32_t* prog, uint32_t plen, const uin
     return true;
 }
 
-// One CTA per (query, segment tile of WPT * 256 words). Operands are decoded into shared-memory
-// slots of the tile (dense: each thread its own words; sparse: zeroed, then scattered), then every
-// word is run through the program. Grid: x = query (fastest, so all queries of a tile share the
-// tile's postings in L2), y = segment tile.
+// One CTA per (query, segment tile of WPT * 256 words). A chain of dependent loads (offsets, rows, posting
+// heads, postings) bounds a CTA, so tiles are small enough that several CTAs share an SM. Dense operands
+// are read where they lie when the program gets to them; the others are decoded into shared-memory slots
+// of the tile first (bytemaps: each thread its own words; sparse: zeroed, then scattered). A sparse
+// posting holds a few thousand entries at most, so every tile reads all of them and keeps its own: a
+// search for the tile's first entry would be ten dependent loads. Grid: x = query (fastest, so all queries
+// of a tile share the tile's postings in L2), y = segment tile. 64 queries of up to 6 tags over 2M docs with
+// packed postings: 56 us with whole-segment tiles and every operand staged, 38 us now (256 queries over 4M
+// docs 376 -> 257 us a call).
 template <int WPT>
-__global__ void __launch_bounds__(kTile) filter_batch_kernel(FilterLaunch L) {
+__global__ void __launch_bounds__(kTile) filter_batch_kernel(FilterLaunch L, uint32_t tiles_per_cta) {
     constexpr uint32_t TW = kTile * WPT;  // words per CTA
     extern __shared__ uint64_t slots[];   // [nop][TW]
     __shared__ OperandInfo s_op[kMaxOperands];
@@ -239,13 +217,14 @@ __global__ void __launch_bounds__(kTile) filter_batch_kernel(FilterLaunch L) {
     const uint32_t q = blockIdx.x;
     const uint32_t t = threadIdx.x;
     const uint32_t seg_words = L.docs_per_seg / 64;
-    const uint32_t tiles = (seg_words + TW - 1) / TW;
-    const uint32_t seg = blockIdx.y / tiles;
-    const uint32_t w0 = (blockIdx.y % tiles) * TW;
-    const uint32_t nw = min(TW, seg_words - w0);
+    const uint32_t tiles = (seg_words + TW - 1) / TW;                       // of a segment
+    const uint32_t groups = (tiles + tiles_per_cta - 1) / tiles_per_cta;  // CTAs of a segment
+    const uint32_t seg = blockIdx.y / groups;
+    const uint32_t tile0 = (blockIdx.y % groups) * tiles_per_cta, tile1 = min(tiles, tile0 + tiles_per_cta);
+    const uint32_t cta_w0 = tile0 * TW, cta_nw = min(tile1 * TW, seg_words) - cta_w0;
     const uint64_t seg_doc0 = static_cast<uint64_t>(seg) * L.docs_per_seg;
     const uint32_t seg_docs = static_cast<uint32_t>(min(static_cast<uint64_t>(L.docs_per_seg), L.doc_num - seg_doc0));
-    const uint64_t gw0 = static_cast<uint64_t>(seg) * seg_words + w0;
+    const uint64_t seg_w0 = static_cast<uint64_t>(seg) * seg_words;
     uint64_t* out_row = L.out + static_cast<uint64_t>(q) * L.out_stride;
 
     const uint32_t p0 = L.prog_off ? L.prog_off[q] : 0u;
@@ -257,14 +236,10 @@ __global__ void __launch_bounds__(kTile) filter_batch_kernel(FilterLaunch L) {
 
     if (plen == 0) {  // empty program: match all (the reference memsets 0xff, text_filter.cpp:553-559)
         uint32_t c = 0;
-#pragma unroll
-        for (int k = 0; k < WPT; ++k) {
-            const uint32_t w = k * kTile + t;
-            if (w < nw) {
-                const uint64_t v = tail_mask(gw0 + w, L.doc_num);
-                out_row[gw0 + w] = v;
-                c += __popcll(v);
-            }
+        for (uint32_t w = t; w < cta_nw; w += kTile) {
+            const uint64_t v = tail_mask(seg_w0 + cta_w0 + w, L.doc_num);
+            out_row[seg_w0 + cta_w0 + w] = v;
+            c += __popcll(v);
         }
         if (L.pass_count) {
             c = warp_sum(c);
@@ -273,7 +248,7 @@ __global__ void __launch_bounds__(kTile) filter_batch_kernel(FilterLaunch L) {
         return;
     }
     if (nop > L.max_opnd || nop > static_cast<uint32_t>(kMaxOperands) || plen > static_cast<uint32_t>(kMaxProgram)) {
-        for (uint32_t w = t; w < nw; w += kTile) out_row[gw0 + w] = 0;
+        for (uint32_t w = t; w < cta_nw; w += kTile) out_row[seg_w0 + cta_w0 + w] = 0;
         if (t == 0 && L.status) atomicOr(L.status + q, kStatusBadProgram);
         return;
     }
@@ -285,83 +260,89 @@ __global__ void __launch_bounds__(kTile) filter_batch_kernel(FilterLaunch L) {
         const uint64_t row = L.opnd_row ? L.opnd_row[o0 + t] : t;
         const uint64_t a = L.table[row * L.row_stride + static_cast<uint64_t>(seg) * L.seg_stride];
         if (!L.ref_table) {
-            resolve_operand(s_op[t], reinterpret_cast<const uint8_t*>(a), seg_docs, w0 * 4u, (w0 + nw) * 4u, &s_bad);
+            resolve_operand(s_op[t], reinterpret_cast<const uint8_t*>(a), seg_docs, &s_bad);
         } else if (a == 2u || a == 0u) {  // EMPTY_OPERAND_TAG
-            resolve_operand(s_op[t], nullptr, seg_docs, 0u, 0u, &s_bad);
+            resolve_operand(s_op[t], nullptr, seg_docs, &s_bad);
         } else if (a & 1u) {  // SPARSE_OPERAND_TAG: the sparse posting's head
-            resolve_operand(s_op[t], reinterpret_cast<const uint8_t*>(a & ~1ull), seg_docs, w0 * 4u, (w0 + nw) * 4u,
-                            &s_bad);
+            resolve_operand(s_op[t], reinterpret_cast<const uint8_t*>(a & ~1ull), seg_docs, &s_bad);
         } else {  // a dense bitset: the payload of a DENSE_BITMAP posting, no head
             OperandInfo& o = s_op[t];
             o.addr = reinterpret_cast<const uint8_t*>(a) - 8;
             o.layout = kDenseBitmap;
             o.plen = L.docs_per_seg / 8;
             o.k = 0;
-            o.lo = o.hi = 0;
-        }
-    }
-    __syncthreads();
-
-    // Dense operands: each thread its own words (coalesced). Sparse ones: zero, then scatter below.
-    for (uint32_t i = 0; i < nop; ++i) {
-        const OperandInfo& o = s_op[i];
-#pragma unroll
-        for (int k = 0; k < WPT; ++k) {
-            const uint32_t w = k * kTile + t;
-            uint64_t v = 0;
-            if (w < nw) {
-                if (o.layout == kDenseBitmap) v = dense_word(o, w0 + w);
-                else if (o.layout == kDenseBytemap) v = bytemap_word(o, w0 + w);
-            }
-            slots[i * TW + w] = v;
-        }
-    }
-    __syncthreads();
-    for (uint32_t i = 0; i < nop; ++i) {
-        const OperandInfo& o = s_op[i];
-        if (o.layout == kSparseBitmap || o.layout == kSparsePacked) {
-            uint16_t* units = reinterpret_cast<uint16_t*>(slots + i * TW);
-            for (int32_t e = o.lo + static_cast<int32_t>(t); e < o.hi; e += kTile) {
-                uint32_t unit, mask;
-                if (o.layout == kSparseBitmap) {
-                    unit = ld32(o.addr + 8 + 4u * e) / 2u;
-                    mask = ld16(o.addr + 8 + 4u * o.k + 2u * e);
-                } else {
-                    const uint32_t w = ld32(o.addr + 8 + 4u * e);
-                    unit = w >> 16;
-                    mask = w & 0xffffu;
-                }
-                const uint32_t rel = unit - w0 * 4u;
-                if (rel < nw * 4u) units[rel] = static_cast<uint16_t>(mask);
-            }
-        } else if (o.layout == kSparseIdList) {
-            uint32_t* bits = reinterpret_cast<uint32_t*>(slots + i * TW);
-            for (uint32_t e = t; e < o.k; e += kTile) {
-                const uint32_t id = ld32(o.addr + 8 + 4u * e);
-                const uint32_t rel = id - w0 * 64u;
-                if (id < seg_docs && rel < nw * 64u) atomicOr(bits + rel / 32, 1u << (rel % 32));
-            }
         }
     }
     __syncthreads();
 
     const bool bad_posting = s_bad != 0;
-    uint64_t res[WPT];
-    const bool bad = bad_posting || !eval_words<WPT>(s_prog, plen, slots, TW, t, kTile, nop, res);
+    bool bad = false;
     uint32_t c = 0;
+    // the operands' set-up is shared by the CTA's tiles
+    for (uint32_t tile = tile0; tile < tile1; ++tile) {
+        const uint32_t w0 = tile * TW, nw = min(TW, seg_words - w0);
+        if (tile > tile0) __syncthreads();  // the slots are read
+        // bytemaps: each thread its own words; sparse (and all-zero) postings: zero, then scatter below
+        for (uint32_t i = 0; i < nop; ++i) {
+            const OperandInfo& o = s_op[i];
+            if (o.layout == kDenseBitmap) continue;  // uniform
 #pragma unroll
-    for (int k = 0; k < WPT; ++k) {
-        const uint32_t w = k * kTile + t;
-        if (w >= nw) continue;
-        const uint64_t r = bad ? 0ull : res[k] & tail_mask(gw0 + w, L.doc_num);
-        out_row[gw0 + w] = r;
-        c += __popcll(r);
+            for (int k = 0; k < WPT; ++k) {
+                const uint32_t w = k * kTile + t;
+                slots[i * TW + w] = o.layout == kDenseBytemap && w < nw ? bytemap_word(o, w0 + w) : 0ull;
+            }
+        }
+        __syncthreads();
+        for (uint32_t i = 0; i < nop; ++i) {
+            const OperandInfo& o = s_op[i];
+            if (o.layout == kSparseBitmap || o.layout == kSparsePacked) {
+                uint16_t* units = reinterpret_cast<uint16_t*>(slots + i * TW);
+                const bool packed = o.layout == kSparsePacked;
+#pragma unroll 4
+                for (uint32_t e = t; e < o.k; e += kTile) {
+                    const uint32_t x = ld32(o.addr + 8 + 4u * e);
+                    const uint32_t mask = packed ? x & 0xffffu : ld16(o.addr + 8 + 4u * o.k + 2u * e);
+                    const uint32_t rel = (packed ? x >> 16 : x / 2u) - w0 * 4u;
+                    if (rel < nw * 4u) units[rel] = static_cast<uint16_t>(mask);
+                }
+            } else if (o.layout == kSparseIdList) {
+                uint32_t* bits = reinterpret_cast<uint32_t*>(slots + i * TW);
+#pragma unroll 4
+                for (uint32_t e = t; e < o.k; e += kTile) {
+                    const uint32_t id = ld32(o.addr + 8 + 4u * e);
+                    const uint32_t rel = id - w0 * 64u;
+                    if (id < seg_docs && rel < nw * 64u) atomicOr(bits + rel / 32, 1u << (rel % 32));
+                }
+            }
+        }
+        __syncthreads();
+
+        auto operand = [&](uint32_t i, uint64_t (&v)[WPT]) {
+            const OperandInfo& o = s_op[i];
+            if (o.layout == kDenseBitmap) {
+#pragma unroll
+                for (int k = 0; k < WPT; ++k) v[k] = k * kTile + t < nw ? dense_word(o, w0 + k * kTile + t) : 0ull;
+            } else {
+#pragma unroll
+                for (int k = 0; k < WPT; ++k) v[k] = slots[i * TW + k * kTile + t];
+            }
+        };
+        uint64_t res[WPT];
+        bad = bad_posting || !eval_words<WPT>(s_prog, plen, operand, nop, res);
+#pragma unroll
+        for (int k = 0; k < WPT; ++k) {
+            const uint32_t w = k * kTile + t;
+            if (w >= nw) continue;
+            const uint64_t r = bad ? 0ull : res[k] & tail_mask(seg_w0 + w0 + w, L.doc_num);
+            out_row[seg_w0 + w0 + w] = r;
+            c += __popcll(r);
+        }
     }
     if (L.pass_count) {
         c = warp_sum(c);
         if ((t & 31) == 0 && c) atomicAdd(L.pass_count + q, c);
     }
-    if (L.status && bad && t < nw) atomicOr(L.status + q, bad_posting ? kStatusBadPosting : kStatusBadProgram);
+    if (L.status && bad && t == 0) atomicOr(L.status + q, bad_posting ? kStatusBadPosting : kStatusBadProgram);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -436,7 +417,13 @@ __global__ void __launch_bounds__(kDenseT) filter_dense_kernel(DenseFilterLaunch
     cp_async_wait_all();
     __syncthreads();
     uint64_t res[WPT];
-    const bool bad = !eval_words<WPT>(s_prog, plen, dslots, TW, t, kDenseT, nop, res);
+    const bool bad = !eval_words<WPT>(
+        s_prog, plen,
+        [&](uint32_t i, uint64_t (&v)[WPT]) {
+#pragma unroll
+            for (int k = 0; k < WPT; ++k) v[k] = dslots[i * TW + k * kDenseT + t];
+        },
+        nop, res);
     uint32_t c = 0;
 #pragma unroll
     for (int k = 0; k < WPT; ++k) {
@@ -708,11 +695,7 @@ __global__ void __launch_bounds__(256) posting_expand_kernel(const uint64_t* src
     __shared__ int bad;
     if (threadIdx.x == 0) {
         bad = 0;
-        resolve_operand(o, addr, seg_docs, 0u, 0xffffffffu, &bad);
-        if (o.layout == kSparseBitmap || o.layout == kSparsePacked) {
-            o.lo = 0;
-            o.hi = static_cast<int32_t>(o.k);
-        }
+        resolve_operand(o, addr, seg_docs, &bad);
     }
     __syncthreads();
     if (bad && threadIdx.x == 0 && status) atomicOr(status, kStatusBadPosting);
@@ -728,7 +711,7 @@ __global__ void __launch_bounds__(256) posting_expand_kernel(const uint64_t* src
     __syncthreads();
     if (o.layout == kSparseBitmap || o.layout == kSparsePacked) {
         uint16_t* units = reinterpret_cast<uint16_t*>(out);
-        for (int32_t e = threadIdx.x; e < o.hi; e += blockDim.x) {
+        for (uint32_t e = threadIdx.x; e < o.k; e += blockDim.x) {
             uint32_t unit, mask;
             if (o.layout == kSparseBitmap) {
                 unit = ld32(o.addr + 8 + 4u * e) / 2u;
@@ -755,7 +738,11 @@ cudaError_t launch_filter_wpt(const FilterLaunch& L, cudaStream_t stream) {
     constexpr uint32_t TW = kTile * WPT;
     const uint32_t seg_words = L.docs_per_seg / 64;
     const uint32_t tiles = (seg_words + TW - 1) / TW;
-    const uint64_t gy = static_cast<uint64_t>(L.seg_num) * tiles;
+    // a CTA takes up to 4 tiles of a segment, sharing its set-up (half of a tile's time), where that
+    // still leaves four waves of four CTAs per SM (fewer idle in the last one)
+    uint32_t tpc = 4;
+    while (tpc > 1 && static_cast<uint64_t>(L.nq) * L.seg_num * ((tiles + tpc - 1) / tpc) < 4 * 148 * 4) tpc >>= 1;
+    const uint64_t gy = static_cast<uint64_t>(L.seg_num) * ((tiles + tpc - 1) / tpc);
     if (gy > 65535u) return cudaErrorInvalidValue;
     const size_t smem = static_cast<size_t>(L.max_opnd > 0 ? L.max_opnd : 1) * TW * sizeof(uint64_t);
     // opt in always (static plus dynamic shared memory may pass 48 KB even when the dynamic part does
@@ -765,21 +752,26 @@ cudaError_t launch_filter_wpt(const FilterLaunch& L, cudaStream_t stream) {
                                          static_cast<int>(kFilterSmemCeiling));
     if (e != cudaSuccess) return e;
     dim3 grid(L.nq, static_cast<uint32_t>(gy));
-    filter_batch_kernel<WPT><<<grid, kTile, smem, stream>>>(L);
+    filter_batch_kernel<WPT><<<grid, kTile, smem, stream>>>(L, tpc);
     return cudaGetLastError();
 }
 
 }  // namespace
 
-// The tile is as wide as the segment allows (up to 2048 words = 131072 docs) while the operand slots
-// stay within 96 KB of shared memory.
+// The widest tile (8, 4, 2 or 1 words a thread) whose operand slots stay within 52 KB of shared memory, so
+// that four CTAs share an SM (within what the segment and the grid's height allow).
 cudaError_t launch_filter_batch(const FilterLaunch& L, cudaStream_t stream) {
     if (L.nq == 0 || L.seg_num == 0) return cudaSuccess;
     if (L.max_opnd > static_cast<uint32_t>(kMaxOperands)) return cudaErrorInvalidValue;
     const uint32_t seg_words = L.docs_per_seg / 64;
     const size_t per_word = static_cast<size_t>(L.max_opnd > 0 ? L.max_opnd : 1) * sizeof(uint64_t);
+    auto tiles = [&](int w) {
+        return static_cast<uint64_t>(L.seg_num) * ((seg_words + w * kTile - 1) / (w * kTile));
+    };
     int wpt = 8;
-    while (wpt > 1 && (static_cast<size_t>(wpt) * kTile * per_word > 96 * 1024 || static_cast<uint32_t>(wpt / 2) * kTile >= seg_words))
+    while (wpt > 1 && (static_cast<size_t>(wpt) * kTile * per_word > 52 * 1024 ||
+                       static_cast<uint32_t>(wpt / 2) * kTile >= seg_words) &&
+           !(tiles(wpt / 2) > 65535u && static_cast<size_t>(wpt) * kTile * per_word <= 96 * 1024))
         wpt /= 2;
     switch (wpt) {
         case 8: return launch_filter_wpt<8>(L, stream);
