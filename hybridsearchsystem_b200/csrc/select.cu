@@ -323,7 +323,9 @@ __device__ __forceinline__ uint32_t load_list(HistSmem& S, const uint32_t* count
     *key_lo = lo;
     *key_hi = hi;
     *overflow = S.lost != 0;
-    return S.counter;
+    const uint32_t n = S.counter;
+    __syncthreads();  // every thread has read the count: the caller may clear it at once
+    return n;
 }
 
 // Sorts E keys per thread (key of index t + NT e in v[e]) of the first m / E threads descending:

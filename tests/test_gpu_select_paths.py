@@ -57,3 +57,26 @@ def test_select_paths_at_other_dims(torch_cuda, method, dim):
 @pytest.mark.parametrize("sample_docs,cap", [(512, 1 << 18), (4096, 8192), (60001, 1 << 18)])
 def test_small_samples_and_lists(torch_cuda, method, sample_docs, cap):
     _check(60001, 128, method, 17, [3, 128, 256, 257, 1024], sample_docs=sample_docs, cap=cap)
+
+
+@pytest.mark.parametrize("method", [0, 2], ids=["simt", "bf16"])
+@pytest.mark.parametrize("nq", [60, 200], ids=["one_cta", "two_ctas"])
+def test_lists_shorter_than_k_keep_every_entry(torch_cuda, method, nq):
+    # more than 512 candidates but fewer than K: no K-th best is sought, so the kernel goes from reading
+    # the list's length straight to clearing the counter that held it; every warp must have read it first
+    n, k = 60001, 3000
+    mix, vec, bits, table = _world(n, 128)
+    q = mix.queries(nq, seed=71)
+    exprs = data.make_filters(mix, nq, n_tags=(1, 2), seed=72, selectivity_range=(0.01, 0.045))
+    want_s, want_i, want_c = oracle.topk(q, exprs, np.full(nq, k, np.int32), vec, bits, threads=8)
+    assert ((want_c > 512) & (want_c < k)).sum() >= nq // 2
+    s = hss.FullRecallSearcher(table, max_batch=nq, method=method)
+    for _ in range(20):
+        for a, e in zip(q, exprs):
+            s.add_query(e, a, k)
+        scores, ids, counts = s.batch_search(out_stride=k)
+        assert (np.asarray(counts) == want_c).all()
+        for i in range(nq):
+            c = int(want_c[i])
+            assert (ids[i, :c] == want_i[i, :c]).all(), i
+            assert (scores[i, :c].view(np.uint32) == want_s[i, :c].view(np.uint32)).all(), i
