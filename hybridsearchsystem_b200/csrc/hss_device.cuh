@@ -69,7 +69,9 @@ __host__ __device__ inline float result_key_score(uint64_t k) { return key_float
 // Programmatic dependent launch: a kernel launched by launch_dependent (hss_kernels.h) may start while the
 // kernel before it on the stream still runs, as soon as each of that kernel's CTAs has called
 // launch_dependents() or returned. Until wait_for_previous() returns, it must not touch global memory
-// that an earlier kernel reads or writes; after it, every earlier kernel has completed.
+// that an earlier kernel reads or writes; after it, every earlier kernel has completed. The compiler
+// must see that too: no __restrict__ parameter and no __ldg for memory that an earlier kernel writes
+// (either makes the load a read-only one, which may be moved above the wait).
 __device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 

@@ -221,8 +221,8 @@ __device__ __forceinline__ void tile_of(int64_t tile, int N, int* m0, int* n0) {
 }
 
 // A hidden layer of the training pass: Z = A W + b, act = gelu(Z).
-__global__ void __launch_bounds__(kGroup) layer_forward_kernel(Product P, const float* __restrict__ bias,
-                                                               float* __restrict__ Z, float* __restrict__ act) {
+__global__ void __launch_bounds__(kGroup) layer_forward_kernel(Product P, const float* bias,
+                                                               float* Z, float* act) {
     extern __shared__ __align__(16) float gsm[];
     launch_dependents();
     wait_for_previous();
@@ -247,11 +247,11 @@ constexpr int kHeadRows = 8;
 constexpr int kHeadT = 256;
 constexpr int kHeadK = 256;
 
-__global__ void __launch_bounds__(kHeadT) head_kernel(const float* __restrict__ A2, const float* __restrict__ Z2,
-                                                      const float* __restrict__ w3, const float* __restrict__ b3,
-                                                      const float* __restrict__ target, int B, int H, float tau,
-                                                      float* __restrict__ dy, float* __restrict__ term,
-                                                      float* __restrict__ dZ2) {
+__global__ void __launch_bounds__(kHeadT) head_kernel(const float* A2, const float* Z2,
+                                                      const float* w3, const float* b3,
+                                                      const float* target, int B, int H, float tau,
+                                                      float* dy, float* term,
+                                                      float* dZ2) {
     __shared__ float sa[kHeadRows][kHeadK + 1];
     __shared__ float sw[kHeadK];
     __shared__ float sdy[kHeadRows];
@@ -302,12 +302,12 @@ __global__ void __launch_bounds__(kHeadT) head_kernel(const float* __restrict__ 
 // Gradients of the output and second hidden layer, one grid: tiles [0, tilesA) dZ1 = (dZ2 W2^T) *
 // gelu'(Z1), then tilesW of dW2 = A1^T dZ2 (those of the first 32 rows also db2, the columns' sums of
 // dZ2), then blocks of 32 outputs of dw3 = A2^T dy (the first also db3 = sum dy).
-__global__ void __launch_bounds__(kGradThreads) grad_hidden_kernel(Product dA, const float* __restrict__ Z1,
-                                                                   float* __restrict__ dZ1, int64_t tilesA, Product dW,
-                                                                   float* __restrict__ gW2, float* __restrict__ gb2,
-                                                                   int64_t tilesW, const float* __restrict__ A2,
-                                                                   const float* __restrict__ dy, int B, int H,
-                                                                   float* __restrict__ gw3, float* __restrict__ gb3) {
+__global__ void __launch_bounds__(kGradThreads) grad_hidden_kernel(Product dA, const float* Z1,
+                                                                   float* dZ1, int64_t tilesA, Product dW,
+                                                                   float* gW2, float* gb2,
+                                                                   int64_t tilesW, const float* A2,
+                                                                   const float* dy, int B, int H,
+                                                                   float* gw3, float* gb3) {
     extern __shared__ __align__(16) float gsm[];
     launch_dependents();
     wait_for_previous();
@@ -354,8 +354,8 @@ __global__ void __launch_bounds__(kGradThreads) grad_hidden_kernel(Product dA, c
 }
 
 // dW1 = X^T dZ1, db1 = the columns' sums of dZ1.
-__global__ void __launch_bounds__(kGradThreads) grad_input_kernel(Product dW, float* __restrict__ gW1,
-                                                                  float* __restrict__ gb1) {
+__global__ void __launch_bounds__(kGradThreads) grad_input_kernel(Product dW, float* gW1,
+                                                                  float* gb1) {
     extern __shared__ __align__(16) float gsm[];
     launch_dependents();
     wait_for_previous();

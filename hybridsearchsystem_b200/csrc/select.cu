@@ -941,7 +941,7 @@ __global__ void __launch_bounds__(256) aggregate_count_kernel(const uint64_t* __
 }
 
 // Exclusive scan of nb block counts in place (one CTA).
-__global__ void __launch_bounds__(1024) aggregate_scan_kernel(uint32_t* __restrict__ block_count, uint32_t nb) {
+__global__ void __launch_bounds__(1024) aggregate_scan_kernel(uint32_t* block_count, uint32_t nb) {
     __shared__ uint32_t warp_tot[32];
     __shared__ uint32_t carry;
     launch_dependents();
@@ -980,13 +980,13 @@ __global__ void __launch_bounds__(1024) aggregate_scan_kernel(uint32_t* __restri
 }
 
 template <int MODE>
-__global__ void __launch_bounds__(kAggT) aggregate_scatter_kernel(const uint64_t* __restrict__ bits,
-                                                                  const float* __restrict__ scores,
-                                                                  const uint32_t* __restrict__ loc_in, uint32_t n,
-                                                                  const uint32_t* __restrict__ blocks,
-                                                                  float* __restrict__ out_scores,
-                                                                  uint32_t* __restrict__ out_loc,
-                                                                  uint32_t* __restrict__ total) {
+__global__ void __launch_bounds__(kAggT) aggregate_scatter_kernel(const uint64_t* bits,
+                                                                  const float* scores,
+                                                                  const uint32_t* loc_in, uint32_t n,
+                                                                  const uint32_t* blocks,
+                                                                  float* out_scores,
+                                                                  uint32_t* out_loc,
+                                                                  uint32_t* total) {
     __shared__ uint32_t wsum[kAggT / 32];
     __shared__ uint32_t woff[kAggWords];
     __shared__ uint64_t wbits[kAggWords];
@@ -999,7 +999,7 @@ __global__ void __launch_bounds__(kAggT) aggregate_scatter_kernel(const uint64_t
         // whole words below the block; the bitmap is only 8-byte aligned
         const uint32_t words = b * kAggWords;
 #pragma unroll 8
-        for (uint32_t w = t; w < words; w += kAggT) before += __popcll(__ldg(bits + w));
+        for (uint32_t w = t; w < words; w += kAggT) before += __popcll(bits[w]);
     } else if (MODE == kAggSums) {
         for (uint32_t i = t; i < b; i += kAggT) before += blocks[i];
     } else if (t == 0) {
@@ -1075,11 +1075,11 @@ __global__ void __launch_bounds__(kAggT) aggregate_scatter_kernel(const uint64_t
 // 131,072 scores; 16 CTAs take 11 us.
 constexpr uint32_t kTopkSample = 65536;
 
-__global__ void __launch_bounds__(kST) topk_op_kernel(const float* __restrict__ scores,
-                                                      const uint32_t* __restrict__ locs,
-                                                      const uint32_t* __restrict__ count, uint32_t k,
-                                                      float* __restrict__ out_scores, uint32_t* __restrict__ out_locs,
-                                                      uint32_t* __restrict__ out_count) {
+__global__ void __launch_bounds__(kST) topk_op_kernel(const float* scores,
+                                                      const uint32_t* locs,
+                                                      const uint32_t* count, uint32_t k,
+                                                      float* out_scores, uint32_t* out_locs,
+                                                      uint32_t* out_count) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     SelectSmem& S = *reinterpret_cast<SelectSmem*>(smem_raw);
     cg::cluster_group cluster = cg::this_cluster();
@@ -1205,9 +1205,9 @@ __global__ void __launch_bounds__(kST) topk_op_kernel(const float* __restrict__ 
 // Per-query error bounds: eps = c * ||q||_2 * max_doc ||v||_2 (Cauchy-Schwarz on sum |q_i v_i|),
 // computed in double and rounded up to float.
 // Bounds of queries qlist[0..nq) (or 0..nq-1 when qlist is null), written at the query's own index.
-__global__ void query_eps_kernel(const float* __restrict__ qry, const uint32_t* __restrict__ qlist, uint32_t nq,
+__global__ void query_eps_kernel(const float* qry, const uint32_t* qlist, uint32_t nq,
                                  uint32_t dim, float max_norm, double c_main, double c_sample,
-                                 float* __restrict__ eps_main, float* __restrict__ eps_sample) {
+                                 float* eps_main, float* eps_sample) {
     // beside the batch's filter, as stage_queries_kernel
     launch_dependents();
     const uint32_t r = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
