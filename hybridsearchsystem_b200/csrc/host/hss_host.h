@@ -575,6 +575,7 @@ class FullRecallSearcher {
                     float* thetaCopy = nullptr, const float* emitTheta = nullptr);
     uint32_t MaximaGroups(uint32_t rows, uint64_t count, bool simt, uint32_t* docs) const;
     uint64_t SampleOptimum(uint32_t nq, uint32_t maxK) const;
+    bool SplitSelect(uint32_t nq, uint32_t maxK) const;
     bool OnePass(uint32_t nq, uint32_t maxK, uint64_t sampled) const;
     void SampleTiles(uint64_t want, uint32_t rows, bool simt, uint64_t* count, uint64_t* step) const;
     // A batch's small inputs in the pinned staging buffer: per-query program and operand offsets, K,

@@ -809,6 +809,20 @@ uint64_t FullRecallSearcher::SampleOptimum(uint32_t nq, uint32_t maxK) const {
     return static_cast<uint64_t>(std::min(s, n / 8));
 }
 
+// Whether the select step spreads its rescoring over the device (three kernels) instead of leaving each
+// query's rows to its CTA. It pays where a query has more rows, or longer ones, than its SM can read in
+// the time the rest of the batch takes (us a batch, one CTA a query -> spread):
+//   8-bit form, whose error band grows with the row: 768 dims, 300k docs, 128 queries, K 10 1070 -> 398,
+//   K 100 9545 -> 1740; 384 dims, 4 queries, K 10 159 -> 91; 256 dims, K 100 1157 -> 878; 128 dims, 256
+//   queries, K 300 920 -> 901. Not 256 dims, 128 queries, K 10 (263 -> 281) nor 128 dims, K 200 (757 -> 777).
+//   Other forms, batches that leave SMs idle: 768 dims, K 1000: 1 query 537 -> 445, 64 queries 576 -> 528.
+//   Not 256 queries, K 700 (713 -> 750), nor rows of 128 dims (bf16, 64 queries, K 1000 629 -> 632).
+bool FullRecallSearcher::SplitSelect(uint32_t nq, uint32_t maxK) const {
+    const uint64_t dim = m_table->GetDimension(), floats = maxK * dim;
+    if (m_tcFormat == kTcE4M3) return dim >= 384 || floats >= (dim >= 256 ? 25600u : 32768u);
+    return nq <= 64 && floats >= 1ull << 19;
+}
+
 // Whether the corpus is passed over once, at the sample's threshold, instead of in two parts with the
 // threshold raised between them. One pass keeps about K N / s docs per query, two 2 K sqrt(N / s); the
 // second launch, the raise and the gap cost about as much as keeping 400,000 more docs (300,000 docs, 256
@@ -1046,6 +1060,12 @@ int FullRecallSearcher::EnqueueAttempt(uint32_t nq, const BatchInputs& in, float
     // a batch with a large K keeps long candidate lists (K = 1000: about 13k per query at 10M, past
     // the default shared-memory buffer): select K from {10, 100, 1000} 0.302 -> 0.199 ms
     SE.fast_large = maxK > 256 ? 1 : 0;
+    // in the sample's counts, which nothing reads any more (the spread rescoring reads the queries 16
+    // bytes at a time)
+    static_assert(kMaxCandSegs * 4 >= sizeof(uint2), "a query's pending rows fit where its counts were");
+    SE.pending = SplitSelect(nq, maxK) && (reinterpret_cast<uintptr_t>(dQueries) & 15u) == 0
+                     ? reinterpret_cast<uint2*>(D + SL.sampCount)
+                     : nullptr;
     // With a model, theta is the prediction: the passes below run at it (raised like a proven one
     // when pass A's K-th best allows), and the select step checks every query whose theta stayed
     // above its proven threshold; a query that fails is re-run at a proven threshold.
@@ -1086,7 +1106,7 @@ int FullRecallSearcher::EnqueueAttempt(uint32_t nq, const BatchInputs& in, float
 
     // 3. exact rescoring and the top K
     Ck(launch_select_topk(SE, stream));
-    ++m_b.launches;
+    m_b.launches += SE.pending ? 3 : 1;
     if (m_timing) Ck(cudaEventRecord(m_ev[4], stream));
     // the statuses that decide re-runs (and the tensor-core pass's error bits), on the host when
     // m_evStatus (recorded by the caller) completes
@@ -1211,7 +1231,7 @@ int FullRecallSearcher::SearchFinish() {
         SE.qlist = dQlist;
         SE.nq_list = nre;
         Ck(launch_select_topk(SE, stream));
-        m_b.launches += 2;
+        m_b.launches += SE.pending ? 4 : 2;
     }
     if (tc && m_b.ce == cudaSuccess) {
         // the copy made with the statuses covers the first attempt; re-runs need a fresh one (stream

@@ -198,6 +198,9 @@ struct SelectLaunch {
     int32_t* status;
     const uint32_t* qlist;
     uint32_t nq_list;
+    // [nq] or null: the rows to rescore (work from .x to .y) between the step's first kernel and the others;
+    // given, the step takes three kernels, with the rescoring spread over the whole device
+    uint2* pending;
     int fast_large;            // hold up to 32,768 candidate scores in shared memory (else 8,192)
 };
 

@@ -636,7 +636,7 @@ __device__ __forceinline__ void rescore_rows(const float* sq, const float* vec, 
                                              Put put) {
     const uint32_t lane = threadIdx.x & 31, j = lane & 3;
     const uint32_t quads = dim / 4;
-    for (uint32_t r0 = (threadIdx.x >> 5) * 8; r0 < m; r0 += NT / 4) {
+    for (uint32_t r0 = NT == 32 ? 0 : (threadIdx.x >> 5) * 8; r0 < m; r0 += NT / 4) {  // NT = 32: one warp's rows
         const uint32_t r = r0 + (lane >> 2);
         const bool ok = r < m;
         const uint32_t loc = list(ok ? r : r0);
@@ -681,167 +681,27 @@ __device__ __forceinline__ void rescore_rows(const float* sq, const float* vec, 
     }
 }
 
-// ---------------------------------------------------------------------------------------------
-// The select step, one CTA per query: a chain of dependent steps and the rescoring's row reads bound it.
-//   * The list's scores are read once into shared memory (`fast` entries), the first locations with them.
-//   * A list of at most kSelT entries is rescored whole; a longer one is cut: t~ bounds the K-th
-//     best approximate score from below, so only entries of at least t~ - 2 eps can be in the top K. Where
-//     those are more than kSelT, the entries of at least t~ (K of them at least) are rescored
-//     first: the least of their exact scores, s, bounds the K-th exact score, and the rest needs only
-//     s - eps, about half the band.
-//   * Survivors are packed before they are rescored, so that every lane group has a row.
-template <int NT, uint32_t FAST>
-__global__ void __launch_bounds__(NT, NT == kSelT ? 2 : 1) select_topk_kernel(SelectLaunch L) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    SelectSmem& S = *reinterpret_cast<SelectSmem*>(smem_raw);
-    float* sq = reinterpret_cast<float*>(smem_raw + sizeof(SelectSmem));
-    float* cs = reinterpret_cast<float*>(smem_raw + select_cand_offset(L.dim));
-    uint32_t* surv = S.hist;  // survivors' locations: after the last digit
-    launch_dependents();
-    wait_for_previous();
-    const uint32_t qi = L.qlist ? L.qlist[blockIdx.x] : blockIdx.x;
+// A threshold above the proven one (a prediction) has to be checked: the list holds every doc
+// with s~ >= theta, so a doc left out scores s < theta + eps, and the K best candidates are the
+// K best docs when their K-th exact score s_K >= theta + eps. A query that fails goes back to a
+// proven threshold: the larger of its proven one and s_K - eps (every true top-K doc scores at
+// least s_K, the candidates' K-th best, hence s~ >= s_K - eps).
+__device__ __forceinline__ void threshold_miss(const SelectLaunch& L, uint32_t qi, float raised) {
+    if (threadIdx.x == 0) {
+        const float t = fmaxf(L.theta_proven[qi], raised);
+        L.theta[qi] = t;
+        L.theta_proven[qi] = t;
+        L.out_count[qi] = 0;
+        atomicOr(L.status + qi, kStatusOverflow | kStatusThresholdMiss);
+    }
+}
+
+// The end of the select step: the nf keys of a query (in S.sortbuf, or in ws) sorted, a predicted threshold
+// checked, the first kq results written.
+template <int NT>
+__device__ __forceinline__ void finish_select(SelectSmem& S, const SelectLaunch& L, uint32_t qi, uint32_t k, uint32_t kq,
+                                              uint32_t nf, bool in_smem, const unsigned long long* ws) {
     const uint32_t tid = threadIdx.x;
-    const uint32_t k = L.topk[qi];
-    const uint64_t row = static_cast<uint64_t>(qi) * L.cap;
-    if (k > static_cast<uint32_t>(kMaxTopK)) {
-        if (tid == 0) {
-            L.out_count[qi] = 0;
-            atomicOr(L.status + qi, kStatusTopKTooLarge);
-        }
-        return;
-    }
-    const uint32_t* counts = L.cand_count + static_cast<uint64_t>(qi) * kMaxCandSegs;
-    const float* sc = L.cand_score + row;
-    const uint32_t* lc = L.cand_loc + row;
-    const float eps = L.eps_main[qi];
-    const float theta_q = L.theta[qi];
-    for (uint32_t i = tid; i < L.dim; i += NT) sq[i] = L.qry[static_cast<uint64_t>(qi) * L.dim + i];
-    bool overflow = false;
-    uint32_t key_lo, key_hi;
-    const uint32_t n = load_list<NT>(S, counts, L.segs, L.seg_cap, sc, lc, cs, FAST, S.locs, &overflow, &key_lo, &key_hi);
-    auto visit_keys = [&](auto fn) {
-        if (n <= FAST) {
-            for (uint32_t i = tid; i < n; i += NT) fn(float_key(cs[i]));
-        } else {
-            walk_segments<NT>(counts, L.segs, L.seg_cap, sc, [](uint32_t) {}, [&](uint32_t, bool ok, float v) {
-                if (ok) fn(float_key(v));
-            });
-        }
-    };
-    // A threshold above the proven one (a prediction) has to be checked: the list holds every doc
-    // with s~ >= theta, so a doc left out scores s < theta + eps, and the K best candidates are the
-    // K best docs when their K-th exact score s_K >= theta + eps. A query that fails goes back to a
-    // proven threshold: the larger of its proven one and s_K - eps (every true top-K doc scores at
-    // least s_K, the candidates' K-th best, hence s~ >= s_K - eps).
-    const bool unproven = L.theta_proven != nullptr && theta_q > L.theta_proven[qi];
-    auto threshold_miss = [&](float raised) {
-        if (tid == 0) {
-            const float t = fmaxf(L.theta_proven[qi], raised);
-            L.theta[qi] = t;
-            L.theta_proven[qi] = t;
-            L.out_count[qi] = 0;
-            atomicOr(L.status + qi, kStatusOverflow | kStatusThresholdMiss);
-        }
-    };
-    if (overflow) {
-        // The stored candidates are a subset of the qualifying docs, so their K-th best still bounds
-        // the true K-th best from below: raise the threshold and let the host re-run this query.
-        float theta = unproven ? L.theta_proven[qi] : theta_q;
-        if (n >= k && k > 0) {
-            const uint32_t kk = kth_lower_bound<NT>(visit_keys, k, key_lo, key_hi, S);
-            theta = fmaxf(theta, __fsub_rd(key_float(kk), 2.0f * eps));
-        }
-        __syncthreads();  // every thread has read the old thresholds
-        if (tid == 0) {
-            L.theta[qi] = theta;
-            if (L.theta_proven) L.theta_proven[qi] = theta;
-            L.out_count[qi] = 0;
-            atomicOr(L.status + qi, kStatusOverflow);
-        }
-        return;
-    }
-    if (n == 0 || k == 0) {
-        if (unproven && k > 0) {
-            threshold_miss(-INFINITY);
-            return;
-        }
-        if (tid == 0) L.out_count[qi] = 0;
-        return;
-    }
-    const uint32_t kq = min(k, n);
-    unsigned long long* ws = L.work + row;
-    uint32_t nf;
-    bool in_smem;  // the keys: S.sortbuf or ws
-    if (n <= static_cast<uint32_t>(kSelT)) {
-        rescore_rows<NT>(sq, L.vec, L.dim, n, [&](uint32_t i) { return S.locs[i]; },
-                         [&](uint32_t i, uint32_t loc, float e) { S.sortbuf[i] = result_key(e, loc); });
-        nf = n;
-        in_smem = true;
-    } else {
-        const float t = n > kq ? key_float(kth_lower_bound<NT>(visit_keys, kq, key_lo, key_hi, S)) : -INFINITY;
-        const float cut2 = __fsub_rd(t, 2.0f * eps);
-        // fn(score, location) of every entry
-        auto visit_entries = [&](auto fn) {
-            if (n <= min(FAST, static_cast<uint32_t>(kMaxTopK))) {
-                for (uint32_t i = tid; i < n; i += NT) fn(cs[i], [&] { return S.locs[i]; });
-            } else {
-                walk_segments<NT>(counts, L.segs, L.seg_cap, sc, [](uint32_t) {}, [&](uint32_t at, bool ok, float v) {
-                    if (ok) fn(v, [&] { return lc[at]; });
-                });
-            }
-        };
-        // how many clear the cut at all
-        if (tid == 0) S.counter = 0;
-        __syncthreads();
-        uint32_t mine = 0;
-        visit_keys([&](uint32_t key) { mine += key_float(key) >= cut2 ? 1u : 0u; });
-        mine = warp_sum(mine);
-        if ((tid & 31) == 0 && mine) atomicAdd(&S.counter, mine);
-        __syncthreads();
-        const uint32_t all = S.counter;
-        const bool two = all > static_cast<uint32_t>(kSelT) && all > kq && t > -INFINITY;
-        float lo = two ? t : cut2, hi = INFINITY, low_exact = INFINITY;
-        nf = 0;
-        in_smem = all <= static_cast<uint32_t>(kMaxTopK);
-        for (int wave = 0; wave < (two ? 2 : 1); ++wave) {
-            __syncthreads();  // the survivors' list is free
-            if (tid == 0) S.total = 0;
-            __syncthreads();
-            const bool last = !two || wave == 1;
-            visit_entries([&](float v, auto loc) {
-                if (v >= lo && (wave == 0 || v < hi)) {
-                    const uint32_t at = next_place(&S.total);
-                    if (in_smem)
-                        surv[at] = loc();
-                    else
-                        ws[nf + at] = loc();
-                }
-            });
-            __syncthreads();
-            const uint32_t m = S.total;
-            float least = INFINITY;
-            rescore_rows<NT>(
-                sq, L.vec, L.dim, m,
-                [&](uint32_t i) { return in_smem ? surv[i] : static_cast<uint32_t>(ws[nf + i]); },
-                [&](uint32_t i, uint32_t loc, float e) {
-                    const unsigned long long key = result_key(e, loc);
-                    if (in_smem)
-                        S.sortbuf[nf + i] = key;
-                    else
-                        ws[nf + i] = key;
-                    least = fminf(least, e);
-                });
-            nf += m;
-            if (last) break;
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) least = fminf(least, __shfl_xor_sync(0xffffffffu, least, o));
-            if ((tid & 31) == 0) S.wsum[tid >> 5] = float_bits(least);
-            __syncthreads();
-            for (int w = 0; w < NT / 32; ++w) low_exact = fminf(low_exact, bits_float(S.wsum[w]));
-            hi = t;
-            lo = fmaxf(cut2, __fsub_rd(low_exact, eps));
-        }
-    }
     __syncthreads();
     uint32_t m;
     const unsigned long long* sorted = S.sortbuf;
@@ -884,10 +744,12 @@ __global__ void __launch_bounds__(NT, NT == kSelT ? 2 : 1) select_topk_kernel(Se
         m = gather_top_keys<NT>([&](uint32_t i) { return static_cast<uint64_t>(ws[i]); }, nf, kq, S);
     }
     if (m) bitonic_desc<NT>(S, m);
-    if (unproven) {
-        const float lo = kq == k && nf >= kq ? __fsub_rd(result_key_score(sorted[kq - 1]), eps) : -INFINITY;
-        if (!(lo >= theta_q)) {
-            threshold_miss(lo);
+    const float theta_q = L.theta[qi];
+    if (L.theta_proven != nullptr && theta_q > L.theta_proven[qi]) {
+        const float lo = kq == k && nf >= kq ? __fsub_rd(result_key_score(sorted[kq - 1]), L.eps_main[qi]) : -INFINITY;
+        if (!(lo >= theta_q)) {  // uniform
+            __syncthreads();  // every thread has read the thresholds
+            threshold_miss(L, qi, lo);
             return;
         }
     }
@@ -900,6 +762,247 @@ __global__ void __launch_bounds__(NT, NT == kSelT ? 2 : 1) select_topk_kernel(Se
         L.out_id[orow + i] = L.gdocid ? L.gdocid[loc] : static_cast<int64_t>(loc);
     }
     if (tid == 0) L.out_count[qi] = kout;
+}
+
+// ---------------------------------------------------------------------------------------------
+// The select step, one CTA per query: a chain of dependent steps and the rescoring's row reads bound it.
+//   * The list's scores are read once into shared memory (`fast` entries), the first locations with them.
+//   * A list of at most kSelT entries is rescored whole; a longer one is cut: t~ bounds the K-th
+//     best approximate score from below, so only entries of at least t~ - 2 eps can be in the top K. Where
+//     those are more than kSelT, the entries of at least t~ (K of them at least) are rescored
+//     first: the least of their exact scores, s, bounds the K-th exact score, and the rest needs only
+//     s - eps, about half the band.
+//   * Survivors are packed before they are rescored, so that every lane group has a row.
+// SPLIT: the kernel ends with the survivors' list in L.work (and, of a list cut in two waves, the first
+// wave's keys): rescore_kernel scores the rest with all SMs, select_final_kernel sorts. A query's rows
+// are otherwise read by its own CTA, and the query with the most holds up the batch.
+template <int NT, uint32_t FAST, bool SPLIT>
+__global__ void __launch_bounds__(NT, NT == kSelT ? 2 : 1) select_topk_kernel(SelectLaunch L) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    SelectSmem& S = *reinterpret_cast<SelectSmem*>(smem_raw);
+    float* sq = reinterpret_cast<float*>(smem_raw + sizeof(SelectSmem));
+    float* cs = reinterpret_cast<float*>(smem_raw + select_cand_offset(L.dim));
+    uint32_t* surv = S.hist;  // survivors' locations: after the last digit
+    launch_dependents();
+    wait_for_previous();
+    const uint32_t qi = L.qlist ? L.qlist[blockIdx.x] : blockIdx.x;
+    const uint32_t tid = threadIdx.x;
+    const uint32_t k = L.topk[qi];
+    const uint64_t row = static_cast<uint64_t>(qi) * L.cap;
+    if (SPLIT && tid == 0) L.pending[qi] = make_uint2(1, 0);  // answered here, unless rows follow
+    if (k > static_cast<uint32_t>(kMaxTopK)) {
+        if (tid == 0) {
+            L.out_count[qi] = 0;
+            atomicOr(L.status + qi, kStatusTopKTooLarge);
+        }
+        return;
+    }
+    const uint32_t* counts = L.cand_count + static_cast<uint64_t>(qi) * kMaxCandSegs;
+    const float* sc = L.cand_score + row;
+    const uint32_t* lc = L.cand_loc + row;
+    const float eps = L.eps_main[qi];
+    const float theta_q = L.theta[qi];
+    for (uint32_t i = tid; i < L.dim; i += NT) sq[i] = L.qry[static_cast<uint64_t>(qi) * L.dim + i];
+    bool overflow = false;
+    uint32_t key_lo, key_hi;
+    const uint32_t n = load_list<NT>(S, counts, L.segs, L.seg_cap, sc, lc, cs, FAST, S.locs, &overflow, &key_lo, &key_hi);
+    auto visit_keys = [&](auto fn) {
+        if (n <= FAST) {
+            for (uint32_t i = tid; i < n; i += NT) fn(float_key(cs[i]));
+        } else {
+            walk_segments<NT>(counts, L.segs, L.seg_cap, sc, [](uint32_t) {}, [&](uint32_t, bool ok, float v) {
+                if (ok) fn(float_key(v));
+            });
+        }
+    };
+    const bool unproven = L.theta_proven != nullptr && theta_q > L.theta_proven[qi];
+    if (overflow) {
+        // The stored candidates are a subset of the qualifying docs, so their K-th best still bounds
+        // the true K-th best from below: raise the threshold and let the host re-run this query.
+        float theta = unproven ? L.theta_proven[qi] : theta_q;
+        if (n >= k && k > 0) {
+            const uint32_t kk = kth_lower_bound<NT>(visit_keys, k, key_lo, key_hi, S);
+            theta = fmaxf(theta, __fsub_rd(key_float(kk), 2.0f * eps));
+        }
+        __syncthreads();  // every thread has read the old thresholds
+        if (tid == 0) {
+            L.theta[qi] = theta;
+            if (L.theta_proven) L.theta_proven[qi] = theta;
+            L.out_count[qi] = 0;
+            atomicOr(L.status + qi, kStatusOverflow);
+        }
+        return;
+    }
+    if (n == 0 || k == 0) {
+        __syncthreads();  // every thread has read the thresholds
+        if (unproven && k > 0) {
+            threshold_miss(L, qi, -INFINITY);
+            return;
+        }
+        if (tid == 0) L.out_count[qi] = 0;
+        return;
+    }
+    const uint32_t kq = min(k, n);
+    unsigned long long* ws = L.work + row;
+    uint32_t nf;
+    bool in_smem;  // the keys: S.sortbuf or ws
+    if (SPLIT && n <= static_cast<uint32_t>(kSelT)) {
+        for (uint32_t i = tid; i < n; i += NT) ws[i] = S.locs[i];
+        __syncthreads();
+        if (tid == 0) L.pending[qi] = make_uint2(0, n);
+        return;
+    }
+    if (n <= static_cast<uint32_t>(kSelT)) {
+        rescore_rows<NT>(sq, L.vec, L.dim, n, [&](uint32_t i) { return S.locs[i]; },
+                         [&](uint32_t i, uint32_t loc, float e) { S.sortbuf[i] = result_key(e, loc); });
+        nf = n;
+        in_smem = true;
+    } else {
+        const float t = n > kq ? key_float(kth_lower_bound<NT>(visit_keys, kq, key_lo, key_hi, S)) : -INFINITY;
+        const float cut2 = __fsub_rd(t, 2.0f * eps);
+        // fn(score, location) of every entry
+        auto visit_entries = [&](auto fn) {
+            if (n <= min(FAST, static_cast<uint32_t>(kMaxTopK))) {
+                for (uint32_t i = tid; i < n; i += NT) fn(cs[i], [&] { return S.locs[i]; });
+            } else {
+                walk_segments<NT>(counts, L.segs, L.seg_cap, sc, [](uint32_t) {}, [&](uint32_t at, bool ok, float v) {
+                    if (ok) fn(v, [&] { return lc[at]; });
+                });
+            }
+        };
+        // how many clear the cut at all
+        if (tid == 0) S.counter = 0;
+        __syncthreads();
+        uint32_t mine = 0;
+        visit_keys([&](uint32_t key) { mine += key_float(key) >= cut2 ? 1u : 0u; });
+        mine = warp_sum(mine);
+        if ((tid & 31) == 0 && mine) atomicAdd(&S.counter, mine);
+        __syncthreads();
+        const uint32_t all = S.counter;
+        // (split: a first wave of K rows in this CTA pays where it spares the others many)
+        const bool two = all > (SPLIT ? 2 * kq + 256 : static_cast<uint32_t>(kSelT)) && all > kq && t > -INFINITY;
+        float lo = two ? t : cut2, hi = INFINITY, low_exact = INFINITY;
+        nf = 0;
+        in_smem = all <= static_cast<uint32_t>(kMaxTopK);
+        for (int wave = 0; wave < (two ? 2 : 1); ++wave) {
+            __syncthreads();  // the survivors' list is free
+            if (tid == 0) S.total = 0;
+            __syncthreads();
+            const bool last = !two || wave == 1;
+            visit_entries([&](float v, auto loc) {
+                if (v >= lo && (wave == 0 || v < hi)) {
+                    const uint32_t at = next_place(&S.total);
+                    if (in_smem)
+                        surv[at] = loc();
+                    else
+                        ws[nf + at] = loc();
+                }
+            });
+            __syncthreads();
+            const uint32_t m = S.total;
+            if (SPLIT && last) {
+                if (in_smem)
+                    for (uint32_t i = tid; i < m; i += NT) ws[nf + i] = surv[i];
+                if (tid == 0) L.pending[qi] = make_uint2(nf, nf + m);
+                return;
+            }
+            float least = INFINITY;
+            rescore_rows<NT>(
+                sq, L.vec, L.dim, m,
+                [&](uint32_t i) { return in_smem ? surv[i] : static_cast<uint32_t>(ws[nf + i]); },
+                [&](uint32_t i, uint32_t loc, float e) {
+                    const unsigned long long key = result_key(e, loc);
+                    if (in_smem && !SPLIT)
+                        S.sortbuf[nf + i] = key;
+                    else
+                        ws[nf + i] = key;
+                    least = fminf(least, e);
+                });
+            nf += m;
+            if (last) break;
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) least = fminf(least, __shfl_xor_sync(0xffffffffu, least, o));
+            if ((tid & 31) == 0) S.wsum[tid >> 5] = float_bits(least);
+            __syncthreads();
+            for (int w = 0; w < NT / 32; ++w) low_exact = fminf(low_exact, bits_float(S.wsum[w]));
+            hi = t;
+            lo = fmaxf(cut2, __fsub_rd(low_exact, eps));
+        }
+    }
+    finish_select<NT>(S, L, qi, k, kq, nf, in_smem, ws);
+}
+
+// Exact scores of every query's pending rows (L.work from L.pending.x to .y), eight rows to a warp, the
+// groups of eight dealt out evenly over all warps of the grid: bound by the rows' reads, where the query
+// with the most rows bound the one-kernel step (8-bit form, 768 dims, 300k docs, 128 queries, K 10: select
+// step 975 -> 239 us; K 100: 10.0 -> 1.37 ms).
+constexpr int kRescoreT = 256;
+
+__global__ void __launch_bounds__(kRescoreT, 4) rescore_kernel(SelectLaunch L) {
+    extern __shared__ uint32_t group_end[];  // [nq_list] groups of the queries up to and with this one
+    __shared__ uint32_t wsum[kRescoreT / 32];
+    launch_dependents();
+    wait_for_previous();
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    uint32_t carry = 0;
+    for (uint32_t i0 = 0; i0 < L.nq_list; i0 += kRescoreT) {
+        const uint32_t i = i0 + tid;
+        uint32_t x = 0;
+        if (i < L.nq_list) {
+            const uint2 p = L.pending[L.qlist ? L.qlist[i] : i];
+            x = p.y > p.x ? (p.y - p.x + 7) / 8 : 0u;
+        }
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= static_cast<uint32_t>(o)) x += y;
+        }
+        if (lane == 31) wsum[warp] = x;
+        __syncthreads();
+        uint32_t before = 0, all = 0;
+        for (uint32_t w = 0; w < kRescoreT / 32; ++w) {
+            if (w < warp) before += wsum[w];
+            all += wsum[w];
+        }
+        if (i < L.nq_list) group_end[i] = carry + before + x;
+        carry += all;
+        __syncthreads();
+    }
+    const uint32_t step = gridDim.x * (kRescoreT / 32);
+    for (uint32_t g = blockIdx.x * (kRescoreT / 32) + warp; g < carry; g += step) {
+        uint32_t lo = 0, hi = L.nq_list - 1;  // the first query whose end is past g
+        while (lo < hi) {
+            const uint32_t mid = (lo + hi) >> 1;
+            if (group_end[mid] > g)
+                hi = mid;
+            else
+                lo = mid + 1;
+        }
+        const uint32_t qi = L.qlist ? L.qlist[lo] : lo;
+        const uint2 p = L.pending[qi];
+        const uint32_t first = p.x + 8 * (g - (lo ? group_end[lo - 1] : 0u));
+        unsigned long long* ws = L.work + static_cast<uint64_t>(qi) * L.cap + first;
+        rescore_rows<32>(L.qry + static_cast<uint64_t>(qi) * L.dim, L.vec, L.dim, min(8u, p.y - first),
+                         [&](uint32_t i) { return static_cast<uint32_t>(ws[i]); },
+                         [&](uint32_t i, uint32_t loc, float e) { ws[i] = result_key(e, loc); });
+    }
+}
+
+// The keys of L.work sorted and written out, one CTA per query.
+__global__ void __launch_bounds__(kSelT, 2) select_final_kernel(SelectLaunch L) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    SelectSmem& S = *reinterpret_cast<SelectSmem*>(smem_raw);
+    launch_dependents();
+    wait_for_previous();
+    const uint32_t qi = L.qlist ? L.qlist[blockIdx.x] : blockIdx.x;
+    const uint2 p = L.pending[qi];
+    if (p.x > p.y) return;  // the first kernel has written this query's outcome
+    const uint32_t nf = p.y, k = L.topk[qi];
+    const unsigned long long* ws = L.work + static_cast<uint64_t>(qi) * L.cap;
+    const bool in_smem = nf <= static_cast<uint32_t>(kMaxTopK);
+    if (in_smem)
+        for (uint32_t i = threadIdx.x; i < nf; i += kSelT) S.sortbuf[i] = ws[i];
+    finish_select<kSelT>(S, L, qi, k, min(k, nf), nf, in_smem, ws);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -1283,10 +1386,18 @@ cudaError_t launch_select_topk(const SelectLaunch& L, cudaStream_t stream) {
     if (bad_segments(L.segs, L.seg_cap, L.cap) || L.segs > static_cast<uint32_t>(kST)) return cudaErrorInvalidValue;
     const bool wide = L.fast_large || L.nq_list <= kWideQueries;
     const size_t smem = select_cand_offset(L.dim) + (wide ? kFastLarge : kFast) * sizeof(float);
-    auto kernel = wide ? select_topk_kernel<kST, kFastLarge> : select_topk_kernel<kSelT, kFast>;
+    const bool split = L.pending != nullptr;
+    auto kernel = wide ? (split ? select_topk_kernel<kST, kFastLarge, true> : select_topk_kernel<kST, kFastLarge, false>)
+                       : (split ? select_topk_kernel<kSelT, kFast, true> : select_topk_kernel<kSelT, kFast, false>);
     cudaError_t e = set_smem(kernel, smem);
     if (e != cudaSuccess) return e;
-    return launch_dependent(kernel, dim3(L.nq_list), wide ? kST : kSelT, smem, stream, 1, L);
+    e = launch_dependent(kernel, dim3(L.nq_list), wide ? kST : kSelT, smem, stream, 1, L);
+    if (e != cudaSuccess || !split) return e;
+    e = launch_dependent(rescore_kernel, dim3(148 * 4), kRescoreT, L.nq_list * sizeof(uint32_t), stream, 1, L);
+    if (e != cudaSuccess) return e;
+    e = set_smem(select_final_kernel, sizeof(SelectSmem));
+    if (e != cudaSuccess) return e;
+    return launch_dependent(select_final_kernel, dim3(L.nq_list), kSelT, sizeof(SelectSmem), stream, 1, L);
 }
 
 cudaError_t launch_query_eps(const float* qry, const uint32_t* qlist, uint32_t nq, uint32_t dim, float max_norm,

@@ -80,3 +80,12 @@ def test_lists_shorter_than_k_keep_every_entry(torch_cuda, method, nq):
             c = int(want_c[i])
             assert (ids[i, :c] == want_i[i, :c]).all(), i
             assert (scores[i, :c].view(np.uint32) == want_s[i, :c].view(np.uint32)).all(), i
+
+
+@pytest.mark.parametrize("method,dim,nq,topks", [
+    (3, 384, 1, [1]), (3, 384, 40, [1, 10, 300, 1000]), (3, 256, 130, [2048, 7]), (3, 128, 9, [256, 1024]),
+    (2, 704, 7, [745]), (2, 704, 64, [2049, 1, 745]), (1, 352, 5, [1490, 4096])])
+@pytest.mark.parametrize("n", [300, 20003])
+def test_rescoring_spread_over_the_device(torch_cuda, method, dim, nq, topks, n):
+    # (300 docs: every list is rescored whole; a filter that passes fewer docs than K, or none)
+    _check(n, dim, method, nq, topks)
