@@ -767,15 +767,19 @@ __device__ __forceinline__ void finish_select(SelectSmem& S, const SelectLaunch&
 // ---------------------------------------------------------------------------------------------
 // The select step, one CTA per query: a chain of dependent steps and the rescoring's row reads bound it.
 //   * The list's scores are read once into shared memory (`fast` entries), the first locations with them.
-//   * A list of at most kSelT entries is rescored whole; a longer one is cut: t~ bounds the K-th
+//   * A list of at most kWholeFloats floats is rescored whole; a longer one is cut: t~ bounds the K-th
 //     best approximate score from below, so only entries of at least t~ - 2 eps can be in the top K. Where
-//     those are more than kSelT, the entries of at least t~ (K of them at least) are rescored
-//     first: the least of their exact scores, s, bounds the K-th exact score, and the rest needs only
-//     s - eps, about half the band.
+//     those are many, the entries of at least t~ (K of them at least) are rescored first: the least of
+//     their exact scores, s, bounds the K-th exact score, and the rest needs only s - eps, about half the
+//     band. (Lists of up to 512 entries whole, and two waves only past 512: 768 dims, 256 queries, K 10
+//     473 us a batch, now 412; 1M docs x 128 dims, 256 queries, K 10 189, now 175; 131k docs, 32 queries,
+//     K 100 82, now 72. Two waves from 2 K entries at any K: 768 dims, 256 queries, K 1000 832 -> 849.)
 //   * Survivors are packed before they are rescored, so that every lane group has a row.
 // SPLIT: the kernel ends with the survivors' list in L.work (and, of a list cut in two waves, the first
 // wave's keys): rescore_kernel scores the rest with all SMs, select_final_kernel sorts. A query's rows
 // are otherwise read by its own CTA, and the query with the most holds up the batch.
+constexpr uint32_t kWholeFloats = 16384;
+
 template <int NT, uint32_t FAST, bool SPLIT>
 __global__ void __launch_bounds__(NT, NT == kSelT ? 2 : 1) select_topk_kernel(SelectLaunch L) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -846,13 +850,14 @@ __global__ void __launch_bounds__(NT, NT == kSelT ? 2 : 1) select_topk_kernel(Se
     unsigned long long* ws = L.work + row;
     uint32_t nf;
     bool in_smem;  // the keys: S.sortbuf or ws
-    if (SPLIT && n <= static_cast<uint32_t>(kSelT)) {
+    const bool whole = n <= static_cast<uint32_t>(kSelT) && (n <= kq || n * L.dim <= kWholeFloats);
+    if (SPLIT && whole) {
         for (uint32_t i = tid; i < n; i += NT) ws[i] = S.locs[i];
         __syncthreads();
         if (tid == 0) L.pending[qi] = make_uint2(0, n);
         return;
     }
-    if (n <= static_cast<uint32_t>(kSelT)) {
+    if (whole) {
         rescore_rows<NT>(sq, L.vec, L.dim, n, [&](uint32_t i) { return S.locs[i]; },
                          [&](uint32_t i, uint32_t loc, float e) { S.sortbuf[i] = result_key(e, loc); });
         nf = n;
@@ -879,8 +884,10 @@ __global__ void __launch_bounds__(NT, NT == kSelT ? 2 : 1) select_topk_kernel(Se
         if ((tid & 31) == 0 && mine) atomicAdd(&S.counter, mine);
         __syncthreads();
         const uint32_t all = S.counter;
-        // (split: a first wave of K rows in this CTA pays where it spares the others many)
-        const bool two = all > (SPLIT ? 2 * kq + 256 : static_cast<uint32_t>(kSelT)) && all > kq && t > -INFINITY;
+        // a first wave pays where it spares reading about as many rows again, or kSelT; in the split form,
+        // where this CTA alone reads it and all SMs the rest, later
+        const uint32_t limit = SPLIT ? 2 * kq + 256 : min(static_cast<uint32_t>(kSelT), max(2 * kq, 128u));
+        const bool two = all > limit && all > kq && t > -INFINITY;
         float lo = two ? t : cut2, hi = INFINITY, low_exact = INFINITY;
         nf = 0;
         in_smem = all <= static_cast<uint32_t>(kMaxTopK);

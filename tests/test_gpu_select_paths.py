@@ -89,3 +89,10 @@ def test_lists_shorter_than_k_keep_every_entry(torch_cuda, method, nq):
 def test_rescoring_spread_over_the_device(torch_cuda, method, dim, nq, topks, n):
     # (300 docs: every list is rescored whole; a filter that passes fewer docs than K, or none)
     _check(n, dim, method, nq, topks)
+
+
+@pytest.mark.parametrize("method,dim", [(2, 64), (2, 128), (0, 36), (3, 128)])
+@pytest.mark.parametrize("n", [127, 128, 129, 257, 511, 513])
+def test_short_lists_around_the_whole_and_wave_limits(torch_cuda, method, dim, n):
+    # a corpus no larger than the doc sample: list lengths on both sides of the limits, K around half of them
+    _check(n, dim, method, 12, [1, 7, 63, 64, 65, 128, 255])
