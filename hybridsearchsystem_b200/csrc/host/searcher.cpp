@@ -813,7 +813,7 @@ uint64_t FullRecallSearcher::SampleOptimum(uint32_t nq, uint32_t maxK) const {
 // query's rows to its CTA. It pays where a query has more rows, or longer ones, than its SM can read in
 // the time the rest of the batch takes (us a batch, one CTA a query -> spread):
 //   8-bit form, whose error band grows with the row: 768 dims, 300k docs, 128 queries, K 10 1070 -> 398,
-//   K 100 9545 -> 1740; 384 dims, 4 queries, K 10 159 -> 91; 256 dims, K 100 1157 -> 878; 128 dims, 256
+//   K 100 9545 -> 1740 (1677 with later changes); 384 dims, 4 queries, K 10 159 -> 91; 256 dims, K 100 1157 -> 878; 128 dims, 256
 //   queries, K 300 920 -> 901. Not 256 dims, 128 queries, K 10 (263 -> 281) nor 128 dims, K 200 (757 -> 777).
 //   Other forms, batches that leave SMs idle: 768 dims, K 1000: 1 query 537 -> 445, 64 queries 576 -> 528.
 //   Not 256 queries, K 700 (713 -> 750), nor rows of 128 dims (bf16, 64 queries, K 1000 629 -> 632).

@@ -240,11 +240,12 @@ __device__ __forceinline__ uint64_t kth_bound_u64(KeyFn key, uint32_t n, uint32_
 // segment that starts at or before it, found by five shuffles, so the loads are coalesced within a
 // segment, independent and eight per thread in flight, and no block-wide scan or barrier is needed. Every
 // call is made by a full warp (valid = false past the end), so fn may use warp collectives; begin(m) is
-// called by the full warp before a group's m entries. Returns whether a segment of this lane lost entries.
-template <int NT, class Begin, class Fn>
+// called by the full warp before a group's m entries. LONG: segments of 64 entries or more on average are
+// walked one after the other, without the lookups (doc-sample lists hold about 110 a segment). Returns whether a segment of this lane lost entries.
+template <int NT, bool LONG, class Begin, class Fn>
 __device__ __forceinline__ bool walk_segments(const uint32_t* counts, uint32_t segs, uint32_t seg_cap, const float* src,
                                               Begin begin, Fn fn) {
-    constexpr uint32_t U = 8, kWarps = NT / 32;
+    constexpr uint32_t U = 8, kLong = 4, kWarps = NT / 32;
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     // segments per warp and round: as even a share as 32 lanes allow
     const uint32_t rounds = (segs + 32 * kWarps - 1) / (32 * kWarps);
@@ -262,6 +263,28 @@ __device__ __forceinline__ bool walk_segments(const uint32_t* counts, uint32_t s
         }
         const uint32_t off = x - c, total = __shfl_sync(0xffffffffu, x, 31);
         if (total == 0) continue;
+        if (LONG && total >= 64 * per) {
+            for (uint32_t j = 0; j < per; ++j) {
+                const uint32_t m = __shfl_sync(0xffffffffu, c, j);
+                if (m == 0) continue;
+                begin(m);
+                const uint32_t first = (g0 + j) * seg_cap;
+                for (uint32_t b = 0; b < m; b += 32 * kLong) {
+                    float v[kLong];
+#pragma unroll
+                    for (uint32_t u = 0; u < kLong; ++u) {
+                        const uint32_t idx = b + 32 * u + lane;
+                        v[u] = idx < m ? src[first + idx] : 0.0f;
+                    }
+#pragma unroll
+                    for (uint32_t u = 0; u < kLong; ++u) {
+                        if (b + 32 * u >= m) break;  // warp-uniform
+                        fn(first + b + 32 * u + lane, b + 32 * u + lane < m, v[u]);
+                    }
+                }
+            }
+            continue;
+        }
         begin(total);
         for (uint32_t b = 0; b < total; b += 32 * U) {
             uint32_t at[U];
@@ -291,7 +314,7 @@ __device__ __forceinline__ bool walk_segments(const uint32_t* counts, uint32_t s
 // The first walk of a list: scores into `cache` (as many as fit), where locs is given the locations of the
 // first kMaxTopK too, and the smallest and largest key. Returns the number of entries; *overflow = some
 // segment lost entries. Synchronised at its end.
-template <int NT>
+template <int NT, bool LONG>
 __device__ __forceinline__ uint32_t load_list(HistSmem& S, const uint32_t* counts, uint32_t segs, uint32_t seg_cap,
                                               const float* src, const uint32_t* loc_src, float* cache, uint32_t cap,
                                               uint32_t* locs, bool* overflow, uint32_t* key_lo, uint32_t* key_hi) {
@@ -302,7 +325,7 @@ __device__ __forceinline__ uint32_t load_list(HistSmem& S, const uint32_t* count
     __syncthreads();
     uint32_t pos = 0, lo = 0xffffffffu, hi = 0;
     const uint32_t lane = threadIdx.x & 31;
-    const bool lost = walk_segments<NT>(
+    const bool lost = walk_segments<NT, LONG>(
         counts, segs, seg_cap, src,
         [&](uint32_t m) {
             if (lane == 0) pos = atomicAdd(&S.counter, m);
@@ -470,9 +493,12 @@ __device__ __forceinline__ uint32_t gather_top_keys(KeyFn key, uint32_t n, uint3
 // ---------------------------------------------------------------------------------------------
 // The threshold of a sample or of a first candidate pass. One CTA per query; bound by a chain of
 // dependent steps (counts, entries, two digits), so the list is read once, into shared memory where it
-// fits (kFastSample entries), with the first digit counted on the way.
-template <int NT>
-__global__ void __launch_bounds__(NT, 1024 / NT) sample_threshold_kernel(SampleThresholdLaunch L) {
+// fits (kFastSample entries). 1,024 threads and long segments walked as they lie: with a threshold model,
+// whose sample is kept as lists, 256 queries on 10M docs 1214 us a batch (K 1000: 1866) with 512 threads and
+// a lookup per entry, 1190 (1785) now; 8-bit form, whose raises read long lists, 1M docs, 256 queries, K 100
+// 877 -> 819; other raises even.
+__global__ void __launch_bounds__(kST) sample_threshold_kernel(SampleThresholdLaunch L) {
+    constexpr int NT = kST;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     HistSmem& S = *reinterpret_cast<HistSmem*>(smem_raw);
     float* cs = reinterpret_cast<float*>(smem_raw + sizeof(HistSmem));
@@ -484,13 +510,13 @@ __global__ void __launch_bounds__(NT, 1024 / NT) sample_threshold_kernel(SampleT
     const float* sc = L.score + static_cast<uint64_t>(qi) * L.cap;
     bool lost = false;  // a sample segment that overflowed only lowers the sample's K-th best
     uint32_t key_lo, key_hi;
-    const uint32_t n = load_list<NT>(S, counts, L.segs, L.seg_cap, sc, nullptr, cs, kFastSample, nullptr, &lost, &key_lo,
+    const uint32_t n = load_list<NT, true>(S, counts, L.segs, L.seg_cap, sc, nullptr, cs, kFastSample, nullptr, &lost, &key_lo,
                                      &key_hi);
     auto visit = [&](auto fn) {
         if (n <= kFastSample) {
             for (uint32_t i = threadIdx.x; i < n; i += NT) fn(float_key(cs[i]));
         } else {
-            walk_segments<NT>(counts, L.segs, L.seg_cap, sc, [](uint32_t) {}, [&](uint32_t, bool ok, float v) {
+            walk_segments<NT, true>(counts, L.segs, L.seg_cap, sc, [](uint32_t) {}, [&](uint32_t, bool ok, float v) {
                 if (ok) fn(float_key(v));
             });
         }
@@ -809,12 +835,12 @@ __global__ void __launch_bounds__(NT, NT == kSelT ? 2 : 1) select_topk_kernel(Se
     for (uint32_t i = tid; i < L.dim; i += NT) sq[i] = L.qry[static_cast<uint64_t>(qi) * L.dim + i];
     bool overflow = false;
     uint32_t key_lo, key_hi;
-    const uint32_t n = load_list<NT>(S, counts, L.segs, L.seg_cap, sc, lc, cs, FAST, S.locs, &overflow, &key_lo, &key_hi);
+    const uint32_t n = load_list<NT, SPLIT>(S, counts, L.segs, L.seg_cap, sc, lc, cs, FAST, S.locs, &overflow, &key_lo, &key_hi);
     auto visit_keys = [&](auto fn) {
         if (n <= FAST) {
             for (uint32_t i = tid; i < n; i += NT) fn(float_key(cs[i]));
         } else {
-            walk_segments<NT>(counts, L.segs, L.seg_cap, sc, [](uint32_t) {}, [&](uint32_t, bool ok, float v) {
+            walk_segments<NT, SPLIT>(counts, L.segs, L.seg_cap, sc, [](uint32_t) {}, [&](uint32_t, bool ok, float v) {
                 if (ok) fn(float_key(v));
             });
         }
@@ -870,7 +896,7 @@ __global__ void __launch_bounds__(NT, NT == kSelT ? 2 : 1) select_topk_kernel(Se
             if (n <= min(FAST, static_cast<uint32_t>(kMaxTopK))) {
                 for (uint32_t i = tid; i < n; i += NT) fn(cs[i], [&] { return S.locs[i]; });
             } else {
-                walk_segments<NT>(counts, L.segs, L.seg_cap, sc, [](uint32_t) {}, [&](uint32_t at, bool ok, float v) {
+                walk_segments<NT, SPLIT>(counts, L.segs, L.seg_cap, sc, [](uint32_t) {}, [&](uint32_t at, bool ok, float v) {
                     if (ok) fn(v, [&] { return lc[at]; });
                 });
             }
@@ -1369,11 +1395,9 @@ cudaError_t launch_sample_threshold(const SampleThresholdLaunch& L, cudaStream_t
     if (L.nq_list == 0) return cudaSuccess;
     if (bad_segments(L.segs, L.seg_cap, L.cap)) return cudaErrorInvalidValue;
     const size_t smem = sizeof(HistSmem) + kFastSample * sizeof(float);
-    const bool wide = L.nq_list <= kWideQueries;
-    auto kernel = wide ? sample_threshold_kernel<kST> : sample_threshold_kernel<kSelT>;
-    cudaError_t e = set_smem(kernel, smem);
+    cudaError_t e = set_smem(sample_threshold_kernel, smem);
     if (e != cudaSuccess) return e;
-    return launch_dependent(kernel, dim3(L.nq_list), wide ? kST : kSelT, smem, stream, 1, L);
+    return launch_dependent(sample_threshold_kernel, dim3(L.nq_list), kST, smem, stream, 1, L);
 }
 
 cudaError_t launch_maxima_threshold(const MaximaThresholdLaunch& L, cudaStream_t stream) {

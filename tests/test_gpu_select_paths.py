@@ -96,3 +96,10 @@ def test_rescoring_spread_over_the_device(torch_cuda, method, dim, nq, topks, n)
 def test_short_lists_around_the_whole_and_wave_limits(torch_cuda, method, dim, n):
     # a corpus no larger than the doc sample: list lengths on both sides of the limits, K around half of them
     _check(n, dim, method, 12, [1, 7, 63, 64, 65, 128, 255])
+
+
+@pytest.mark.parametrize("sample_docs", [4096, 16384, 60001])
+def test_listed_samples_of_short_and_long_segments(torch_cuda, sample_docs):
+    # K past half the sample's groups keeps the sample as lists of docs: segments on both sides of the
+    # 64 entries at which they are walked one after the other
+    _check(60001, 128, 2, 20, [sample_docs // 16 + 1 if sample_docs < 60001 else 4000, 2048], sample_docs=sample_docs)
