@@ -565,15 +565,20 @@ class FullRecallSearcher {
     uint32_t SegsOf(uint32_t rows, uint64_t countTiles, uint32_t cap, bool simt) const;
     uint32_t SegCapOf(uint32_t rows, uint64_t countTiles, uint32_t cap, uint32_t segs, bool simt) const;
     void Stage(const uint32_t* dList, uint32_t rows);
+    struct MaximaSample {
+        uint32_t groups = 0, docs = 0;  // group maxima (0: the sample is kept as lists); docs of a group
+        uint64_t tiles = 0;             // of UnitOf() docs
+        uint64_t blockStep = 0;         // sample_tile_of
+    };
     void Cand(const float* theta, float* score, uint32_t* loc, uint32_t* count, uint32_t cap, uint32_t segBase,
               uint32_t segCap, uint64_t begin, uint64_t step, uint32_t skip, uint64_t countTiles, const uint32_t* dList,
-              uint32_t rows, bool simt,
-              float* best = nullptr, bool coarse = false);
+              uint32_t rows, bool simt, const MaximaSample* maxima = nullptr);
     // The doc sample of m_b.want docs and its threshold (raised, with raiseOnly); the pass keeps the
     // filtered docs at or above emitTheta (null: every filtered doc).
     uint64_t Sample(const uint32_t* dList, uint32_t rows, bool simt, bool raiseOnly = false, float* stats = nullptr,
                     float* thetaCopy = nullptr, const float* emitTheta = nullptr);
-    uint32_t MaximaGroups(uint32_t rows, uint64_t count, bool simt, uint32_t* docs) const;
+    uint32_t SampleTileNum() const;
+    MaximaSample Maxima(uint32_t rows, uint64_t want, bool simt) const;
     uint64_t SampleOptimum(uint32_t nq, uint32_t maxK) const;
     bool SplitSelect(uint32_t nq, uint32_t maxK) const;
     bool OnePass(uint32_t nq, uint32_t maxK, uint64_t sampled) const;
@@ -654,6 +659,7 @@ class FullRecallSearcher {
     int m_tcFormat = -1;  // TcFormat, or -1 for the SIMT pass
     uint32_t m_tcKblocks = 0;
     CUtensorMap m_docMap{};
+    CUtensorMap m_sampleMap{};  // the corpus in sample tiles (group maxima)
     CUtensorMap m_qryMap{};
     void* m_dStaged = nullptr;  // [256][dim] staged queries in the pass's format
     float* m_dQScale = nullptr;

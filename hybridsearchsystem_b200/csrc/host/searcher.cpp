@@ -262,7 +262,9 @@ bool FullRecallSearcher::Allocate(void* dArena, size_t arenaBytes) {
         m_dStaged = W + A.staged;
         m_dQScale = reinterpret_cast<float*>(W + A.qScale);
         m_dError = reinterpret_cast<int32_t*>(m_dStage + L.errWord);
-        if (!make_tc_map(&m_docMap, m_tcFormat, m_table->DeviceRows(m_tcFormat), m_table->GetTileNum() * 128, dim) ||
+        const void* rows = m_table->DeviceRows(m_tcFormat);
+        if (!make_tc_map(&m_docMap, m_tcFormat, rows, m_table->GetTileNum() * 128, dim) ||
+            (SampleTileNum() && !make_tc_sample_map(&m_sampleMap, m_tcFormat, rows, SampleTileNum(), dim)) ||
             !make_tc_map(&m_qryMap, m_tcFormat, m_dStaged, 256, dim)) {
             m_err = "cuTensorMapEncodeTiled failed";
             return false;
@@ -560,7 +562,8 @@ void FullRecallSearcher::Stage(const uint32_t* dList, uint32_t rows) {
 // SIMT pass and the single-SM tensor-core pass, 256 for the SM-pair pass.
 void FullRecallSearcher::Cand(const float* theta, float* score, uint32_t* loc, uint32_t* count, uint32_t cap,
                               uint32_t segBase, uint32_t segCap, uint64_t begin, uint64_t step, uint32_t skip,
-                              uint64_t countTiles, const uint32_t* dList, uint32_t rows, bool simt, float* best, bool coarse) {
+                              uint64_t countTiles, const uint32_t* dList, uint32_t rows, bool simt,
+                              const MaximaSample* maxima) {
     const DataTable& T = *m_table;
     const uint32_t g = CtasOf(rows, countTiles, cap, simt);
     if (UseSimt(simt)) {
@@ -579,7 +582,11 @@ void FullRecallSearcher::Cand(const float* theta, float* score, uint32_t* loc, u
         C.segs = g;
         C.seg_cap = segCap;
         C.seg_base = segBase;
-        C.best = best;
+        if (maxima) {
+            C.best = m_dSampScore;
+            C.sample_tiles = SampleTileNum();
+            C.block_step = maxima->blockStep;
+        }
         C.dim = T.GetDimension();
         C.tile_begin = begin;
         C.tile_step = step;
@@ -605,8 +612,12 @@ void FullRecallSearcher::Cand(const float* theta, float* score, uint32_t* loc, u
     C.ctas = g;
     C.seg_cap = segCap;
     C.seg_base = segBase;
-    C.best = best;
-    C.coarse = coarse ? 1 : 0;
+    if (maxima) {
+        C.best = m_dSampScore;
+        C.coarse = maxima->docs == kTcCoarseGroup ? 1 : 0;
+        C.sample_tiles = SampleTileNum();
+        C.block_step = maxima->blockStep;
+    }
     C.tile_begin = begin;
     C.tile_step = step;
     C.tile_count = countTiles;
@@ -619,11 +630,9 @@ void FullRecallSearcher::Cand(const float* theta, float* score, uint32_t* loc, u
         C.wait_budget = m_testBudget;
         m_testHold = 0;
     }
-    Ck(launch_tc_cand(C, m_docMap, m_qryMap, m_numSms, m_b.stream));
+    Ck(launch_tc_cand(C, maxima ? m_sampleMap : m_docMap, m_qryMap, m_numSms, m_b.stream));
 }
 
-// The doc sample: evenly spaced tiles, every filtered doc kept; its K-th best bounds the threshold.
-// Returns the sample's tile count.
 // Tiles (and their step) of a doc sample of `want` docs for `rows` queries.
 void FullRecallSearcher::SampleTiles(uint64_t want, uint32_t rows, bool simt, uint64_t* count, uint64_t* step) const {
     const uint32_t unit = UnitOf(rows, simt);
@@ -633,35 +642,53 @@ void FullRecallSearcher::SampleTiles(uint64_t want, uint32_t rows, bool simt, ui
     *count = std::min<uint64_t>(sampTiles, (tilesU + *step - 1) / *step);
 }
 
-// Groups of a sample of `count` tiles that is kept as group maxima, 0 where it is kept as lists of docs: a
-// K past half the groups would find its threshold far below the docs' K-th best (at K = groups it is
-// the least maximum). *docs: docs of a group. Coarse groups, a quarter of the stores and of the
-// threshold's entries, where K is an eighth of them at most (the K-th maximum is then at rank 1.07 K or
-// better among the docs).
-uint32_t FullRecallSearcher::MaximaGroups(uint32_t rows, uint64_t count, bool simt, uint32_t* docs) const {
-    const uint64_t all = count * UnitOf(rows, simt);
-    *docs = UseSimt(simt) ? kSimtGroup : all / kTcCoarseGroup >= 8ull * m_b.maxK ? kTcCoarseGroup : kTcGroup;
-    const uint64_t groups = all / *docs;
-    return groups >= 2ull * m_b.maxK && groups <= m_sampCap ? static_cast<uint32_t>(groups) : 0u;
+// Sample tiles of the corpus (none below 1,024 docs).
+uint32_t FullRecallSearcher::SampleTileNum() const {
+    return static_cast<uint32_t>(m_table->GetTileNum() / kSampleBlock * kSampleBlock);
 }
 
+// A sample of `want` docs that is kept as group maxima; no groups where it is kept as lists of docs: a K past
+// half the groups would find its threshold far below the docs' K-th best (at K = groups it is the least
+// maximum). Coarse groups, half the stores and the threshold's entries, where K is an eighth of them at most
+// (the K-th maximum is then at rank 1.07 K or better among the docs). Both hold for any order of the corpus: a
+// group's docs lie far apart (kSampleRuns), and the sample's blocks are spread over all of it.
+FullRecallSearcher::MaximaSample FullRecallSearcher::Maxima(uint32_t rows, uint64_t want, bool simt) const {
+    MaximaSample M;
+    const uint64_t all = SampleTileNum() / kSampleBlock, docs = 128ull * kSampleBlock;
+    if (all == 0) return M;
+    uint64_t blocks = std::min<uint64_t>(all, std::max<uint64_t>(1, (want + docs - 1) / docs));
+    // a sample of several blocks a CTA gives every CTA as many
+    const uint64_t ctas = CtasOf(rows, blocks * kSampleBlock, m_sampCap, simt) / (UnitOf(rows, simt) / 128);
+    if (blocks >= 2 * ctas) blocks -= blocks % ctas;
+    const uint64_t sampled = blocks * docs;
+    M.blockStep = (all << 32) / blocks;
+    M.tiles = sampled / UnitOf(rows, simt);
+    M.docs = UseSimt(simt) ? kSimtGroup : sampled / kTcCoarseGroup >= 8ull * m_b.maxK ? kTcCoarseGroup : kTcGroup;
+    const uint64_t groups = sampled / M.docs;
+    if (groups >= 2ull * m_b.maxK && groups <= m_sampCap) M.groups = static_cast<uint32_t>(groups);
+    return M;
+}
+
+// The doc sample of evenly spaced tiles, and the threshold its K-th best proves: kept as the maxima of groups
+// of its filtered docs where K allows it, else (and for the model's statistics) as lists of them.
+// Returns its tile count.
 uint64_t FullRecallSearcher::Sample(const uint32_t* dList, uint32_t rows, bool simt, bool raiseOnly, float* stats,
                                     float* thetaCopy, const float* emitTheta) {
     const StageLayout SL = MakeLayout(m_cfg.maxBatch);
     uint8_t* D = m_dStage;
-    uint64_t count = 0, step = 1;
-    SampleTiles(m_b.want, rows, simt, &count, &step);
+    auto* dSampCount = reinterpret_cast<uint32_t*>(D + SL.sampCount);
+    const MaximaSample maxima = stats || raiseOnly ? MaximaSample{} : Maxima(rows, m_b.want, simt);
+    uint64_t count = maxima.tiles, step = 1;
+    if (!maxima.groups) SampleTiles(m_b.want, rows, simt, &count, &step);
     const uint32_t segs = SegsOf(rows, count, m_sampCap, simt);
     const uint32_t segCap = SegCapOf(rows, count, m_sampCap, segs, simt);
-    auto* dSampCount = reinterpret_cast<uint32_t*>(D + SL.sampCount);
-    uint32_t groupDocs = 0;
-    if (const uint32_t groups = MaximaGroups(rows, count, simt, &groupDocs); groups && !stats && !raiseOnly) {
-        Cand(reinterpret_cast<const float*>(D + SL.negInf), m_dSampScore, m_dSampLoc, dSampCount, m_sampCap, 0, segCap, 0,
-             step, 0, count, dList, rows, simt, m_dSampScore, groupDocs == kTcCoarseGroup);
+    if (maxima.groups) {
+        Cand(reinterpret_cast<const float*>(D + SL.negInf), m_dSampScore, m_dSampLoc, dSampCount, m_sampCap, 0, segCap,
+             0, 1, 0, count, dList, rows, simt, &maxima);
         MaximaThresholdLaunch MT{};
         MT.best = m_dSampScore;
         MT.cap = m_sampCap;
-        MT.groups = groups;
+        MT.groups = maxima.groups;
         MT.topk = reinterpret_cast<const uint32_t*>(D + SL.topk);
         MT.eps_sample = reinterpret_cast<const float*>(D + SL.epsSamp);
         MT.eps_main = reinterpret_cast<const float*>(D + SL.epsMain);
@@ -825,15 +852,22 @@ bool FullRecallSearcher::SplitSelect(uint32_t nq, uint32_t maxK) const {
 
 // Whether the corpus is passed over once, at the sample's threshold, instead of in two parts with the
 // threshold raised between them. One pass keeps about K N / s docs per query, two 2 K sqrt(N / s); the
-// second launch, the raise and the gap cost about as much as keeping 400,000 more docs (300,000 docs, 256
-// queries, K = 100: 165 -> 146 us; 131,072 docs, 32 queries: 108 -> 92; 1M x 768, 256 queries, 570,000
-// more docs: 551 -> 557). Not where the lists would fill past an eighth, nor for the 8-bit form (1M docs,
-// 128 queries: 512 -> 675 us: its band keeps far more than that estimate).
+// second launch, the raise and the gap cost about as much as keeping 400,000 more docs, and the line is
+// drawn at 300,000 (300,000 docs, 256 queries, K = 100: 165 -> 146 us; 131,072 docs, 32 queries: 108 -> 92;
+// 1M x 768, 256 queries, 570,000 more docs: 551 -> 557). Not where the lists would fill past an eighth, nor for
+// the 8-bit form (1M docs, 128 queries: 512 -> 675 us: its band keeps far more than that estimate).
+// Nor from a thin sample, unless K is small: in a corpus in the order of its clusters a thin sample may hold
+// fewer than K docs of the query's own, its threshold then lies among other clusters' scores, and one pass
+// has no raise to recover with (BF16, 1M docs in the order of 1,024 clusters, 32 queries, K = 100: ratio 30 in
+// one pass 277 us, in two 200, and in random order 158 and 144; 10M, one query: 709 and 569, 628 and 553; 1M,
+// 256 queries, K = 10, random order: 160 and 176). The FP32 SIMT form's passes cost more than what such a
+// threshold keeps (1M docs, 64 queries, K = 100: one pass 533 us, two 547).
 bool FullRecallSearcher::OnePass(uint32_t nq, uint32_t maxK, uint64_t sampled) const {
     if (m_tcFormat == kTcE4M3 || sampled == 0) return false;
     const double ratio = static_cast<double>(m_table->GetDocNum()) / static_cast<double>(sampled);
     const double more = static_cast<double>(nq) * maxK * (ratio - 2.0 * std::sqrt(ratio));
-    return more <= 300e3 && 8.0 * maxK * ratio <= m_cfg.candidateCap;
+    const bool dense = ratio <= (m_tcFormat < 0 ? 32.0 : 10.0) || maxK * ratio <= 512.0;
+    return dense && more <= 300e3 && 8.0 * maxK * ratio <= m_cfg.candidateCap;
 }
 
 uint32_t FullRecallSearcher::PlanTopK(uint32_t maxK) const {
@@ -968,7 +1002,7 @@ int FullRecallSearcher::EnqueueAttempt(uint32_t nq, const BatchInputs& in, float
     ++m_b.launches;
     if (m_timing) Ck(cudaEventRecord(m_ev[1], stream));
 
-    // 1. doc sample: evenly spaced tiles, every filtered doc kept; its K-th best bounds the threshold.
+    // 1. doc sample: evenly spaced tiles; its K-th best bounds the threshold.
     // Without a model it grows with K so that its threshold keeps the full pass within the list
     // capacity; with one, the prediction sets the threshold and the sample only feeds the features
     // (which are made from the same sample size, with or without a model set).
@@ -981,10 +1015,8 @@ int FullRecallSearcher::EnqueueAttempt(uint32_t nq, const BatchInputs& in, float
     // statuses (a copy here would stall the stream between the sample and the passes)
     auto* dTheta1 = reinterpret_cast<float*>(D + SL.theta1);
     if (!wantStats) m_b.want = std::max<uint64_t>(m_b.want, SampleOptimum(nq, maxK));
-    uint64_t sampCount = 0, grownStep = 1;
-    uint32_t groupDocs = 0;
-    SampleTiles(m_b.want, nq, false, &sampCount, &grownStep);
-    if (m_b.want > m_cfg.sampleDocs && !MaximaGroups(nq, sampCount, false, &groupDocs)) {
+    uint64_t sampCount = 0;
+    if (m_b.want > m_cfg.sampleDocs && !Maxima(nq, m_b.want, false).groups) {
         m_b.want = m_b.wantRerun;
         // A sample grown with K, kept as lists, in two steps: the sample_docs sample's proven threshold first, then the
         // grown sample keeps only the docs above it. Its K-th best is the same whenever it has K docs

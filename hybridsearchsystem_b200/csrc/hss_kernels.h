@@ -113,14 +113,40 @@ struct CandLaunch {
     uint32_t cap;
     uint32_t segs, seg_cap;    // CTAs of the launch (cand_simt_segments) and entries per segment
     uint32_t seg_base;         // first segment this pass writes
-    // [nq][cap] or null: instead of candidates the pass writes, for the it-th tile it visits, the best
+    // [nq][cap] or null: instead of candidates the pass writes, for the it-th sample tile it visits, the best
     // score of each kSimtGroup docs whose filter bit is set (-inf: none) at it * (128 / kSimtGroup) + group
     float* best;
+    uint32_t sample_tiles;     // with best: T of the sample tiles
+    uint64_t block_step;       // with best: the sample's blocks (sample_tile_of)
     uint32_t dim;              // multiple of 4
     uint64_t tile_begin, tile_step, tile_count;
     uint32_t tile_skip;
 };
-constexpr uint32_t kSimtGroup = 4, kTcGroup = 8, kTcCoarseGroup = 32;  // docs per group maximum
+constexpr uint32_t kSimtGroup = 4, kTcGroup = 8, kTcCoarseGroup = 16;  // docs per group maximum
+// A doc sample kept as group maxima is made of sample tiles. The corpus (up to the last 1,023 docs) is cut into
+// kSampleRuns equal parts of 16 T docs, and tile v < T takes the kSampleRun docs from 16 v of every part: doc i of
+// the tile is doc (i / 16) 16 T + 16 v + i % 16. A group's docs come from four parts (one doc from each, a
+// tensor-core group two that are eight docs apart, a coarse one four), so that docs that lie together in the
+// corpus -- one tag's, one cluster's -- fall in about half as many groups as there are such docs in the sample,
+// and the K-th best maximum stays close to the sample's K-th best score in any order of the corpus. With groups
+// of 8 or 32 neighbours and docs in the order of their tags or clusters, fewer than K groups could hold a
+// filtered doc: 10M docs, one query for a tag of 263,000 docs in a row, K = 100, 565 us a batch with lists of
+// docs, 1316 with such groups.
+// A sample takes whole blocks of kSampleBlock neighbouring tiles, spread evenly over the corpus: a block's filter
+// bits are 16 bytes of every part. (16 parts of 8 docs: twice the cache lines of filter bits, of which an SM that
+// gives its shared memory to the pass has about 200 in flight; 10M docs, 256 queries, the sample's pass 28 us with
+// whole tiles of neighbours, 76 with those.)
+constexpr uint32_t kSampleRun = 16, kSampleRuns = 8, kSampleBlock = 8;
+// The i-th tile of a sample whose blocks lie step / 2^32 blocks apart, and whether `tiles` of them are whole
+// blocks of the first T tiles.
+__host__ __device__ inline uint32_t sample_tile_of(uint32_t i, uint64_t step) {
+    return static_cast<uint32_t>((i / kSampleBlock * step) >> 32) * kSampleBlock + i % kSampleBlock;
+}
+inline bool sample_fits(uint64_t tiles, uint64_t step, uint32_t sample_tiles) {
+    const uint64_t blocks = tiles / kSampleBlock, all = sample_tiles / kSampleBlock;
+    return blocks > 0 && tiles % kSampleBlock == 0 && sample_tiles % kSampleBlock == 0 && blocks <= all &&
+           step >= (1ull << 32) && step <= (all << 32) / blocks;
+}
 // Largest query count of one SIMT candidate pass (its per-query counts live in shared memory).
 constexpr uint32_t kMaxSimtBatch = 4096;
 // CTAs of a SIMT candidate pass over tile_count tiles into lists of `cap` entries (one list segment
@@ -228,10 +254,13 @@ struct TcCandLaunch {
     uint32_t ctas, seg_cap;    // CTAs of the launch (tc_cand_ctas); entries per list segment
     uint32_t seg_base;         // first segment this pass writes (it writes 2 per CTA)
     float* best;               // or null: group maxima instead of candidates, as in CandLaunch
-    int coarse;                // their groups: kTcGroup docs (0) or kTcCoarseGroup (1)
+    int coarse;                // their groups: kTcGroup docs (0) or kTcCoarseGroup (1); doc_map: the sample's
     uint64_t tile_begin, tile_step, tile_count;  // tiles of tc_tile_docs(nq_rows, kblocks) docs
     uint32_t tile_skip;
     uint64_t tiles128;         // 128-doc tiles of the corpus (rows of the tensor map / 128)
+    uint32_t sample_tiles;     // with best: T of the sample tiles
+    uint64_t block_step;       // with best: the sample's blocks (sample_tile_of)
+    uint32_t chunk_log;        // with best: 2^chunk_log consecutive tiles a CTA takes at a time (set by launch_tc_cand)
     int32_t* error;            // device error bits (bounded waits that expired)
     // Pipeline test knobs (single-SM kernel): wait_budget > 0 replaces the clock budget of the waits
     // that can abort the pass; hold_load > 0 makes the producer stop before issuing its
@@ -265,6 +294,8 @@ bool make_tc_map(CUtensorMap* map, int format, const void* base, uint64_t rows, 
 // per-doc scale (e4m3), per-doc norm and quantisation-error norm (FP64, rounded up to float).
 cudaError_t launch_quantize_docs(const float* vec, uint64_t rows, uint64_t valid_rows, uint32_t dim, int format,
                                  void* out, float* scale, float* norm, float* err_norm, cudaStream_t stream);
+// The tensor map of the corpus in sample_tiles sample tiles: a box is one k-block of a tile.
+bool make_tc_sample_map(CUtensorMap* map, int format, const void* base, uint64_t sample_tiles, uint32_t dim);
 // Stage a batch of queries in a tensor-core format (rows past nq zero) and compute the per-query error
 // bounds of the candidate pass (see score_tc.cu / searcher.cpp).
 struct StageQueriesLaunch {

@@ -170,6 +170,8 @@ constexpr uint32_t kCWarps = kCT / 32;
 constexpr int kCK = 32;            // dims per stage
 constexpr int kCPitch = kCK + 4;
 static_assert(kSimtGroup == 4, "a thread's docs of a tile are one group");
+static_assert(kSampleRun * kSampleRuns == kDocTile && kCT / 8 == 2 * kSampleRun && kSampleRun == 16,
+              "a sample tile's rows");
 
 __device__ __forceinline__ void fma2(unsigned long long& acc, unsigned long long a, unsigned long long b) {
     asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc) : "l"(a), "l"(b));
@@ -183,7 +185,7 @@ struct SimtTile {
     static constexpr size_t fixed = 3 * stage_floats * sizeof(float) + 4 * QT * 16;
 };
 
-// MAXIMA: the pass writes group maxima (CandLaunch::best) instead of candidates.
+// MAXIMA: the pass writes group maxima (CandLaunch::best) of sample tiles instead of candidates.
 template <int TQ, bool MAXIMA>
 __global__ void __launch_bounds__(kCT, 2) cand_simt_kernel(CandLaunch L) {
     using T = SimtTile<TQ>;
@@ -214,10 +216,16 @@ __global__ void __launch_bounds__(kCT, 2) cand_simt_kernel(CandLaunch L) {
         const uint32_t k0 = kc * kCK, part = tid & 7;
         float* sd = ring + stage * T::stage_floats + (tid >> 3) * kCPitch + part * 4;
         if (part * 4 < L.dim - k0) {
-            const float* v = L.vec + (static_cast<uint64_t>(tile) * kDocTile + (tid >> 3)) * L.dim + k0 + part * 4;
+            // row tid / 8, then every 32nd: of the tile, or (MAXIMA) of the sample tile, whose rows 32 apart
+            // are two runs apart
+            const uint64_t row = tid >> 3;
+            const uint64_t doc = MAXIMA ? (row / kSampleRun * L.sample_tiles + tile) * kSampleRun + row % kSampleRun
+                                        : static_cast<uint64_t>(tile) * kDocTile + row;
+            const uint64_t step = MAXIMA ? static_cast<uint64_t>(L.sample_tiles) * (kCT / 8) : kCT / 8;
+            const float* v = L.vec + doc * L.dim + k0 + part * 4;
 #pragma unroll
             for (uint32_t i = 0; i < kDocTile * 8 / kCT; ++i)
-                copy16(sd + i * (kCT / 8) * kCPitch, v + static_cast<uint64_t>(i * (kCT / 8)) * L.dim);
+                copy16(sd + i * (kCT / 8) * kCPitch, v + i * step * L.dim);
 #pragma unroll
             for (uint32_t i = 0; i < (T::QT * 8 + kCT - 1) / kCT; ++i) {
                 const uint32_t r = (tid >> 3) + i * (kCT / 8);
@@ -231,14 +239,25 @@ __global__ void __launch_bounds__(kCT, 2) cand_simt_kernel(CandLaunch L) {
         if (kc == 0 && tid < T::QT) {
             const uint32_t li = min(chunk * T::QT + tid, L.nq_list - 1);
             const uint32_t qi = L.qlist ? L.qlist[li] : li;
-            // bitmap rows and tiles are multiples of 16 bytes (segments of 128 docs)
-            copy16(sBits + bits * T::QT + tid, L.bits + static_cast<uint64_t>(qi) * L.bits_stride + tile * 2ull);
+            const uint64_t* brow = L.bits + static_cast<uint64_t>(qi) * L.bits_stride;
+            if (MAXIMA) {  // 16 bits of every run
+                const uint16_t* p = reinterpret_cast<const uint16_t*>(brow) + tile;
+                uint32_t b[kSampleRuns];
+#pragma unroll
+                for (uint32_t r = 0; r < kSampleRuns; ++r) b[r] = p[static_cast<uint64_t>(r) * L.sample_tiles];
+                sBits[bits * T::QT + tid] =
+                    make_uint4(b[0] | b[1] << 16, b[2] | b[3] << 16, b[4] | b[5] << 16, b[6] | b[7] << 16);
+            } else {
+                // bitmap rows and tiles are multiples of 16 bytes (segments of 128 docs)
+                copy16(sBits + bits * T::QT + tid, brow + tile * 2ull);
+            }
         }
     };
     auto commit = [] { asm volatile("cp.async.commit_group;" ::: "memory"); };
 
     // The it-th tile of the pass (32-bit: the launcher checks tile_walk_fits).
     auto tile_at = [&](uint32_t it) {
+        if (MAXIMA) return sample_tile_of(it, L.block_step);
         return L.tile_skip >= 2 ? it + it / (L.tile_skip - 1) + 1
                                 : static_cast<uint32_t>(L.tile_begin) + it * static_cast<uint32_t>(L.tile_step);
     };
@@ -398,7 +417,9 @@ cudaError_t launch_cand_simt(const CandLaunch& L, int num_sms, cudaStream_t stre
         seg_end * L.seg_cap > L.cap || L.nq_list > kMaxSimtBatch ||
         !tile_walk_fits(L.tile_begin, L.tile_step, L.tile_skip, L.tile_count, L.segs))
         return cudaErrorInvalidValue;
-    if (L.best && L.tile_count * (kDocTile / kSimtGroup) > L.cap) return cudaErrorInvalidValue;
+    if (L.best && (L.tile_count * (kDocTile / kSimtGroup) > L.cap || L.bits_stride < 2ull * L.sample_tiles ||
+                   !sample_fits(L.tile_count, L.block_step, L.sample_tiles)))
+        return cudaErrorInvalidValue;
     // the filter words and rows are copied 16 bytes at a time
     if ((L.bits_stride & 1u) || (reinterpret_cast<uintptr_t>(L.bits) & 15u) || (reinterpret_cast<uintptr_t>(L.vec) & 15u) ||
         (reinterpret_cast<uintptr_t>(L.qry) & 15u))

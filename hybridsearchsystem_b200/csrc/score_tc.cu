@@ -101,6 +101,14 @@ __device__ inline void tma_load_2d(void* dst, const CUtensorMap* map, int x, int
         : "memory");
 }
 
+__device__ inline void tma_load_3d(void* dst, const CUtensorMap* map, int x, int y, int z, unsigned long long* bar) {
+    asm volatile(
+        "cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::
+            "r"(smem_u32(dst)),
+        "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
+        : "memory");
+}
+
 // UMMA shared-memory descriptor: K-major operand with the 128-byte swizzle, 8-row groups 1024 bytes
 // apart (stride byte offset), sm_100 descriptor version 1.
 __device__ inline uint64_t smem_desc(uint32_t addr) {
@@ -353,34 +361,101 @@ __device__ __forceinline__ void emit_lane(uint32_t m, const uint32_t (&v)[32], f
     }
 }
 
-// One 32-doc chunk's group maxima (the doc sample): the best score of each kTcGroup docs whose filter bit is
-// set, -inf where none is, as one 16-byte store at out[4 * chunk]; coarse: of the whole chunk, at
-// out[chunk]. live: the chunk was read (some lane has a bit).
-template <int F>
-__device__ __forceinline__ void store_maxima(bool live, uint32_t m, const uint32_t (&v)[32], float qs, float* out,
-                                             uint32_t chunk, bool coarse) {
-    float g[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-    if (live) {
+// ---- the doc sample's tiles (kSampleRuns, hss_kernels.h) ----
+// The runs of a thread's 64 columns of a sample tile, and of a 32-doc chunk of them.
+constexpr uint32_t kThreadRuns = 64 / kSampleRun, kChunkRuns = 32 / kSampleRun;
+static_assert(kSampleRun == 16 && kSampleRuns == 8 && kSampleBlock == 8,
+              "a tile is 128 docs; a block's filter bits are 16 bytes of every part");
+
+// The n-th unit (a tile, or a pair's two) that CTA (or pair) b of `of` visits of a sample. A CTA takes 2^chunk_log
+// consecutive units of a block at a time, whose filter bits it loads together.
+__device__ __forceinline__ uint32_t sample_unit(const TcCandLaunch& L, uint32_t b, uint32_t of, uint32_t n) {
+    return (((n >> L.chunk_log) * of + b) << L.chunk_log) | (n & ((1u << L.chunk_log) - 1u));
+}
+// How many units it visits.
+__device__ __forceinline__ uint32_t sample_units(const TcCandLaunch& L, uint32_t b, uint32_t of) {
+    const uint32_t chunks = static_cast<uint32_t>(L.tile_count) >> L.chunk_log;
+    return b < chunks ? (chunks - b + of - 1) / of << L.chunk_log : 0u;
+}
+
+// Filter bits of the runs run0 .. run0 + 3 of tile v's block (16 bits a tile), and tile v's 64 of them.
+__device__ __forceinline__ void load_block_bits(uint4 (&w)[kThreadRuns], const uint64_t* brow, uint32_t sample_tiles,
+                                                uint32_t v, uint32_t run0) {
+    const uint4* p = reinterpret_cast<const uint4*>(brow) + static_cast<uint64_t>(run0) * (sample_tiles / kSampleBlock) +
+                     v / kSampleBlock;
 #pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            float x[8];
+    for (uint32_t r = 0; r < kThreadRuns; ++r) w[r] = p[static_cast<uint64_t>(r) * (sample_tiles / kSampleBlock)];
+}
+__device__ __forceinline__ void tile_bits(const uint4 (&w)[kThreadRuns], uint32_t v, uint32_t (&m)[2]) {
+    const uint32_t j = v % kSampleBlock, half = j & 1u ? 0x7632u : 0x5410u;
+    uint32_t x[kThreadRuns];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-                float s = __uint_as_float(v[8 * k + j]);
-                if (F == kTcE4M3) s *= qs;
-                x[j] = (m >> (8 * k + j)) & 1u ? s : -INFINITY;
-            }
-            g[k] = max3(max3(x[0], x[1], x[2]), max3(x[3], x[4], x[5]), fmaxf(x[6], x[7]));
+    for (uint32_t r = 0; r < kThreadRuns; ++r)
+        x[r] = j & 4u ? (j & 2u ? w[r].w : w[r].z) : (j & 2u ? w[r].y : w[r].x);
+#pragma unroll
+    for (uint32_t c = 0; c < 2; ++c) m[c] = __byte_perm(x[2 * c], x[2 * c + 1], half);
+}
+
+// E4M3: scale_chunk for the runs run0, run0 + 1 of sample tile v.
+__device__ __forceinline__ void scale_sample_chunk(uint32_t (&x)[32], const float* __restrict__ doc_scale,
+                                                   uint64_t sample_tiles, uint32_t v, uint32_t run0) {
+#pragma unroll
+    for (uint32_t r = 0; r < kChunkRuns; ++r) {
+        const float4* s = reinterpret_cast<const float4*>(doc_scale + ((run0 + r) * sample_tiles + v) * kSampleRun);
+#pragma unroll
+        for (uint32_t h = 0; h < kSampleRun / 4; ++h) {
+            const float4 f = __ldg(s + h);
+            uint32_t* y = x + r * kSampleRun + 4 * h;
+            y[0] = __float_as_uint(__uint_as_float(y[0]) * f.x);
+            y[1] = __float_as_uint(__uint_as_float(y[1]) * f.y);
+            y[2] = __float_as_uint(__uint_as_float(y[2]) * f.z);
+            y[3] = __float_as_uint(__uint_as_float(y[3]) * f.w);
         }
     }
-    if (coarse)
-        out[chunk] = fmaxf(max3(g[0], g[1], g[2]), g[3]);
-    else
-        *reinterpret_cast<float4*>(out + 4u * chunk) = make_float4(g[0], g[1], g[2], g[3]);
 }
-static_assert(kTcGroup == 8 && kTcCoarseGroup == 32, "a chunk of 32 docs holds 4 groups, or is one");
 
-// MAXIMA: the pass writes group maxima (TcCandLaunch::best) instead of candidates.
+// A 32-doc chunk's scores of docs whose filter bit is set, into g: g[p] is the best so far of the docs at
+// places p and p + 8 of their runs.
+template <int F>
+__device__ __forceinline__ void fold_maxima(uint32_t m, const uint32_t (&v)[32], float qs, float (&g)[8]) {
+#pragma unroll
+    for (uint32_t p = 0; p < 8; ++p) {
+        float x[4];
+#pragma unroll
+        for (uint32_t r = 0; r < 4; ++r) {
+            float s = __uint_as_float(v[8 * r + p]);
+            if (F == kTcE4M3) s *= qs;
+            x[r] = (m >> (8 * r + p)) & 1u ? s : -INFINITY;
+        }
+        g[p] = max3(max3(g[p], x[0], x[1]), x[2], x[3]);
+    }
+}
+
+// The maxima of the n-th 64 docs of a sample: eight groups of kTcGroup docs, or four of kTcCoarseGroup (every
+// fourth place of the runs).
+__device__ __forceinline__ void store_maxima(const float (&g)[8], float* out, uint32_t n, bool coarse) {
+    if (coarse) {
+        *reinterpret_cast<float4*>(out + 4u * n) =
+            make_float4(fmaxf(g[0], g[4]), fmaxf(g[1], g[5]), fmaxf(g[2], g[6]), fmaxf(g[3], g[7]));
+    } else {
+        float4* o = reinterpret_cast<float4*>(out + 8u * n);
+        o[0] = make_float4(g[0], g[1], g[2], g[3]);
+        o[1] = make_float4(g[4], g[5], g[6], g[7]);
+    }
+}
+static_assert(kTcGroup == 8 && kTcCoarseGroup == 16, "64 docs hold 8 groups, or 4");
+
+// One k-block of a tile's docs: rows y .. y + 127, or (sample) the run from row y of every part.
+template <bool SAMPLE>
+__device__ __forceinline__ void load_docs(void* dst, const CUtensorMap* map, int x, int y, unsigned long long* bar) {
+    if (SAMPLE)
+        tma_load_3d(dst, map, x, y, 0, bar);
+    else
+        tma_load_2d(dst, map, x, y, bar);
+}
+
+// MAXIMA: the pass writes group maxima (TcCandLaunch::best) of sample tiles instead of candidates; doc_map is
+// then the sample's (make_tc_sample_map).
 template <int F, int H, bool MAXIMA>
 __global__ void __launch_bounds__(64 + 256 * H, 1) tc_cand_kernel(const __grid_constant__ CUtensorMap doc_map,
                                                                   const __grid_constant__ CUtensorMap qry_map,
@@ -424,7 +499,9 @@ __global__ void __launch_bounds__(64 + 256 * H, 1) tc_cand_kernel(const __grid_c
     fence_after();
     launch_dependents();
     const uint32_t tmem = S.tmem_base;
-    const uint64_t ntiles = L.tile_count;
+    // a sample's CTAs have their own numbers of tiles
+    const uint64_t ntiles =
+        MAXIMA ? blockIdx.x + static_cast<uint64_t>(sample_units(L, blockIdx.x, gridDim.x)) * gridDim.x : L.tile_count;
     const long long budget = L.wait_budget > 0 ? L.wait_budget : kWaitBudget;
 
     if (warp == 0) {
@@ -441,11 +518,14 @@ __global__ void __launch_bounds__(64 + 256 * H, 1) tc_cand_kernel(const __grid_c
                         tma_load_2d(qsm + (static_cast<size_t>(h) * kb_n + kb) * kStageBytes, &qry_map,
                                     static_cast<int>(kb * (128 / Fmt<F>::elem)), h * kRows, &S.qbar);
             };
-            uint32_t n = 0;
+            uint32_t n = 0, visited = 0;
             bool held = false;
             TileWalk walk(L.tile_begin, L.tile_step, L.tile_skip, blockIdx.x, gridDim.x);
-            for (uint64_t it = blockIdx.x; it < ntiles && !S.abort && !held; it += gridDim.x, walk.advance()) {
-                const int y = static_cast<int>(walk.tile() * kRows);
+            for (uint64_t it = blockIdx.x; it < ntiles && !S.abort && !held;
+                 it += gridDim.x, walk.advance(), ++visited) {
+                const int y = static_cast<int>(
+                    MAXIMA ? sample_tile_of(sample_unit(L, blockIdx.x, gridDim.x, visited), L.block_step) * kSampleRun
+                           : walk.tile() * kRows);
                 for (uint32_t g = 0; g < sg_n; ++g, ++n) {
                     const uint32_t s = n % stages, ph = (n / stages) & 1u;
                     if (L.hold_load && n + 1 >= L.hold_load) {  // pipeline test: stop issuing here
@@ -456,8 +536,8 @@ __global__ void __launch_bounds__(64 + 256 * H, 1) tc_cand_kernel(const __grid_c
                     if (!mbar_wait(&S.empty[s], ph ^ 1u, S, L.error, 1, budget)) break;
                     mbar_expect_tx(&S.full[s], static_cast<uint32_t>(stage_bytes));
                     for (uint32_t j = 0; j < G; ++j)
-                        tma_load_2d(ring + s * stage_bytes + j * kStageBytes, &doc_map,
-                                    static_cast<int>((g * G + j) * (128 / Fmt<F>::elem)), y, &S.full[s]);
+                        load_docs<MAXIMA>(ring + s * stage_bytes + j * kStageBytes, &doc_map,
+                                          static_cast<int>((g * G + j) * (128 / Fmt<F>::elem)), y, &S.full[s]);
                 }
             }
             if (!queries) load_queries();
@@ -532,15 +612,33 @@ __global__ void __launch_bounds__(64 + 256 * H, 1) tc_cand_kernel(const __grid_c
         TileWalk walk(L.tile_begin, L.tile_step, L.tile_skip, blockIdx.x, gridDim.x);
         uint64_t tile_next = walk.tile();
         uint64_t fw_next = 0;
-        if (valid && blockIdx.x < ntiles) fw_next = brow[tile_next * 2 + colh];
+        uint4 block_bits[kThreadRuns] = {};  // sample: a chunk's, loaded while the one before ends
+        auto load_bits = [&](uint32_t n) {
+            load_block_bits(block_bits, brow, L.sample_tiles,
+                            sample_tile_of(sample_unit(L, blockIdx.x, gridDim.x, n), L.block_step), colh * kThreadRuns);
+        };
+        if (valid && blockIdx.x < ntiles) {
+            if (MAXIMA)
+                load_bits(0);
+            else
+                fw_next = brow[tile_next * 2 + colh];
+        }
         for (uint64_t it = blockIdx.x; it < ntiles; it += gridDim.x, ++iter) {
             const uint32_t buf = iter & 1u;
-            const uint64_t tile = tile_next;
-            const uint64_t fw = fw_next;
-            walk.advance();
-            tile_next = walk.tile();
-            if (valid && it + gridDim.x < ntiles) fw_next = brow[tile_next * 2 + colh];
-            const uint32_t m[2] = {static_cast<uint32_t>(fw), static_cast<uint32_t>(fw >> 32)};
+            uint64_t tile = tile_next;
+            uint32_t m[2] = {static_cast<uint32_t>(fw_next), static_cast<uint32_t>(fw_next >> 32)};
+            uint32_t unit = 0;
+            if constexpr (MAXIMA) {
+                unit = sample_unit(L, blockIdx.x, gridDim.x, iter);
+                tile = sample_tile_of(unit, L.block_step);
+                tile_bits(block_bits, static_cast<uint32_t>(tile), m);
+                if (valid && ((iter + 1) & ((1u << L.chunk_log) - 1u)) == 0 && it + gridDim.x < ntiles)
+                    load_bits(iter + 1);
+            } else {
+                walk.advance();
+                tile_next = walk.tile();
+                if (valid && it + gridDim.x < ntiles) fw_next = brow[tile_next * 2 + colh];
+            }
             // 32-doc chunks that no query of the warp lets through are not read from TMEM at all
             bool live[2];
 #pragma unroll
@@ -562,16 +660,26 @@ __global__ void __launch_bounds__(64 + 256 * H, 1) tc_cand_kernel(const __grid_c
             fence_before();
             __syncwarp();
             if (lane == 0) mbar_arrive(&S.acc_empty[buf]);
+            if constexpr (MAXIMA) {
+                float best[8];
 #pragma unroll
-            for (int c = 0; c < 2; ++c) {
-                const uint64_t doc0 = tile * kRows + colh * 64u + c * 32u;
-                if (F == kTcE4M3 && live[c]) scale_chunk(v[c], L.doc_scale, doc0);
-                if constexpr (MAXIMA) {
-                    if (valid)
-                        store_maxima<F>(live[c], m[c], v[c], qs, L.best + static_cast<uint64_t>(qi) * L.cap,
-                                        static_cast<uint32_t>(it) * 4u + colh * 2u + c, L.coarse != 0);
-                } else if (live[c]) {
-                    emit_lane<F>(m[c], v[c], t, qs, doc0, out_score, out_loc, seg_cap, ncand);
+                for (uint32_t p = 0; p < 8; ++p) best[p] = -INFINITY;
+#pragma unroll
+                for (uint32_t c = 0; c < 2; ++c)
+                    if (live[c]) {
+                        if (F == kTcE4M3)
+                            scale_sample_chunk(v[c], L.doc_scale, L.sample_tiles, static_cast<uint32_t>(tile),
+                                               colh * kThreadRuns + c * kChunkRuns);
+                        fold_maxima<F>(m[c], v[c], qs, best);
+                    }
+                if (valid)
+                    store_maxima(best, L.best + static_cast<uint64_t>(qi) * L.cap, unit * 2u + colh, L.coarse != 0);
+            } else {
+#pragma unroll
+                for (int c = 0; c < 2; ++c) {
+                    const uint64_t doc0 = tile * kRows + colh * 64u + c * 32u;
+                    if (F == kTcE4M3 && live[c]) scale_chunk(v[c], L.doc_scale, doc0);
+                    if (live[c]) emit_lane<F>(m[c], v[c], t, qs, doc0, out_score, out_loc, seg_cap, ncand);
                 }
             }
         }
@@ -696,7 +804,9 @@ __global__ void __launch_bounds__(kPairThreads, 1) tc2_cand_kernel(const __grid_
     fence_after();
     launch_dependents();
     const uint32_t tmem = S.tmem_base;
-    const uint64_t ntiles = L.tile_count;
+    const uint64_t ntiles = EMIT == kEmitMaxima
+                                ? pair + static_cast<uint64_t>(sample_units(L, pair, npairs)) * npairs
+                                : L.tile_count;
 
     if (warp == 0) {
         if (lane == 0) {
@@ -712,10 +822,13 @@ __global__ void __launch_bounds__(kPairThreads, 1) tc2_cand_kernel(const __grid_
                                 static_cast<int>(kb * (128 / Fmt<F>::elem)), static_cast<int>(rank * kRows), &S.qbar);
             };
             if (SQ) load_queries();
-            uint32_t n = 0, s = 0, ph = 0;  // stages issued; ring slot and phase of the next
+            uint32_t n = 0, s = 0, ph = 0, visited = 0;  // stages issued; ring slot and phase of the next; tiles
             TileWalk walk(L.tile_begin, L.tile_step, L.tile_skip, pair, npairs);
-            for (uint64_t it = pair; it < ntiles && !S.abort; it += npairs, walk.advance()) {
-                const int y = static_cast<int>(walk.tile() * 2 * kRows + rank * kRows);
+            for (uint64_t it = pair; it < ntiles && !S.abort; it += npairs, walk.advance(), ++visited) {
+                const int y = static_cast<int>(
+                    EMIT == kEmitMaxima
+                        ? (sample_tile_of(2 * sample_unit(L, pair, npairs, visited), L.block_step) + rank) * kSampleRun
+                        : (walk.tile() * 2 + rank) * kRows);
                 for (uint32_t g = 0; g < sg_n; ++g, ++n, s = s + 1 == stages ? 0 : s + 1, ph ^= s == 0 ? 1u : 0u) {
                     if (!SQ && n == stages) load_queries();
                     if (!pair_wait<F>(&S.empty[s], ph ^ 1u, S, L.error, 1, false)) break;
@@ -724,12 +837,13 @@ __global__ void __launch_bounds__(kPairThreads, 1) tc2_cand_kernel(const __grid_
                     if (SQ) {
                         tma_load_2d(st, &qry_map, static_cast<int>(g * (128 / Fmt<F>::elem)),
                                     static_cast<int>(rank * kRows), &S.full[s]);
-                        tma_load_2d(st + kStageBytes, &doc_map, static_cast<int>(g * (128 / Fmt<F>::elem)), y,
-                                    &S.full[s]);
+                        load_docs<EMIT == kEmitMaxima>(st + kStageBytes, &doc_map,
+                                                       static_cast<int>(g * (128 / Fmt<F>::elem)), y, &S.full[s]);
                     } else {
                         for (uint32_t j = 0; j < G; ++j)
-                            tma_load_2d(st + j * kStageBytes, &doc_map,
-                                        static_cast<int>((g * G + j) * (128 / Fmt<F>::elem)), y, &S.full[s]);
+                            load_docs<EMIT == kEmitMaxima>(st + j * kStageBytes, &doc_map,
+                                                           static_cast<int>((g * G + j) * (128 / Fmt<F>::elem)), y,
+                                                           &S.full[s]);
                     }
                 }
             }
@@ -827,15 +941,28 @@ __global__ void __launch_bounds__(kPairThreads, 1) tc2_cand_kernel(const __grid_
         TileWalk walk(L.tile_begin, L.tile_step, L.tile_skip, pair, npairs);
         const uint32_t nt = static_cast<uint32_t>(ntiles);
         uint32_t tile_next = static_cast<uint32_t>(walk.tile());
-        uint64_t fw_next = pair < nt ? word_of(tile_next) : 0ull;
+        uint64_t fw_next = EMIT != kEmitMaxima && pair < nt ? word_of(tile_next) : 0ull;
+        uint4 block_bits[kThreadRuns] = {};  // as in tc_cand_kernel
+        auto load_bits = [&](uint32_t n) {
+            load_block_bits(block_bits, brow, L.sample_tiles,
+                            sample_tile_of(2 * sample_unit(L, pair, npairs, n), L.block_step), (g & 1u) * kThreadRuns);
+        };
+        if (EMIT == kEmitMaxima && valid && pair < nt) load_bits(0);
         for (uint32_t it = pair; it < nt; it += npairs, ++iter) {
             const uint32_t buf = iter & 1u;
-            const uint64_t tile = tile_next;
-            const uint64_t fw = fw_next;
-            walk.advance();
-            tile_next = static_cast<uint32_t>(walk.tile());
-            if (it + npairs < nt) fw_next = word_of(tile_next);
-            const uint32_t m[2] = {static_cast<uint32_t>(fw), static_cast<uint32_t>(fw >> 32)};
+            uint64_t tile = tile_next;  // (sample: the 128-doc tile of this thread's columns)
+            uint32_t m[2] = {static_cast<uint32_t>(fw_next), static_cast<uint32_t>(fw_next >> 32)};
+            uint32_t unit = 0;
+            if constexpr (EMIT == kEmitMaxima) {
+                unit = sample_unit(L, pair, npairs, iter);
+                tile = sample_tile_of(2 * unit, L.block_step) + g / 2;
+                tile_bits(block_bits, static_cast<uint32_t>(tile), m);
+                if (valid && ((iter + 1) & ((1u << L.chunk_log) - 1u)) == 0 && it + npairs < nt) load_bits(iter + 1);
+            } else {
+                walk.advance();
+                tile_next = static_cast<uint32_t>(walk.tile());
+                if (it + npairs < nt) fw_next = word_of(tile_next);
+            }
             bool live[2];
 #pragma unroll
             for (int c = 0; c < 2; ++c) live[c] = __any_sync(0xffffffffu, m[c] != 0u);
@@ -868,6 +995,11 @@ __global__ void __launch_bounds__(kPairThreads, 1) tc2_cand_kernel(const __grid_
                 // one 32-doc chunk in registers at a time (79 registers, where both chunks at once
                 // spilled at the 96-register ceiling); the buffer goes back to the issuer once the
                 // second is loaded
+                float best[8];
+                if constexpr (EMIT == kEmitMaxima) {
+#pragma unroll
+                    for (uint32_t p = 0; p < 8; ++p) best[p] = -INFINITY;
+                }
 #pragma unroll
                 for (int c = 0; c < 2; ++c) {
                     uint32_t v[32];
@@ -879,16 +1011,22 @@ __global__ void __launch_bounds__(kPairThreads, 1) tc2_cand_kernel(const __grid_
                         __syncwarp();
                         if (lane == 0) mbar_arrive_cluster(buf ? acc_empty_addr1 : acc_empty_addr0);
                     }
-                    const uint64_t doc0 = tile * 256u + g * 64u + c * 32u;
+                    if (!live[c]) continue;
                     // (a live chunk has a filtered doc, so its docs are rows of the corpus and have scales)
-                    if (F == kTcE4M3 && live[c]) scale_chunk(v, L.doc_scale, doc0);
                     if constexpr (EMIT == kEmitMaxima) {
-                        if (valid)
-                            store_maxima<F>(live[c], m[c], v, qs, L.best + static_cast<uint64_t>(qi) * L.cap,
-                                            it * 8u + g * 2u + c, L.coarse != 0);
-                    } else if (live[c]) {
+                        if (F == kTcE4M3)
+                            scale_sample_chunk(v, L.doc_scale, L.sample_tiles, static_cast<uint32_t>(tile),
+                                               (g & 1u) * kThreadRuns + c * kChunkRuns);
+                        fold_maxima<F>(m[c], v, qs, best);
+                    } else {
+                        const uint64_t doc0 = tile * 256u + g * 64u + c * 32u;
+                        if (F == kTcE4M3) scale_chunk(v, L.doc_scale, doc0);
                         emit_lane<F>(m[c], v, t, qs, doc0, out_score, out_loc, seg_cap, ncand);
                     }
+                }
+                if constexpr (EMIT == kEmitMaxima) {
+                    if (valid)
+                        store_maxima(best, L.best + static_cast<uint64_t>(qi) * L.cap, unit * 4u + g, L.coarse != 0);
                 }
             }
         }
@@ -1003,10 +1141,22 @@ cudaError_t launch_tc_cand(const TcCandLaunch& Lin, const CUtensorMap& doc_map, 
     if (L.ctas != tc_cand_ctas(L.nq_rows, L.kblocks, L.tile_count, sms, L.cap) || L.seg_cap == 0 || seg_end > kMaxCandSegs ||
         seg_end * L.seg_cap > L.cap)
         return cudaErrorInvalidValue;
-    // a tile's group maxima stay inside a query's row, in 16-byte stores
-    if (L.best && (L.tile_count * (tc_tile_docs(L.nq_rows, L.kblocks) / (L.coarse ? kTcCoarseGroup : kTcGroup)) > L.cap || L.cap % 4 ||
-                   (reinterpret_cast<uintptr_t>(L.best) & 15u)))
-        return cudaErrorInvalidValue;
+    if (L.best) {
+        // whole blocks of sample tiles inside the corpus; a tile's group maxima stay inside a query's row, in
+        // 16-byte stores
+        const uint64_t tiles = L.tile_count * (pair ? 2u : 1u);
+        const uint32_t groups = tc_tile_docs(L.nq_rows, L.kblocks) / (L.coarse ? kTcCoarseGroup : kTcGroup);
+        if (L.sample_tiles > L.tiles128 || !sample_fits(tiles, L.block_step, L.sample_tiles) ||
+            L.bits_stride < 2ull * L.sample_tiles || L.bits_stride % 2 ||
+            (reinterpret_cast<uintptr_t>(L.bits) & 15u) || L.tile_count * groups > L.cap || L.cap % 4 ||
+            (reinterpret_cast<uintptr_t>(L.best) & 15u))
+            return cudaErrorInvalidValue;
+        // the longest chunks, within a block, that leave no CTA more tiles than an even share
+        const uint64_t of = L.ctas / (pair ? 2u : 1u), share = (L.tile_count + of - 1) / of;
+        L.chunk_log = 0;
+        for (uint32_t c = 2; c <= kSampleBlock / (pair ? 2u : 1u); c *= 2)
+            if ((L.tile_count / c + of - 1) / of * c <= share) L.chunk_log = c == 2 ? 1 : c == 4 ? 2 : 3;
+    }
     switch (L.format) {
         case kTcTF32: return sq ? launch_tc2_typed<kTcTF32, true>(L, doc_map, qry_map, stream)
                                 : pair ? launch_tc2_typed<kTcTF32, false>(L, doc_map, qry_map, stream)
@@ -1037,7 +1187,8 @@ PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
 }
 }  // namespace
 
-bool make_tc_map(CUtensorMap* map, int format, const void* base, uint64_t rows, uint32_t dim) {
+static bool encode_map(CUtensorMap* map, int format, const void* base, uint32_t dim, uint32_t rank,
+                       const cuuint64_t (&rows)[2], const cuuint32_t (&box_rows)[2]) {
     auto fn = encode_fn();
     if (!fn) return false;
     const uint32_t elem = format == kTcTF32 ? 4 : (format == kTcBF16 ? 2 : 1);
@@ -1045,14 +1196,22 @@ bool make_tc_map(CUtensorMap* map, int format, const void* base, uint64_t rows, 
                                    : format == kTcBF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16
                                                        : CU_TENSOR_MAP_DATA_TYPE_UINT8;
     if ((reinterpret_cast<uintptr_t>(base) & 15u) || (static_cast<uint64_t>(dim) * elem) % 128 != 0) return false;
-    cuuint64_t gdim[2] = {dim, rows};
-    cuuint64_t gstride[1] = {static_cast<cuuint64_t>(dim) * elem};
-    cuuint32_t box[2] = {128u / elem, 128u};
-    cuuint32_t estride[2] = {1, 1};
-    const CUresult r = fn(map, dt, 2, const_cast<void*>(base), gdim, gstride, box, estride, CU_TENSOR_MAP_INTERLEAVE_NONE,
+    cuuint64_t gdim[3] = {dim, rows[0], rows[1]};
+    cuuint64_t gstride[2] = {static_cast<cuuint64_t>(dim) * elem, rows[0] * static_cast<cuuint64_t>(dim) * elem};
+    cuuint32_t box[3] = {128u / elem, box_rows[0], box_rows[1]};
+    cuuint32_t estride[3] = {1, 1, 1};
+    const CUresult r = fn(map, dt, rank, const_cast<void*>(base), gdim, gstride, box, estride, CU_TENSOR_MAP_INTERLEAVE_NONE,
                           CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS;
+}
+
+bool make_tc_map(CUtensorMap* map, int format, const void* base, uint64_t rows, uint32_t dim) {
+    return encode_map(map, format, base, dim, 2, {rows, 1}, {128u, 1u});
+}
+
+bool make_tc_sample_map(CUtensorMap* map, int format, const void* base, uint64_t sample_tiles, uint32_t dim) {
+    return encode_map(map, format, base, dim, 3, {sample_tiles * kSampleRun, kSampleRuns}, {kSampleRun, kSampleRuns});
 }
 
 }  // namespace hss
