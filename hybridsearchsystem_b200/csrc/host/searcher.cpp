@@ -1016,8 +1016,9 @@ int FullRecallSearcher::EnqueueAttempt(uint32_t nq, const BatchInputs& in, float
     auto* dTheta1 = reinterpret_cast<float*>(D + SL.theta1);
     if (!wantStats) m_b.want = std::max<uint64_t>(m_b.want, SampleOptimum(nq, maxK));
     uint64_t sampCount = 0;
+    // lists have no use for a sample past what the list capacity asks for
+    if (!wantStats && !Maxima(nq, m_b.want, false).groups) m_b.want = m_b.wantRerun;
     if (m_b.want > m_cfg.sampleDocs && !Maxima(nq, m_b.want, false).groups) {
-        m_b.want = m_b.wantRerun;
         // A sample grown with K, kept as lists, in two steps: the sample_docs sample's proven threshold first, then the
         // grown sample keeps only the docs above it. Its K-th best is the same whenever it has K docs
         // above that threshold (and raises theta_1 then); otherwise theta_1 stays. Every doc of the
