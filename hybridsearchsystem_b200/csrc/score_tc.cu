@@ -626,8 +626,7 @@ __global__ void __launch_bounds__(64 + 256 * H, 1) tc_cand_kernel(const __grid_c
         for (uint64_t it = blockIdx.x; it < ntiles; it += gridDim.x, ++iter) {
             const uint32_t buf = iter & 1u;
             uint64_t tile = tile_next;
-            uint32_t m[2] = {static_cast<uint32_t>(fw_next), static_cast<uint32_t>(fw_next >> 32)};
-            uint32_t unit = 0;
+            uint32_t m[2], unit = 0;
             if constexpr (MAXIMA) {
                 unit = sample_unit(L, blockIdx.x, gridDim.x, iter);
                 tile = sample_tile_of(unit, L.block_step);
@@ -635,9 +634,12 @@ __global__ void __launch_bounds__(64 + 256 * H, 1) tc_cand_kernel(const __grid_c
                 if (valid && ((iter + 1) & ((1u << L.chunk_log) - 1u)) == 0 && it + gridDim.x < ntiles)
                     load_bits(iter + 1);
             } else {
+                const uint64_t fw = fw_next;
                 walk.advance();
                 tile_next = walk.tile();
                 if (valid && it + gridDim.x < ntiles) fw_next = brow[tile_next * 2 + colh];
+                m[0] = static_cast<uint32_t>(fw);
+                m[1] = static_cast<uint32_t>(fw >> 32);
             }
             // 32-doc chunks that no query of the warp lets through are not read from TMEM at all
             bool live[2];
@@ -951,17 +953,19 @@ __global__ void __launch_bounds__(kPairThreads, 1) tc2_cand_kernel(const __grid_
         for (uint32_t it = pair; it < nt; it += npairs, ++iter) {
             const uint32_t buf = iter & 1u;
             uint64_t tile = tile_next;  // (sample: the 128-doc tile of this thread's columns)
-            uint32_t m[2] = {static_cast<uint32_t>(fw_next), static_cast<uint32_t>(fw_next >> 32)};
-            uint32_t unit = 0;
+            uint32_t m[2], unit = 0;
             if constexpr (EMIT == kEmitMaxima) {
                 unit = sample_unit(L, pair, npairs, iter);
                 tile = sample_tile_of(2 * unit, L.block_step) + g / 2;
                 tile_bits(block_bits, static_cast<uint32_t>(tile), m);
                 if (valid && ((iter + 1) & ((1u << L.chunk_log) - 1u)) == 0 && it + npairs < nt) load_bits(iter + 1);
             } else {
+                const uint64_t fw = fw_next;
                 walk.advance();
                 tile_next = static_cast<uint32_t>(walk.tile());
                 if (it + npairs < nt) fw_next = word_of(tile_next);
+                m[0] = static_cast<uint32_t>(fw);
+                m[1] = static_cast<uint32_t>(fw >> 32);
             }
             bool live[2];
 #pragma unroll
@@ -1011,17 +1015,18 @@ __global__ void __launch_bounds__(kPairThreads, 1) tc2_cand_kernel(const __grid_
                         __syncwarp();
                         if (lane == 0) mbar_arrive_cluster(buf ? acc_empty_addr1 : acc_empty_addr0);
                     }
-                    if (!live[c]) continue;
                     // (a live chunk has a filtered doc, so its docs are rows of the corpus and have scales)
                     if constexpr (EMIT == kEmitMaxima) {
-                        if (F == kTcE4M3)
-                            scale_sample_chunk(v, L.doc_scale, L.sample_tiles, static_cast<uint32_t>(tile),
-                                               (g & 1u) * kThreadRuns + c * kChunkRuns);
-                        fold_maxima<F>(m[c], v, qs, best);
+                        if (live[c]) {
+                            if (F == kTcE4M3)
+                                scale_sample_chunk(v, L.doc_scale, L.sample_tiles, static_cast<uint32_t>(tile),
+                                                   (g & 1u) * kThreadRuns + c * kChunkRuns);
+                            fold_maxima<F>(m[c], v, qs, best);
+                        }
                     } else {
                         const uint64_t doc0 = tile * 256u + g * 64u + c * 32u;
-                        if (F == kTcE4M3) scale_chunk(v, L.doc_scale, doc0);
-                        emit_lane<F>(m[c], v, t, qs, doc0, out_score, out_loc, seg_cap, ncand);
+                        if (F == kTcE4M3 && live[c]) scale_chunk(v, L.doc_scale, doc0);
+                        if (live[c]) emit_lane<F>(m[c], v, t, qs, doc0, out_score, out_loc, seg_cap, ncand);
                     }
                 }
                 if constexpr (EMIT == kEmitMaxima) {
