@@ -524,7 +524,7 @@ class FullRecallSearcher {
     static uint32_t GraphTopK(uint32_t maxK);
     static uint32_t GraphOperands(uint32_t maxOpnd);
     // The K a batch's launch plan is made for under graph replay.
-    uint32_t PlanTopK(uint32_t maxK) const;
+    uint32_t PlanTopK(uint32_t nq, uint32_t maxK) const;
 
     const StageTimes& LastTimes() const { return m_times; }
     void SetTiming(bool on) { m_timing = on; }
@@ -578,10 +578,22 @@ class FullRecallSearcher {
     uint64_t Sample(const uint32_t* dList, uint32_t rows, bool simt, bool raiseOnly = false, float* stats = nullptr,
                     float* thetaCopy = nullptr, const float* emitTheta = nullptr);
     uint32_t SampleTileNum() const;
-    MaximaSample Maxima(uint32_t rows, uint64_t want, bool simt) const;
+    MaximaSample Maxima(uint32_t rows, uint64_t want, uint32_t maxK, bool simt) const;
     uint64_t SampleOptimum(uint32_t nq, uint32_t maxK) const;
     bool SplitSelect(uint32_t nq, uint32_t maxK) const;
     bool OnePass(uint32_t nq, uint32_t maxK, uint64_t sampled) const;
+    struct Plan {
+        uint64_t want = 0, wantRerun = 0;    // docs of the sample, and of a re-run's
+        uint32_t groups = 0, groupDocs = 0;  // its group maxima (0: lists)
+        bool twoStep = false;                // lists of a grown sample
+        bool onePass = false;
+        bool spread = false, large = false;  // the select step's forms
+        bool operator==(const Plan& o) const {
+            return want == o.want && wantRerun == o.wantRerun && groups == o.groups && groupDocs == o.groupDocs &&
+                   twoStep == o.twoStep && onePass == o.onePass && spread == o.spread && large == o.large;
+        }
+    };
+    Plan PlanOf(uint32_t nq, uint32_t maxK, bool stats) const;
     void SampleTiles(uint64_t want, uint32_t rows, bool simt, uint64_t* count, uint64_t* step) const;
     // A batch's small inputs in the pinned staging buffer: per-query program and operand offsets, K,
     // the programs and then their operands (operand offsets count from the program array's start);

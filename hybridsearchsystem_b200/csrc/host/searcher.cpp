@@ -652,7 +652,8 @@ uint32_t FullRecallSearcher::SampleTileNum() const {
 // maximum). Coarse groups, half the stores and the threshold's entries, where K is an eighth of them at most
 // (the K-th maximum is then at rank 1.07 K or better among the docs). Both hold for any order of the corpus: a
 // group's docs lie far apart (kSampleRuns), and the sample's blocks are spread over all of it.
-FullRecallSearcher::MaximaSample FullRecallSearcher::Maxima(uint32_t rows, uint64_t want, bool simt) const {
+FullRecallSearcher::MaximaSample FullRecallSearcher::Maxima(uint32_t rows, uint64_t want, uint32_t maxK,
+                                                            bool simt) const {
     MaximaSample M;
     const uint64_t all = SampleTileNum() / kSampleBlock, docs = 128ull * kSampleBlock;
     if (all == 0) return M;
@@ -663,9 +664,9 @@ FullRecallSearcher::MaximaSample FullRecallSearcher::Maxima(uint32_t rows, uint6
     const uint64_t sampled = blocks * docs;
     M.blockStep = (all << 32) / blocks;
     M.tiles = sampled / UnitOf(rows, simt);
-    M.docs = UseSimt(simt) ? kSimtGroup : sampled / kTcCoarseGroup >= 8ull * m_b.maxK ? kTcCoarseGroup : kTcGroup;
+    M.docs = UseSimt(simt) ? kSimtGroup : sampled / kTcCoarseGroup >= 8ull * maxK ? kTcCoarseGroup : kTcGroup;
     const uint64_t groups = sampled / M.docs;
-    if (groups >= 2ull * m_b.maxK && groups <= m_sampCap) M.groups = static_cast<uint32_t>(groups);
+    if (groups >= 2ull * maxK && groups <= m_sampCap) M.groups = static_cast<uint32_t>(groups);
     return M;
 }
 
@@ -677,7 +678,7 @@ uint64_t FullRecallSearcher::Sample(const uint32_t* dList, uint32_t rows, bool s
     const StageLayout SL = MakeLayout(m_cfg.maxBatch);
     uint8_t* D = m_dStage;
     auto* dSampCount = reinterpret_cast<uint32_t*>(D + SL.sampCount);
-    const MaximaSample maxima = stats || raiseOnly ? MaximaSample{} : Maxima(rows, m_b.want, simt);
+    const MaximaSample maxima = stats || raiseOnly ? MaximaSample{} : Maxima(rows, m_b.want, m_b.maxK, simt);
     uint64_t count = maxima.tiles, step = 1;
     if (!maxima.groups) SampleTiles(m_b.want, rows, simt, &count, &step);
     const uint32_t segs = SegsOf(rows, count, m_sampCap, simt);
@@ -762,7 +763,7 @@ int FullRecallSearcher::SearchEnqueue(const float* dQueries, uint32_t nq, const 
     BatchInputs in = PrepareInputs(nq, rows, exprs, topks, std::min(1u, outStride));
     int rc;
     if (graph) {
-        in.maxK = PlanTopK(in.maxK);
+        in.maxK = PlanTopK(rows, in.maxK);
         in.maxOpnd = GraphOperands(in.maxOpnd);
         GraphKey key;
         key.rows = rows;
@@ -870,12 +871,38 @@ bool FullRecallSearcher::OnePass(uint32_t nq, uint32_t maxK, uint64_t sampled) c
     return dense && more <= 300e3 && 8.0 * maxK * ratio <= m_cfg.candidateCap;
 }
 
-uint32_t FullRecallSearcher::PlanTopK(uint32_t maxK) const {
-    // A batch's K enters its launch plan through the doc sample's size (without a model: the sample;
-    // with one: pass A's share) and the select variant (K > 256): every K up to `flat` plans as
-    // K = 1 does.
+// What a batch's rows and largest K decide of its launches.
+FullRecallSearcher::Plan FullRecallSearcher::PlanOf(uint32_t nq, uint32_t maxK, bool stats) const {
+    Plan P;
+    P.wantRerun = SampleWant(maxK);
+    // Without a model the sample grows with K so that its threshold keeps the full pass within the list
+    // capacity; with one, the prediction sets the threshold and the sample only feeds the features (which are
+    // made from the same sample size, with or without a model set).
+    P.want = stats ? m_cfg.sampleDocs : std::max<uint64_t>(P.wantRerun, SampleOptimum(nq, maxK));
+    uint64_t tiles = 0, step = 1;
+    if (!stats) {
+        const MaximaSample M = Maxima(nq, P.want, maxK, false);
+        P.groups = M.groups;
+        P.groupDocs = M.docs;
+        tiles = M.tiles;
+        // lists have no use for a sample past what the list capacity asks for
+        if (!P.groups) P.want = P.wantRerun;
+    }
+    P.twoStep = !stats && !P.groups && P.want > m_cfg.sampleDocs;
+    if (!P.groups) SampleTiles(P.want, nq, false, &tiles, &step);
+    P.onePass = !stats && OnePass(nq, maxK, std::min<uint64_t>(tiles * UnitOf(nq, false), m_table->GetDocNum()));
+    P.spread = SplitSelect(nq, maxK);
+    P.large = maxK > 256;
+    return P;
+}
+
+uint32_t FullRecallSearcher::PlanTopK(uint32_t nq, uint32_t maxK) const {
+    // K is rounded up to a power of two, and to the largest one up to 256 whose plan is that of K = 1: a replayed
+    // batch takes the launches that it would take directly, but for a sample of a K up to twice its own.
+    const bool stats = static_cast<bool>(m_model);
+    const Plan least = PlanOf(nq, 1, stats);
     uint32_t flat = 1;
-    while (flat < 256 && SampleWant(flat * 2) == SampleWant(1)) flat <<= 1;
+    while (flat < 256 && PlanOf(nq, flat * 2, stats) == least) flat <<= 1;
     return maxK == 0 ? 0u : std::max(GraphTopK(maxK), flat);
 }
 
@@ -1003,30 +1030,24 @@ int FullRecallSearcher::EnqueueAttempt(uint32_t nq, const BatchInputs& in, float
     if (m_timing) Ck(cudaEventRecord(m_ev[1], stream));
 
     // 1. doc sample: evenly spaced tiles; its K-th best bounds the threshold.
-    // Without a model it grows with K so that its threshold keeps the full pass within the list
-    // capacity; with one, the prediction sets the threshold and the sample only feeds the features
-    // (which are made from the same sample size, with or without a model set).
     const bool learned = static_cast<bool>(m_model);
-    m_b.wantRerun = SampleWant(maxK);
-    m_b.want = learned || m_featuresOut != nullptr ? m_cfg.sampleDocs : m_b.wantRerun;
-    m_b.learned = learned;
     const bool wantStats = learned || m_featuresOut != nullptr;
+    const Plan plan = PlanOf(nq, maxK, wantStats);
+    m_b.wantRerun = plan.wantRerun;
+    m_b.want = plan.want;
+    m_b.learned = learned;
     // the sample's proven thresholds (theta_1) are also kept in theta1, copied to the host with the
     // statuses (a copy here would stall the stream between the sample and the passes)
     auto* dTheta1 = reinterpret_cast<float*>(D + SL.theta1);
-    if (!wantStats) m_b.want = std::max<uint64_t>(m_b.want, SampleOptimum(nq, maxK));
     uint64_t sampCount = 0;
-    // lists have no use for a sample past what the list capacity asks for
-    if (!wantStats && !Maxima(nq, m_b.want, false).groups) m_b.want = m_b.wantRerun;
-    if (m_b.want > m_cfg.sampleDocs && !Maxima(nq, m_b.want, false).groups) {
+    if (plan.twoStep) {
         // A sample grown with K, kept as lists, in two steps: the sample_docs sample's proven threshold first, then the
         // grown sample keeps only the docs above it. Its K-th best is the same whenever it has K docs
         // above that threshold (and raises theta_1 then); otherwise theta_1 stays. Every doc of the
         // grown sample is otherwise stored and walked (K = 1000 at 10M: about 76k per query).
-        const uint64_t grown = m_b.want;
         m_b.want = m_cfg.sampleDocs;
         (void)Sample(nullptr, nq, false, false, nullptr, dTheta1);
-        m_b.want = grown;
+        m_b.want = plan.want;
         sampCount = Sample(nullptr, nq, false, true, nullptr, dTheta1, dTheta);
         m_b.launches += 4;
     } else {
@@ -1069,7 +1090,7 @@ int FullRecallSearcher::EnqueueAttempt(uint32_t nq, const BatchInputs& in, float
     }
     uint32_t split = static_cast<uint32_t>(std::sqrt(static_cast<double>(tilesM) / static_cast<double>(splitSample)));
     split = std::min<uint32_t>(split, 64);
-    if (!learned && OnePass(nq, maxK, std::min<uint64_t>(sampCount * UnitOf(nq, false), T.GetDocNum()))) split = 1;
+    if (plan.onePass) split = 1;
     SelectLaunch& SE = m_b.se;
     SE.vec = T.DeviceVectors();
     SE.qry = dQueries;
@@ -1092,11 +1113,11 @@ int FullRecallSearcher::EnqueueAttempt(uint32_t nq, const BatchInputs& in, float
     SE.nq_list = nq;
     // a batch with a large K keeps long candidate lists (K = 1000: about 13k per query at 10M, past
     // the default shared-memory buffer): select K from {10, 100, 1000} 0.302 -> 0.199 ms
-    SE.fast_large = maxK > 256 ? 1 : 0;
+    SE.fast_large = plan.large ? 1 : 0;
     // in the sample's counts, which nothing reads any more (the spread rescoring reads the queries 16
     // bytes at a time)
     static_assert(kMaxCandSegs * 4 >= sizeof(uint2), "a query's pending rows fit where its counts were");
-    SE.pending = SplitSelect(nq, maxK) && (reinterpret_cast<uintptr_t>(dQueries) & 15u) == 0
+    SE.pending = plan.spread && (reinterpret_cast<uintptr_t>(dQueries) & 15u) == 0
                      ? reinterpret_cast<uint2*>(D + SL.sampCount)
                      : nullptr;
     // With a model, theta is the prediction: the passes below run at it (raised like a proven one

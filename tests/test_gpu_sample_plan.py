@@ -46,3 +46,32 @@ def test_a_sample_that_does_not_grow_is_taken_once(torch_cuda):
         assert t["retries"] == 0
         launches[k] = t["launches"]
     assert launches[2400] == launches[2300]
+
+
+@pytest.mark.parametrize("method,n,nq,k", [(BF16, 300_000, 256, 8), (E4M3, 100_000, 16, 10)], ids=["bf16", "e4m3"])
+def test_a_replayed_batch_is_planned_as_a_direct_one(torch_cuda, method, n, nq, k):
+    # a small K: the same sample (its thresholds, bit for bit), the same docs kept and the same launches, whether
+    # they are replayed from a graph, which is shared by other K, or not
+    torch = torch_cuda
+    mix, vec, bits, table = _world(n)
+    s = hss.FullRecallSearcher(table, max_batch=nq, method=method)
+    q = mix.queries(nq, seed=35)
+    exprs = data.make_filters(mix, nq, n_tags=(1, 2), seed=36)
+    f = s.compile_filters(exprs)
+    d_q = torch.from_numpy(q).to("cuda:0")
+    sc = torch.zeros((nq, k), dtype=torch.float32, device="cuda:0")
+    ids = torch.zeros((nq, k), dtype=torch.int64, device="cuda:0")
+    cnt = torch.zeros(nq, dtype=torch.int32, device="cuda:0")
+    stream = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    seen = []
+    for graphs in (False, True, True):  # direct, captured, replayed
+        s.set_graphs(graphs)
+        assert s.search_device(d_q.data_ptr(), nq, f, [k] * nq, sc.data_ptr(), ids.data_ptr(), cnt.data_ptr(), k,
+                               stream.cuda_stream) == 0
+        stream.synchronize()
+        seen.append((s.last_thresholds(nq)[0].tobytes(), s.last_candidate_counts(nq).tobytes(),
+                     s.last_times()["launches"], s.last_times()["retries"]))
+    assert s.graph_stats()["replays"] == 1
+    assert seen[1:] == [seen[0]] * 2
+    _check(sc.cpu().numpy(), ids.cpu().numpy(), cnt.cpu().numpy(), oracle.topk(q, exprs, [k] * nq, vec, bits, threads=8))
