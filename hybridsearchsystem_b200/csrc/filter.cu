@@ -25,6 +25,7 @@ struct OperandInfo {
     uint32_t layout;  // kEmpty for an all-zero or absent posting
     uint32_t plen;    // payload bytes (clamped to what the layout can legally hold)
     uint32_t k;       // sparse entries
+    uint32_t lo, hi;  // those of them that a tile reads
 };
 constexpr uint32_t kEmpty = 0xffu;
 
@@ -84,7 +85,7 @@ __device__ inline void resolve_operand(OperandInfo& o, const uint8_t* addr, uint
     o.addr = addr;
     o.layout = kEmpty;
     o.plen = 0;
-    o.k = 0;
+    o.k = o.lo = o.hi = 0;
     if (addr == nullptr) return;
     const uint64_t both = ld64(addr);  // [layout:4|hits:28] and the payload's bytes
     const uint32_t head = static_cast<uint32_t>(both);
@@ -100,6 +101,30 @@ __device__ inline void resolve_operand(OperandInfo& o, const uint8_t* addr, uint
     if (layout == kSparseBitmap) o.k = o.plen / 6;
     if (layout == kSparsePacked) o.k = o.plen / 4;
     if (layout == kSparseIdList) o.k = o.plen / 4;
+    o.hi = o.k;
+}
+
+// The entries of a sparse bitmap or packed posting (sorted by unit) with units in [u0, u1), into o.lo and o.hi, by a
+// full warp: 16 lanes look for the first entry from u0 on, the others for the first from u1 on, each step
+// cutting what is left to a sixteenth (4,096 entries: three dependent loads).
+__device__ inline void find_entries(OperandInfo& o, uint32_t u0, uint32_t u1) {
+    const uint32_t lane = threadIdx.x & 31, l = lane & 15, shift = o.layout == kSparsePacked ? 16u : 1u;
+    const uint32_t u = lane < 16 ? u0 : u1;
+    uint32_t lo = 0, hi = o.k;  // entries before lo are below u, those from hi on are not
+    while (__any_sync(0xffffffffu, lo < hi)) {
+        const uint32_t step = (hi - lo + 15) / 16, at = lo + l * step;
+        const bool below = at < hi && ld32(o.addr + 8 + 4u * at) >> shift < u;
+        const uint32_t n = __popc((__ballot_sync(0xffffffffu, below) >> (lane & 16u)) & 0xffffu);  // a prefix of the 16
+        if (n == 0) {
+            hi = lo;
+        } else {
+            hi = min(hi, lo + n * step);
+            lo += (n - 1) * step + 1;
+        }
+    }
+    if (lane == 0) o.lo = lo;
+    if (lane == 16) o.hi = lo;
+    __syncwarp();
 }
 
 __device__ inline uint64_t tail_mask(uint64_t gw, uint64_t doc_num) {
@@ -119,6 +144,9 @@ __device__ inline uint64_t tail_mask(uint64_t gw, uint64_t doc_num) {
 template <int W, class Operand>
 __device__ __forceinline__ bool eval_words(const uint32_t* prog, uint32_t plen, Operand operand, uint32_t nop,
                                            uint64_t (&result)[W]) {
+    // two operands' loads in flight; at one or two words a thread the second only costs instructions (segments of
+    // 8,192 docs, 2M docs, 64 queries 103 and 96 us)
+    constexpr int kInFlight = W > 2 ? 2 : 1;
     uint64_t st[kMaxStack][W];
     uint32_t sp = 0, next = 0, pc = 0;
     while (pc < plen) {
@@ -146,7 +174,7 @@ __device__ __forceinline__ bool eval_words(const uint32_t* prog, uint32_t plen, 
                 const bool is_and = op == kOpAnd;
 #pragma unroll
                 for (int k = 0; k < W; ++k) acc[k] = is_and ? ~0ull : 0ull;
-#pragma unroll 2  // two operands' loads in flight
+#pragma unroll kInFlight
                 for (uint32_t j = 0; j < pn; ++j) {
                     operand(next + j, v);
 #pragma unroll
@@ -171,7 +199,7 @@ __device__ __forceinline__ bool eval_words(const uint32_t* prog, uint32_t plen, 
                 uint64_t o[W];
 #pragma unroll
                 for (int k = 0; k < W; ++k) o[k] = 0ull;
-#pragma unroll 2
+#pragma unroll kInFlight
                 for (uint32_t j = 0; j < pn; ++j) {
                     operand(next + j, v);
 #pragma unroll
@@ -199,13 +227,19 @@ __device__ __forceinline__ bool eval_words(const uint32_t* prog, uint32_t plen, 
 // One CTA per (query, segment tile of WPT * 256 words). A chain of dependent loads (offsets, rows, posting
 // heads, postings) bounds a CTA, so tiles are small enough that several CTAs share an SM. Dense operands
 // are read where they lie when the program gets to them; the others are decoded into shared-memory slots
-// of the tile first (bytemaps: each thread its own words; sparse: zeroed, then scattered). A sparse
-// posting holds a few thousand entries at most, so every tile reads all of them and keeps its own: a
-// search for the tile's first entry would be ten dependent loads. Grid: x = query (fastest, so all queries
-// of a tile share the tile's postings in L2), y = segment tile. 64 queries of up to 6 tags over 2M docs with
-// packed postings: 56 us with whole-segment tiles and every operand staged, 38 us now (256 queries over 4M
-// docs 376 -> 257 us a call).
-template <int WPT>
+// of the tile first (bytemaps: each thread its own words; sparse: zeroed, then scattered). A tile reads a short
+// sparse posting whole and keeps its own entries, and looks up where its entries of a long one lie (kScanEntries).
+// Grid: x = query (fastest, so all queries of a tile share the tile's postings in L2), y = segment tile. 64 queries
+// of up to 6 tags over 2M docs with packed postings: 56 us with whole-segment tiles and every operand staged, 38 us
+// now (256 queries over 4M docs 376 -> 257 us a call).
+// Us a call, 64 queries, read whole by every tile -> looked up from 1,024 entries on: 2M docs in segments of 1M, up to
+// 12 tags 472 -> 108; 4M docs in one segment 991 -> 96; segments of 131,072, 256 queries 420 -> 345. Looked up from 256
+// on: 312 in the last case, but 85 -> 92 with 64 queries of packed postings.
+constexpr uint32_t kScanEntries = 1024;
+
+// SPLIT: a segment has several tiles (without it the kernel needs no tile arithmetic and fewer registers: segments
+// of 16,384 docs, 2M docs, 64 queries 76 and 64 us).
+template <int WPT, bool SPLIT>
 __global__ void __launch_bounds__(kTile) filter_batch_kernel(FilterLaunch L, uint32_t tiles_per_cta) {
     constexpr uint32_t TW = kTile * WPT;  // words per CTA
     extern __shared__ uint64_t slots[];   // [nop][TW]
@@ -217,10 +251,11 @@ __global__ void __launch_bounds__(kTile) filter_batch_kernel(FilterLaunch L, uin
     const uint32_t q = blockIdx.x;
     const uint32_t t = threadIdx.x;
     const uint32_t seg_words = L.docs_per_seg / 64;
-    const uint32_t tiles = (seg_words + TW - 1) / TW;                       // of a segment
-    const uint32_t groups = (tiles + tiles_per_cta - 1) / tiles_per_cta;  // CTAs of a segment
-    const uint32_t seg = blockIdx.y / groups;
-    const uint32_t tile0 = (blockIdx.y % groups) * tiles_per_cta, tile1 = min(tiles, tile0 + tiles_per_cta);
+    const uint32_t tiles = SPLIT ? (seg_words + TW - 1) / TW : 1u;                       // of a segment
+    const uint32_t groups = SPLIT ? (tiles + tiles_per_cta - 1) / tiles_per_cta : 1u;  // CTAs of a segment
+    const uint32_t seg = SPLIT ? blockIdx.y / groups : blockIdx.y;
+    const uint32_t tile0 = SPLIT ? blockIdx.y % groups * tiles_per_cta : 0u;
+    const uint32_t tile1 = SPLIT ? min(tiles, tile0 + tiles_per_cta) : 1u;
     const uint32_t cta_w0 = tile0 * TW, cta_nw = min(tile1 * TW, seg_words) - cta_w0;
     const uint64_t seg_doc0 = static_cast<uint64_t>(seg) * L.docs_per_seg;
     const uint32_t seg_docs = static_cast<uint32_t>(min(static_cast<uint64_t>(L.docs_per_seg), L.doc_num - seg_doc0));
@@ -270,7 +305,7 @@ __global__ void __launch_bounds__(kTile) filter_batch_kernel(FilterLaunch L, uin
             o.addr = reinterpret_cast<const uint8_t*>(a) - 8;
             o.layout = kDenseBitmap;
             o.plen = L.docs_per_seg / 8;
-            o.k = 0;
+            o.k = o.lo = o.hi = 0;
         }
     }
     __syncthreads();
@@ -282,6 +317,12 @@ __global__ void __launch_bounds__(kTile) filter_batch_kernel(FilterLaunch L, uin
     for (uint32_t tile = tile0; tile < tile1; ++tile) {
         const uint32_t w0 = tile * TW, nw = min(TW, seg_words - w0);
         if (tile > tile0) __syncthreads();  // the slots are read
+        if (SPLIT)
+            for (uint32_t i = t / 32; i < nop; i += kTile / 32) {
+                OperandInfo& o = s_op[i];
+                if ((o.layout == kSparseBitmap || o.layout == kSparsePacked) && o.k > kScanEntries)
+                    find_entries(o, w0 * 4u, (w0 + nw) * 4u);
+            }
         // bytemaps: each thread its own words; sparse (and all-zero) postings: zero, then scatter below
         for (uint32_t i = 0; i < nop; ++i) {
             const OperandInfo& o = s_op[i];
@@ -299,7 +340,7 @@ __global__ void __launch_bounds__(kTile) filter_batch_kernel(FilterLaunch L, uin
                 uint16_t* units = reinterpret_cast<uint16_t*>(slots + i * TW);
                 const bool packed = o.layout == kSparsePacked;
 #pragma unroll 4
-                for (uint32_t e = t; e < o.k; e += kTile) {
+                for (uint32_t e = (SPLIT ? o.lo : 0u) + t; e < (SPLIT ? o.hi : o.k); e += kTile) {
                     const uint32_t x = ld32(o.addr + 8 + 4u * e);
                     const uint32_t mask = packed ? x & 0xffffu : ld16(o.addr + 8 + 4u * o.k + 2u * e);
                     const uint32_t rel = (packed ? x >> 16 : x / 2u) - w0 * 4u;
@@ -748,11 +789,12 @@ cudaError_t launch_filter_wpt(const FilterLaunch& L, cudaStream_t stream) {
     // opt in always (static plus dynamic shared memory may pass 48 KB even when the dynamic part does
     // not), to the one ceiling every caller sets: searchers on other threads launch it concurrently
     if (smem > kFilterSmemCeiling) return cudaErrorInvalidValue;
-    cudaError_t e = cudaFuncSetAttribute(filter_batch_kernel<WPT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    auto kernel = tiles > 1 ? filter_batch_kernel<WPT, true> : filter_batch_kernel<WPT, false>;
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          static_cast<int>(kFilterSmemCeiling));
     if (e != cudaSuccess) return e;
     dim3 grid(L.nq, static_cast<uint32_t>(gy));
-    filter_batch_kernel<WPT><<<grid, kTile, smem, stream>>>(L, tpc);
+    kernel<<<grid, kTile, smem, stream>>>(L, tpc);
     return cudaGetLastError();
 }
 
