@@ -409,8 +409,6 @@ class ThresholdModel {
     uint32_t m_cap = 0;
     float *m_dP = nullptr, *m_dG = nullptr, *m_dM = nullptr, *m_dV = nullptr;
     float *m_dZ1 = nullptr, *m_dA1 = nullptr, *m_dZ2 = nullptr, *m_dA2 = nullptr;
-    float* m_hPin = nullptr;  // pinned: gradient and loss terms on their way out
-    size_t m_pinFloats = 0;
     float *m_dDy = nullptr, *m_dD1 = nullptr, *m_dD2 = nullptr, *m_dSq = nullptr;
 };
 
