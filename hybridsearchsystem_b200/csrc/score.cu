@@ -64,7 +64,9 @@ __global__ void __launch_bounds__(kExactT) exact_score_kernel(const float* __res
     const uint32_t q0 = blockIdx.y * T::QT;
     const uint32_t chunks = (dim + kExactK - 1) / kExactK;
 
-    // rows past the matrices copy the last row instead (in bounds; their outputs are not stored)
+    // Rows past the matrices are not written and their outputs not stored: docs copy the last row (in bounds),
+    // absent queries nothing (copies of the last query by every CTA met in one place: 100,000 docs x 100, 6
+    // queries 47 us, 19 now)
     auto stage = [&](uint32_t c) {
         float* sd = exact_smem + (c & 1u) * T::stage_floats;
         float* sq = sd + T::DT * kExactPitch;
@@ -78,9 +80,9 @@ __global__ void __launch_bounds__(kExactT) exact_score_kernel(const float* __res
         }
         for (uint32_t f = t; f < T::QT * (kExactK / 4); f += kExactT) {
             const uint32_t r = f / (kExactK / 4), part = f % (kExactK / 4);
-            if (part < k4)
+            if (part < k4 && q0 + r < m)
                 copy4_async<VEC>(sq + r * kExactK + part * 4,
-                                 qry + static_cast<uint64_t>(min(q0 + r, m - 1)) * dim + k0 + part * 4);
+                                 qry + static_cast<uint64_t>(q0 + r) * dim + k0 + part * 4);
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
@@ -149,6 +151,62 @@ cudaError_t launch_exact_tile(const float* qry, const float* docs, float* out, u
     }
     const dim3 grid(static_cast<uint32_t>((static_cast<uint64_t>(n) + T::DT - 1) / T::DT), (m + T::QT - 1) / T::QT);
     kernel<<<grid, kExactT, T::smem, stream>>>(qry, docs, out, m, n, dim, ldc);
+    return cudaGetLastError();
+}
+
+// Rows of at most kShortDim floats: bound by the doc rows' and the outputs' bytes, at launch latency in the sizes in
+// use, and a staged tile would wait for a copy of a few sectors a row through shared memory. A thread reads its doc's
+// row into registers and forms every query's chain from it, up to 32 queries to a CTA (broadcast from shared memory).
+// 300,000 docs, us staged -> so: 4 dims 1 query 7.0 -> 3.6, 8 queries 21.9 -> 3.9, 32 queries 16.8 -> 7.8; 16 dims 1
+// query 7.0 -> 5.2, 32 queries 19.6 -> 18.4; 28 dims 1 query 8.0 -> 6.3, 8 queries 40.5 -> 11.5, 32 queries even. Past
+// 16 dims a second CTA's worth of queries is better staged (100,000 docs x 28, 100 queries: 40 us).
+constexpr uint32_t kShortDim = 28, kShortDimMany = 16, kShortQueries = 32;
+constexpr int kShortT = 128;
+
+template <int QUADS, bool VEC>
+__global__ void __launch_bounds__(kShortT) exact_short_kernel(const float* __restrict__ qry,
+                                                              const float* __restrict__ docs, float* __restrict__ out,
+                                                              uint32_t m, uint32_t n, uint64_t ldc, uint32_t per) {
+    __shared__ __align__(16) float sq[kShortQueries * QUADS * 4];
+    const uint32_t q0 = blockIdx.y * per, queries = min(per, m - q0);
+    for (uint32_t i = threadIdx.x; i < queries * QUADS * 4; i += kShortT)
+        sq[i] = qry[static_cast<uint64_t>(q0) * QUADS * 4 + i];
+    const uint64_t doc = static_cast<uint64_t>(blockIdx.x) * kShortT + threadIdx.x;
+    float4 v[QUADS];
+    if (doc < n) {
+        const float* row = docs + doc * (QUADS * 4);
+#pragma unroll
+        for (int i = 0; i < QUADS; ++i)
+            v[i] = VEC ? *reinterpret_cast<const float4*>(row + 4 * i)
+                       : make_float4(row[4 * i], row[4 * i + 1], row[4 * i + 2], row[4 * i + 3]);
+    }
+    __syncthreads();
+    if (doc >= n) return;
+    for (uint32_t q = 0; q < queries; ++q) {
+        float s = 0.0f;
+#pragma unroll
+        for (int i = 0; i < QUADS; ++i) {
+            const float4 x = *reinterpret_cast<const float4*>(sq + (q * QUADS + i) * 4);
+            s = __fadd_rn(s, __fmul_rn(x.x, v[i].x));
+            s = __fadd_rn(s, __fmul_rn(x.y, v[i].y));
+            s = __fadd_rn(s, __fmul_rn(x.z, v[i].z));
+            s = __fadd_rn(s, __fmul_rn(x.w, v[i].w));
+        }
+        out[(static_cast<uint64_t>(q0) + q) * ldc + doc] = s;
+    }
+}
+
+template <int QUADS>
+cudaError_t launch_exact_short(const float* qry, const float* docs, float* out, uint32_t m, uint32_t n, uint64_t ldc,
+                               cudaStream_t stream) {
+    const bool vec = (reinterpret_cast<uintptr_t>(docs) & 15u) == 0;
+    auto kernel = vec ? exact_short_kernel<QUADS, true> : exact_short_kernel<QUADS, false>;
+    // fewer queries to a CTA where the docs alone would leave SMs with less than four CTAs
+    const uint64_t tiles = (n - 1) / kShortT + 1;
+    uint32_t per = kShortQueries;
+    while (per > 2 && tiles * ((m - 1) / per + 1) < 4 * 148) per /= 2;
+    const dim3 grid(static_cast<uint32_t>(tiles), (m - 1) / per + 1);
+    kernel<<<grid, kShortT, 0, stream>>>(qry, docs, out, m, n, ldc, per);
     return cudaGetLastError();
 }
 
@@ -383,7 +441,7 @@ cudaError_t launch_cand_simt_tile(const CandLaunch& L, cudaStream_t stream) {
 
 }  // namespace
 
-// The tile: few queries take narrow ones (the pass is then bound by the doc rows, so no thread should
+// Short rows go straight to registers. The tile of longer ones: few queries take narrow ones (the pass is then bound by the doc rows, so no thread should
 // carry chains of absent queries); from 5 queries on, 32 x 128 where that pads the batch to at most a
 // tenth more queries than 16 x 64 does and still gives every SM a CTA, else 16 x 64.
 cudaError_t launch_exact_score(const float* qry, const float* docs, float* out, uint32_t m, uint32_t n, uint32_t dim,
@@ -391,6 +449,17 @@ cudaError_t launch_exact_score(const float* qry, const float* docs, float* out, 
     if (m == 0 || n == 0) return cudaSuccess;
     if ((static_cast<uint64_t>(m) + 7) / 8 > 65535u) return cudaErrorInvalidValue;
     constexpr uint64_t kSms = 148;
+    if (dim <= (m <= kShortQueries ? kShortDim : kShortDimMany)) {
+        switch (dim / 4) {
+            case 1: return launch_exact_short<1>(qry, docs, out, m, n, ldc, stream);
+            case 2: return launch_exact_short<2>(qry, docs, out, m, n, ldc, stream);
+            case 3: return launch_exact_short<3>(qry, docs, out, m, n, ldc, stream);
+            case 4: return launch_exact_short<4>(qry, docs, out, m, n, ldc, stream);
+            case 5: return launch_exact_short<5>(qry, docs, out, m, n, ldc, stream);
+            case 6: return launch_exact_short<6>(qry, docs, out, m, n, ldc, stream);
+            case 7: return launch_exact_short<7>(qry, docs, out, m, n, ldc, stream);
+        }
+    }
     if (m <= 2) return launch_exact_tile<2, 1, 1>(qry, docs, out, m, n, dim, ldc, stream);
     if (m <= 4)
         return n >= kSms * 256 ? launch_exact_tile<4, 2, 1>(qry, docs, out, m, n, dim, ldc, stream)
