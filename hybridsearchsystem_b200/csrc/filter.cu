@@ -782,7 +782,8 @@ cudaError_t launch_filter_wpt(const FilterLaunch& L, cudaStream_t stream) {
     // a CTA takes up to 4 tiles of a segment, sharing its set-up (half of a tile's time), where that
     // still leaves four waves of four CTAs per SM (fewer idle in the last one)
     uint32_t tpc = 4;
-    while (tpc > 1 && static_cast<uint64_t>(L.nq) * L.seg_num * ((tiles + tpc - 1) / tpc) < 4 * 148 * 4) tpc >>= 1;
+    const uint64_t waves = 4ull * 4 * device_sms();
+    while (tpc > 1 && static_cast<uint64_t>(L.nq) * L.seg_num * ((tiles + tpc - 1) / tpc) < waves) tpc >>= 1;
     const uint64_t gy = static_cast<uint64_t>(L.seg_num) * ((tiles + tpc - 1) / tpc);
     if (gy > 65535u) return cudaErrorInvalidValue;
     const size_t smem = static_cast<size_t>(L.max_opnd > 0 ? L.max_opnd : 1) * TW * sizeof(uint64_t);
@@ -836,7 +837,7 @@ cudaError_t launch_filter_dense(const DenseFilterLaunch& L, cudaStream_t stream)
         // More tiles per CTA share its program setup over more words, fewer leave more CTAs: take the
         // most (4, 2, 1) that still leaves 4 waves of resident CTAs (small batches and tables take 1),
         // but no fewer than the grid's height limit needs.
-        const uint64_t want = 4ull * kWideCtasPerSm * (L.sm_count ? L.sm_count : 148u);
+        const uint64_t want = 4ull * kWideCtasPerSm * (L.sm_count ? L.sm_count : device_sms());
         uint32_t tpc = kWideMaxTilesPerCta;
         while (tpc > 1 && static_cast<uint64_t>(L.nq) * ((total + tpc - 1) / tpc) < want &&
                (total + tpc / 2 - 1) / (tpc / 2) <= 65535u)

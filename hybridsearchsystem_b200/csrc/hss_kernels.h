@@ -11,6 +11,14 @@
 
 namespace hss {
 
+// SMs of the current device (148 where it cannot be asked), for the launch rules.
+inline uint32_t device_sms() {
+    int dev = 0, n = 0;
+    const bool ok = cudaGetDevice(&dev) == cudaSuccess &&
+                    cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess;
+    return ok && n > 0 ? static_cast<uint32_t>(n) : 148u;
+}
+
 // Launches a kernel that calls wait_for_previous() (hss_device.cuh), so that its launch and its
 // set-up overlap the end of the kernel before it: a batch's chain of short kernels otherwise idles
 // 1 to 3 us between each two. cluster > 1: clusters of that many CTAs along x.
@@ -81,7 +89,7 @@ struct DenseFilterLaunch {
     uint32_t seg_num;
     uint64_t doc_num;
     uint32_t max_opnd;         // largest operand count of any query in the batch (<= 64)
-    uint32_t sm_count;         // SMs of the device (sizes the grid; 0: 148)
+    uint32_t sm_count;         // SMs of the device (sizes the grid; 0: asked)
 };
 cudaError_t launch_filter_dense(const DenseFilterLaunch& L, cudaStream_t stream);
 

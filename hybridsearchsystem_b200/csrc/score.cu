@@ -204,7 +204,8 @@ cudaError_t launch_exact_short(const float* qry, const float* docs, float* out, 
     // fewer queries to a CTA where the docs alone would leave SMs with less than four CTAs
     const uint64_t tiles = (n - 1) / kShortT + 1;
     uint32_t per = kShortQueries;
-    while (per > 2 && tiles * ((m - 1) / per + 1) < 4 * 148) per /= 2;
+    const uint64_t ctas = 4ull * device_sms();
+    while (per > 2 && tiles * ((m - 1) / per + 1) < ctas) per /= 2;
     const dim3 grid(static_cast<uint32_t>(tiles), (m - 1) / per + 1);
     kernel<<<grid, kShortT, 0, stream>>>(qry, docs, out, m, n, ldc, per);
     return cudaGetLastError();
@@ -448,7 +449,7 @@ cudaError_t launch_exact_score(const float* qry, const float* docs, float* out, 
                                uint64_t ldc, cudaStream_t stream) {
     if (m == 0 || n == 0) return cudaSuccess;
     if ((static_cast<uint64_t>(m) + 7) / 8 > 65535u) return cudaErrorInvalidValue;
-    constexpr uint64_t kSms = 148;
+    const uint64_t sms = device_sms();
     if (dim <= (m <= kShortQueries ? kShortDim : kShortDimMany)) {
         switch (dim / 4) {
             case 1: return launch_exact_short<1>(qry, docs, out, m, n, ldc, stream);
@@ -462,11 +463,11 @@ cudaError_t launch_exact_score(const float* qry, const float* docs, float* out, 
     }
     if (m <= 2) return launch_exact_tile<2, 1, 1>(qry, docs, out, m, n, dim, ldc, stream);
     if (m <= 4)
-        return n >= kSms * 256 ? launch_exact_tile<4, 2, 1>(qry, docs, out, m, n, dim, ldc, stream)
+        return n >= sms * 256 ? launch_exact_tile<4, 2, 1>(qry, docs, out, m, n, dim, ldc, stream)
                                : launch_exact_tile<4, 1, 1>(qry, docs, out, m, n, dim, ldc, stream);
     const uint32_t pad32 = (m + 31) / 32 * 32, pad16 = (m + 15) / 16 * 16;
     const uint64_t ctas = static_cast<uint64_t>(pad32 / 32) * ((static_cast<uint64_t>(n) + 127) / 128);
-    if (10ull * pad32 <= 11ull * pad16 && ctas >= kSms)
+    if (10ull * pad32 <= 11ull * pad16 && ctas >= sms)
         return launch_exact_tile<8, 4, 4>(qry, docs, out, m, n, dim, ldc, stream);
     return launch_exact_tile<4, 2, 4>(qry, docs, out, m, n, dim, ldc, stream);
 }

@@ -1387,9 +1387,8 @@ bool bad_segments(uint32_t segs, uint32_t seg_cap, uint32_t cap) {
 }
 }  // namespace
 
-// Up to this many queries every CTA has an SM to itself: the selection kernels then take 1,024 threads
+// Up to as many queries as SMs every CTA has one to itself: the selection kernels then take 1,024 threads
 // (more, and two CTAs of 512 threads per SM hide each other's steps better).
-constexpr uint32_t kWideQueries = 148;
 
 cudaError_t launch_sample_threshold(const SampleThresholdLaunch& L, cudaStream_t stream) {
     if (L.nq_list == 0) return cudaSuccess;
@@ -1405,7 +1404,7 @@ cudaError_t launch_maxima_threshold(const MaximaThresholdLaunch& L, cudaStream_t
     if (L.groups == 0 || L.groups % 4 || L.cap % 4 || L.groups > L.cap || (reinterpret_cast<uintptr_t>(L.best) & 15u))
         return cudaErrorInvalidValue;
     const size_t smem = sizeof(HistSmem) + (L.groups < kFastSample ? L.groups : kFastSample) * sizeof(float);
-    const bool wide = L.nq_list <= kWideQueries;
+    const bool wide = L.nq_list <= device_sms();
     auto kernel = wide ? maxima_threshold_kernel<kST> : maxima_threshold_kernel<kSelT>;
     cudaError_t e = set_smem(kernel, smem);
     if (e != cudaSuccess) return e;
@@ -1415,7 +1414,7 @@ cudaError_t launch_maxima_threshold(const MaximaThresholdLaunch& L, cudaStream_t
 cudaError_t launch_select_topk(const SelectLaunch& L, cudaStream_t stream) {
     if (L.nq_list == 0) return cudaSuccess;
     if (bad_segments(L.segs, L.seg_cap, L.cap) || L.segs > static_cast<uint32_t>(kST)) return cudaErrorInvalidValue;
-    const bool wide = L.fast_large || L.nq_list <= kWideQueries;
+    const bool wide = L.fast_large || L.nq_list <= device_sms();
     const size_t smem = select_cand_offset(L.dim) + (wide ? kFastLarge : kFast) * sizeof(float);
     const bool split = L.pending != nullptr;
     auto kernel = wide ? (split ? select_topk_kernel<kST, kFastLarge, true> : select_topk_kernel<kST, kFastLarge, false>)
@@ -1424,7 +1423,7 @@ cudaError_t launch_select_topk(const SelectLaunch& L, cudaStream_t stream) {
     if (e != cudaSuccess) return e;
     e = launch_dependent(kernel, dim3(L.nq_list), wide ? kST : kSelT, smem, stream, 1, L);
     if (e != cudaSuccess || !split) return e;
-    e = launch_dependent(rescore_kernel, dim3(148 * 4), kRescoreT, L.nq_list * sizeof(uint32_t), stream, 1, L);
+    e = launch_dependent(rescore_kernel, dim3(4 * device_sms()), kRescoreT, L.nq_list * sizeof(uint32_t), stream, 1, L);
     if (e != cudaSuccess) return e;
     e = set_smem(select_final_kernel, sizeof(SelectSmem));
     if (e != cudaSuccess) return e;
