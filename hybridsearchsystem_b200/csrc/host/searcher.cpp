@@ -838,17 +838,22 @@ uint64_t FullRecallSearcher::SampleOptimum(uint32_t nq, uint32_t maxK) const {
 }
 
 // Whether the select step spreads its rescoring over the device (three kernels) instead of leaving each
-// query's rows to its CTA. It pays where a query has more rows, or longer ones, than its SM can read in
-// the time the rest of the batch takes (us a batch, one CTA a query -> spread):
-//   8-bit form, whose error band grows with the row: 768 dims, 300k docs, 128 queries, K 10 1070 -> 398,
-//   K 100 9545 -> 1740 (1677 with later changes); 384 dims, 4 queries, K 10 159 -> 91; 256 dims, K 100 1157 -> 878; 128 dims, 256
-//   queries, K 300 920 -> 901. Not 256 dims, 128 queries, K 10 (263 -> 281) nor 128 dims, K 200 (757 -> 777).
+// query's rows to its CTA. It pays where the query with the most rows, or the longest ones, has more than its SM can
+// read in the time the rest of the batch takes.
+//   8-bit form, whose error band keeps far more than K rows and more for some queries than for others: at any batch
+//   size, except for short rows and a small K, where two launches more are the larger part. us a batch, one CTA a
+//   query -> spread, at 1 / 16 / 128 / 256 queries:
+//     128 dims, 300k docs, K 10    106 -> 110,  103 -> 108,  127 -> 133,  166 -> 174
+//     128 dims, 300k docs, K 30    141 -> 132,  157 -> 152,  169 -> 173,  271 -> 268
+//     128 dims, 1M docs, K 100     474 -> 416,  536 -> 489,  631 -> 592,  832 -> 747
+//     256 dims, 1M docs, K 10      199 -> 178,  326 -> 318,  446 -> 415,  705 -> 608
+//     768 dims, 300k docs, K 10    145 -> 129,  272 -> 205, 2360 -> 432, 2616 -> 633
 //   Other forms, batches that leave SMs idle: 768 dims, K 1000: 1 query 537 -> 445, 64 queries 576 -> 528.
 //   Not 256 queries, K 700 (713 -> 750), nor rows of 128 dims (bf16, 64 queries, K 1000 629 -> 632).
 bool FullRecallSearcher::SplitSelect(uint32_t nq, uint32_t maxK) const {
-    const uint64_t dim = m_table->GetDimension(), floats = maxK * dim;
-    if (m_tcFormat == kTcE4M3) return dim >= 384 || floats >= (dim >= 256 ? 25600u : 32768u);
-    return nq <= 64 && floats >= 1ull << 19;
+    const uint64_t dim = m_table->GetDimension();
+    if (m_tcFormat == kTcE4M3) return dim > 128 || maxK >= 32;
+    return nq <= 64 && maxK * dim >= 1ull << 19;
 }
 
 // Whether the corpus is passed over once, at the sample's threshold, instead of in two parts with the

@@ -75,3 +75,21 @@ def test_a_replayed_batch_is_planned_as_a_direct_one(torch_cuda, method, n, nq, 
     assert s.graph_stats()["replays"] == 1
     assert seen[1:] == [seen[0]] * 2
     _check(sc.cpu().numpy(), ids.cpu().numpy(), cnt.cpu().numpy(), oracle.topk(q, exprs, [k] * nq, vec, bits, threads=8))
+
+
+@pytest.mark.parametrize("k,spread", [(31, 0), (32, 2), (100, 2)])
+def test_the_8_bit_select_step_is_spread_over_the_device(torch_cuda, k, spread):
+    # two more launches from K = 32 on (rows of 128 dims); results exact either way
+    mix, vec, bits, table = _world(100_000)
+    launches = []
+    for kk in (1, k):
+        s = hss.FullRecallSearcher(table, max_batch=3, method=E4M3)
+        q = mix.queries(3, seed=37)
+        exprs = ["1", "2 OR 3", "NOT 4"]
+        for e, v in zip(exprs, q):
+            s.add_query(e, v, kk)
+        sc, ids, cnt = s.batch_search(out_stride=kk)
+        _check(sc, ids, cnt, oracle.topk(q, exprs, [kk] * 3, vec, bits, threads=8))
+        assert s.last_times()["retries"] == 0
+        launches.append(s.last_times()["launches"])
+    assert launches[1] - launches[0] == spread
