@@ -902,13 +902,15 @@ FullRecallSearcher::Plan FullRecallSearcher::PlanOf(uint32_t nq, uint32_t maxK, 
 }
 
 uint32_t FullRecallSearcher::PlanTopK(uint32_t nq, uint32_t maxK) const {
-    // K is rounded up to a power of two, and to the largest one up to 256 whose plan is that of K = 1: a replayed
-    // batch takes the launches that it would take directly, but for a sample of a K up to twice its own.
+    // K is rounded up to a power of two, and on to the largest one up to 256 with the same plan: a replayed batch
+    // takes the launches that it would take directly, but for a sample of a K up to twice its own, and the K of one
+    // plan share a graph (a capture takes 0.2 ms of the host, now and then far more).
+    if (maxK == 0) return 0u;
     const bool stats = static_cast<bool>(m_model);
-    const Plan least = PlanOf(nq, 1, stats);
-    uint32_t flat = 1;
-    while (flat < 256 && PlanOf(nq, flat * 2, stats) == least) flat <<= 1;
-    return maxK == 0 ? 0u : std::max(GraphTopK(maxK), flat);
+    uint32_t k = GraphTopK(maxK);
+    const Plan plan = PlanOf(nq, k, stats);
+    while (k < 256 && PlanOf(nq, 2 * k, stats) == plan) k <<= 1;
+    return k;
 }
 
 uint32_t FullRecallSearcher::GraphOperands(uint32_t maxOpnd) {

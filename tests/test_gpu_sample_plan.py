@@ -93,3 +93,30 @@ def test_the_8_bit_select_step_is_spread_over_the_device(torch_cuda, k, spread):
         assert s.last_times()["retries"] == 0
         launches.append(s.last_times()["launches"])
     assert launches[1] - launches[0] == spread
+
+
+def test_the_k_of_one_plan_share_a_graph(torch_cuda):
+    # 400,000 docs, 4 queries: K up to 32 are planned with one pass (12.2 K <= 512), K from 33 to 256 with two;
+    # every other part of the plan is the same for them
+    torch = torch_cuda
+    mix, vec, bits, table = _world(400_000)
+    s = hss.FullRecallSearcher(table, max_batch=4, method=BF16)
+    s.set_graphs(True)
+    q = mix.queries(4, seed=38)
+    exprs = ["1", "2 OR 3", "NOT 4", "5"]
+    f = s.compile_filters(exprs)
+    d_q = torch.from_numpy(q).to("cuda:0")
+    sc = torch.zeros((4, 256), dtype=torch.float32, device="cuda:0")
+    ids = torch.zeros((4, 256), dtype=torch.int64, device="cuda:0")
+    cnt = torch.zeros(4, dtype=torch.int32, device="cuda:0")
+    stream = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    captures = []
+    for k in (1, 10, 32, 50, 100, 200, 256):
+        assert s.search_device(d_q.data_ptr(), 4, f, [k] * 4, sc.data_ptr(), ids.data_ptr(), cnt.data_ptr(), 256,
+                               stream.cuda_stream) == 0
+        stream.synchronize()
+        captures.append(s.graph_stats()["captures"])
+        _check(sc.cpu().numpy(), ids.cpu().numpy(), cnt.cpu().numpy(),
+               oracle.topk(q, exprs, [k] * 4, vec, bits, threads=8))
+    assert captures == [1, 1, 1, 2, 2, 2, 2]
