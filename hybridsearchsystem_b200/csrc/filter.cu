@@ -144,9 +144,9 @@ __device__ inline uint64_t tail_mask(uint64_t gw, uint64_t doc_num) {
 template <int W, class Operand>
 __device__ __forceinline__ bool eval_words(const uint32_t* prog, uint32_t plen, Operand operand, uint32_t nop,
                                            uint64_t (&result)[W]) {
-    // two operands' loads in flight; at one or two words a thread the second only costs instructions (segments of
-    // 8,192 docs, 2M docs, 64 queries 103 and 96 us)
-    constexpr int kInFlight = W > 2 ? 2 : 1;
+    // two operands' loads in flight; at one word a thread the second only costs instructions (segments of 8,192 docs,
+    // 2M docs, 64 queries 103 and 96 us), at two it pays (byte maps, up to 12 tags, 256 queries 1264 -> 1096 us)
+    constexpr int kInFlight = W > 1 ? 2 : 1;
     uint64_t st[kMaxStack][W];
     uint32_t sp = 0, next = 0, pc = 0;
     while (pc < plen) {
