@@ -790,7 +790,12 @@ cudaError_t launch_filter_wpt(const FilterLaunch& L, cudaStream_t stream) {
     // opt in always (static plus dynamic shared memory may pass 48 KB even when the dynamic part does
     // not), to the one ceiling every caller sets: searchers on other threads launch it concurrently
     if (smem > kFilterSmemCeiling) return cudaErrorInvalidValue;
-    auto kernel = tiles > 1 ? filter_batch_kernel<WPT, true> : filter_batch_kernel<WPT, false>;
+    auto kernel = filter_batch_kernel<WPT, false>;
+    if constexpr (WPT < 8) {
+        if (tiles > 1) kernel = filter_batch_kernel<WPT, true>;
+    } else {
+        if (tiles > 1) return cudaErrorInvalidValue;
+    }
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          static_cast<int>(kFilterSmemCeiling));
     if (e != cudaSuccess) return e;
@@ -802,7 +807,9 @@ cudaError_t launch_filter_wpt(const FilterLaunch& L, cudaStream_t stream) {
 }  // namespace
 
 // The widest tile (8, 4, 2 or 1 words a thread) whose operand slots stay within 52 KB of shared memory, so
-// that four CTAs share an SM (within what the segment and the grid's height allow).
+// that four CTAs share an SM (within what the segment and the grid's height allow). 8 words only where one tile is the
+// segment: with several, the kernel takes 128 registers, two CTAs an SM (256 queries of up to 2 tags, segments of 1M
+// docs: 135 us with 8 words, 97 with 4).
 cudaError_t launch_filter_batch(const FilterLaunch& L, cudaStream_t stream) {
     if (L.nq == 0 || L.seg_num == 0) return cudaSuccess;
     if (L.max_opnd > static_cast<uint32_t>(kMaxOperands)) return cudaErrorInvalidValue;
@@ -811,7 +818,7 @@ cudaError_t launch_filter_batch(const FilterLaunch& L, cudaStream_t stream) {
     auto tiles = [&](int w) {
         return static_cast<uint64_t>(L.seg_num) * ((seg_words + w * kTile - 1) / (w * kTile));
     };
-    int wpt = 8;
+    int wpt = seg_words > 8u * kTile ? 4 : 8;
     while (wpt > 1 && (static_cast<size_t>(wpt) * kTile * per_word > 52 * 1024 ||
                        static_cast<uint32_t>(wpt / 2) * kTile >= seg_words) &&
            !(tiles(wpt / 2) > 65535u && static_cast<size_t>(wpt) * kTile * per_word <= 96 * 1024))
