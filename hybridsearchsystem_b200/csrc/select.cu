@@ -457,12 +457,14 @@ __device__ __forceinline__ uint32_t pad_sort(SelectSmem& S, uint32_t got) {
 }
 
 // Brings the top `kq` (<= kMaxTopK) of n u64 keys key(i) (and possibly more) into S.sortbuf, unsorted,
-// filled up with zeros to sort_size() entries, which it returns. Long lists are cut at a lower bound of
-// the kq-th key first, so that the sort takes about kq keys.
+// filled up with zeros to sort_size() entries, which it returns. Lists past 512 keys of which less than half is
+// wanted are cut at a lower bound of the kq-th key first, so that the sort takes about kq keys.
+constexpr uint32_t kCutKeys = 512;
+
 template <int NT, class KeyFn>
 __device__ __forceinline__ uint32_t gather_top_keys(KeyFn key, uint32_t n, uint32_t kq, SelectSmem& S) {
     uint32_t got;
-    if (n <= static_cast<uint32_t>(NT) || (n <= static_cast<uint32_t>(kMaxTopK) && n <= 2 * kq)) {
+    if (n <= kCutKeys || (n <= static_cast<uint32_t>(kMaxTopK) && n <= 2 * kq)) {
         for (uint32_t i = threadIdx.x; i < n; i += NT) S.sortbuf[i] = key(i);
         got = n;
     } else {
