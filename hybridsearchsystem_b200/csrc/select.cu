@@ -495,11 +495,11 @@ __device__ __forceinline__ uint32_t gather_top_keys(KeyFn key, uint32_t n, uint3
 // ---------------------------------------------------------------------------------------------
 // The threshold of a sample or of a first candidate pass. One CTA per query; bound by a chain of
 // dependent steps (counts, entries, two digits), so the list is read once, into shared memory where it
-// fits (kFastSample entries). 1,024 threads and long segments walked as they lie: with a threshold model,
+// fits (`held` entries). 1,024 threads and long segments walked as they lie: with a threshold model,
 // whose sample is kept as lists, 256 queries on 10M docs 1214 us a batch (K 1000: 1866) with 512 threads and
 // a lookup per entry, 1190 (1785) now; 8-bit form, whose raises read long lists, 1M docs, 256 queries, K 100
 // 877 -> 819; other raises even.
-__global__ void __launch_bounds__(kST) sample_threshold_kernel(SampleThresholdLaunch L) {
+__global__ void __launch_bounds__(kST) sample_threshold_kernel(SampleThresholdLaunch L, uint32_t held) {
     constexpr int NT = kST;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     HistSmem& S = *reinterpret_cast<HistSmem*>(smem_raw);
@@ -512,10 +512,10 @@ __global__ void __launch_bounds__(kST) sample_threshold_kernel(SampleThresholdLa
     const float* sc = L.score + static_cast<uint64_t>(qi) * L.cap;
     bool lost = false;  // a sample segment that overflowed only lowers the sample's K-th best
     uint32_t key_lo, key_hi;
-    const uint32_t n = load_list<NT, true>(S, counts, L.segs, L.seg_cap, sc, nullptr, cs, kFastSample, nullptr, &lost, &key_lo,
-                                     &key_hi);
+    const uint32_t n = load_list<NT, true>(S, counts, L.segs, L.seg_cap, sc, nullptr, cs, held, nullptr, &lost, &key_lo,
+                                           &key_hi);
     auto visit = [&](auto fn) {
-        if (n <= kFastSample) {
+        if (n <= held) {
             for (uint32_t i = threadIdx.x; i < n; i += NT) fn(float_key(cs[i]));
         } else {
             walk_segments<NT, true>(counts, L.segs, L.seg_cap, sc, [](uint32_t) {}, [&](uint32_t, bool ok, float v) {
@@ -1395,12 +1395,15 @@ bool bad_segments(uint32_t segs, uint32_t seg_cap, uint32_t cap) {
 cudaError_t launch_sample_threshold(const SampleThresholdLaunch& L, cudaStream_t stream) {
     if (L.nq_list == 0) return cudaSuccess;
     if (bad_segments(L.segs, L.seg_cap, L.cap)) return cudaErrorInvalidValue;
-    const size_t smem = sizeof(HistSmem) + kFastSample * sizeof(float);
+    const uint32_t held = L.stats && L.nq_list <= device_sms() ? kFastLarge : kFastSample;
+    const size_t smem = sizeof(HistSmem) + held * sizeof(float);
     cudaError_t e = set_smem(sample_threshold_kernel, smem);
     if (e != cudaSuccess) return e;
-    return launch_dependent(sample_threshold_kernel, dim3(L.nq_list), kST, smem, stream, 1, L);
+    return launch_dependent(sample_threshold_kernel, dim3(L.nq_list), kST, smem, stream, 1, L, held);
 }
 
+// Up to as many queries as SMs every CTA has one to itself: this kernel and the select step then take 1,024
+// threads (more, and two CTAs of 512 threads per SM hide each other's steps better).
 cudaError_t launch_maxima_threshold(const MaximaThresholdLaunch& L, cudaStream_t stream) {
     if (L.nq_list == 0) return cudaSuccess;
     if (L.groups == 0 || L.groups % 4 || L.cap % 4 || L.groups > L.cap || (reinterpret_cast<uintptr_t>(L.best) & 15u))
