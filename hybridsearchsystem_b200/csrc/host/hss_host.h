@@ -573,8 +573,8 @@ class FullRecallSearcher {
               uint32_t rows, bool simt, const MaximaSample* maxima = nullptr);
     // The doc sample of m_b.want docs and its threshold (raised, with raiseOnly); the pass keeps the
     // filtered docs at or above emitTheta (null: every filtered doc).
-    uint64_t Sample(const uint32_t* dList, uint32_t rows, bool simt, bool raiseOnly = false, float* stats = nullptr,
-                    float* thetaCopy = nullptr, const float* emitTheta = nullptr);
+    void Sample(const uint32_t* dList, uint32_t rows, bool simt, bool raiseOnly = false, float* stats = nullptr,
+                float* thetaCopy = nullptr, const float* emitTheta = nullptr);
     uint32_t SampleTileNum() const;
     MaximaSample Maxima(uint32_t rows, uint64_t want, uint32_t maxK, bool simt) const;
     uint64_t SampleOptimum(uint32_t nq, uint32_t maxK) const;
