@@ -531,14 +531,14 @@ cudaError_t launch_train_gradients(const TrainLaunch& L, cudaStream_t stream) {
         if (e != cudaSuccess) return e;
     }
     const dim3 gF(static_cast<unsigned>(tF));
-    cudaError_t e = launch_dependent(layer_forward_kernel, gF, kGroup, kFwdSmem, stream, 1, Product{L.X, W1, B, H, D, D, H},
-                                     b1, L.Z1, L.A1);
+    cudaError_t e = launch_dependent(layer_forward_kernel, gF, kGroup, kFwdSmem, stream, 1,
+                                     Product{L.X, W1, B, H, D, D, H}, b1, L.Z1, L.A1);
     if (e == cudaSuccess)
-        e = launch_dependent(layer_forward_kernel, gF, kGroup, kFwdSmem, stream, 1, Product{L.A1, W2, B, H, H, H, H}, b2,
-                             L.Z2, L.A2);
+        e = launch_dependent(layer_forward_kernel, gF, kGroup, kFwdSmem, stream, 1, Product{L.A1, W2, B, H, H, H, H},
+                             b2, L.Z2, L.A2);
     if (e == cudaSuccess)
-        e = launch_dependent(head_kernel, dim3((B + kHeadRows - 1) / kHeadRows), kHeadT, 0, stream, 1, L.A2, L.Z2, w3, b3,
-                             L.T, B, H, L.tau, L.dy, L.term, L.dZ2);
+        e = launch_dependent(head_kernel, dim3((B + kHeadRows - 1) / kHeadRows), kHeadT, 0, stream, 1, L.A2, L.Z2, w3,
+                             b3, L.T, B, H, L.tau, L.dy, L.term, L.dZ2);
     if (e == cudaSuccess)
         e = launch_dependent(grad_hidden_kernel, dim3(static_cast<unsigned>(tF + tW2 + tw3)), kGradThreads, kGradSmem,
                              stream, 1, Product{L.dZ2, W2, B, H, H, H, H}, L.Z1, L.dZ1, tF,

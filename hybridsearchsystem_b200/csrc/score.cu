@@ -442,9 +442,10 @@ cudaError_t launch_cand_simt_tile(const CandLaunch& L, cudaStream_t stream) {
 
 }  // namespace
 
-// Short rows go straight to registers. The tile of longer ones: few queries take narrow ones (the pass is then bound by the doc rows, so no thread should
-// carry chains of absent queries); from 5 queries on, 32 x 128 where that pads the batch to at most a
-// tenth more queries than 16 x 64 does and still gives every SM a CTA, else 16 x 64.
+// Short rows go straight to registers (exact_short_kernel). The tile of longer ones: few queries take narrow ones
+// (the pass is then bound by the doc rows, so no thread should carry chains of absent queries); from 5 queries on,
+// 32 x 128 where that pads the batch to at most a tenth more queries than 16 x 64 does and still gives every SM a
+// CTA, else 16 x 64.
 cudaError_t launch_exact_score(const float* qry, const float* docs, float* out, uint32_t m, uint32_t n, uint32_t dim,
                                uint64_t ldc, cudaStream_t stream) {
     if (m == 0 || n == 0) return cudaSuccess;

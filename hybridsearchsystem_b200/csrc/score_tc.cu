@@ -381,8 +381,8 @@ __device__ __forceinline__ uint32_t sample_units(const TcCandLaunch& L, uint32_t
 // Filter bits of the runs run0 .. run0 + 3 of tile v's block (16 bits a tile), and tile v's 64 of them.
 __device__ __forceinline__ void load_block_bits(uint4 (&w)[kThreadRuns], const uint64_t* brow, uint32_t sample_tiles,
                                                 uint32_t v, uint32_t run0) {
-    const uint4* p = reinterpret_cast<const uint4*>(brow) + static_cast<uint64_t>(run0) * (sample_tiles / kSampleBlock) +
-                     v / kSampleBlock;
+    const uint4* p = reinterpret_cast<const uint4*>(brow) +
+                     static_cast<uint64_t>(run0) * (sample_tiles / kSampleBlock) + v / kSampleBlock;
 #pragma unroll
     for (uint32_t r = 0; r < kThreadRuns; ++r) w[r] = p[static_cast<uint64_t>(r) * (sample_tiles / kSampleBlock)];
 }
@@ -1143,8 +1143,8 @@ cudaError_t launch_tc_cand(const TcCandLaunch& Lin, const CUtensorMap& doc_map, 
     L.stages = static_cast<uint32_t>(st < static_cast<size_t>(kMaxTcStages) ? st : kMaxTcStages);
     // every CTA writes segments seg_base + 2 b and seg_base + 2 b + 1 (pair: 4 per pair)
     const uint64_t seg_end = static_cast<uint64_t>(L.seg_base) + 2ull * L.ctas;
-    if (L.ctas != tc_cand_ctas(L.nq_rows, L.kblocks, L.tile_count, sms, L.cap) || L.seg_cap == 0 || seg_end > kMaxCandSegs ||
-        seg_end * L.seg_cap > L.cap)
+    if (L.ctas != tc_cand_ctas(L.nq_rows, L.kblocks, L.tile_count, sms, L.cap) || L.seg_cap == 0 ||
+        seg_end > kMaxCandSegs || seg_end * L.seg_cap > L.cap)
         return cudaErrorInvalidValue;
     if (L.best) {
         // whole blocks of sample tiles inside the corpus; a tile's group maxima stay inside a query's row, in
@@ -1205,8 +1205,8 @@ static bool encode_map(CUtensorMap* map, int format, const void* base, uint32_t 
     cuuint64_t gstride[2] = {static_cast<cuuint64_t>(dim) * elem, rows[0] * static_cast<cuuint64_t>(dim) * elem};
     cuuint32_t box[3] = {128u / elem, box_rows[0], box_rows[1]};
     cuuint32_t estride[3] = {1, 1, 1};
-    const CUresult r = fn(map, dt, rank, const_cast<void*>(base), gdim, gstride, box, estride, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                          CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+    const CUresult r = fn(map, dt, rank, const_cast<void*>(base), gdim, gstride, box, estride,
+                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS;
 }

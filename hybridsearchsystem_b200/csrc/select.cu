@@ -21,11 +21,13 @@ namespace cg = cooperative_groups;
 namespace hss {
 namespace {
 
-constexpr int kST = 1024;             // threads of the TOPK operator's CTAs and of the large select form
-constexpr int kSelT = 512;            // threads of the threshold kernel and of the usual select form
+// threads of a CTA: 1,024 in the TOPK operator, the threshold of a listed sample or pass, and, for batches of at most
+// as many queries as SMs, the select step and the threshold of group maxima; else these two take 512
+constexpr int kST = 1024;
+constexpr int kSelT = 512;
 constexpr int kBins = 4096;           // histogram bins: 12-bit digits
 // candidate scores a CTA holds in shared memory: the usual select form (two CTAs of 512 threads per SM),
-// the form for batches whose lists run long (large K; one CTA of 1,024), the threshold kernel (two CTAs)
+// the form for few queries or for lists that run long (large K; one CTA of 1,024), the threshold kernels
 constexpr uint32_t kFast = 8192;
 constexpr uint32_t kFastLarge = 32768;
 constexpr uint32_t kFastSample = 20480;
@@ -241,7 +243,8 @@ __device__ __forceinline__ uint64_t kth_bound_u64(KeyFn key, uint32_t n, uint32_
 // segment, independent and eight per thread in flight, and no block-wide scan or barrier is needed. Every
 // call is made by a full warp (valid = false past the end), so fn may use warp collectives; begin(m) is
 // called by the full warp before a group's m entries. LONG: segments of 64 entries or more on average are
-// walked one after the other, without the lookups (doc-sample lists hold about 110 a segment). Returns whether a segment of this lane lost entries.
+// walked one after the other, without the lookups (doc-sample lists hold about 110 a segment). Returns whether
+// a segment of this lane lost entries.
 template <int NT, bool LONG, class Begin, class Fn>
 __device__ __forceinline__ bool walk_segments(const uint32_t* counts, uint32_t segs, uint32_t seg_cap, const float* src,
                                               Begin begin, Fn fn) {
@@ -536,7 +539,8 @@ __global__ void __launch_bounds__(kST) sample_threshold_kernel(SampleThresholdLa
         // a true top-K doc therefore scores >= t - eps_s - eps_m under the main pass's arithmetic.
         const float t = __fsub_rd(__fsub_rd(key_float(kk), L.eps_sample[qi]), L.eps_main[qi]);
         theta = L.raise_only ? fmaxf(theta, t) : t;
-        if (L.stats && threadIdx.x == 0) L.stats[static_cast<uint64_t>(qi) * kSampleStats + kSampleRanks] = key_float(kk);
+        if (L.stats && threadIdx.x == 0)
+            L.stats[static_cast<uint64_t>(qi) * kSampleStats + kSampleRanks] = key_float(kk);
         if (L.theta_also && L.raise_only && threadIdx.x == 0) L.theta_also[qi] = fmaxf(L.theta_also[qi], t);
     } else if (L.stats && threadIdx.x == 0) {
         L.stats[static_cast<uint64_t>(qi) * kSampleStats + kSampleRanks] = -2.0f;  // no K-th best
@@ -727,8 +731,8 @@ __device__ __forceinline__ void threshold_miss(const SelectLaunch& L, uint32_t q
 // The end of the select step: the nf keys of a query (in S.sortbuf, or in ws) sorted, a predicted threshold
 // checked, the first kq results written.
 template <int NT>
-__device__ __forceinline__ void finish_select(SelectSmem& S, const SelectLaunch& L, uint32_t qi, uint32_t k, uint32_t kq,
-                                              uint32_t nf, bool in_smem, const unsigned long long* ws) {
+__device__ __forceinline__ void finish_select(SelectSmem& S, const SelectLaunch& L, uint32_t qi, uint32_t k,
+                                              uint32_t kq, uint32_t nf, bool in_smem, const unsigned long long* ws) {
     const uint32_t tid = threadIdx.x;
     __syncthreads();
     uint32_t m;
@@ -765,7 +769,8 @@ __device__ __forceinline__ void finish_select(SelectSmem& S, const SelectLaunch&
         __syncthreads();
 #pragma unroll
         for (int i = 0; i < kOwn; ++i)
-            if (tid + NT * i < nf && static_cast<uint32_t>(own[i] >> 32) >= lb) S.sortbuf[next_place(&S.counter)] = own[i];
+            if (tid + NT * i < nf && static_cast<uint32_t>(own[i] >> 32) >= lb)
+                S.sortbuf[next_place(&S.counter)] = own[i];
         __syncthreads();
         m = pad_sort<NT>(S, S.counter);
     } else {
@@ -837,7 +842,8 @@ __global__ void __launch_bounds__(NT, NT == kSelT ? 2 : 1) select_topk_kernel(Se
     for (uint32_t i = tid; i < L.dim; i += NT) sq[i] = L.qry[static_cast<uint64_t>(qi) * L.dim + i];
     bool overflow = false;
     uint32_t key_lo, key_hi;
-    const uint32_t n = load_list<NT, SPLIT>(S, counts, L.segs, L.seg_cap, sc, lc, cs, FAST, S.locs, &overflow, &key_lo, &key_hi);
+    const uint32_t n = load_list<NT, SPLIT>(S, counts, L.segs, L.seg_cap, sc, lc, cs, FAST, S.locs, &overflow, &key_lo,
+                                            &key_hi);
     auto visit_keys = [&](auto fn) {
         if (n <= FAST) {
             for (uint32_t i = tid; i < n; i += NT) fn(float_key(cs[i]));
@@ -898,9 +904,10 @@ __global__ void __launch_bounds__(NT, NT == kSelT ? 2 : 1) select_topk_kernel(Se
             if (n <= min(FAST, static_cast<uint32_t>(kMaxTopK))) {
                 for (uint32_t i = tid; i < n; i += NT) fn(cs[i], [&] { return S.locs[i]; });
             } else {
-                walk_segments<NT, SPLIT>(counts, L.segs, L.seg_cap, sc, [](uint32_t) {}, [&](uint32_t at, bool ok, float v) {
-                    if (ok) fn(v, [&] { return lc[at]; });
-                });
+                walk_segments<NT, SPLIT>(counts, L.segs, L.seg_cap, sc, [](uint32_t) {},
+                                         [&](uint32_t at, bool ok, float v) {
+                                             if (ok) fn(v, [&] { return lc[at]; });
+                                         });
             }
         };
         // how many clear the cut at all
@@ -1149,7 +1156,7 @@ __global__ void __launch_bounds__(kAggT) aggregate_scatter_kernel(const uint64_t
         wbits[t] = v;
         c = static_cast<uint32_t>(__popcll(v));
     }
-    // exclusive offsets of the block's words (the first four warps), and the sum of every thread's share
+    // exclusive offsets of the block's words (the first two warps), and the sum of every thread's share
     uint32_t x = c;
     if (t < kAggWords) {
 #pragma unroll
@@ -1389,9 +1396,8 @@ bool bad_segments(uint32_t segs, uint32_t seg_cap, uint32_t cap) {
 }
 }  // namespace
 
-// Up to as many queries as SMs every CTA has one to itself: the selection kernels then take 1,024 threads
-// (more, and two CTAs of 512 threads per SM hide each other's steps better).
-
+// Two CTAs an SM, but one with room for a whole sample of the default size where the statistics of few queries walk
+// it five more times (64 queries, 32,768 docs: 57 -> 36 us).
 cudaError_t launch_sample_threshold(const SampleThresholdLaunch& L, cudaStream_t stream) {
     if (L.nq_list == 0) return cudaSuccess;
     if (bad_segments(L.segs, L.seg_cap, L.cap)) return cudaErrorInvalidValue;
@@ -1459,8 +1465,8 @@ cudaError_t launch_aggregate(const uint64_t* bits, const float* scores, const ui
     const uint32_t nb = static_cast<uint32_t>((static_cast<uint64_t>(n) + kAggDocs - 1) / kAggDocs);
     if (nb == 0) return cudaMemsetAsync(total, 0, sizeof(uint32_t), stream);
     if (n <= kOwnDocs) {
-        return launch_dependent(aggregate_scatter_kernel<kAggOwn>, dim3(nb), kAggT, 0, stream, 1, bits, scores, loc_in, n,
-                                workspace, out_scores, out_loc, total);
+        return launch_dependent(aggregate_scatter_kernel<kAggOwn>, dim3(nb), kAggT, 0, stream, 1, bits, scores, loc_in,
+                                n, workspace, out_scores, out_loc, total);
     }
     aggregate_count_kernel<<<(nb + 7) / 8, 256, 0, stream>>>(bits, n, nb, workspace);
     if (nb <= kSumBlocks) {
@@ -1469,17 +1475,18 @@ cudaError_t launch_aggregate(const uint64_t* bits, const float* scores, const ui
     }
     cudaError_t e = launch_dependent(aggregate_scan_kernel, dim3(1), 1024, 0, stream, 1, workspace, nb);
     if (e != cudaSuccess) return e;
-    return launch_dependent(aggregate_scatter_kernel<kAggScanned>, dim3(nb), kAggT, 0, stream, 1, bits, scores, loc_in, n,
-                            workspace, out_scores, out_loc, total);
+    return launch_dependent(aggregate_scatter_kernel<kAggScanned>, dim3(nb), kAggT, 0, stream, 1, bits, scores, loc_in,
+                            n, workspace, out_scores, out_loc, total);
 }
 
 // Scratch of the allocation-free aggregator: one word per 1,024 docs, kAggStaticBlocks of them (64 KB,
-// docNumber <= 16,777,216; the count kernel writes one per kAggDocs docs). Module-scope, so it exists once per device for the life of
-// the process and every call on that device shares it. The count kernel writes every entry a call
-// reads before the scan reads it, so a call never sees an earlier call's contents and nothing has to
-// be cleared; two calls that overlap on the GPU (different streams, no ordering) do race on it.
+// docNumber <= 16,777,216; the count kernel writes one per kAggDocs docs). Module-scope, so it exists once per
+// device for the life of the process and every call on that device shares it. The count kernel writes every
+// entry a call reads before the scan reads it, so a call never sees an earlier call's contents and nothing has
+// to be cleared; two calls that overlap on the GPU (different streams, no ordering) do race on it.
 static __device__ __align__(256) uint32_t g_aggregate_scratch[kAggStaticBlocks];
-static_assert(kAggStaticMaxDocs == kAggStaticBlocks * 1024u && kAggDocs >= 1024u, "a block count per 1,024 docs at most");
+static_assert(kAggStaticMaxDocs == kAggStaticBlocks * 1024u && kAggDocs >= 1024u,
+              "a block count per 1,024 docs at most");
 
 cudaError_t aggregate_static_scratch(uint32_t** scratch) {
     return cudaGetSymbolAddress(reinterpret_cast<void**>(scratch), g_aggregate_scratch);
@@ -1559,9 +1566,9 @@ __device__ inline uint32_t preceding(const float* sc, uint32_t n, float x, bool 
 }
 
 constexpr int kMergeT = 1024;
-// Up to as many keys a CTA has a thread for each and cuts nothing: the cut's steps, and 1,024 threads, would be most of
-// the time (2 lists of 10, 256 queries 3.9 -> 3.0 us, 4 of 100 4.3 -> 3.7). Of more than eight lists half as many, since
-// a thread searches every list (16 lists of 16: 6.4 us cut, 7.5 not).
+// Up to as many keys a CTA has a thread for each and cuts nothing: the cut's steps, and 1,024 threads, would be most
+// of the time (2 lists of 10, 256 queries 3.9 -> 3.0 us, 4 of 100 4.3 -> 3.7). Of more than eight lists half as many,
+// since a thread searches every list (16 lists of 16: 6.4 us cut, 7.5 not).
 constexpr int kMergeFew = 512;
 constexpr uint32_t kMergeCap = 12000;  // keys held in shared memory (with the rest within 48 KB)
 
